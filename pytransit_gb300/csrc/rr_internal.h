@@ -43,9 +43,11 @@ struct Carve {
   }
 };
 
-// Per-parameter-vector record of the plain FP64 path (16 doubles):
-// c[0..9] Taylor coefficients, [10] t1, [11] t4 (contact times), [12] valid.
-constexpr int ORB64 = 16;
+// Per-parameter-vector record of the plain FP64 path (24 doubles):
+// c[0..9] Taylor coefficients, [10] t1, [11] t4 (contact times), [12] valid,
+// [13..21] coefficients of r^2(t).
+constexpr int ORB64 = 24;
+constexpr int ORB64_R2 = 13;
 // Per-parameter-vector record of the split path (16 floats):
 // c[0..9], [10] p_hi, [11] p_lo, [12] 1/p, [13] fast-test error bound,
 // [14] flags (int bits), [15] unused.
