@@ -190,6 +190,18 @@ int rr_prepare_split(double t_ref, double t_absmax, const double *k, int nkc, co
                      const float *basis, int nb);
 int rr_flux_split(const float *times_ff, int npt, const int32_t *lcids, int npv, int nlc, int npb, int ng,
                   double dg, const void *workspace, float *flux, int ldflux, void *stream);
+/* The plain FP64 prologue with the limb-darkening tables in one launch, for the
+ * affine laws with an analytic disk integral (uniform, linear, quadratic,
+ * quadratic-tri) and their basis tables: evaluate_ld / evaluate_ldi
+ * (ldmodels.py:143-174) and model_full.py:39-71.  Other laws run
+ * rr_ld_tables_f64 and rr_prepare_f64.  istar[npv, npb] is written; of
+ * ldp[npv, npb, nz] only the rows of vectors whose k lies outside the weight
+ * table (all rows for the other laws). */
+int rr_prepare_f64_ld(const double *k, int nkc, const double *p, const double *a, const double *inc,
+                      const double *e, const double *w, int npv, int npb, int law, const double *ldc, int npar,
+                      const double *mu, int nz, const double *basis, int nb, const double *weights, int nk,
+                      int ng, double dk, double kmin, double kmax, const double *z_edges, double *ldp,
+                      double *istar, void *workspace, size_t workspace_bytes, void *stream);
 /* rr_ld_tables_f32 followed by rr_prepare_split, as one launch for the
  * affine laws with an analytic disk integral (uniform, linear, quadratic,
  * quadratic-tri) given their basis tables: ldp[npv, npb, nz] and

@@ -45,6 +45,8 @@ def _sig(L):
                                  _d, _d, _vp, _vp, _sz, _vp, _i, _vp])
     L.rr_prepare_f64.argtypes = ([_vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp, _vp, _i, _i, _i, _d, _d, _d,
                                   _vp, _vp, _sz, _vp, _i, _vp, _i, _vp, _i])
+    L.rr_prepare_f64_ld.argtypes = ([_vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _i, _vp, _i, _vp, _i, _vp,
+                                     _i, _i, _d, _d, _d, _vp, _vp, _vp, _vp, _sz, _vp])
     L.rr_basis_count.argtypes = [_i, _i]
     L.rr_basis_tables.argtypes = [_i, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp]
     L.rr_flux_f64.argtypes = ([_vp, _i, _vp, _i, _vp, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i,

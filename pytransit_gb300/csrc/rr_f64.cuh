@@ -164,17 +164,42 @@ __device__ __forceinline__ double f64_floor_div(double a, double b, float inv_b)
 }
 
 // ---------------------------------------------------------------------------
+// Outer contact times for the bounding box, by the FP32 bisection
+// (contact_points14_f32) on the rounded coefficients.  The box decides only
+// which points are evaluated: F = 1 from the contacts outwards, in or out of
+// it.  So the FP32 times are moved outwards by their own error, the shift dt
+// with |d(z^2)| = 2 z v dt below 4e-6 or, for a grazing orbit, the whole time
+// in which z^2 moves by that much.
+// ---------------------------------------------------------------------------
+__device__ inline void contact_box(double k, const double* c, double& t1, double& t4) {
+  float cf[10];
+#pragma unroll
+  for (int i = 0; i < 10; ++i) cf[i] = (float)c[i];
+  float a, b;
+  contact_points14_f32((float)k, cf, a, b);
+  const float iv = 1.0f / fabsf(cf[1]), most = 2e-3f * iv;
+  t1 = (double)(a - fmaf(fabsf(a), 1e-6f, fminf(most, 2e-6f * iv * iv / fabsf(a))));
+  t4 = (double)(b + fmaf(fabsf(b), 1e-6f, fminf(most, 2e-6f * iv * iv / fabsf(b))));
+}
+
+// ---------------------------------------------------------------------------
 // r^2(t) = x(t)^2 + y(t)^2 of a Taylor orbit c[0..9], degree 8.
 // ---------------------------------------------------------------------------
 constexpr int R2_N = 9;
 __device__ inline void r2_poly(const double* c, double* d) {
+#pragma unroll
   for (int m = 0; m < R2_N; ++m) {
-    double s = 0.0;
-    for (int j = 0; j < 5; ++j) {
-      const int i = m - j;
-      if (i < 0 || i > 4) continue;
-      s = __fma_rn(c[j], c[i], s);
-      s = __fma_rn(c[5 + j], c[5 + i], s);
+    double s = 0.0;   // twice the products c_j c_{m-j}, j < m - j, then the square
+#pragma unroll
+    for (int j = 0; 2 * j < m; ++j) {
+      if (m - j > 4) continue;
+      s = __fma_rn(c[j], c[m - j], s);
+      s = __fma_rn(c[5 + j], c[5 + m - j], s);
+    }
+    s = __dadd_rn(s, s);
+    if (m % 2 == 0) {
+      s = __fma_rn(c[m / 2], c[m / 2], s);
+      s = __fma_rn(c[5 + m / 2], c[5 + m / 2], s);
     }
     d[m] = s;
   }

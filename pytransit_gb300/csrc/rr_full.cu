@@ -291,20 +291,27 @@ __device__ inline void ld_coefs_f32(const OrbitArgs& A, int pv, int pb, float* c
   for (int i = 0; i < ORB_MAX_LDPAR; ++i) c[i] = i < A.npar ? (float)src[i] : 0.0f;
 }
 
-// Plain FP64 path: validity, the FP64 Taylor coefficients and the contact
-// times of one pv.
+// Plain FP64 path: validity, the FP64 Taylor coefficients, the contact times
+// and r^2(t) of one pv.
 __device__ __forceinline__ void orbit_pv_f64(const OrbitArgs& A, int pv) {
   const double a = A.a[pv], e = A.e[pv], p = A.p[pv];
-  const bool ldbad = A.ldp_is_f32 ? isnan(((const float*)A.ldp)[(size_t)pv * A.npb * A.nz])
-                                  : isnan(((const double*)A.ldp)[(size_t)pv * A.npb * A.nz]);
+  bool ldbad;
+  if (A.ld_direct) {
+    double u[ORB_MAX_LDPAR];
+#pragma unroll
+    for (int i = 0; i < ORB_MAX_LDPAR; ++i) u[i] = i < A.npar ? A.ldc[(size_t)pv * A.npb * A.npar + i] : 0.0;
+    ldbad = isnan(ld_value<double>(A.law, A.mu[0], u, A.npar));
+  } else {
+    ldbad = A.ldp_is_f32 ? isnan(((const float*)A.ldp)[(size_t)pv * A.npb * A.nz])
+                         : isnan(((const double*)A.ldp)[(size_t)pv * A.npb * A.nz]);
+  }
   const bool valid = !(isnan(a) || a <= 1.0 || e < 0.0 || ldbad);
   double c[10];
   double t1 = 0.0, t4 = 0.0;
   const double k0 = A.k[(size_t)pv * A.nkc];
   if (valid) {
     solve2d_conj(p, a, A.inc[pv], e, A.w[pv], c);
-    t1 = contact_point(k0, 1, c);
-    t4 = contact_point(k0, 4, c);
+    contact_box(k0, c, t1, t4);
   } else {
     for (int i = 0; i < 10; ++i) c[i] = 0.0;
   }
@@ -531,6 +538,82 @@ __global__ void __launch_bounds__(PRO_THREADS, 8) prologue_split_kernel(ProArgs 
 }
 
 // ---------------------------------------------------------------------------
+// The same for the plain FP64 path: ld_tables_kernel<double>,
+// ldm_basis_kernel<double> and orbit_kernel<false> in one launch.  The three
+// took 74 + 63 + 53 us for 8192 pv x 4 passbands, each bound by the FP64 pipe
+// or by one thread's chain of FP64 instructions; this one takes 52 us (77 pv
+// x 1: 9 us, against 4 + 4 + 51).  Here the chains run beside
+// the LD blocks; the two k rows of a basis column are blended once for all
+// passbands (2 NB + NB npb FP64 instructions per column instead of
+// 2 (NB + 1) npb); and the profile on the mu grid is evaluated only for a k
+// outside the tables, which alone reads it.
+// ---------------------------------------------------------------------------
+struct Pro64Args {
+  OrbitArgs orb;
+  int npv, npb, npar, nz, nk, ng, kw_stride;
+  const double *ldc, *mu, *kw, *ze;
+  double kmin, kmax, dk;
+  const double* B;
+  double *ldp, *istar, *ldm;
+};
+
+template <int LAW>
+__global__ void __launch_bounds__(PRO_THREADS) prologue_f64_kernel(Pro64Args P, int norb) {
+  constexpr int NB = LAW == LD_UNIFORM ? 1 : (LAW == LD_LINEAR ? 2 : 3);   // basis_count of the law
+  __shared__ double s_coef[PRO_WARPS][PRO_MAX_COEF];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if ((int)blockIdx.x < norb) {
+    if (warp != 0) return;
+    const int pv = blockIdx.x * 32 + lane;
+    if (pv < P.npv) orbit_pv<false>(P.orb, pv);
+    return;
+  }
+  const int pv = ((int)blockIdx.x - norb) * PRO_WARPS + warp;
+  if (pv >= P.npv) return;   // warp-uniform; no block barrier follows
+  const int npb = P.npb, ng = P.ng;
+  double* coef = s_coef[warp];
+  const double* ldc = P.ldc + (size_t)pv * npb * P.npar;
+  for (int pb = lane; pb < npb; pb += 32) {
+    double is;
+    ld_integral<double>(LAW, ldc + pb * P.npar, is);
+    P.istar[(size_t)pv * npb + pb] = is;
+    basis_coefs(LAW, ldc + pb * P.npar, P.npar, coef + pb * NB);
+  }
+  __syncwarp();
+  double* out = P.ldm + (size_t)pv * npb * ng;
+  const double k = P.kw[(size_t)pv * P.kw_stride];
+  int ik = -1;
+  double ak = 0.0;
+  if (P.kmin <= k && k <= P.kmax) {   // model_full.py:46-51
+    ik = (int)floor((k - P.kmin) / P.dk);
+    ak = (k - P.kmin - ik * P.dk) / P.dk;
+    if (ik + 1 >= P.nk || ik < 0) ik = -1;
+  }
+  if (ik >= 0) {
+    const double a0 = 1.0 - ak;
+    const double* B0 = P.B + (size_t)ik * NB * ng;
+    const double* B1 = B0 + (size_t)NB * ng;
+    for (int g = lane; g < ng; g += 32) {
+      double eb[NB];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) eb[b] = fma(ak, __ldg(B1 + b * ng + g), a0 * __ldg(B0 + b * ng + g));
+      for (int pb = 0; pb < npb; ++pb) {
+        double d = coef[pb * NB] * eb[0];
+#pragma unroll
+        for (int b = 1; b < NB; ++b) d = fma(coef[pb * NB + b], eb[b], d);
+        out[(size_t)pb * ng + g] = d;
+      }
+    }
+  } else {
+    double* ldp_pv = P.ldp + (size_t)pv * npb * P.nz;
+    for (int i = lane; i < npb * P.nz; i += 32)
+      ldp_pv[i] = ld_value<double>(LAW, P.mu[i % P.nz], ldc + (i / P.nz) * P.npar, P.npar);
+    __syncwarp();
+    for (int g = lane; g < ng; g += 32) ldm_direct_g(k, g, ng, P.nz, P.ze, (const double*)ldp_pv, npb, out);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Plain FP64 flux, model_full.py:75-99, one thread per (pv, point).  The phase
 // fold uses explicitly rounded operations so no multiply-add is fused: at
 // BJD-scale times the reference's rounding sequence matters at 1e-10 d.
@@ -568,8 +651,8 @@ __device__ __forceinline__ void f64_orbit(const double* o, F64Orbit& P) {
     P.d[m] = o[ORB64_R2 + m];
     P.df[m] = f32_of(P.d[m]);
   }
-  P.t1 = f32_of(o[10]);
-  P.t4 = f32_of(o[11]);
+  P.t1 = (float)o[10];
+  P.t4 = (float)o[11];
   P.even = r2_is_even(P.d);
 }
 
@@ -1715,6 +1798,46 @@ int rr_prepare_split_ld(double t_ref, double t_absmax, const double* k, int nkc,
     default: prologue_split_kernel<LD_QUADRATIC_TRI><<<norb + nld, PRO_THREADS, 0, s>>>(P, norb); break;
   }
   return check_launch("rr_prepare_split_ld");
+}
+
+int rr_prepare_f64_ld(const double* k, int nkc, const double* p, const double* a, const double* inc, const double* e,
+                      const double* w, int npv, int npb, int law, const double* ldc, int npar, const double* mu,
+                      int nz, const double* basis, int nb, const double* weights, int nk, int ng, double dk,
+                      double kmin, double kmax, const double* z_edges, double* ldp, double* istar, void* workspace,
+                      size_t workspace_bytes, void* stream) {
+  const bool analytic = law == LD_UNIFORM || law == LD_LINEAR || law == LD_QUADRATIC || law == LD_QUADRATIC_TRI;
+  const bool fused = analytic && basis && ldc && mu && nb > 0 && nb <= MAX_BASIS && nb == basis_count(law, npar) &&
+                     npar >= 0 && npar <= ORB_MAX_LDPAR && npb * nb <= PRO_MAX_COEF;
+  if (!fused) {
+    const int st = rr_ld_tables_f64(law, ldc, npv, npb, npar, mu, nz, ldp, istar, stream);
+    if (st) return st;
+    return rr_prepare_f64(k, nkc, p, a, inc, e, w, npv, npb, ldp, weights, nk, ng, nz, dk, kmin, kmax, z_edges,
+                          workspace, workspace_bytes, stream, law, ldc, npar, basis, nb);
+  }
+  if (nkc > 1 && nkc != npb) return RR_ERR_SHAPE;
+  if (npv < 0 || npb < 1 || nk < 2 || ng < 2 || nz < 1 || nz > MAX_NZ || nkc < 1 || !ldp || !istar) return RR_ERR_ARG;
+  if (npv == 0) return RR_OK;
+  if (workspace_bytes < rr_full_f64_workspace_bytes(npv, npb, ng)) return RR_ERR_WORKSPACE;
+  Carve cv(workspace);
+  Pro64Args P{};
+  OrbitArgs& oa = P.orb;
+  oa.orb64 = cv.take<double>((size_t)npv * ORB64);
+  P.ldm = cv.take<double>((size_t)npv * npb * ng);
+  oa.k = k; oa.p = p; oa.a = a; oa.inc = inc; oa.e = e; oa.w = w;
+  oa.nkc = nkc; oa.npv = npv; oa.npb = npb; oa.nz = nz;
+  oa.ld_direct = 1; oa.law = law; oa.npar = npar; oa.ldc = ldc; oa.mu = mu;
+  P.npv = npv; P.npb = npb; P.npar = npar; P.nz = nz; P.nk = nk; P.ng = ng; P.kw_stride = nkc;
+  P.ldc = ldc; P.mu = mu; P.kw = k; P.ze = z_edges; P.kmin = kmin; P.kmax = kmax; P.dk = dk;
+  P.B = basis; P.ldp = ldp; P.istar = istar;
+  cudaStream_t s = as_stream(stream);
+  const int norb = (npv + 31) / 32, nblk = norb + (npv + PRO_WARPS - 1) / PRO_WARPS;
+  switch (law) {
+    case LD_UNIFORM: prologue_f64_kernel<LD_UNIFORM><<<nblk, PRO_THREADS, 0, s>>>(P, norb); break;
+    case LD_LINEAR: prologue_f64_kernel<LD_LINEAR><<<nblk, PRO_THREADS, 0, s>>>(P, norb); break;
+    case LD_QUADRATIC: prologue_f64_kernel<LD_QUADRATIC><<<nblk, PRO_THREADS, 0, s>>>(P, norb); break;
+    default: prologue_f64_kernel<LD_QUADRATIC_TRI><<<nblk, PRO_THREADS, 0, s>>>(P, norb); break;
+  }
+  return check_launch("rr_prepare_f64_ld");
 }
 
 int rr_flux_split(const float* times_ff, int npt, const int32_t* lcids, int npv, int nlc, int npb, int ng,

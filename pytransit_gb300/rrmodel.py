@@ -566,11 +566,12 @@ class RoadRunnerModel(TransitModel):
         ldc_d = args.get('ldc')
         npar = int(ldc_d.shape[2]) if ldc_d is not None else 0
         basis, nb = self._basis(device, npar, split) if ldc_d is not None else (None, 0)
-        # a named law in the split path: the LD tables are made by the prologue launch itself
-        fused = split and self.ld_law is not None and ldc_d is not None
+        # a named law: the LD tables are made by the prologue call itself
+        fused = self.ld_law is not None and ldc_d is not None
         if fused:
-            ldp = torch.empty((npv, npb, nz), dtype=torch.float32, device=device)
-            istar = torch.empty((npv, npb), dtype=torch.float32, device=device)
+            dt = torch.float32 if split else torch.float64
+            ldp = torch.empty((npv, npb, nz), dtype=dt, device=device)
+            istar = torch.empty((npv, npb), dtype=dt, device=device)
         else:
             ldp, istar = self._ld_tables(ldc, npv, npb, device, split, ldc_d)
         kmin, kmax = float(self.klims[0]), float(self.klims[1])
@@ -626,10 +627,16 @@ class RoadRunnerModel(TransitModel):
             res = None if pipe else torch.empty((npv, npt), dtype=torch.float64, device=device)
             wsb = L.rr_full_f64_workspace_bytes(npv, npb, self.ng)
             ws = self._workspace(wsb, device)
-            st = L.rr_prepare_f64(P(args['k']), k.shape[1], P(args['p']), P(args['a']), P(args['i']),
-                                  P(args['e']), P(args['w']), npv, npb, P(ldp), P(tb['W64']), self.nk, self.ng, nz,
-                                  self.dk, kmin, kmax, P(tb['ze']), P(ws), ws.numel(), stream,
-                                  self.ld_law or 0, P(ldc_d), npar, P(basis), nb)
+            orbit = (P(args['k']), k.shape[1], P(args['p']), P(args['a']), P(args['i']), P(args['e']), P(args['w']),
+                     npv, npb)
+            if fused:
+                st = L.rr_prepare_f64_ld(*orbit, self.ld_law, P(ldc_d), npar, P(tb['mu']), nz, P(basis), nb,
+                                         P(tb['W64']), self.nk, self.ng, self.dk, kmin, kmax, P(tb['ze']), P(ldp),
+                                         P(istar), P(ws), ws.numel(), stream)
+            else:
+                st = L.rr_prepare_f64(*orbit, P(ldp), P(tb['W64']), self.nk, self.ng, nz, self.dk, kmin, kmax,
+                                      P(tb['ze']), P(ws), ws.numel(), stream, self.ld_law or 0, P(ldc_d), npar,
+                                      P(basis), nb)
             if st == 0 and pipe:
                 st = self._flux64_to_host(args, dd, istar, npt, npv, nlc, npb, ws, host_rows, device)
             elif st == 0:
