@@ -319,17 +319,24 @@ __device__ __forceinline__ F64Limb f64_limb(const F64Disk& D, double r2, double 
 // The LD means' lerp at separation z (common.py:225-233 with the two
 // divisions folded into D.cg): the cell from the FP32 position, moved by one
 // where its FP64 fraction falls outside [0, 1).
-__device__ __forceinline__ double f64_ld_mean(const F64Disk& D, double z, const double* __restrict__ lda, int ng) {
+__device__ __forceinline__ void f64_ld_cell(const F64Disk& D, double z, const double* __restrict__ lda, int ng, int& i,
+                                            double& fr, double& l0, double& dl) {
   float fi = fminf(truncf(f32_of_pos(z) * D.cgf), (float)(ng - 2));
-  double fr = __fma_rn(z, D.cg, -f64_of_pos(fi));
+  fr = __fma_rn(z, D.cg, -f64_of_pos(fi));
   const float ff = f32_of(fr);
   if ((ff < 0.0f && fi > 0.0f) || (ff >= 1.0f && fi < (float)(ng - 2))) {
     fi += ff < 0.0f ? -1.0f : 1.0f;
     fr = __fma_rn(z, D.cg, -f64_of_pos(fi));
   }
-  const int i = (int)fi;
-  const double l0 = __ldg(lda + i);
-  return __fma_rn(fr, __dadd_rn(__ldg(lda + i + 1), -l0), l0);
+  i = (int)fi;
+  l0 = __ldg(lda + i);
+  dl = __dadd_rn(__ldg(lda + i + 1), -l0);
+}
+__device__ __forceinline__ double f64_ld_mean(const F64Disk& D, double z, const double* __restrict__ lda, int ng) {
+  int i;
+  double fr, l0, dl;
+  f64_ld_cell(D, z, lda, ng, i, fr, l0, dl);
+  return __fma_rn(fr, dl, l0);
 }
 
 }  // namespace rr

@@ -1,0 +1,351 @@
+// The points of the plain FP64 RoadRunner path (model_full.py:75-99): fold,
+// box, samples, and the walk of a warp over its tiles that the flux and the
+// log-likelihood kernels share.
+#pragma once
+#include "rr_f64.cuh"
+#include "rr_internal.h"
+
+namespace rr {
+
+// Data, parameters and prologue tables of one call.
+struct F64Args {
+  const double* times;
+  const double *k, *t0, *p, *exptimes, *istar, *ldm, *orb64;
+  const int32_t *lcids, *pbids, *epids, *nsamples;
+  int npt, npv, nkc, ldt0, npb, nlc, ng;
+  double dg;
+  bool nan_istar;      // a non-finite disk integral makes in-box points NaN
+};
+
+// Phase fold of the reference (model_full.py:84-86) with its rounding: the
+// epoch's conjunction t0 + epoch p, epoch = floor(((t - t0) + p/2) / p).
+__device__ __forceinline__ double f64_conjunction(double t, double t0, double p, float inv_p) {
+  const double epoch = f64_floor_div(__dadd_rn(__dsub_rn(t, t0), __dmul_rn(0.5, p)), p, inv_p);
+  return __dadd_rn(t0, __dmul_rn(epoch, p));
+}
+
+// Constants of one parameter vector: r^2(t) in FP64 and FP32.
+struct F64Orbit {
+  double d[R2_N];
+  float df[R2_N];
+  float t1, t4;        // contacts
+  int even;
+};
+
+__device__ __forceinline__ void f64_orbit(const double* o, F64Orbit& P) {
+#pragma unroll
+  for (int m = 0; m < R2_N; ++m) {
+    P.d[m] = o[ORB64_R2 + m];
+    P.df[m] = f32_of(P.d[m]);
+  }
+  P.t1 = (float)o[10];
+  P.t4 = (float)o[11];
+  P.even = r2_is_even(P.d);
+}
+
+// Constants of one light curve of one pv.
+struct F64Lc {
+  F64Disk disk;
+  double w;            // 1 / (istar nsamples); NaN for a non-finite istar (A.nan_istar)
+  double ex, step;     // exposure time and its share of one sample
+  float lo, hi;        // box
+  int ns, pb;
+};
+
+template <bool IK = false>
+__device__ __forceinline__ void f64_lc(const F64Args& A, int pv, int lc, const F64Orbit& P, F64Lc& R) {
+  R.pb = A.pbids[lc];
+  R.ns = max(A.nsamples[lc], 0);
+  R.ex = A.exptimes[lc];
+  R.step = R.ns > 1 ? __ddiv_rn(R.ex, (double)R.ns) : R.ex;
+  // Box: the contact times padded by 0.003 d + exposure (model_full.py:87-89).
+  // It only separates points that may overlap the star from points that
+  // cannot (F = 1 on both sides of its edges), so it is FP32.
+  const float ex = f32_of(R.ex), pad = 0.003f + ex;
+  R.lo = P.t1 - pad;
+  R.hi = P.t4 + pad;
+  // bound of the FP32 r^2's error at any sample: 16 roundings of the largest partial sums
+  const float tb = fmaxf(fabsf(R.lo), fabsf(R.hi)) + ex;
+  float sum = fabsf(P.df[R2_N - 1]);
+#pragma unroll
+  for (int m = R2_N - 2; m >= 0; --m) sum = fmaf(sum, tb, fabsf(P.df[m]));
+  f64_disk<IK>(A.k[(size_t)pv * A.nkc + (A.nkc == A.npb ? R.pb : 0)], A.dg, fmaf(4e-6f, sum, 2e-6f), R.disk);
+  const double is = A.istar[(size_t)pv * A.npb + R.pb];
+  R.w = isfinite(is) || !A.nan_istar ? f64_recip(R.ns == 1 ? is : __dmul_rn(is, (double)R.ns)) : CUDART_NAN;
+}
+
+// Time of sample s (0 based) from conjunction: tc + ex ((s + 1/2) / ns - 1/2).
+__device__ __forceinline__ double f64_sample_time(const F64Lc& R, double tc, int s) {
+  if (R.ns == 1) return tc;
+  return __fma_rn(f64_of_pos((float)s + 0.5f), R.step, __fma_rn(-0.5, R.ex, tc));
+}
+
+// LD means of one passband and, for the general form, the orbit they belong to.
+struct F64Table {
+  const double *o, *lda;
+  int ng;
+  double dg;
+};
+
+// The term I(z) A(z) of one sample by the reference's own expressions
+// (model_full.py:93-98), for the separations and radius ratios that the
+// kernels' forms leave out: z = 0, k <= 0, k >= 1, NaN.
+static __device__ __noinline__ double f64_term_general(const F64Table& T, double k, double t) {
+  double c[10];
+  for (int i = 0; i < 10; ++i) c[i] = T.o[i];
+  const double z = sep_c_f64(t, c);
+  double kap;
+  return interp_ldm_f64(z / (1.0 + k), T.dg, T.lda, T.ng) * ccia_star<double>(k, z, kap);
+}
+
+// Class of the sample at t from the FP32 r^2: 0 surely outside the star (its
+// term is 0), 1 surely inside (the planet's whole disk), 2 the limb or unsure.
+__device__ __forceinline__ int f64_class(const F64Lc& R, const F64Orbit& P, double t) {
+  const float tf = f32_of(t);
+  float r = P.df[R2_N - 1];
+#pragma unroll
+  for (int m = R2_N - 2; m >= 0; --m) r = fmaf(r, tf, P.df[m]);
+  return r > R.disk.r2out ? 0 : (r < R.disk.r2in ? 1 : 2);
+}
+
+__device__ __forceinline__ double f64_term_inner(const F64Lc& R, const F64Orbit& P, const F64Table& T, double t) {
+  const double r2 = r2_at(P.d, P.even, t);
+  if (!f64_moderate(r2)) return f64_term_general(T, R.disk.k, t);
+  return __dmul_rn(f64_ld_mean(R.disk, f64_sqrt(f64_root(r2)), T.lda, T.ng), R.disk.area_in);
+}
+
+__device__ __forceinline__ double f64_term_limb(const F64Lc& R, const F64Orbit& P, const F64Table& T, double t) {
+  const double r2 = r2_at(P.d, P.even, t);
+  if (!R.disk.fast || !f64_moderate(r2)) return f64_term_general(T, R.disk.k, t);
+  const F64Root q = f64_root(r2);
+  const double ip = f64_ld_mean(R.disk, f64_sqrt(q), T.lda, T.ng);
+  return __dmul_rn(ip, f64_limb<false>(R.disk, r2, f64_rsqrt(q)).area);
+}
+
+constexpr int F64_Q = 256;        // points and (point, sample) pairs a warp holds
+constexpr int F64_LC_SMEM = 32;   // light-curve constants staged per block
+struct F64Queue {
+  double tc[F64_Q];
+  double term[F64_Q];
+  int pt[F64_Q];
+  unsigned short list[F64_Q];
+};
+
+__device__ __forceinline__ void f64_box(const F64Args& A, const F64Orbit& P, int lc, const F64Lc* recs, float& lo,
+                                        float& hi) {
+  if (lc < F64_LC_SMEM) {
+    lo = recs[lc].lo;
+    hi = recs[lc].hi;
+  } else {
+    const float pad = 0.003f + f32_of(A.exptimes[lc]);
+    lo = P.t1 - pad;
+    hi = P.t4 + pad;
+  }
+}
+
+// The terms of the samples [s0, s0 + ns) of the ni items from i0 on: each pair
+// (item, sample) classified in FP32, then the inner and the limb pairs as full
+// warps.  inner(f, it, s) and limb(f, it, s) do one pair (f = it ns + s - s0, at
+// most F64_Q pairs), none(f) a pair outside the star.
+template <class Inner, class Limb, class None>
+__device__ __forceinline__ void f64_pairs(const F64Lc& R, const F64Orbit& P, F64Queue& Q, int i0, int ni, int s0,
+                                          int ns, Inner inner, Limb limb, None none) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const int np = ni * ns;
+  const float ins = 1.0f / (float)ns;
+  int nin = 0, nlimb = 0;   // pairs on the inner list (from the front) and the limb list (from the back)
+  for (int f0 = 0; f0 < np; f0 += 32) {
+    const int f = f0 + lane;
+    int cls = 0;
+    if (f < np) {
+      const int it = (ns == 1) ? f : (int)(((float)f + 0.5f) * ins);
+      cls = f64_class(R, P, f64_sample_time(R, Q.tc[i0 + it], s0 + f - it * ns));
+      if (cls == 0) none(f);
+    }
+    const unsigned m1 = __ballot_sync(FULL, cls == 1), m2 = __ballot_sync(FULL, cls == 2);
+    if (cls == 1) Q.list[nin + __popc(m1 & below)] = (unsigned short)f;
+    if (cls == 2) Q.list[F64_Q - 1 - nlimb - __popc(m2 & below)] = (unsigned short)f;
+    nin += __popc(m1);
+    nlimb += __popc(m2);
+  }
+  __syncwarp();
+  for (int j = lane; j < nin; j += 32) {
+    const int f = Q.list[j], it = (ns == 1) ? f : (int)(((float)f + 0.5f) * ins);
+    inner(f, it, s0 + f - it * ns);
+  }
+  for (int j = lane; j < nlimb; j += 32) {
+    const int f = Q.list[F64_Q - 1 - j], it = (ns == 1) ? f : (int)(((float)f + 0.5f) * ins);
+    limb(f, it, s0 + f - it * ns);
+  }
+  __syncwarp();
+}
+
+// The sums D = sum_s I A of the n queued points, all of the light curve R:
+// point(i, D) is called once per point by one lane, chunk(i0, ni) by the warp
+// after the points [i0, i0 + ni).
+template <class Point, class Chunk>
+__device__ __forceinline__ void f64_sums(const F64Lc& R, const F64Orbit& P, const F64Table& T, F64Queue& Q, int n,
+                                         Point point, Chunk chunk) {
+  const int lane = threadIdx.x & 31;
+  // R, P and Q arrive as generic pointers (the callers are not inlined)
+  __builtin_assume(__isShared(&R));
+  __builtin_assume(__isShared(&P));
+  __builtin_assume(__isShared(&Q));
+  __syncwarp();
+  const int sc = min(max(R.ns, 1), F64_Q);   // samples and points of a chunk of pairs
+  const int ic = F64_Q / sc;
+  for (int i0 = 0; i0 < n; i0 += ic) {
+    const int ni = min(ic, n - i0);
+    double D = 0.0;
+    for (int s0 = 0; s0 < max(R.ns, 1); s0 += sc) {
+      const int ns = min(sc, R.ns - s0);
+      f64_pairs(R, P, Q, i0, ni, s0, ns,
+                [&](int f, int it, int s) { Q.term[f] = f64_term_inner(R, P, T, f64_sample_time(R, Q.tc[i0 + it], s)); },
+                [&](int f, int it, int s) { Q.term[f] = f64_term_limb(R, P, T, f64_sample_time(R, Q.tc[i0 + it], s)); },
+                [&](int f) { Q.term[f] = 0.0; });
+      if (s0 + ns == R.ns) {
+        for (int i = lane; i < ni; i += 32) {
+          if (s0 == 0) D = ns > 0 ? Q.term[i * ns] : 0.0;
+          for (int s = s0 == 0 ? 1 : 0; s < ns; ++s) D = __dadd_rn(D, Q.term[i * ns + s]);
+          point(i0 + i, D);
+        }
+      } else if (lane == 0) {
+        // more samples than a chunk holds: one point at a time, its sum carried by lane 0
+        for (int s = 0; s < ns; ++s) D = s0 + s == 0 ? Q.term[0] : __dadd_rn(D, Q.term[s]);
+      }
+      __syncwarp();
+    }
+    chunk(i0, ni);
+  }
+}
+
+// A warp's walk over its share of one pv's row: slots / 4 tiles from the
+// block's first, or, in launches too small to fill the GPU, `slots` < 4 of one
+// tile's four 32-point slots.  sink.tile(p0, q0, q1) gets a tile (slots q0 to
+// q1) without in-box points, sink.outside(pt) a point out of the box,
+// sink.flush(lc, n) the queued points.
+template <class Sink>
+__device__ __forceinline__ void f64_walk(const F64Args& A, int pv, const double* __restrict__ tiles64, int slots,
+                                         bool valid, const F64Orbit& P, const F64Lc* recs, F64Queue& Q, const Sink& sink) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int ntiles = (A.npt + TIME_TILE - 1) / TIME_TILE;
+  const int slot0 = blockIdx.x * slots;
+  const int tb0 = slot0 >> 2, tb1 = min(ntiles, tb0 + max(slots >> 2, 1));
+  const int q0 = slot0 & 3, q1 = slots < 4 ? q0 + slots : 4;
+  const double p = A.p[pv], hp = __dmul_rn(0.5, p);
+  const float inv_p = 1.0f / f32_of(p);
+  int n = 0, qlc = -1;   // queued points and their light curve
+  for (int tbase = tb0; tbase < tb1; tbase += 32) {
+    const int jn = min(32, tb1 - tbase);
+    bool cull = !valid, tileone = false;   // tileone: one light curve and one epoch
+    double conj = 0.0;
+    int tlc = -1;
+    float blo = 0.0f, bhi = 0.0f;
+    if (valid && lane < jn) {
+      const double2 tm = __ldg(reinterpret_cast<const double2*>(tiles64 + 4 * (size_t)(tbase + lane)));
+      tlc = (int)f32_of(__ldg(tiles64 + 4 * (size_t)(tbase + lane) + 2));
+      if (tlc >= 0) {
+        const double t0 = A.t0[(size_t)pv * A.ldt0 + A.epids[tlc]];
+        f64_box(A, P, tlc, recs, blo, bhi);
+        // the epoch of both ends: in FP32 where that leaves no doubt
+        const double h0 = __dadd_rn(__dsub_rn(tm.x, t0), hp);
+        const float span = f32_of(__dsub_rn(tm.y, tm.x)) * 1.000001f;
+        const float qe = f32_of(h0) * inv_p;
+        float n0, n1;
+        const bool sure0 = f64_floor_sure(qe, n0), sure1 = f64_floor_sure(fmaf(span, inv_p, qe), n1);
+        const double e0 = sure0 ? f64_int(n0) : floor(__ddiv_rn(h0, p));
+        conj = __dadd_rn(t0, __dmul_rn(e0, p));
+        const float tc0 = f32_of(__dsub_rn(tm.x, conj));
+        if (sure0 && sure1 && n0 == n1) {
+          tileone = true;
+          cull = tc0 > bhi || tc0 + span + 1e-6f * (fabsf(tc0) + span) < blo;
+        } else {
+          // an epoch or more begins inside the tile: its first points end at
+          // +p/2, its last ones start at -p/2
+          const double e1 = sure1 ? f64_int(n1) : floor(__ddiv_rn(__dadd_rn(__dsub_rn(tm.y, t0), hp), p));
+          const float tc1 = f32_of(__dsub_rn(tm.y, __dadd_rn(t0, __dmul_rn(e1, p))));
+          tileone = e0 == e1;
+          cull = tileone ? (tc0 > bhi || tc1 < blo) : (e1 == e0 + 1.0 && tc0 > bhi && tc1 < blo);
+        }
+      }
+    }
+    const unsigned jmask = jn == 32 ? FULL : (1u << jn) - 1u;
+    const unsigned cmask = __ballot_sync(FULL, cull) & jmask;
+    for (unsigned m = cmask; m; m &= m - 1u) sink.tile((tbase + __ffs(m) - 1) * TIME_TILE, q0, q1);
+    for (unsigned m = ~cmask & jmask; m; m &= m - 1u) {
+      const int j = __ffs(m) - 1;
+      const int p0 = (tbase + j) * TIME_TILE;
+      const int lc = __shfl_sync(FULL, tlc, j);
+      const double cj = __shfl_sync(FULL, conj, j);
+      const float lo = __shfl_sync(FULL, blo, j), hi = __shfl_sync(FULL, bhi, j);
+      const bool one = __shfl_sync(FULL, (int)tileone, j) != 0;
+      for (int q = q0; q < q1; ++q) {
+        const int pt = p0 + 32 * q + lane;
+        bool in = false;
+        double tc = 0.0;
+        int l = lc;
+        if (pt < A.npt) {
+          const double t = __ldg(A.times + pt);
+          float plo = lo, phi = hi;
+          if (one) {
+            tc = __dsub_rn(t, cj);
+          } else {
+            if (lc < 0) {
+              l = A.lcids[pt];
+              f64_box(A, P, l, recs, plo, phi);
+            }
+            tc = __dsub_rn(t, f64_conjunction(t, A.t0[(size_t)pv * A.ldt0 + A.epids[l]], p, inv_p));
+          }
+          const float tf = f32_of(tc);
+          in = plo <= tf && tf <= phi;
+          if (!in) sink.outside(pt);
+        }
+        // the in-box points to the queue, one light curve at a time
+        for (unsigned pend = __ballot_sync(FULL, in); pend;) {
+          const int kl = __shfl_sync(FULL, l, __ffs(pend) - 1);
+          const unsigned mem = __ballot_sync(FULL, l == kl) & pend;
+          if (n > 0 && (kl != qlc || n > F64_Q - 32)) {
+            sink.flush(qlc, n);
+            n = 0;
+          }
+          qlc = kl;
+          if (mem >> lane & 1u) {
+            const int at = n + __popc(mem & ((1u << lane) - 1u));
+            Q.tc[at] = tc;
+            Q.pt[at] = pt;
+          }
+          n += __popc(mem);
+          pend &= ~mem;
+        }
+      }
+    }
+  }
+  if (n > 0) sink.flush(qlc, n);
+}
+
+// Launch shape of a walk: slots of 32 points per warp.  Below two rounds of 16
+// warps per SM single slots or pairs, so that a small call's chain of FP64
+// operations is as short as it can be (77 x 1501: 329 us with 32 tiles a warp,
+// 14 us).  Above, whole tiles, evenly over the row's warps: up to 64 while that
+// leaves four rounds (flux of 8192 x 19,700: 515 us with at most 32 tiles a
+// warp, 491 with 64, 493 with 96), and down to 8 while that leaves one, since a
+// warp's own cost (constants, cull test, partly filled last lists) is that of
+// about two tiles (log-likelihood of 1500 x 2999: 156 us with 3, 142 with 8).
+inline int f64_slots(int npt, int npv) {
+  const int ntiles = (npt + TIME_TILE - 1) / TIME_TILE;
+  const long long tiles = (long long)ntiles * npv, round = 16LL * sm_count();
+  if (tiles < round) return 4 * tiles <= round ? 1 : (4 * tiles <= 2 * round ? 2 : 4);
+  long long want = tiles / (4 * round);
+  const long long least = tiles / round < 8 ? tiles / round : 8;
+  want = want < least ? least : (want > 64 ? 64 : want);
+  const int nblk = (int)((ntiles + want - 1) / want);
+  return 4 * ((ntiles + nblk - 1) / nblk);
+}
+inline int f64_warps(int npt, int slots) {
+  return (4 * ((npt + TIME_TILE - 1) / TIME_TILE) + slots - 1) / slots;
+}
+
+}  // namespace rr

@@ -12,10 +12,12 @@
 // bounding box and the epoch count are piecewise constant and contribute no
 // derivative.  Out-of-box points (F = 1 exactly) only enter through the
 // pv-independent constant sum_i -log sigma_i - log(2 pi)/2 - (o_i - 1)^2/(2 sigma_i^2).
+#include <algorithm>
 #include <cmath>
 
 #include "rr_device.cuh"
 #include "rr_dual.cuh"
+#include "rr_f64_points.cuh"
 #include "rr_internal.h"
 
 namespace rr {
@@ -146,27 +148,78 @@ grad_ld_kernel(int law, const double* __restrict__ ldc, int npb, int npar, const
 // ---------------------------------------------------------------------------
 // Observations: dobs[i] = o_i - 1 and isig2[i] = 1/sigma_lc^2 in R, and the
 // pv-independent constant of lnL in per-block parts (FP64, fixed order), one
-// block per OBS_CHUNK points.
+// block per OBS_CHUNK points.  With tiles64 also the FP64 summaries of the
+// chunk's 128-point tiles (rr_time_tiles_f64), a warp per tile.
 // ---------------------------------------------------------------------------
 constexpr int OBS_THREADS = 128;
 constexpr int OBS_CHUNK = OBS_THREADS * 4;
+constexpr int OBS_LC = 128;   // light curves whose constants a block stages
 
 template <typename R>
 __global__ void __launch_bounds__(OBS_THREADS) obs_kernel(const double* __restrict__ obs,
                                                           const double* __restrict__ sigma,
-                                                          const int32_t* __restrict__ lcids, int npt,
+                                                          const int32_t* __restrict__ lcids, int npt, int nlc,
                                                           R* __restrict__ dobs, R* __restrict__ isig2,
-                                                          double* __restrict__ cpart) {
+                                                          double* __restrict__ cpart,
+                                                          const double* __restrict__ times,
+                                                          double* __restrict__ tiles64) {
   __shared__ double red[OBS_THREADS / 32];
-  double acc = 0.0;
+  static_assert(OBS_CHUNK == (OBS_THREADS / 32) * TIME_TILE, "a warp summarises one tile of the block's chunk");
+  if (tiles64) {
+    const int tile = blockIdx.x * (OBS_CHUNK / TIME_TILE) + (threadIdx.x >> 5);
+    if (tile * TIME_TILE < npt) {   // warp-uniform
+      const int lane = threadIdx.x & 31;
+      const int lc0 = lcids[tile * TIME_TILE];
+      double tmin = INFINITY, tmax = -INFINITY;
+      bool same = true;
+      for (int q = 0; q < TIME_TILE / 32; ++q) {
+        const int i = tile * TIME_TILE + 32 * q + lane;
+        if (i >= npt) break;
+        tmin = fmin(tmin, times[i]);
+        tmax = fmax(tmax, times[i]);
+        same = same && lcids[i] == lc0;
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        tmin = fmin(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
+        tmax = fmax(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+      }
+      same = __all_sync(0xffffffffu, same);
+      if (lane == 0) {
+        double* t = tiles64 + 4 * (size_t)tile;
+        t[0] = tmin;
+        t[1] = tmax;
+        t[2] = same ? (double)lc0 : -1.0;
+        t[3] = 0.0;
+      }
+    }
+  }
+  // A light curve's constants once per block (a logarithm and two divisions
+  // per point made this kernel 13.5 us for 3000 points; now 8)
+  __shared__ double s_c[OBS_LC][3];   // -log(sigma) - log(2 pi) / 2, 1 / sigma, 1 / sigma^2
   const double hl2pi = 0.5 * log(2.0 * PI);
+  auto constants = [&](int lc, double* c) {
+    const double sg = sigma[lc];
+    c[0] = -log(sg) - hl2pi;
+    c[1] = 1.0 / sg;
+    c[2] = 1.0 / (sg * sg);
+  };
+  const bool staged = nlc <= OBS_LC;
+  if (staged)
+    for (int lc = threadIdx.x; lc < nlc; lc += blockDim.x) constants(lc, s_c[lc]);
+  __syncthreads();
+  double acc = 0.0;
   const int i0 = blockIdx.x * OBS_CHUNK, i1 = min(npt, i0 + OBS_CHUNK);
   for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-    const double s = sigma[lcids[i]];
+    double c[3];
+    if (staged) {
+      for (int j = 0; j < 3; ++j) c[j] = s_c[lcids[i]][j];
+    } else {
+      constants(lcids[i], c);
+    }
     const double d = obs[i] - 1.0;
     dobs[i] = (R)d;
-    isig2[i] = (R)(1.0 / (s * s));
-    acc += -log(s) - hl2pi - 0.5 * (d / s) * (d / s);
+    isig2[i] = (R)c[2];
+    acc += c[0] - 0.5 * (d * c[1]) * (d * c[1]);
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -190,21 +243,15 @@ __global__ void __launch_bounds__(OBS_THREADS) obs_kernel(const double* __restri
 template <typename R>
 struct GradArgs {
   // data
-  const double* times;          // FP64 path
-  const float2* times_ff;       // split path
-  const int32_t *lcids, *pbids, *epids, *nsamples;
-  const double* exptimes;
+  const float2* times_ff;
+  const int32_t *lcids, *pbids, *epids;
   const R *dobs, *isig2;
-  // parameters (FP64 path reads them directly)
-  const double *k, *t0, *p, *istar64;
-  int nkc, ldt0, nep;
+  int nkc, nep;
   // prologue tables
-  const double* orb64;
   const float *orb32, *lc32;
   const R *ldm, *dc, *tab, *dis;
   int npt, npv, npb, nlc, ng, npar, ngrad;
   double dg;
-  int grad;
   double* partials;
 };
 
@@ -231,62 +278,35 @@ constexpr int LNL_NW = LNL_THREADS / 32;
 // deficit D and with it the residual weight -(r / sigma^2) / (ns istar); the
 // second recomputes each sample and adds its derivative terms, already
 // scaled by that weight, straight into acc (no per-point sums are kept).
-template <typename R, bool SPLIT, bool GRAD>
+template <typename R, bool GRAD>
 __device__ __forceinline__ void lnlike_point(const GradArgs<R>& A, int pv, int pt, int lc, const float* lcs,
                                              bool lc_smem, const R* orbc, const R* dcs, R* acc) {
   const int pb = A.pbids[lc], ep = A.epids[lc];
   bool inbox;
   R tc, nep_count;
-  if (SPLIT) {
-    const float* LCR = lc_smem ? lcs + lc * LC32 : A.lc32 + ((size_t)pv * A.nlc + lc) * LC32;
-    const float* o = A.orb32 + (size_t)pv * ORB32;
-    const float p_hi = o[10], p_lo = o[11], inv_p = o[12];
-    const float2 tt = A.times_ff[pt];
-    const float d0h = LCR[LC_D0H], d0l = LCR[LC_D0L];
-    float n = floorf(fmaf(tt.x - d0h, inv_p, 0.5f));
-    float s1, e1, q1, e2, s2, e3;
-    two_sum(tt.x, -d0h, s1, e1);
+  const float* LCR = lc_smem ? lcs + lc * LC32 : A.lc32 + ((size_t)pv * A.nlc + lc) * LC32;
+  const float* o = A.orb32 + (size_t)pv * ORB32;
+  const float p_hi = o[10], p_lo = o[11], inv_p = o[12];
+  const float2 tt = A.times_ff[pt];
+  const float d0h = LCR[LC_D0H], d0l = LCR[LC_D0L];
+  float n = floorf(fmaf(tt.x - d0h, inv_p, 0.5f));
+  float s1, e1, q1, e2, s2, e3;
+  two_sum(tt.x, -d0h, s1, e1);
+  two_prod(n, p_hi, q1, e2);
+  two_sum(s1, -q1, s2, e3);
+  float t = s2 + (((e1 + e3) - e2) + (tt.y - d0l) - n * p_lo);
+  if (t >= 0.5f * p_hi || t < -0.5f * p_hi) {
+    n += (t >= 0.5f * p_hi) ? 1.0f : -1.0f;
     two_prod(n, p_hi, q1, e2);
     two_sum(s1, -q1, s2, e3);
-    float t = s2 + (((e1 + e3) - e2) + (tt.y - d0l) - n * p_lo);
-    if (t >= 0.5f * p_hi || t < -0.5f * p_hi) {
-      n += (t >= 0.5f * p_hi) ? 1.0f : -1.0f;
-      two_prod(n, p_hi, q1, e2);
-      two_sum(s1, -q1, s2, e3);
-      t = s2 + (((e1 + e3) - e2) + (tt.y - d0l) - n * p_lo);
-    }
-    inbox = (LCR[LC_LO] <= t && t <= LCR[LC_HI]);
-    tc = (R)t;
-    nep_count = (R)n;
-  } else {
-    const double t = A.times[pt];
-    const double t0 = A.t0[(size_t)pv * A.ldt0 + ep];
-    const double p = A.p[pv];
-    const double epoch = floor(__ddiv_rn(__dadd_rn(__dsub_rn(t, t0), __dmul_rn(0.5, p)), p));
-    const double tcd = __dsub_rn(t, __dadd_rn(t0, __dmul_rn(epoch, p)));
-    const double pad = __dadd_rn(0.003, A.exptimes[lc]);
-    const double* o = A.orb64 + (size_t)pv * ORB64;
-    inbox = (__dsub_rn(o[10], pad) <= tcd && tcd <= __dadd_rn(o[11], pad));
-    tc = (R)tcd;
-    nep_count = (R)epoch;
+    t = s2 + (((e1 + e3) - e2) + (tt.y - d0l) - n * p_lo);
   }
+  inbox = (LCR[LC_LO] <= t && t <= LCR[LC_HI]);
+  tc = (R)t;
+  nep_count = (R)n;
   if (!inbox) return;
-  R kk, inv_is, ex, inv_ns;
-  int ns;
-  if (SPLIT) {
-    const float* LCR = lc_smem ? lcs + lc * LC32 : A.lc32 + ((size_t)pv * A.nlc + lc) * LC32;
-    kk = (R)LCR[LC_K];
-    inv_is = (R)LCR[LC_INVIS];
-    ex = (R)LCR[LC_EXPT];
-    inv_ns = (R)LCR[LC_INVNS];
-    ns = __float_as_int(LCR[LC_NS]);
-  } else {
-    kk = (R)A.k[(size_t)pv * A.nkc + (A.nkc == A.npb ? pb : 0)];
-    inv_is = R(1) / (R)A.istar64[(size_t)pv * A.npb + pb];
-    ex = (R)A.exptimes[lc];
-    ns = A.nsamples[lc];
-    inv_ns = R(1) / (R)ns;
-  }
+  const R kk = (R)LCR[LC_K], inv_is = (R)LCR[LC_INVIS], ex = (R)LCR[LC_EXPT], inv_ns = (R)LCR[LC_INVNS];
+  const int ns = __float_as_int(LCR[LC_NS]);
   const R inv1pk = R(1) / (R(1) + kk);
   const R inv_dg = R(1) / (R)A.dg;
   const size_t ppb = (size_t)pv * A.npb + pb;
@@ -428,25 +448,23 @@ __device__ __forceinline__ void lnlike_flush(const GradArgs<R>& A, R* acc, int k
 // depend on its passband and epoch), flushing to its warp's row of shared
 // sums when the light curve changes and at the end; the block writes the sum
 // of the warps' rows, in warp order, to its slot of partials.
-template <typename R, bool SPLIT, bool GRAD>
-__global__ void __launch_bounds__(LNL_THREADS, sizeof(R) == 4 ? 4 : 2) lnlike_kernel(GradArgs<R> A) {
+template <typename R, bool GRAD>
+__global__ void __launch_bounds__(LNL_THREADS, 4) lnlike_kernel(GradArgs<R> A) {
   constexpr int NS = GRAD ? GS_NSLOT : 1;
   __shared__ double wred[LNL_NW][1 + MAX_NGRAD];
-  __shared__ __align__(16) float lcs[SPLIT ? GLC_SMEM * LC32 : 1];
+  __shared__ __align__(16) float lcs[GLC_SMEM * LC32];
   __shared__ R orbc[10];
   __shared__ R dcs[50];
   const int pv = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5;
   for (int i = tid; i < LNL_NW * (1 + MAX_NGRAD); i += blockDim.x) (&wred[0][0])[i] = 0.0;
-  if (tid < 10)
-    orbc[tid] = SPLIT ? (R)A.orb32[(size_t)pv * ORB32 + tid] : (R)A.orb64[(size_t)pv * ORB64 + tid];
+  if (tid < 10) orbc[tid] = (R)A.orb32[(size_t)pv * ORB32 + tid];
   if (GRAD && tid < 50) dcs[tid] = A.dc[(size_t)pv * 50 + tid];
-  const bool lc_smem = SPLIT && A.nlc <= GLC_SMEM;
+  const bool lc_smem = A.nlc <= GLC_SMEM;
   if (lc_smem)
     for (int i = tid; i < A.nlc * LC32; i += blockDim.x) lcs[i] = A.lc32[(size_t)pv * A.nlc * LC32 + i];
   __syncthreads();
-  const bool valid = SPLIT ? (__float_as_int(A.orb32[(size_t)pv * ORB32 + 14]) & FLAG_VALID)
-                           : (A.orb64[(size_t)pv * ORB64 + 12] != 0.0);
+  const bool valid = __float_as_int(A.orb32[(size_t)pv * ORB32 + 14]) & FLAG_VALID;
   R acc[NS];
 #pragma unroll
   for (int s = 0; s < NS; ++s) acc[s] = R(0);
@@ -460,7 +478,7 @@ __global__ void __launch_bounds__(LNL_THREADS, sizeof(R) == 4 ? 4 : 2) lnlike_ke
       if (flush) key = -1;
     }
     if (lc < 0) continue;
-    lnlike_point<R, SPLIT, GRAD>(A, pv, pt, lc, lcs, lc_smem, orbc, dcs, acc);
+    lnlike_point<R, GRAD>(A, pv, pt, lc, lcs, lc_smem, orbc, dcs, acc);
     key = lc;
   }
   lnlike_flush<R, NS>(A, acc, key, key >= 0, wred[warp]);
@@ -474,6 +492,282 @@ __global__ void __launch_bounds__(LNL_THREADS, sizeof(R) == 4 ? 4 : 2) lnlike_ke
   }
 }
 
+// ---------------------------------------------------------------------------
+// The FP64 likelihood and its adjoint, one warp per share of a pv's row, on the
+// walk, queue and sample arithmetic of the FP64 flux (rr_f64_points.cuh): the
+// FP64 pipe bounds both, so the in-box points are collected and their inner
+// and limb samples run as full warps.
+//
+// The adjoint's sums are taken in the form that needs the fewest FP64
+// instructions per sample:
+//   * orbit coefficients: z depends on theta through x(t) and y(t), polynomials
+//     whose coefficients' derivatives dc belong to the pv, so the samples only
+//     accumulate the moments sum (x / z) t^m dL/dz and sum (y / z) t^m dL/dz
+//     (18 instructions a sample, against 55 for five derivative polynomials);
+//     the five columns follow from the ten moments once per share;
+//   * disk integral: one sum of r D / sigma^2 per light curve.
+// Sums are per lane in a fixed order, over lanes in lane order and over shares
+// in order: reproducible bit for bit.
+// ---------------------------------------------------------------------------
+enum FSlot { FS_LNL = 0, FS_KK, FS_KW, FS_IS, FS_T, FS_P, FS_C0, FS_M0 = FS_C0 + MAX_GRAD_PAR, FS_NSLOT = FS_M0 + 10 };
+
+struct LnlF64Args : F64Args {
+  const double *dobs, *isig2, *dc, *tab, *dis;
+  int npar, nep, ngrad;
+  double* partials;
+};
+
+template <bool GRAD>
+struct LnlF64Smem {
+  static constexpr int NS = GRAD ? FS_NSLOT : 1;
+  double acc[NS][33];                      // per-lane sums of the current light curve
+  double tot[NS];
+  double row[GRAD ? 1 + MAX_NGRAD : 1];    // the share's columns
+  double g[GRAD ? F64_Q : 1];              // per point of a chunk: -(r / sigma^2) w
+  float ep[GRAD ? F64_Q : 1];              // per point of a chunk: epoch
+  int lc;                                  // light curve of acc, or -1
+};
+
+// I(z) A(z)'s value and partial derivatives at one sample.
+struct F64Partials {
+  double x, y, iz, ip, slope, ar, dadk, dadz, z, fr;   // slope = dI/dz
+  int i;
+  bool none;
+};
+
+static __device__ __noinline__ void f64_partials_general(const F64Disk& K, const F64Table& T, double r2, F64Partials& S) {
+  const double z = sqrt(r2);
+  S.z = z;
+  S.none = !(z < 1.0 + K.k);
+  S.iz = 1.0 / z;
+  const double gg = z / (1.0 + K.k) / T.dg;
+  S.i = min(max((int)gg, 0), T.ng - 2);
+  S.fr = gg - (double)S.i;
+  const double l0 = T.lda[S.i], l1 = T.lda[S.i + 1];
+  S.ip = l0 + S.fr * (l1 - l0);
+  S.slope = (l1 - l0) / ((1.0 + K.k) * T.dg);
+  S.ar = ccia_star_grad<double>(K.k, z, S.dadk, S.dadz);
+}
+
+__device__ __forceinline__ void f64_partials(const F64Lc& R, const F64Table& T, double t, bool limb, F64Partials& S) {
+  const F64Disk& K = R.disk;
+  const double* c = T.o;
+  double x = c[4], y = c[9];
+#pragma unroll
+  for (int m = 3; m >= 0; --m) {
+    x = __fma_rn(x, t, c[m]);
+    y = __fma_rn(y, t, c[5 + m]);
+  }
+  S.x = x;
+  S.y = y;
+  S.none = false;
+  const double r2 = __fma_rn(x, x, __dmul_rn(y, y));
+  if (!f64_moderate(r2) || (limb && !K.fast)) {
+    f64_partials_general(K, T, r2, S);
+    return;
+  }
+  const F64Root q = f64_root(r2);
+  S.z = f64_sqrt(q);
+  S.iz = f64_rsqrt(q);
+  double l0, dl;
+  f64_ld_cell(K, S.z, T.lda, T.ng, S.i, S.fr, l0, dl);
+  S.ip = __fma_rn(S.fr, dl, l0);
+  S.slope = __dmul_rn(dl, K.cg);
+  if (limb) {
+    const F64Limb L = f64_limb<true>(K, r2, S.iz);
+    S.ar = L.area;
+    S.dadk = __dmul_rn(__dadd_rn(K.k, K.k), L.kappa0);
+    S.dadz = __dmul_rn(-2.0 * L.kite, S.iz);
+  } else {
+    S.ar = K.area_in;
+    S.dadk = __dmul_rn(2.0 * PI, K.k);
+    S.dadz = 0.0;
+  }
+}
+
+// The lanes' sums of light curve S.lc into the share's columns.
+template <bool GRAD>
+__device__ __noinline__ void lnl_f64_reduce(const LnlF64Args& A, LnlF64Smem<GRAD>& S, int pv) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  // lnL in the same order with and without the gradient
+  double l = S.acc[FS_LNL][lane];
+  for (int d = 16; d > 0; d >>= 1) l = __dadd_rn(l, __shfl_down_sync(0xffffffffu, l, d));
+  if (lane == 0) S.row[0] += l;
+  if constexpr (GRAD) {
+    // a lane per slot, over the lanes in order: 31 FP64 instructions for all slots
+    if (lane > FS_LNL && lane < S.NS) {
+      double v = S.acc[lane][0];
+      for (int i = 1; i < 32; ++i) v = __dadd_rn(v, S.acc[lane][i]);
+      S.tot[lane] = v;
+    }
+    __syncwarp();
+    const int pb = A.pbids[S.lc], ep = A.epids[S.lc], nkc = A.nkc, nep = A.nep;
+    double* col = S.row + 1;
+    if (lane < 5) {
+      const double* d = A.dc + (size_t)pv * 50 + lane * 10;
+      double v = lane == 0 ? -S.tot[FS_P] : 0.0;
+      for (int m = 0; m < 10; ++m) v += d[m] * S.tot[FS_M0 + m];
+      col[nkc + nep + lane] += v;
+    } else if (lane == 6) {
+      col[nkc == 1 ? 0 : pb] += S.tot[FS_KK];
+      col[0] += S.tot[FS_KW];
+    } else if (lane == 7) {
+      col[nkc + ep] -= S.tot[FS_T];
+    } else if (lane >= 8 && lane < 8 + A.npar) {
+      const int j = lane - 8;
+      const size_t ppb = (size_t)pv * A.npb + pb;
+      col[nkc + nep + 5 + pb * A.npar + j] +=
+          S.tot[FS_C0 + j] + S.tot[FS_IS] * A.dis[ppb * A.npar + j] / A.istar[ppb];
+    }
+  }
+  __syncwarp();
+  for (int i = lane; i < S.NS * 33; i += 32) (&S.acc[0][0])[i] = 0.0;
+  __syncwarp();
+}
+
+// The terms of the n queued points, all of light curve lc, into the lanes' sums.
+template <bool GRAD>
+__device__ __noinline__ void lnl_f64_flush(const LnlF64Args& A, const F64Orbit& P, F64Lc* recs, F64Queue& Q,
+                                           const double* o, LnlF64Smem<GRAD>& S, int pv, int lc, int n) {
+  const int lane = threadIdx.x & 31, nrec = min(A.nlc, F64_LC_SMEM);
+  if (lc != S.lc) {
+    if (S.lc >= 0) lnl_f64_reduce<GRAD>(A, S, pv);
+    if (lane == 0) S.lc = lc;
+    __syncwarp();
+  }
+  if (lc >= F64_LC_SMEM) {
+    if (lane == 0) f64_lc<GRAD>(A, pv, lc, P, recs[nrec]);
+    __syncwarp();
+  }
+  const F64Lc& R = recs[min(lc, nrec)];
+  const size_t ppb = (size_t)pv * A.npb + R.pb;
+  const F64Table T{o, A.ldm + ppb * A.ng, A.ng, A.dg};
+  double lnl = S.acc[FS_LNL][lane], is = GRAD ? S.acc[GRAD ? FS_IS : 0][lane] : 0.0;
+  const double t0 = GRAD ? A.t0[(size_t)pv * A.ldt0 + A.epids[lc]] : 0.0;
+  const float inv_p = 1.0f / f32_of(A.p[pv]);
+  f64_sums(
+      R, P, T, Q, n,
+      [&](int i, double SQ) {
+        const int pt = Q.pt[i];
+        const double D = __dmul_rn(SQ, R.w), d = A.dobs[pt], w = A.isig2[pt];
+        lnl = __fma_rn(-__dmul_rn(__fma_rn(0.5, D, d), D), w, lnl);
+        if constexpr (GRAD) {
+          const int j = i % (F64_Q / min(max(R.ns, 1), F64_Q));   // the point's place in its chunk
+          const double rw = __dmul_rn(__dadd_rn(d, D), w);
+          S.g[j] = __dmul_rn(-rw, R.w);
+          is = __fma_rn(rw, D, is);
+          S.ep[j] = rintf(f32_of(__dsub_rn(__dsub_rn(A.times[pt], t0), Q.tc[i])) * inv_p);
+        }
+      },
+      [&](int i0, int ni) {
+        if constexpr (GRAD) {
+          double a[FS_NSLOT];
+#pragma unroll
+          for (int s = 0; s < FS_NSLOT; ++s) a[s] = S.acc[s][lane];
+          const double* tab = A.tab + ppb * (size_t)(1 + A.npar) * A.ng;
+          const double inv1pk = __dmul_rn(R.disk.cg, A.dg);
+          const int sc = min(max(R.ns, 1), F64_Q);
+          __syncwarp();
+          auto sample = [&](int it, int smp, bool limb) {
+            const double t = f64_sample_time(R, Q.tc[i0 + it], smp);
+            F64Partials q;
+            f64_partials(R, T, t, limb, q);
+            if (q.none) return;
+            const double g = S.g[it], ga = __dmul_rn(g, q.ar);
+            const double gi = __dmul_rn(g, q.ip);
+            a[FS_KK] = __fma_rn(gi, q.dadk, a[FS_KK]);
+            a[FS_KK] = __fma_rn(-__dmul_rn(__dmul_rn(q.slope, q.z), inv1pk), ga, a[FS_KK]);
+            const double* Tt = tab + q.i;
+#pragma unroll
+            for (int j = -1; j < MAX_GRAD_PAR; ++j) {
+              if (j >= A.npar) break;
+              const double* Tj = Tt + (size_t)(1 + j) * A.ng;
+              const double v = __fma_rn(q.fr, __dadd_rn(__ldg(Tj + 1), -__ldg(Tj)), __ldg(Tj));
+              double& s = a[j < 0 ? FS_KW : FS_C0 + j];
+              s = __fma_rn(v, ga, s);
+            }
+            // dL/dz over z, then its moments
+            const double gz = __dmul_rn(__fma_rn(q.slope, ga, __dmul_rn(gi, q.dadz)), q.iz);
+            double u = __dmul_rn(gz, q.x), v = __dmul_rn(gz, q.y);
+            double xd = __dmul_rn(4.0, o[4]), yd = __dmul_rn(4.0, o[9]);
+#pragma unroll
+            for (int m = 3; m >= 1; --m) {
+              xd = __fma_rn(xd, t, (double)m * o[m]);
+              yd = __fma_rn(yd, t, (double)m * o[5 + m]);
+            }
+            const double gt = __fma_rn(u, xd, __dmul_rn(v, yd));   // dL/dz dz/dt
+            a[FS_T] = __dadd_rn(a[FS_T], gt);
+            if (S.ep[it] != 0.0f) a[FS_P] = __fma_rn(gt, f64_of(S.ep[it]), a[FS_P]);
+#pragma unroll
+            for (int m = 0; m < 5; ++m) {
+              a[FS_M0 + m] = __dadd_rn(a[FS_M0 + m], u);
+              a[FS_M0 + 5 + m] = __dadd_rn(a[FS_M0 + 5 + m], v);
+              if (m < 4) {
+                u = __dmul_rn(u, t);
+                v = __dmul_rn(v, t);
+              }
+            }
+          };
+          for (int s0 = 0; s0 < R.ns; s0 += sc)
+            f64_pairs(
+                R, P, Q, i0, ni, s0, min(sc, R.ns - s0),
+                [&](int, int it, int smp) { sample(it, smp, false); },
+                [&](int, int it, int smp) { sample(it, smp, true); }, [](int) {});
+#pragma unroll
+          for (int s = 0; s < FS_NSLOT; ++s)
+            if (s != FS_LNL && s != FS_IS) S.acc[s][lane] = a[s];
+          __syncwarp();
+        }
+      });
+  S.acc[FS_LNL][lane] = lnl;
+  if constexpr (GRAD) S.acc[FS_IS][lane] = is;
+}
+
+template <bool GRAD>
+struct LnlF64Sink {
+  const LnlF64Args& A;
+  const F64Orbit& P;
+  F64Lc* recs;
+  F64Queue& Q;
+  const double* o;
+  LnlF64Smem<GRAD>& S;
+  int pv;
+
+  __device__ __forceinline__ void tile(int, int, int) const {}
+  __device__ __forceinline__ void outside(int) const {}
+  __device__ __forceinline__ void flush(int lc, int n) const { lnl_f64_flush<GRAD>(A, P, recs, Q, o, S, pv, lc, n); }
+};
+
+template <bool GRAD>
+__global__ void __launch_bounds__(32, GRAD ? 12 : 20) lnlike_f64_kernel(const __grid_constant__ LnlF64Args A, const double* tiles64,
+                                                                         int slots) {
+  __shared__ double o[ORB64];
+  __shared__ F64Orbit P;
+  __shared__ F64Queue Q;
+  __shared__ LnlF64Smem<GRAD> S;
+  extern __shared__ __align__(16) unsigned char lnl_smem[];
+  F64Lc* recs = reinterpret_cast<F64Lc*>(lnl_smem);
+  const int pv = blockIdx.y, lane = threadIdx.x;
+  if (lane < ORB64) o[lane] = A.orb64[(size_t)pv * ORB64 + lane];
+  const int ncol = GRAD ? 1 + A.ngrad : 1;
+  for (int i = lane; i < ncol; i += 32) S.row[i] = 0.0;
+  if (lane == 0) S.lc = -1;
+  for (int i = lane; i < S.NS * 33; i += 32) (&S.acc[0][0])[i] = 0.0;
+  __syncwarp();
+  const bool valid = o[12] != 0.0;
+  if (valid) {
+    if (lane == 0) f64_orbit(o, P);
+    __syncwarp();
+    for (int lc = lane; lc < min(A.nlc, F64_LC_SMEM); lc += 32) f64_lc<GRAD>(A, pv, lc, P, recs[lc]);
+    __syncwarp();
+    f64_walk(A, pv, tiles64, slots, true, P, recs, Q, LnlF64Sink<GRAD>{A, P, recs, Q, o, S, pv});
+    if (S.lc >= 0) lnl_f64_reduce<GRAD>(A, S, pv);
+  }
+  double* out = A.partials + ((size_t)pv * gridDim.x + blockIdx.x) * (1 + A.ngrad);
+  for (int i = lane; i < ncol; i += 32) out[i] = S.row[i];
+}
+
 // Sum the block partials of each pv in a fixed order; invalid pv -> NaN.
 __global__ void lnlike_reduce_kernel(const double* __restrict__ partials, int nblk, int ngrad, int npv,
                                      const double* __restrict__ cpart, int ncpart, const double* __restrict__ orb64,
@@ -482,7 +776,7 @@ __global__ void lnlike_reduce_kernel(const double* __restrict__ partials, int nb
   const int pv = blockIdx.x;
   const bool valid = orb32 ? (__float_as_int(orb32[(size_t)pv * ORB32 + 14]) & FLAG_VALID)
                            : (orb64[(size_t)pv * ORB64 + 12] != 0.0);
-  for (int i = threadIdx.x; i <= ngrad; i += blockDim.x) {
+  for (int i = threadIdx.x; i <= (grad ? ngrad : 0); i += blockDim.x) {
     double s = 0.0;
     for (int b = 0; b < nblk; ++b) s += partials[((size_t)pv * nblk + b) * (1 + ngrad) + i];
     if (!valid) s = CUDART_NAN;
@@ -499,6 +793,7 @@ template <typename R>
 struct GradWs {
   R *dc, *tab, *dis, *dobs, *isig2;
   double *partials, *cconst;   // cconst: the constant of lnL in per-block parts
+  double* tiles64;             // FP64 path: tile summaries
 };
 
 template <typename R>
@@ -511,7 +806,13 @@ static GradWs<R> carve_grad(Carve& cv, int npv, int npb, int npar, int ng, int n
   g.isig2 = cv.take<R>((size_t)npt);
   g.partials = cv.take<double>((size_t)npv * nblk * (1 + ngrad));
   g.cconst = cv.take<double>((size_t)(npt + OBS_CHUNK - 1) / OBS_CHUNK);
+  g.tiles64 = sizeof(R) == 8 ? cv.take<double>(4 * (((size_t)npt + TIME_TILE - 1) / TIME_TILE)) : nullptr;
   return g;
+}
+
+// Shares of a pv's row: the partial sums' count.
+static int lnlike_blocks(int split, int npt, int npv) {
+  return split ? (npt + LNL_CHUNK - 1) / LNL_CHUNK : f64_warps(npt, f64_slots(npt, npv));
 }
 
 }  // namespace rr
@@ -524,7 +825,7 @@ int rr_lnlike_ngrad(int nkc, int nep, int npb, int npar) { return nkc + nep + 5 
 
 size_t rr_lnlike_workspace_bytes(int split, int npv, int npb, int nlc, int nep, int ng, int npar, int npt,
                                  int nkc) {
-  const int nblk = (npt + LNL_CHUNK - 1) / LNL_CHUNK;
+  const int nblk = lnlike_blocks(split, npt, npv);
   const int ngrad = rr_lnlike_ngrad(nkc, nep, npb, npar);
   size_t base = split ? rr_full_split_workspace_bytes(npv, npb, nlc, nep, ng) : rr_full_f64_workspace_bytes(npv, npb, ng);
   Carve c(nullptr);
@@ -567,7 +868,7 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
     st = rr_prepare_f64(k, nkc, p, a, inc, e, w, npv, npb, (const double*)ldp, (const double*)weights, nk, ng, nz,
                         dk, kmin, kmax, z_edges, workspace, base, stream, 0, nullptr, 0, nullptr, 0);
   if (st) return st;
-  const int nblk = (npt + LNL_CHUNK - 1) / LNL_CHUNK;
+  const int nblk = lnlike_blocks(split, npt, npv);
   Carve cv(static_cast<char*>(workspace) + base);
   GradWs<R> g = carve_grad<R>(cv, npv, npb, npar, ng, npt, nblk, ngrad);
   // prologue tables of the forward pass (inside the base workspace)
@@ -583,27 +884,38 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
     orb64 = pcv.take<double>((size_t)npv * ORB64);
     ldm = (const R*)pcv.take<double>((size_t)npv * npb * ng);
   }
-  grad_orbit_kernel<R><<<(npv + 63) / 64, 64, 0, s>>>(p, a, inc, e, w, npv, g.dc);
-  grad_ld_kernel<R><<<dim3(npv, npb), 128, 0, s>>>(law, ldc, npb, npar, mu, nz, ldp, k, nkc, weights, nk, ng, dk,
-                                                   kmin, kmax, z_edges, g.tab, g.dis);
+  if (grad) {   // the derivative tables, read by the adjoint alone
+    grad_orbit_kernel<R><<<(npv + 63) / 64, 64, 0, s>>>(p, a, inc, e, w, npv, g.dc);
+    grad_ld_kernel<R><<<dim3(npv, npb), 128, 0, s>>>(law, ldc, npb, npar, mu, nz, ldp, k, nkc, weights, nk, ng, dk,
+                                                     kmin, kmax, z_edges, g.tab, g.dis);
+  }
   const int nobs = (npt + OBS_CHUNK - 1) / OBS_CHUNK;
-  obs_kernel<R><<<nobs, OBS_THREADS, 0, s>>>(obs, sigma, lcids, npt, g.dobs, g.isig2, g.cconst);
-  GradArgs<R> A{};
-  A.times = times; A.times_ff = reinterpret_cast<const float2*>(times_ff);
-  A.lcids = lcids; A.pbids = pbids; A.epids = epids; A.nsamples = nsamples; A.exptimes = exptimes;
-  A.dobs = g.dobs; A.isig2 = g.isig2;
-  A.k = k; A.t0 = t0; A.p = p; A.istar64 = (const double*)istar; A.nkc = nkc; A.ldt0 = ldt0; A.nep = nep;
-  A.orb64 = orb64; A.orb32 = orb32; A.lc32 = lc32;
-  A.ldm = ldm; A.dc = g.dc; A.tab = g.tab; A.dis = g.dis;
-  A.npt = npt; A.npv = npv; A.npb = npb; A.nlc = nlc; A.ng = ng; A.npar = npar; A.ngrad = ngrad;
-  A.dg = dg; A.grad = grad != nullptr; A.partials = g.partials;
-  dim3 grid(nblk, npv);
-  if (split) {
-    if (A.grad) lnlike_kernel<R, true, true><<<grid, LNL_THREADS, 0, s>>>(A);
-    else lnlike_kernel<R, true, false><<<grid, LNL_THREADS, 0, s>>>(A);
+  obs_kernel<R><<<nobs, OBS_THREADS, 0, s>>>(obs, sigma, lcids, npt, nlc, g.dobs, g.isig2, g.cconst, times, g.tiles64);
+  if constexpr (sizeof(R) == 4) {
+    GradArgs<R> A{};
+    A.times_ff = reinterpret_cast<const float2*>(times_ff);
+    A.lcids = lcids; A.pbids = pbids; A.epids = epids;
+    A.dobs = g.dobs; A.isig2 = g.isig2; A.nkc = nkc; A.nep = nep;
+    A.orb32 = orb32; A.lc32 = lc32;
+    A.ldm = ldm; A.dc = g.dc; A.tab = g.tab; A.dis = g.dis;
+    A.npt = npt; A.npv = npv; A.npb = npb; A.nlc = nlc; A.ng = ng; A.npar = npar; A.ngrad = ngrad;
+    A.dg = dg; A.partials = g.partials;
+    const dim3 grid(nblk, npv);
+    if (grad) lnlike_kernel<R, true><<<grid, LNL_THREADS, 0, s>>>(A);
+    else lnlike_kernel<R, false><<<grid, LNL_THREADS, 0, s>>>(A);
   } else {
-    if (A.grad) lnlike_kernel<R, false, true><<<grid, LNL_THREADS, 0, s>>>(A);
-    else lnlike_kernel<R, false, false><<<grid, LNL_THREADS, 0, s>>>(A);
+    LnlF64Args A{};
+    A.times = times; A.k = k; A.t0 = t0; A.p = p; A.exptimes = exptimes; A.istar = (const double*)istar;
+    A.ldm = (const double*)ldm; A.orb64 = orb64;
+    A.lcids = lcids; A.pbids = pbids; A.epids = epids; A.nsamples = nsamples;
+    A.npt = npt; A.npv = npv; A.nkc = nkc; A.ldt0 = ldt0; A.npb = npb; A.nlc = nlc; A.ng = ng; A.dg = dg;
+    A.dobs = g.dobs; A.isig2 = g.isig2; A.dc = g.dc; A.tab = g.tab; A.dis = g.dis;
+    A.npar = npar; A.nep = nep; A.ngrad = ngrad; A.partials = g.partials;
+    const dim3 grid(nblk, npv);
+    const int slots = f64_slots(npt, npv);
+    const size_t smem = sizeof(F64Lc) * (std::min(nlc, F64_LC_SMEM) + 1);
+    if (grad) lnlike_f64_kernel<true><<<grid, 32, smem, s>>>(A, g.tiles64, slots);
+    else lnlike_f64_kernel<false><<<grid, 32, smem, s>>>(A, g.tiles64, slots);
   }
   lnlike_reduce_kernel<<<npv, 64, 0, s>>>(g.partials, nblk, ngrad, npv, g.cconst, nobs, orb64, orb32, lnl, grad);
   return check_launch("rr_lnlike");
