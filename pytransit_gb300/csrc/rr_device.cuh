@@ -342,54 +342,6 @@ __device__ inline void basis_coefs(int law, const double* pv, int npar, double* 
 // r'' = -mu r/|r|^3.  c[0..4] are the x coefficients, c[5..9] the y ones
 // (x(t) = sum c[j] t^j, layout of gdmodel.py:441-442); sky axes as
 // taylor_z.py:62-76.
-// Eccentric anomaly from the mean anomaly by Newton's method, |err| <= 1e-8
-// (ea_newton_s, pytransit/orbits/orbits_py.py:145-154).
-__device__ inline double ea_newton(double M, double e) {
-  double E = M, err = 0.05;
-  for (int k = 0; fabs(err) > 1e-8 && k < 1000; ++k) {
-    err = E - e * sin(E) - M;
-    E = E - err / (1.0 - e * cos(E));
-  }
-  return E;
-}
-
-// solve2d about t = phase (days from mid-transit; the mid-eclipse for the
-// eclipse models): the Keplerian state at that time (mean anomaly from the
-// one at conjunction, f = pi/2 - w, plus n phase), then the Taylor jet of
-// solve2d_conj below.
-__device__ inline void solve2d_phase(double phase, double p, double a, double inc, double e, double w, double* c) {
-  const double n = 2.0 * PI / p;
-  const double se = sqrt(1.0 - e * e);
-  const double f0 = 0.5 * PI - w;
-  const double E0 = atan2(se * sin(f0), e + cos(f0));
-  const double M = E0 - e * sin(E0) + n * phase;
-  const double E = ea_newton(M, e);
-  const double f = atan2(se * sin(E) / (1.0 - e * cos(E)), (cos(E) - e) / (1.0 - e * cos(E)));
-  const double sf = sin(f), cf = cos(f);
-  const double cth = cos(w + f), sth = sin(w + f);
-  const double r = a * (1.0 - e * e) / (1.0 + e * cf);
-  const double vr = n * a * e * sf / se;
-  const double vt = n * a * (1.0 + e * cf) / se;
-  double P0x = r * cth, P0y = r * sth;
-  double P1x = vr * cth - vt * sth, P1y = vr * sth + vt * cth;
-  const double mu = n * n * a * a * a;
-  const double alpha = -1.5;
-  const double q0 = P0x * P0x + P0y * P0y;
-  const double q1 = 2.0 * (P0x * P1x + P0y * P1y);
-  const double s0 = 1.0 / (q0 * sqrt(q0));
-  const double P2x = -mu * s0 * P0x / 2.0, P2y = -mu * s0 * P0y / 2.0;
-  const double s1 = alpha * q1 * s0 / q0;
-  const double P3x = -mu * (s0 * P1x + s1 * P0x) / 6.0;
-  const double P3y = -mu * (s0 * P1y + s1 * P0y) / 6.0;
-  const double q2 = 2.0 * (P0x * P2x + P0y * P2y) + (P1x * P1x + P1y * P1y);
-  const double s2 = ((alpha - 1.0) * q1 * s1 + 2.0 * alpha * q2 * s0) / (2.0 * q0);
-  const double P4x = -mu * (s0 * P2x + s1 * P1x + s2 * P0x) / 12.0;
-  const double P4y = -mu * (s0 * P2y + s1 * P1y + s2 * P0y) / 12.0;
-  const double ci = cos(inc);
-  c[0] = -P0x; c[1] = -P1x; c[2] = -P2x; c[3] = -P3x; c[4] = -P4x;
-  c[5] = -ci * P0y; c[6] = -ci * P1y; c[7] = -ci * P2y; c[8] = -ci * P3y; c[9] = -ci * P4y;
-}
-
 // The jet at conjunction, f = pi/2 - w, with what vanishes there left out:
 // the position is (0, r), so with g = mu / r^3 the series of r'' = -mu r/|r|^3
 // is, per order,
@@ -400,12 +352,11 @@ __device__ inline void solve2d_phase(double phase, double p, double a, double in
 // One thread's FP64 instructions are issued ~75 cycles apart, so their number
 // is the kernel's time: 4 divisions and a root here, against 12 and 2 for the
 // general recurrence, and no sine of w for a circular orbit.
-__device__ inline void solve2d_conj(double p, double a, double inc, double e, double w, double* c) {
+// (sf, cf): sine and cosine of the true anomaly there, read for e != 0.
+__device__ inline void solve2d_apsis(double p, double a, double inc, double e, double sf, double cf, double* c) {
   const double n = 2.0 * PI / p;
   double r = a, vr = 0.0, vt = n * a;
   if (e != 0.0) {
-    double sf = 1.0, cf = 0.0;
-    sincos(w, &cf, &sf);   // f = pi/2 - w: sin f = cos w, cos f = sin w
     const double se2 = 1.0 - e * e, q = 1.0 + e * cf;
     const double v = n * a / sqrt(se2);
     r = a * se2 / q;
@@ -427,6 +378,24 @@ __device__ inline void solve2d_conj(double p, double a, double inc, double e, do
   c[7] = -ci * P2y;
   c[8] = -ci * (2.0 * gs * vr);
   c[9] = ci * (0.5 * gs * (P2y + 1.5 * ir * (3.0 * vr * vr - q2)));
+}
+
+__device__ inline void solve2d_conj(double p, double a, double inc, double e, double w, double* c) {
+  double sf = 1.0, cf = 0.0;
+  if (e != 0.0) sincos(w, &cf, &sf);   // f = pi/2 - w: sin f = cos w, cos f = sin w
+  solve2d_apsis(p, a, inc, e, sf, cf, c);
+}
+
+// The same about the eclipse, f = 3 pi/2 - w: the other conjunction of the
+// orbit turned by pi, so every coefficient changes its sign.  (The state
+// propagated there from the transit by Newton's method on Kepler's equation,
+// as the reference's solve2d(eclipse offset, ...) takes it, agrees to 2e-15.)
+__device__ inline void solve2d_ecl(double p, double a, double inc, double e, double w, double* c) {
+  double sf = 1.0, cf = 0.0;
+  if (e != 0.0) sincos(w, &cf, &sf);
+  solve2d_apsis(p, a, inc, e, -sf, -cf, c);
+#pragma unroll
+  for (int i = 0; i < 10; ++i) c[i] = -c[i];
 }
 
 // solve2d_conj in FP32 for the split path, whose flux kernel reads the

@@ -4,23 +4,31 @@
 // model_ecspec.py:13-63, npb flux ratios).  Same orbit layer as the transit
 // model, expanded about mid-eclipse, the eclipse time shifted by the light
 // travel time across the orbit.
+#include <algorithm>
 #include <cmath>
 
-#include "rr_device.cuh"
+#include "rr_f64_points.cuh"
 #include "rr_internal.h"
 
 namespace rr {
 
-constexpr int ECL_REC = 16;   // c[0..9], [10] t1, [11] t4, [12] shift, [13] valid, [14] ltt, [15] unused
+// Per-pv record of the FP64 models: the ORB64 record (about mid-eclipse), then
+// [22] shift, [23] light travel time.
+constexpr int ECL_SHIFT = ORB64_R2 + R2_N;
+static_assert(ECL_SHIFT + 2 <= ORB64, "the eclipse's two times follow r^2(t) in the record");
 
 // Time from mid-transit to mid-eclipse from the mean anomalies at the two
 // conjunctions, wrapped to (0, p] (meepmeep's eclipse_time_offset; the
 // reference's own eclipse_phase, pytransit/orbits/orbits_py.py:544-555).
-__device__ inline double eclipse_time_offset(double p, double e, double w) {
+// Split into the mean anomaly at the conjunction f = f0 + pi/2 - w (f0 = 0 the
+// transit, pi the eclipse) and the time between the two.
+__device__ inline double conjunction_anomaly(double e, double w, double f0) {
   const double se = sqrt(1.0 - e * e);
-  const double etr = atan2(se * sin(0.5 * PI - w), e + cos(0.5 * PI - w));
-  const double eec = atan2(se * sin(0.5 * PI + PI - w), e + cos(0.5 * PI + PI - w));
-  const double mtr = etr - e * sin(etr), mec = eec - e * sin(eec);
+  const double f = 0.5 * PI + f0 - w;
+  const double E = atan2(se * sin(f), e + cos(f));
+  return E - e * sin(E);
+}
+__device__ inline double eclipse_time_offset(double p, double mtr, double mec) {
   const double ph = (mec - mtr) * p / (2.0 * PI);
   return ph > 0.0 ? ph : p + ph;
 }
@@ -36,175 +44,248 @@ __device__ inline double eclipse_ltt(double a, double inc, double e, double w, d
 }
 
 // Per pv: validity, eclipse shift, light travel time, Taylor coefficients
-// about mid-eclipse and the contact points (model_eclipse.py:38-60).
-__global__ void eclipse_prepare_kernel(const double* __restrict__ k, const double* __restrict__ p,
-                                       const double* __restrict__ a, const double* __restrict__ inc,
-                                       const double* __restrict__ e, const double* __restrict__ w,
-                                       const double* __restrict__ rstar, int npv, double* __restrict__ rec) {
-  const int pv = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pv >= npv) return;
-  double* o = rec + (size_t)pv * ECL_REC;
-  for (int i = 0; i < ECL_REC; ++i) o[i] = 0.0;
-  if (isnan(a[pv]) || a[pv] <= 1.0 || e[pv] < 0.0) return;
-  const double shift = eclipse_time_offset(p[pv], e[pv], w[pv]);
-  double c[10];
-  solve2d_phase(shift, p[pv], a[pv], inc[pv], e[pv], w[pv], c);
-  for (int i = 0; i < 10; ++i) o[i] = c[i];
-  o[10] = contact_point(k[pv], 1, c);
-  o[11] = contact_point(k[pv], 4, c);
-  o[12] = shift;
-  o[13] = 1.0;
-  o[14] = eclipse_ltt(a[pv], inc[pv], e[pv], w[pv], rstar[pv]);
+// about mid-eclipse, contact points and r^2(t) (model_eclipse.py:38-60).  One
+// thread's FP64 instructions are issued ~75 cycles apart, so the four parts
+// run on four warps, lane = pv: the mean anomalies at the two conjunctions, the
+// orbit, and the light travel time (1000 pv: 76 us on one thread per pv, with
+// the FP64 bisections and Kepler's equation; 12 us).
+constexpr int ECL_PREP_THREADS = 128;
+
+__global__ void __launch_bounds__(ECL_PREP_THREADS)
+eclipse_prepare_kernel(const double* __restrict__ k, const double* __restrict__ p, const double* __restrict__ a,
+                       const double* __restrict__ inc, const double* __restrict__ e, const double* __restrict__ w,
+                       const double* __restrict__ rstar, int npv, double* __restrict__ rec) {
+  __shared__ double s_m[2][32], s_ltt[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int pv = blockIdx.x * 32 + lane;
+  double* o = rec + (size_t)pv * ORB64;
+  const bool valid = pv < npv && !(isnan(a[pv]) || a[pv] <= 1.0 || e[pv] < 0.0);
+  if (valid) {
+    if (warp < 2) {
+      s_m[warp][lane] = conjunction_anomaly(e[pv], w[pv], warp == 0 ? 0.0 : PI);
+    } else if (warp == 2) {
+      double c[10], t1, t4;
+      solve2d_ecl(p[pv], a[pv], inc[pv], e[pv], w[pv], c);
+      contact_box(k[pv], c, t1, t4);
+      for (int i = 0; i < 10; ++i) o[i] = c[i];
+      o[10] = t1;
+      o[11] = t4;
+      r2_poly(c, o + ORB64_R2);
+    } else {
+      s_ltt[lane] = eclipse_ltt(a[pv], inc[pv], e[pv], w[pv], rstar[pv]);
+    }
+  }
+  __syncthreads();
+  if (warp == 0 && pv < npv) {
+    o[12] = valid ? 1.0 : 0.0;
+    if (valid) {
+      o[ECL_SHIFT] = eclipse_time_offset(p[pv], s_m[0][lane], s_m[1][lane]);
+      o[ECL_SHIFT + 1] = s_ltt[lane];
+    }
+  }
 }
 
-// eclipse_model's light curve loop (model_eclipse.py:62-80), one thread per
-// (pv, point): pi k^2 outside the padded box, else the mean over the exposure
-// samples of the visible area pi k^2 - A(1, k, z).
-struct EclF64Args {
-  const double* times;
-  int npt;
-  const double *k, *t0;
-  int ldt0;
-  const double* p;
-  const int32_t *lcids, *epids, *nsamples;
-  const double *exptimes, *rec;
-  int npv;
+// eclipse_model's light curve loop (model_eclipse.py:62-80) on the walk, queue
+// and limb area of the FP64 transit flux (rr_f64_points.cuh): pi k^2 outside
+// the padded box, else the mean over the exposure samples of the visible area
+// pi k^2 - A(1, k, z).  A sample inside the star leaves nothing visible and
+// needs no FP64 work; one on the limb takes 30 FP64 instructions, against ~170
+// with two arctangents.  1000 x 19,699: 547 us point by point, 87 us.
+struct EclF64Args : F64Args {
   double* flux;
   int ldflux;
 };
 
-// One point of a valid pv: pi k^2 outside the padded box, else the mean over
-// the exposure samples of the visible area pi k^2 - A(1, k, z).  Compiled
-// once and called by both flux kernels, so that the compiler's fusing of
-// multiplies and adds is the same in both and so are their bits.
-__device__ __noinline__ double ecl_point_f64(const EclF64Args& A, int pv, int pt, const double* o) {
-  const int lc = A.lcids[pt];
-  const double kk = A.k[pv];
-  const double pik2 = PI * (kk * kk);
-  const double pp = A.p[pv];
-  const double te = __dadd_rn(__dadd_rn(A.t0[(size_t)pv * A.ldt0 + A.epids[lc]], o[12]), o[14]);
-  const double t = A.times[pt];
-  const double epoch = floor(__ddiv_rn(__dadd_rn(__dsub_rn(t, te), __dmul_rn(0.5, pp)), pp));
-  const double tc = __dsub_rn(t, __dadd_rn(te, __dmul_rn(epoch, pp)));
-  const double ex = A.exptimes[lc];
-  const double pad = __dadd_rn(0.003, ex);
-  if (!(__dsub_rn(o[10], pad) <= tc && tc <= __dadd_rn(o[11], pad))) return pik2;
-  double c[10];
-  for (int i = 0; i < 10; ++i) c[i] = o[i];
-  const int ns = A.nsamples[lc];
-  double f = 0.0;
-  for (int s = 1; s < ns + 1; ++s) {
-    const double z = sep_c_f64(tc + ex * ((s - 0.5) / ns - 0.5), c);
-    double kap;
-    f += pik2 - ccia_star<double>(kk, z, kap);
-  }
-  return f / ns;
+// One point of a valid pv by one thread.
+__device__ __noinline__ double ecl_point_f64(const EclF64Args& A, int pv, int lc, double tc, const double* o) {
+  F64Orbit P;
+  f64_orbit(o, P);
+  F64Lc R;
+  f64_lc(A, pv, lc, P, R);
+  const float tf = f32_of(tc);
+  if (!(R.lo <= tf && tf <= R.hi)) return R.disk.area_in;
+  return f64_point_value(R, P, F64Eclipse{o}, tc);
 }
 
-// eclipse_model's light curve loop (model_eclipse.py:62-80), one thread per
-// (pv, point).
-__global__ void __launch_bounds__(256) eclipse_flux_kernel(EclF64Args A) {
+// Every point through the reference's fold, one thread per (pv, point).
+__global__ void __launch_bounds__(256) eclipse_flux_kernel(const __grid_constant__ EclF64Args A) {
   const int pv = blockIdx.z * 65535 + blockIdx.y;
   const int pt = blockIdx.x * blockDim.x + threadIdx.x;
   if (pt >= A.npt || pv >= A.npv) return;
-  const double* o = A.rec + (size_t)pv * ECL_REC;
-  A.flux[(size_t)pv * A.ldflux + pt] = o[13] == 0.0 ? CUDART_NAN : ecl_point_f64(A, pv, pt, o);
+  const double* o = A.orb64 + (size_t)pv * ORB64;
+  double f = CUDART_NAN;
+  if (o[12] != 0.0) {
+    const int lc = A.lcids[pt];
+    const double t = A.times[pt], p = A.p[pv];
+    f = ecl_point_f64(A, pv, lc, __dsub_rn(t, f64_conjunction(t, f64_t0(A, pv, lc), p, 1.0f / (float)p)), o);
+  }
+  A.flux[(size_t)pv * A.ldflux + pt] = f;
 }
 
-// The same with the fold once per 128-point tile for tiles that reach no box
-// (tiles64 from rr_time_tiles_f64).  The fold about the eclipse epoch te is
-// non-decreasing in t with the reference's rounding, so a one-light-curve
-// tile whose two ends share an epoch and whose two ends' tc miss the padded
-// box is pi k^2 at every point: the same bits as eclipse_flux_kernel.  A warp
-// tests 32 tiles at once, one per lane.
-constexpr int ECL64_WARPS = 4;
-
-__global__ void __launch_bounds__(ECL64_WARPS * 32) eclipse_flux_culled_kernel(EclF64Args A, const double* tiles64) {
-  const int pv = blockIdx.z * 65535 + blockIdx.y;
-  if (pv >= A.npv) return;   // block-uniform
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ntiles = (A.npt + TIME_TILE - 1) / TIME_TILE;
-  const int tbase = (blockIdx.x * ECL64_WARPS + warp) * 32;
-  if (tbase >= ntiles) return;   // warp-uniform
-  const unsigned FULL = 0xffffffffu;
-  const double* o = A.rec + (size_t)pv * ECL_REC;
+static __device__ __noinline__ void ecl_flush(const EclF64Args& A, const F64Orbit& P, F64Lc* recs, F64Queue& Q,
+                                              const double* o, int pv, int lc, int n) {
+  const int nrec = min(A.nlc, F64_LC_SMEM);
+  if (lc >= F64_LC_SMEM) {
+    if ((threadIdx.x & 31) == 0) f64_lc(A, pv, lc, P, recs[nrec]);
+    __syncwarp();
+  }
+  const F64Lc& R = recs[min(lc, nrec)];
+  const F64Eclipse T{o};
   double* row = A.flux + (size_t)pv * A.ldflux;
-  const bool valid = o[13] != 0.0;
+  f64_sums(R, P, T, Q, n, [&](int i, double D) { __stcs(row + Q.pt[i], T.value(R, D)); }, [](int, int) {});
+}
+
+struct EclSink {
+  const EclF64Args& A;
+  const F64Orbit& P;
+  F64Lc* recs;
+  F64Queue& Q;
+  const double* o;
+  double* row;
+  int pv;
+  double fill;
+  bool vec;
+
+  __device__ __forceinline__ void tile(int p0, int q0, int q1) const {
+    f64_fill_tile(row, A.npt, p0, q0, q1, fill, vec);
+  }
+  __device__ __forceinline__ void outside(int pt) const { __stcs(row + pt, fill); }
+  __device__ __forceinline__ void flush(int lc, int n) const { ecl_flush(A, P, recs, Q, o, pv, lc, n); }
+};
+
+__global__ void __launch_bounds__(32, 24)
+eclipse_flux_culled_kernel(const __grid_constant__ EclF64Args A, const double* tiles64, int slots) {
+  __shared__ double o[ORB64];
+  __shared__ F64Orbit P;
+  __shared__ F64Queue Q;
+  extern __shared__ __align__(16) unsigned char ecl64_smem[];
+  F64Lc* recs = reinterpret_cast<F64Lc*>(ecl64_smem);
+  const int pv = blockIdx.z * 65535 + blockIdx.y, lane = threadIdx.x;
+  if (pv >= A.npv) return;
+  if (lane < ORB64) o[lane] = A.orb64[(size_t)pv * ORB64 + lane];
+  __syncwarp();
+  const bool valid = o[12] != 0.0;
+  if (valid) {
+    if (lane == 0) f64_orbit(o, P);
+    __syncwarp();
+    for (int lc = lane; lc < min(A.nlc, F64_LC_SMEM); lc += 32) f64_lc(A, pv, lc, P, recs[lc]);
+  }
+  __syncwarp();
   const double kk = A.k[pv];
-  const int tile = tbase + lane;
-  bool cull = !valid;
-  if (valid && tile < ntiles) {
-    const double tmin = tiles64[4 * (size_t)tile], tmax = tiles64[4 * (size_t)tile + 1];
-    const int lc = (int)tiles64[4 * (size_t)tile + 2];
-    if (lc >= 0) {
-      const double pp = A.p[pv];
-      const double te = __dadd_rn(__dadd_rn(A.t0[(size_t)pv * A.ldt0 + A.epids[lc]], o[12]), o[14]);
-      const double e0 = floor(__ddiv_rn(__dadd_rn(__dsub_rn(tmin, te), __dmul_rn(0.5, pp)), pp));
-      const double e1 = floor(__ddiv_rn(__dadd_rn(__dsub_rn(tmax, te), __dmul_rn(0.5, pp)), pp));
-      if (e0 == e1) {
-        const double c = __dadd_rn(te, __dmul_rn(e0, pp));
-        const double pad = __dadd_rn(0.003, A.exptimes[lc]);
-        cull = __dsub_rn(tmax, c) < __dsub_rn(o[10], pad) || __dsub_rn(tmin, c) > __dadd_rn(o[11], pad);
+  f64_walk(A, pv, tiles64, slots, valid, P, recs, Q,
+           EclSink{A, P, recs, Q, o, A.flux + (size_t)pv * A.ldflux, pv,
+                   valid ? __dmul_rn(PI, __dmul_rn(kk, kk)) : CUDART_NAN,
+                   ((A.ldflux & 1) == 0) && ((reinterpret_cast<uintptr_t>(A.flux) & 15) == 0)});
+}
+
+// esmodel's light curve loop (model_ecspec.py:49-62): 1 outside the box padded
+// by 0.0015 d + exptime, else the mean over the samples of 1 - (f_b A(1, k, z)
+// / pi) / (1 + f_b k^2) = 1 - c_b <A>, c_b = f_b / (pi (1 + f_b k^2)).  The
+// area's mean over a point's samples is taken once for all channels, in full
+// warps of queued in-box points, and each output is one FP64 multiply-add and
+// one store; the kernel was bound by two FP64 divisions per channel, point and
+// sample, and by adding each sample to every output in memory.
+//
+// One warp per share of `slots` 32-point slots of a pv.  Without tile
+// summaries the box test is per point: one FP64 subtraction, the fold in FP32
+// with its error allowed for, and the exact fold only near the box.
+constexpr int ES_C_SMEM = 512;   // channel factors staged per block
+
+struct EsF64Args : F64Args {
+  const double* fratio;
+  int nch;
+  double* flux;
+  int ldflux;
+};
+
+__device__ __forceinline__ double es_factor(double f, double k2) {
+  return __dmul_rn(f, f64_recip(__dmul_rn(PI, __fma_rn(f, k2, 1.0))));
+}
+
+static __device__ __noinline__ void es_flush(const EsF64Args& A, const F64Orbit& P, const F64Lc& R, F64Queue& Q,
+                                             const double* o, const double* cb, double* fpv, const double* fr,
+                                             int n) {
+  struct Area : F64Eclipse {   // the occulted area itself
+    __device__ __forceinline__ double none(const F64Lc&) const { return 0.0; }
+    __device__ __forceinline__ double inner(const F64Lc& r, const F64Orbit&, double) const { return r.disk.area_in; }
+    __device__ __forceinline__ double limb(const F64Lc& r, const F64Orbit& p, double t) const {
+      const double r2 = r2_at(p.d, p.even, t);
+      if (!r.disk.fast || !f64_moderate(r2)) return general(o, r.disk.k, t);
+      return f64_limb<false>(r.disk, r2, f64_rsqrt(f64_root(r2))).area;
+    }
+  };
+  f64_sums(
+      R, P, Area{o}, Q, n,
+      [&](int i, double D) {
+        const double ar = -(R.ns == 1 ? D : __dmul_rn(D, R.w));
+        double* out = fpv + Q.pt[i];
+        for (int b = 0; b < A.nch; ++b, out += A.ldflux)
+          __stcs(out, __fma_rn(b < ES_C_SMEM ? cb[b] : es_factor(fr[b], R.disk.k2), ar, 1.0));
+      },
+      [](int, int) {});
+}
+
+__global__ void __launch_bounds__(32, 20) es_flux_kernel(const __grid_constant__ EsF64Args A, int slots) {
+  __shared__ double o[ORB64];
+  __shared__ F64Orbit P;
+  __shared__ F64Queue Q;
+  __shared__ F64Lc R;
+  __shared__ double cb[ES_C_SMEM];
+  const unsigned FULL = 0xffffffffu;
+  const int pv = blockIdx.z * 65535 + blockIdx.y, lane = threadIdx.x;
+  if (pv >= A.npv) return;
+  const int s0 = blockIdx.x * slots, s1 = min(s0 + slots, (A.npt + 31) / 32);
+  if (lane < ORB64) o[lane] = A.orb64[(size_t)pv * ORB64 + lane];
+  __syncwarp();
+  double* fpv = A.flux + (size_t)pv * A.nch * A.ldflux;
+  const double* fr = A.fratio + (size_t)pv * A.nch;
+  const bool valid = o[12] != 0.0;
+  const double fill = valid ? 1.0 : CUDART_NAN;
+  if (valid) {
+    if (lane == 0) {
+      f64_orbit(o, P);
+      f64_lc(A, pv, 0, P, R);
+    }
+    __syncwarp();
+    for (int b = lane; b < min(A.nch, ES_C_SMEM); b += 32) cb[b] = es_factor(fr[b], R.disk.k2);
+    __syncwarp();
+  }
+  const double te = valid ? f64_t0(A, pv, 0) : 0.0, p = A.p[pv];
+  const float pf = f32_of(p), inv_p = 1.0f / pf;
+  int n = 0;
+  for (int s = s0; s < s1; ++s) {
+    const int pt = 32 * s + lane;
+    bool in = false;
+    double tc = 0.0;
+    if (valid && pt < A.npt) {
+      const double t = A.times[pt];
+      const float sf = f32_of(__dsub_rn(t, te)), err = 1e-6f * (fabsf(sf) + fabsf(pf)) + 1e-6f;
+      const float r = fmaf(-rintf(sf * inv_p), pf, sf);
+      // near the box, near a change of epoch, or beyond what the FP32 fold resolves
+      if (!(r < R.lo - err || r > R.hi + err) || fabsf(r) > 0.5f * fabsf(pf) - err || !(fabsf(sf * inv_p) < 1e5f)) {
+        tc = __dsub_rn(t, f64_conjunction(t, te, p, inv_p));
+        const float tf = f32_of(tc);
+        in = R.lo <= tf && tf <= R.hi;
       }
     }
-  }
-  const int jn = min(32, ntiles - tbase);
-  const unsigned jmask = jn == 32 ? FULL : (1u << jn) - 1u;
-  const unsigned cmask = __ballot_sync(FULL, cull) & jmask;
-  const double fill = valid ? PI * (kk * kk) : CUDART_NAN;
-  for (unsigned m = cmask; m; m &= m - 1u) {
-    const int p0 = (tbase + __ffs(m) - 1) * TIME_TILE;
-    for (int q = 0; q < 4; ++q)
-      if (p0 + 32 * q + lane < A.npt) row[p0 + 32 * q + lane] = fill;
-  }
-  for (unsigned m = ~cmask & jmask; m; m &= m - 1u) {
-    const int p0 = (tbase + __ffs(m) - 1) * TIME_TILE;
-    for (int q = 0; q < 4; ++q) {
-      const int pt = p0 + 32 * q + lane;
-      if (pt < A.npt) row[pt] = ecl_point_f64(A, pv, pt, o);
+    const unsigned bm = __ballot_sync(FULL, in);
+    if (!in && pt < A.npt) {
+      double* out = fpv + pt;
+      for (int b = 0; b < A.nch; ++b, out += A.ldflux) __stcs(out, fill);
     }
+    if (!bm) continue;
+    if (n > F64_Q - 32) {
+      es_flush(A, P, R, Q, o, cb, fpv, fr, n);
+      n = 0;
+    }
+    if (in) {
+      const int at = n + __popc(bm & ((1u << lane) - 1u));
+      Q.tc[at] = tc;
+      Q.pt[at] = pt;
+    }
+    n += __popc(bm);
   }
-}
-
-// esmodel's light curve loop (model_ecspec.py:49-62), one thread per (pv,
-// point), all channels: 1 outside the box padded by 0.0015 d + exptime, else
-// the mean over the samples of 1 - (f_b A(1, k, z) / pi) / (1 + f_b k^2).
-__global__ void __launch_bounds__(256)
-es_flux_kernel(const double* __restrict__ times, int npt, const double* __restrict__ k,
-               const double* __restrict__ t0, const double* __restrict__ p, const double* __restrict__ fratio,
-               int npb, int nsamples0, double exptime0, const double* __restrict__ rec, int npv,
-               double* __restrict__ flux, int ldflux) {
-  const int pv = blockIdx.z * 65535 + blockIdx.y;
-  const int pt = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pt >= npt || pv >= npv) return;
-  const double* o = rec + (size_t)pv * ECL_REC;
-  double* out = flux + (size_t)pv * npb * ldflux + pt;
-  if (o[13] == 0.0) {
-    for (int b = 0; b < npb; ++b) out[(size_t)b * ldflux] = CUDART_NAN;
-    return;
-  }
-  const double kk = k[pv], pp = p[pv];
-  const double te = __dadd_rn(__dadd_rn(t0[pv], o[12]), o[14]);
-  const double t = times[pt];
-  const double epoch = floor(__ddiv_rn(__dadd_rn(__dsub_rn(t, te), __dmul_rn(0.5, pp)), pp));
-  const double tc = __dsub_rn(t, __dadd_rn(te, __dmul_rn(epoch, pp)));
-  const double pad = __dadd_rn(0.0015, exptime0);
-  if (!(__dsub_rn(o[10], pad) <= tc && tc <= __dadd_rn(o[11], pad))) {
-    for (int b = 0; b < npb; ++b) out[(size_t)b * ldflux] = 1.0;
-    return;
-  }
-  double c[10];
-  for (int i = 0; i < 10; ++i) c[i] = o[i];
-  const double* fr = fratio + (size_t)pv * npb;
-  for (int b = 0; b < npb; ++b) out[(size_t)b * ldflux] = 0.0;
-  for (int s = 1; s < nsamples0 + 1; ++s) {
-    const double z = sep_c_f64(tc + exptime0 * ((s - 0.5) / nsamples0 - 0.5), c);
-    double kap;
-    const double ar = ccia_star<double>(kk, z, kap);
-    for (int b = 0; b < npb; ++b)
-      out[(size_t)b * ldflux] += 1.0 - (fr[b] * ar / PI) / (1.0 + fr[b] * (kk * kk));
-  }
-  for (int b = 0; b < npb; ++b) out[(size_t)b * ldflux] /= nsamples0;
+  if (n > 0) es_flush(A, P, R, Q, o, cb, fpv, fr, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -237,16 +318,12 @@ struct EclSplitArgs {
 // any.  The light travel time is FP32: it is ~1e-4 d, so its rounding is
 // ~1e-11 d.
 //
-// The jet is about the eclipse conjunction, f = 3 pi/2 - w.  solve2d_phase
-// reaches the same Keplerian state by a Newton solve from the mean anomaly at
-// mid-transit plus n times the offset.  Here the state is taken in closed
-// form, as solve2d_conj_f32 takes the transit's, and it is in FP32:
+// The jet is about the eclipse conjunction, f = 3 pi/2 - w, its state in closed
+// form as solve2d_conj_f32 takes the transit's, in FP32:
 //   r  = a (1 - e^2) / (1 - e sin w)
 //   vr = -n a e cos w / sqrt(1 - e^2)
 //   vt = n a (1 - e sin w) / sqrt(1 - e^2)
-// with w + f = 3 pi/2, so P0 = (0, -r) and P1 = (vt, -vr).  This agrees with
-// the FP64 Newton route to ~2e-15 relative, far below the FP32 rounding of
-// the coefficients.
+// with w + f = 3 pi/2, so P0 = (0, -r) and P1 = (vt, -vr).
 __device__ inline double eclipse_time_offset_split(double p, double e, double w) {
   if (e == 0.0) return 0.5 * p;
   double sw, cw;
@@ -542,7 +619,7 @@ using namespace rr;
 
 extern "C" {
 
-size_t rr_eclipse_workspace_bytes(int npv) { return sizeof(double) * (size_t)(npv > 0 ? npv : 1) * ECL_REC + 256; }
+size_t rr_eclipse_workspace_bytes(int npv) { return sizeof(double) * (size_t)(npv > 0 ? npv : 1) * ORB64 + 256; }
 
 static int eclipse_f64_launch(const double* times, const double* tiles64, int npt, const double* k, const double* t0,
                               int ldt0, const double* p, const double* a, const double* inc, const double* e,
@@ -554,14 +631,16 @@ static int eclipse_f64_launch(const double* times, const double* tiles64, int np
   if (workspace_bytes < rr_eclipse_workspace_bytes(npv)) return RR_ERR_WORKSPACE;
   cudaStream_t s = as_stream(stream);
   double* rec = static_cast<double*>(workspace);
-  eclipse_prepare_kernel<<<(npv + 63) / 64, 64, 0, s>>>(k, p, a, inc, e, w, rstar, npv, rec);
+  eclipse_prepare_kernel<<<(npv + 31) / 32, ECL_PREP_THREADS, 0, s>>>(k, p, a, inc, e, w, rstar, npv, rec);
   EclF64Args A{};
   A.times = times; A.npt = npt; A.k = k; A.t0 = t0; A.ldt0 = ldt0; A.p = p; A.lcids = lcids; A.epids = epids;
-  A.nsamples = nsamples; A.exptimes = exptimes; A.rec = rec; A.npv = npv; A.flux = flux; A.ldflux = ldflux;
+  A.nsamples = nsamples; A.exptimes = exptimes; A.orb64 = rec; A.shift = rec + ECL_SHIFT; A.npv = npv; A.nlc = nlc;
+  A.nkc = A.npb = 1; A.dg = 1.0; A.flux = flux; A.ldflux = ldflux;
   if (tiles64) {
-    const int ntiles = (npt + TIME_TILE - 1) / TIME_TILE, per = ECL64_WARPS * 32;
-    dim3 fg((ntiles + per - 1) / per, npv < 65535 ? npv : 65535, (npv + 65534) / 65535);
-    eclipse_flux_culled_kernel<<<fg, ECL64_WARPS * 32, 0, s>>>(A, tiles64);
+    const int slots = f64_slots(npt, npv);
+    dim3 fg(f64_warps(npt, slots), npv < 65535 ? npv : 65535, (npv + 65534) / 65535);
+    const size_t smem = sizeof(F64Lc) * (std::min(nlc, F64_LC_SMEM) + 1);
+    eclipse_flux_culled_kernel<<<fg, 32, smem, s>>>(A, tiles64, slots);
   } else {
     dim3 fg((npt + 255) / 256, npv < 65535 ? npv : 65535, (npv + 65534) / 65535);
     eclipse_flux_kernel<<<fg, 256, 0, s>>>(A);
@@ -597,9 +676,17 @@ int rr_es_f64(const double* times, int npt, const double* k, const double* t0, c
   if (workspace_bytes < rr_eclipse_workspace_bytes(npv)) return RR_ERR_WORKSPACE;
   cudaStream_t s = as_stream(stream);
   double* rec = static_cast<double*>(workspace);
-  eclipse_prepare_kernel<<<(npv + 63) / 64, 64, 0, s>>>(k, p, a, inc, e, w, rstar, npv, rec);
-  dim3 fg((npt + 255) / 256, npv < 65535 ? npv : 65535, (npv + 65534) / 65535);
-  es_flux_kernel<<<fg, 256, 0, s>>>(times, npt, k, t0, p, fratio, npb, nsamples0, exptime0, rec, npv, flux, ldflux);
+  eclipse_prepare_kernel<<<(npv + 31) / 32, ECL_PREP_THREADS, 0, s>>>(k, p, a, inc, e, w, rstar, npv, rec);
+  EsF64Args A{};
+  A.times = times; A.npt = npt; A.k = k; A.t0 = t0; A.ldt0 = 1; A.p = p;
+  A.orb64 = rec; A.shift = rec + ECL_SHIFT; A.npv = npv; A.nlc = 1; A.nkc = A.npb = 1; A.dg = 1.0;
+  A.pad0 = 0.0015f; A.ns0 = nsamples0; A.ex0 = exptime0;
+  A.fratio = fratio; A.nch = npb; A.flux = flux; A.ldflux = ldflux;
+  // 32-point slots per warp: four rounds of 16 warps per SM, at most 32 slots
+  const long long total = (long long)((npt + 31) / 32) * npv, want = total / (64LL * sm_count());
+  const int slots = want < 1 ? 1 : (want > 32 ? 32 : (int)want);
+  dim3 fg(((npt + 31) / 32 + slots - 1) / slots, npv < 65535 ? npv : 65535, (npv + 65534) / 65535);
+  es_flux_kernel<<<fg, 32, 0, s>>>(A, slots);
   return check_launch("rr_es_f64");
 }
 

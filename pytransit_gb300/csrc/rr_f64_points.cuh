@@ -15,7 +15,21 @@ struct F64Args {
   int npt, npv, nkc, ldt0, npb, nlc, ng;
   double dg;
   bool nan_istar;      // a non-finite disk integral makes in-box points NaN
+  // the eclipse models: no LD tables (istar, pbids null, npb = nkc = 1); the
+  // eclipse's shift and light travel time at shift[pv * ORB64]
+  const double* shift;
+  float pad0 = 0.003f; // box padding beyond the contacts and the exposure
+  int ns0;             // for null nsamples / exptimes
+  double ex0;
 };
+
+// Zero epoch of a light curve: t0, or ((t0 + shift) + light travel time).
+__device__ __forceinline__ double f64_t0(const F64Args& A, int pv, int lc) {
+  const double t0 = A.t0[(size_t)pv * A.ldt0 + (A.epids ? A.epids[lc] : 0)];
+  if (!A.shift) return t0;
+  const double* s = A.shift + (size_t)pv * ORB64;
+  return __dadd_rn(__dadd_rn(t0, s[0]), s[1]);
+}
 
 // Phase fold of the reference (model_full.py:84-86) with its rounding: the
 // epoch's conjunction t0 + epoch p, epoch = floor(((t - t0) + p/2) / p).
@@ -54,14 +68,14 @@ struct F64Lc {
 
 template <bool IK = false>
 __device__ __forceinline__ void f64_lc(const F64Args& A, int pv, int lc, const F64Orbit& P, F64Lc& R) {
-  R.pb = A.pbids[lc];
-  R.ns = max(A.nsamples[lc], 0);
-  R.ex = A.exptimes[lc];
+  R.pb = A.pbids ? A.pbids[lc] : 0;
+  R.ns = max(A.nsamples ? A.nsamples[lc] : A.ns0, 0);
+  R.ex = A.exptimes ? A.exptimes[lc] : A.ex0;
   R.step = R.ns > 1 ? __ddiv_rn(R.ex, (double)R.ns) : R.ex;
   // Box: the contact times padded by 0.003 d + exposure (model_full.py:87-89).
   // It only separates points that may overlap the star from points that
   // cannot (F = 1 on both sides of its edges), so it is FP32.
-  const float ex = f32_of(R.ex), pad = 0.003f + ex;
+  const float ex = f32_of(R.ex), pad = A.pad0 + ex;
   R.lo = P.t1 - pad;
   R.hi = P.t4 + pad;
   // bound of the FP32 r^2's error at any sample: 16 roundings of the largest partial sums
@@ -70,7 +84,7 @@ __device__ __forceinline__ void f64_lc(const F64Args& A, int pv, int lc, const F
 #pragma unroll
   for (int m = R2_N - 2; m >= 0; --m) sum = fmaf(sum, tb, fabsf(P.df[m]));
   f64_disk<IK>(A.k[(size_t)pv * A.nkc + (A.nkc == A.npb ? R.pb : 0)], A.dg, fmaf(4e-6f, sum, 2e-6f), R.disk);
-  const double is = A.istar[(size_t)pv * A.npb + R.pb];
+  const double is = A.istar ? A.istar[(size_t)pv * A.npb + R.pb] : 1.0;
   R.w = isfinite(is) || !A.nan_istar ? f64_recip(R.ns == 1 ? is : __dmul_rn(is, (double)R.ns)) : CUDART_NAN;
 }
 
@@ -80,26 +94,8 @@ __device__ __forceinline__ double f64_sample_time(const F64Lc& R, double tc, int
   return __fma_rn(f64_of_pos((float)s + 0.5f), R.step, __fma_rn(-0.5, R.ex, tc));
 }
 
-// LD means of one passband and, for the general form, the orbit they belong to.
-struct F64Table {
-  const double *o, *lda;
-  int ng;
-  double dg;
-};
-
-// The term I(z) A(z) of one sample by the reference's own expressions
-// (model_full.py:93-98), for the separations and radius ratios that the
-// kernels' forms leave out: z = 0, k <= 0, k >= 1, NaN.
-static __device__ __noinline__ double f64_term_general(const F64Table& T, double k, double t) {
-  double c[10];
-  for (int i = 0; i < 10; ++i) c[i] = T.o[i];
-  const double z = sep_c_f64(t, c);
-  double kap;
-  return interp_ldm_f64(z / (1.0 + k), T.dg, T.lda, T.ng) * ccia_star<double>(k, z, kap);
-}
-
-// Class of the sample at t from the FP32 r^2: 0 surely outside the star (its
-// term is 0), 1 surely inside (the planet's whole disk), 2 the limb or unsure.
+// Class of the sample at t from the FP32 r^2: 0 surely outside the star, 1
+// surely inside (the planet's whole disk), 2 the limb or unsure.
 __device__ __forceinline__ int f64_class(const F64Lc& R, const F64Orbit& P, double t) {
   const float tf = f32_of(t);
   float r = P.df[R2_N - 1];
@@ -108,18 +104,72 @@ __device__ __forceinline__ int f64_class(const F64Lc& R, const F64Orbit& P, doub
   return r > R.disk.r2out ? 0 : (r < R.disk.r2in ? 1 : 2);
 }
 
-__device__ __forceinline__ double f64_term_inner(const F64Lc& R, const F64Orbit& P, const F64Table& T, double t) {
-  const double r2 = r2_at(P.d, P.even, t);
-  if (!f64_moderate(r2)) return f64_term_general(T, R.disk.k, t);
-  return __dmul_rn(f64_ld_mean(R.disk, f64_sqrt(f64_root(r2)), T.lda, T.ng), R.disk.area_in);
-}
+// The terms that a point sums over its samples, and its value from the sum:
+// the flux 1 - sum_s I A / (ns istar) (F64Transit) and the visible planet area
+// sum_s (pi k^2 - A) / ns (F64Eclipse).  general(): a sample by the reference's
+// own expressions, for the separations and radius ratios that the kernels'
+// forms leave out: z = 0, k <= 0, k >= 1, NaN.
+struct F64Transit {
+  const double *o, *lda;
+  int ng;
+  double dg;
 
-__device__ __forceinline__ double f64_term_limb(const F64Lc& R, const F64Orbit& P, const F64Table& T, double t) {
-  const double r2 = r2_at(P.d, P.even, t);
-  if (!R.disk.fast || !f64_moderate(r2)) return f64_term_general(T, R.disk.k, t);
-  const F64Root q = f64_root(r2);
-  const double ip = f64_ld_mean(R.disk, f64_sqrt(q), T.lda, T.ng);
-  return __dmul_rn(ip, f64_limb<false>(R.disk, r2, f64_rsqrt(q)).area);
+  __device__ __forceinline__ double none(const F64Lc&) const { return 0.0; }
+  __device__ __forceinline__ double inner(const F64Lc& R, const F64Orbit& P, double t) const {
+    const double r2 = r2_at(P.d, P.even, t);
+    if (!f64_moderate(r2)) return general(*this, R.disk.k, t);
+    return __dmul_rn(f64_ld_mean(R.disk, f64_sqrt(f64_root(r2)), lda, ng), R.disk.area_in);
+  }
+  __device__ __forceinline__ double limb(const F64Lc& R, const F64Orbit& P, double t) const {
+    const double r2 = r2_at(P.d, P.even, t);
+    if (!R.disk.fast || !f64_moderate(r2)) return general(*this, R.disk.k, t);
+    const F64Root q = f64_root(r2);
+    const double ip = f64_ld_mean(R.disk, f64_sqrt(q), lda, ng);
+    return __dmul_rn(ip, f64_limb<false>(R.disk, r2, f64_rsqrt(q)).area);
+  }
+  __device__ __forceinline__ double value(const F64Lc& R, double D) const { return __fma_rn(-D, R.w, 1.0); }
+
+  static __device__ __noinline__ double general(const F64Transit& T, double k, double t) {
+    double c[10];
+    for (int i = 0; i < 10; ++i) c[i] = T.o[i];
+    const double z = sep_c_f64(t, c);
+    double kap;   // model_full.py:93-98
+    return interp_ldm_f64(z / (1.0 + k), T.dg, T.lda, T.ng) * ccia_star<double>(k, z, kap);
+  }
+};
+
+struct F64Eclipse {
+  const double* o;
+
+  __device__ __forceinline__ double none(const F64Lc& R) const { return R.disk.area_in; }
+  __device__ __forceinline__ double inner(const F64Lc&, const F64Orbit&, double) const { return 0.0; }
+  __device__ __forceinline__ double limb(const F64Lc& R, const F64Orbit& P, double t) const {
+    const double r2 = r2_at(P.d, P.even, t);
+    if (!R.disk.fast || !f64_moderate(r2)) return __dadd_rn(R.disk.area_in, -general(o, R.disk.k, t));
+    return __dadd_rn(R.disk.area_in, -f64_limb<false>(R.disk, r2, f64_rsqrt(f64_root(r2))).area);
+  }
+  __device__ __forceinline__ double value(const F64Lc& R, double D) const { return R.ns == 1 ? D : __dmul_rn(D, R.w); }
+
+  static __device__ __noinline__ double general(const double* o, double k, double t) {
+    double c[10];
+    for (int i = 0; i < 10; ++i) c[i] = o[i];
+    double kap;
+    return ccia_star<double>(k, sep_c_f64(t, c), kap);
+  }
+};
+
+// The value of one in-box point at tc from conjunction by one thread: the same
+// operations in the same order as f64_sums'.
+template <class Terms>
+__device__ __forceinline__ double f64_point_value(const F64Lc& R, const F64Orbit& P, const Terms& T, double tc) {
+  double D = 0.0;
+  for (int s = 0; s < R.ns; ++s) {
+    const double t = f64_sample_time(R, tc, s);
+    const int cls = f64_class(R, P, t);
+    const double term = cls == 0 ? T.none(R) : (cls == 1 ? T.inner(R, P, t) : T.limb(R, P, t));
+    D = s == 0 ? term : __dadd_rn(D, term);
+  }
+  return T.value(R, D);
 }
 
 constexpr int F64_Q = 256;        // points and (point, sample) pairs a warp holds
@@ -137,7 +187,7 @@ __device__ __forceinline__ void f64_box(const F64Args& A, const F64Orbit& P, int
     lo = recs[lc].lo;
     hi = recs[lc].hi;
   } else {
-    const float pad = 0.003f + f32_of(A.exptimes[lc]);
+    const float pad = A.pad0 + f32_of(A.exptimes[lc]);
     lo = P.t1 - pad;
     hi = P.t4 + pad;
   }
@@ -182,11 +232,11 @@ __device__ __forceinline__ void f64_pairs(const F64Lc& R, const F64Orbit& P, F64
   __syncwarp();
 }
 
-// The sums D = sum_s I A of the n queued points, all of the light curve R:
+// The sums D of the n queued points' terms, all of the light curve R:
 // point(i, D) is called once per point by one lane, chunk(i0, ni) by the warp
 // after the points [i0, i0 + ni).
-template <class Point, class Chunk>
-__device__ __forceinline__ void f64_sums(const F64Lc& R, const F64Orbit& P, const F64Table& T, F64Queue& Q, int n,
+template <class Terms, class Point, class Chunk>
+__device__ __forceinline__ void f64_sums(const F64Lc& R, const F64Orbit& P, const Terms& T, F64Queue& Q, int n,
                                          Point point, Chunk chunk) {
   const int lane = threadIdx.x & 31;
   // R, P and Q arrive as generic pointers (the callers are not inlined)
@@ -202,9 +252,9 @@ __device__ __forceinline__ void f64_sums(const F64Lc& R, const F64Orbit& P, cons
     for (int s0 = 0; s0 < max(R.ns, 1); s0 += sc) {
       const int ns = min(sc, R.ns - s0);
       f64_pairs(R, P, Q, i0, ni, s0, ns,
-                [&](int f, int it, int s) { Q.term[f] = f64_term_inner(R, P, T, f64_sample_time(R, Q.tc[i0 + it], s)); },
-                [&](int f, int it, int s) { Q.term[f] = f64_term_limb(R, P, T, f64_sample_time(R, Q.tc[i0 + it], s)); },
-                [&](int f) { Q.term[f] = 0.0; });
+                [&](int f, int it, int s) { Q.term[f] = T.inner(R, P, f64_sample_time(R, Q.tc[i0 + it], s)); },
+                [&](int f, int it, int s) { Q.term[f] = T.limb(R, P, f64_sample_time(R, Q.tc[i0 + it], s)); },
+                [&](int f) { Q.term[f] = T.none(R); });
       if (s0 + ns == R.ns) {
         for (int i = lane; i < ni; i += 32) {
           if (s0 == 0) D = ns > 0 ? Q.term[i * ns] : 0.0;
@@ -248,7 +298,7 @@ __device__ __forceinline__ void f64_walk(const F64Args& A, int pv, const double*
       const double2 tm = __ldg(reinterpret_cast<const double2*>(tiles64 + 4 * (size_t)(tbase + lane)));
       tlc = (int)f32_of(__ldg(tiles64 + 4 * (size_t)(tbase + lane) + 2));
       if (tlc >= 0) {
-        const double t0 = A.t0[(size_t)pv * A.ldt0 + A.epids[tlc]];
+        const double t0 = f64_t0(A, pv, tlc);
         f64_box(A, P, tlc, recs, blo, bhi);
         // the epoch of both ends: in FP32 where that leaves no doubt
         const double h0 = __dadd_rn(__dsub_rn(tm.x, t0), hp);
@@ -297,7 +347,7 @@ __device__ __forceinline__ void f64_walk(const F64Args& A, int pv, const double*
               l = A.lcids[pt];
               f64_box(A, P, l, recs, plo, phi);
             }
-            tc = __dsub_rn(t, f64_conjunction(t, A.t0[(size_t)pv * A.ldt0 + A.epids[l]], p, inv_p));
+            tc = __dsub_rn(t, f64_conjunction(t, f64_t0(A, pv, l), p, inv_p));
           }
           const float tf = f32_of(tc);
           in = plo <= tf && tf <= phi;
@@ -324,6 +374,19 @@ __device__ __forceinline__ void f64_walk(const F64Args& A, int pv, const double*
     }
   }
   if (n > 0) sink.flush(qlc, n);
+}
+
+// The value v at slots q0 to q1 of the tile at p0 (vec: 16-byte aligned rows).
+__device__ __forceinline__ void f64_fill_tile(double* row, int npt, int p0, int q0, int q1, double v, bool vec) {
+  const int lane = threadIdx.x & 31;
+  if (vec && q1 - q0 == 4 && p0 + TIME_TILE <= npt) {
+    double2* q = reinterpret_cast<double2*>(row + p0) + 2 * lane;
+    __stcs(q, make_double2(v, v));
+    __stcs(q + 1, make_double2(v, v));
+  } else {
+    for (int q = q0; q < q1; ++q)
+      if (p0 + 32 * q + lane < npt) row[p0 + 32 * q + lane] = v;
+  }
 }
 
 // Launch shape of a walk: slots of 32 points per warp.  Below two rounds of 16

@@ -622,7 +622,7 @@ struct FluxF64Args : F64Args {
 };
 
 // The flux of one point at tc from conjunction, in or out of the box, by one
-// thread: the same operations in the same order as f64_sums'.
+// thread.
 __device__ __noinline__ double f64_point(const F64Args& A, int pv, int lc, double tc, const double* o) {
   F64Orbit P;
   f64_orbit(o, P);
@@ -630,15 +630,7 @@ __device__ __noinline__ double f64_point(const F64Args& A, int pv, int lc, doubl
   f64_lc(A, pv, lc, P, R);
   const float tf = f32_of(tc);
   if (!(R.lo <= tf && tf <= R.hi)) return 1.0;
-  const F64Table T{o, A.ldm + ((size_t)pv * A.npb + R.pb) * A.ng, A.ng, A.dg};
-  double D = 0.0;
-  for (int s = 0; s < R.ns; ++s) {
-    const double t = f64_sample_time(R, tc, s);
-    const int cls = f64_class(R, P, t);
-    const double term = cls == 1 ? f64_term_inner(R, P, T, t) : (cls == 2 ? f64_term_limb(R, P, T, t) : 0.0);
-    D = s == 0 ? term : __dadd_rn(D, term);
-  }
-  return __fma_rn(-D, R.w, 1.0);
+  return f64_point_value(R, P, F64Transit{o, A.ldm + ((size_t)pv * A.npb + R.pb) * A.ng, A.ng, A.dg}, tc);
 }
 
 // The plain FP64 flux: one thread per point, every point through the
@@ -692,9 +684,9 @@ static __device__ __noinline__ void f64_flux_flush(const FluxF64Args& A, const F
     __syncwarp();
   }
   const F64Lc& R = recs[min(lc, nrec)];
-  const F64Table T{o, A.ldm + ((size_t)pv * A.npb + R.pb) * A.ng, A.ng, A.dg};
+  const F64Transit T{o, A.ldm + ((size_t)pv * A.npb + R.pb) * A.ng, A.ng, A.dg};
   double* row = A.flux + (size_t)pv * A.ldflux;
-  f64_sums(R, P, T, Q, n, [&](int i, double D) { __stcs(row + Q.pt[i], __fma_rn(-D, R.w, 1.0)); },
+  f64_sums(R, P, T, Q, n, [&](int i, double D) { __stcs(row + Q.pt[i], T.value(R, D)); },
            [](int, int) {});
 }
 
@@ -710,15 +702,7 @@ struct F64FluxSink {
   bool vec;
 
   __device__ __forceinline__ void tile(int p0, int q0, int q1) const {
-    const int lane = threadIdx.x & 31;
-    if (vec && q1 - q0 == 4 && p0 + TIME_TILE <= A.npt) {
-      double2* q = reinterpret_cast<double2*>(row + p0) + 2 * lane;
-      __stcs(q, make_double2(fill, fill));
-      __stcs(q + 1, make_double2(fill, fill));
-    } else {
-      for (int q = q0; q < q1; ++q)
-        if (p0 + 32 * q + lane < A.npt) row[p0 + 32 * q + lane] = fill;
-    }
+    f64_fill_tile(row, A.npt, p0, q0, q1, fill, vec);
   }
   __device__ __forceinline__ void outside(int pt) const { __stcs(row + pt, 1.0); }
   __device__ __forceinline__ void flush(int lc, int n) const { f64_flux_flush(A, P, recs, Q, o, pv, lc, n); }

@@ -535,7 +535,7 @@ struct F64Partials {
   bool none;
 };
 
-static __device__ __noinline__ void f64_partials_general(const F64Disk& K, const F64Table& T, double r2, F64Partials& S) {
+static __device__ __noinline__ void f64_partials_general(const F64Disk& K, const F64Transit& T, double r2, F64Partials& S) {
   const double z = sqrt(r2);
   S.z = z;
   S.none = !(z < 1.0 + K.k);
@@ -549,7 +549,7 @@ static __device__ __noinline__ void f64_partials_general(const F64Disk& K, const
   S.ar = ccia_star_grad<double>(K.k, z, S.dadk, S.dadz);
 }
 
-__device__ __forceinline__ void f64_partials(const F64Lc& R, const F64Table& T, double t, bool limb, F64Partials& S) {
+__device__ __forceinline__ void f64_partials(const F64Lc& R, const F64Transit& T, double t, bool limb, F64Partials& S) {
   const F64Disk& K = R.disk;
   const double* c = T.o;
   double x = c[4], y = c[9];
@@ -642,7 +642,7 @@ __device__ __noinline__ void lnl_f64_flush(const LnlF64Args& A, const F64Orbit& 
   }
   const F64Lc& R = recs[min(lc, nrec)];
   const size_t ppb = (size_t)pv * A.npb + R.pb;
-  const F64Table T{o, A.ldm + ppb * A.ng, A.ng, A.dg};
+  const F64Transit T{o, A.ldm + ppb * A.ng, A.ng, A.dg};
   double lnl = S.acc[FS_LNL][lane], is = GRAD ? S.acc[GRAD ? FS_IS : 0][lane] : 0.0;
   const double t0 = GRAD ? A.t0[(size_t)pv * A.ldt0 + A.epids[lc]] : 0.0;
   const float inv_p = 1.0f / f32_of(A.p[pv]);
