@@ -319,8 +319,7 @@ __device__ __forceinline__ F64Limb f64_limb(const F64Disk& D, double r2, double 
 // The LD means' lerp at separation z (common.py:225-233 with the two
 // divisions folded into D.cg): the cell from the FP32 position, moved by one
 // where its FP64 fraction falls outside [0, 1).
-__device__ __forceinline__ void f64_ld_cell(const F64Disk& D, double z, const double* __restrict__ lda, int ng, int& i,
-                                            double& fr, double& l0, double& dl) {
+__device__ __forceinline__ void f64_ld_pos(const F64Disk& D, double z, int ng, int& i, double& fr) {
   float fi = fminf(truncf(f32_of_pos(z) * D.cgf), (float)(ng - 2));
   fr = __fma_rn(z, D.cg, -f64_of_pos(fi));
   const float ff = f32_of(fr);
@@ -329,6 +328,10 @@ __device__ __forceinline__ void f64_ld_cell(const F64Disk& D, double z, const do
     fr = __fma_rn(z, D.cg, -f64_of_pos(fi));
   }
   i = (int)fi;
+}
+__device__ __forceinline__ void f64_ld_cell(const F64Disk& D, double z, const double* __restrict__ lda, int ng, int& i,
+                                            double& fr, double& l0, double& dl) {
+  f64_ld_pos(D, z, ng, i, fr);
   l0 = __ldg(lda + i);
   dl = __dadd_rn(__ldg(lda + i + 1), -l0);
 }

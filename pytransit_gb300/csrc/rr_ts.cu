@@ -20,6 +20,7 @@
 #include <cmath>
 
 #include "rr_ts.cuh"
+#include "rr_ts64.cuh"
 
 namespace rr {
 
@@ -152,6 +153,7 @@ constexpr int TS_L2_ROWS = 16;   // g rows of the 2D table per LD block
 // once and the LD blocks fill the SMs around them.
 // ---------------------------------------------------------------------------
 constexpr int TSP_MAXPAR = 16;
+constexpr int MAX_BASIS_TS = 16;   // basis_coefs writes up to npar values
 
 template <typename R>
 struct TsProArgs {
@@ -451,6 +453,153 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 4) ts_prologue_kerne
   }
 }
 
+// ---------------------------------------------------------------------------
+// FP64 prologue for the affine laws (rr_ts64.cuh):
+//   blocks [0, npv): per-pv blocks: mean and largest k; on separate warps the
+//     orbit and the disk integrals of the basis functions; the box; r^2(t); the
+//     channels' records and coefficients;
+//   blocks [npv, ...): (pv, TS_L2_ROWS rows of the 2D table at kmean): the
+//     areas by the reference's formula, only where the circles cross (~1 in 5
+//     of the (g, z) pairs, gathered to full warps), then NB columns per row.
+// For 100 pv x 200 channels with quadratic limb darkening the general prologue
+// spends 553 us in the FP64 pipe: every (g, z) area, and 40 multiply-adds per
+// (channel, g); this one takes 63 us.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) ts64_prologue_kernel(TsProArgs<double> P, int nb) {
+  __shared__ double s_sum[3], s_max[3];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int npb = P.npb, nz = P.nz, ng = P.ng;
+  if ((int)blockIdx.x < P.npv) {
+    __shared__ double s_c[10], s_t[2], s_d[R2_N], s_J[TS64_MAXNB];
+    const int pv = blockIdx.x;
+    const double av = P.a[pv], ev = P.e[pv], pp = P.p[pv];
+    const bool valid = !(isnan(av) || av <= 1.0 || ev < 0.0);
+    const bool analytic = P.law == LD_UNIFORM || P.law == LD_LINEAR || P.law == LD_QUADRATIC ||
+                          P.law == LD_QUADRATIC_TRI;
+    ts_kstats(P.k + (size_t)pv * npb, npb, s_sum, s_max);
+    if (warp == 3) {
+      if (lane == 0 && valid) solve2d_conj(pp, av, P.inc[pv], ev, P.w[pv], s_c);
+    } else if (!analytic) {
+      // 2 pi trapezoid(z phi_j(mu(z)), z), mu = linspace(1, 0, 200) (rrmodel.py:222-227), a warp per function
+      constexpr int NT = 200;
+      for (int j = warp; j < nb; j += 3) {
+        double sm = 0.0;
+        for (int i = lane + 1; i < NT; i += 32) {
+          const double m0 = (double)(NT - i) / (NT - 1), m1 = (double)(NT - 1 - i) / (NT - 1);
+          const double z0 = sqrt(1.0 - m0 * m0), z1 = sqrt(1.0 - m1 * m1);
+          sm += (z1 - z0) * (z1 * basis_value(P.law, j, m1) + z0 * basis_value(P.law, j, m0)) * 0.5;
+        }
+        for (int o = 16; o > 0; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
+        if (lane == 0) s_J[j] = 2.0 * PI * sm;
+      }
+    }
+    __syncthreads();
+    const double km = ((s_sum[0] + s_sum[1]) + s_sum[2]) / npb;
+    const double kx = fmax(fmax(s_max[0], s_max[1]), s_max[2]);
+    if (valid && tid == 0) {
+      double t1, t4;
+      contact_box(km, s_c, t1, t4);
+      const double pad = 0.0015 + P.exptime0;
+      s_t[0] = t1 - pad;
+      s_t[1] = t4 + pad;
+    }
+    if (valid && tid == 32) r2_poly(s_c, s_d);
+    double* u = P.ldm + (size_t)pv * npb * ng + (size_t)nb * ng;
+    const double ikm2 = 1.0 / (km * km);
+    for (int b = tid; b < npb; b += blockDim.x) {
+      const double* src = P.ldc + ((size_t)pv * npb + b) * P.npar;
+      double c[MAX_BASIS_TS];
+      basis_coefs(P.law, src, P.npar, c);
+      double is;
+      if (!analytic || !ld_integral<double>(P.law, src, is)) {
+        is = 0.0;
+        for (int j = 0; j < nb; ++j) is += c[j] * s_J[j];
+      }
+      for (int j = 0; j < nb; ++j) u[(size_t)b * nb + j] = c[j];
+      double* cr = P.ch + ((size_t)pv * npb + b) * TS_CH;
+      const double kb = P.k[(size_t)pv * npb + b];
+      cr[0] = kb * kb * ikm2;
+      cr[1] = kb - km;
+      cr[2] = isfinite(is) ? 1.0 / is : CUDART_NAN;
+      cr[3] = 0.0;
+    }
+    __syncthreads();
+    if (tid >= TS_ORB) return;
+    double v = 0.0;
+    if (valid) {
+      if (tid < 10) v = s_c[tid];
+      else if (tid < 12) v = s_t[tid - 10];
+      else if (tid == 12) v = km;
+      else if (tid == 13) v = 1.0 / (1.0 + km);
+      else if (tid == 14) v = 1.0 - kx;
+      else if (tid == 15) v = 1.0;
+      else if (tid < TS64_R2 + R2_N) v = s_d[tid - TS64_R2];
+      else if (tid == TS64_NB) v = (double)nb;
+    }
+    P.orb[(size_t)pv * TS_ORB + tid] = v;
+    return;
+  }
+  __shared__ double s_A[TS_L2_ROWS][64], s_phi[TS64_MAXNB][64];
+  __shared__ unsigned short s_list[TS_L2_ROWS * 64];
+  __shared__ int s_n;
+  const int j = (int)blockIdx.x - P.npv, pv = j / P.nrc, rc = j % P.nrc;
+  const int g0 = rc * TS_L2_ROWS, nr = min(TS_L2_ROWS, ng - g0);
+  if (tid == 0) s_n = 0;
+  for (int i = tid; i < nb * nz; i += blockDim.x) s_phi[i / nz][i % nz] = basis_value(P.law, i / nz, P.mu[i % nz]);
+  ts_kstats(P.k + (size_t)pv * npb, npb, s_sum, s_max);
+  __syncthreads();
+  const double k = ((s_sum[0] + s_sum[1]) + s_sum[2]) / npb;
+  const double gstep = (1.0 - 1e-7) / (double)(ng - 1);
+  auto centre = [&](int r) { return (g0 + r == ng - 1 ? 1.0 - 1e-7 : (double)(g0 + r) * gstep) * (1.0 + k); };
+  // areas (calculate_weights_2d, common.py:153-185): the trivial ones at once, the lens-shaped ones from a list
+  for (int i0 = 0; i0 < nr * nz; i0 += blockDim.x) {
+    const int i = i0 + tid;
+    bool lens = false;
+    if (i < nr * nz) {
+      const double b = centre(i / nz), z = P.ze[i % nz];
+      lens = !(z < b - k) && !(z >= b + k) && !(b - k <= -z);
+      if (!lens) s_A[i / nz][i % nz] = cci_acos(z, k, b);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, lens);
+    int at = 0;
+    if (lane == 0 && m) at = atomicAdd(&s_n, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+    if (lens) s_list[at] = (unsigned short)i;
+  }
+  __syncthreads();
+  for (int q = tid; q < s_n; q += blockDim.x) {
+    const int i = s_list[q];
+    s_A[i / nz][i % nz] = cci_acos(P.ze[i % nz], k, centre(i / nz));
+  }
+  __syncthreads();
+  // rows: 8 lanes each, over z; w_z = A(ze_z) - A(ze_{z-1}) normalised by their sum
+  const int r = tid >> 3, l = tid & 7;
+  double sum = 0.0, col[TS64_MAXNB];
+#pragma unroll
+  for (int b = 0; b < TS64_MAXNB; ++b) col[b] = 0.0;
+  if (r < nr)
+    for (int z = l; z < nz; z += 8) {
+      const double d = z == 0 ? s_A[r][0] : s_A[r][z] - s_A[r][z - 1];
+      sum += d;
+#pragma unroll
+      for (int b = 0; b < TS64_MAXNB; ++b)
+        if (b < nb) col[b] = fma(d, s_phi[b][z], col[b]);
+    }
+  for (int o = 4; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+#pragma unroll
+    for (int b = 0; b < TS64_MAXNB; ++b)
+      if (b < nb) col[b] += __shfl_xor_sync(0xffffffffu, col[b], o);
+  }
+  if (r < nr && l < nb) {
+    double v = col[0];
+#pragma unroll
+    for (int b = 1; b < TS64_MAXNB; ++b)
+      if (l == b) v = col[b];
+    P.ldm[(size_t)pv * npb * ng + (size_t)l * ng + g0 + r] = v / sum;
+  }
+}
+
 // Flux launch: blocks of TSF_WARPS warps, each a range of at most 32
 // consecutive tiles of one pv (grid x: tile ranges, y/z: pv), done by
 // ts_range.  The pv's record is staged in shared memory.
@@ -466,6 +615,35 @@ __global__ void __launch_bounds__(TSF_WARPS * 32) ts_flux_kernel(TsArgs<R> A, in
   if (threadIdx.x < TS_ORB) s_o[threadIdx.x] = A.orb[(size_t)pv * TS_ORB + threadIdx.x];
   __syncthreads();
   ts_range<R, SPLIT>(A, pv, tb0, tb1, s_o, S);
+}
+
+// The same for the FP64 workspace: the tiles of a pv whose LD means are kept
+// as basis columns (TS64_NB) by the sums of rr_ts64.cuh, the others by ts_tile.
+__global__ void __launch_bounds__(TSF_WARPS * 32) ts_flux_f64_kernel(const __grid_constant__ TsArgs<double> A, int npv,
+                                                                     int chunk) {
+  __shared__ __align__(16) union Smem {
+    TsSmem<double> full;
+    Ts64Smem basis;
+  } S;
+  __shared__ double s_o[TS_ORB];
+  __shared__ unsigned s_reach;
+  const int pv = blockIdx.y + 65535 * blockIdx.z;
+  if (pv >= npv) return;   // block-uniform
+  const int ntiles = (A.npt + TS_TILE - 1) / TS_TILE;
+  const int tb0 = blockIdx.x * chunk, tb1 = min(ntiles, tb0 + chunk);
+  if (threadIdx.x < TS_ORB) s_o[threadIdx.x] = A.orb[(size_t)pv * TS_ORB + threadIdx.x];
+  __syncthreads();
+  const unsigned reach = ts_reach<double, false>(A, pv, tb0, tb1, s_o, s_reach);
+  if (!reach) return;
+  switch ((int)s_o[TS64_NB]) {
+    case 1: ts64_tiles<1>(A, pv, tb0, reach, s_o, S.basis); return;
+    case 2: ts64_tiles<2>(A, pv, tb0, reach, s_o, S.basis); return;
+    case 3: ts64_tiles<3>(A, pv, tb0, reach, s_o, S.basis); return;
+    case 5: ts64_tiles<5>(A, pv, tb0, reach, s_o, S.basis); return;
+    default:
+      for (unsigned m = reach; m; m &= m - 1u)
+        ts_tile<double, false>(A, pv, tb0 + __ffs(m) - 1, s_o, S.full, true);
+  }
 }
 
 struct TsTables {
@@ -537,6 +715,15 @@ static int ts_prepare_impl(double t_ref, double t_absmax, const double* k, const
     P.ncc = SPLIT ? (npb + 127) / 128 : 1;
     P.exptime0 = exptime0; P.t_ref = t_ref; P.t_absmax = t_absmax;
     P.orb = orb; P.ch = ch; P.ldm = ldm;
+    if constexpr (!SPLIT) {
+      // an affine law with a few basis functions, and channels enough that the
+      // columns and coefficients take no more room than the LD means
+      const int nb = law < 0 ? 0 : basis_count(law, npar);
+      if (nb != 4 && ts64_fits(nb, npb, ng)) {
+        ts64_prologue_kernel<<<npv + npv * P.nrc, 128, 0, s>>>(P, nb);
+        return check_launch("rr_ts_prepare");
+      }
+    }
     const long long nblk = (long long)npv + (long long)npv * P.nrc * P.ncc;
     ts_prologue_kernel<R, SPLIT><<<(unsigned)nblk, 128, 0, s>>>(P);
     return check_launch("rr_ts_prepare");
@@ -585,7 +772,10 @@ static int ts_flux_impl(const double* times, const float* times_ff, int npt, con
   chunk = chunk < 1 ? 1 : (chunk > 32 ? 32 : chunk);
   const long long bx = (ntiles + chunk - 1) / chunk;
   dim3 fg((unsigned)bx, npv < 65535 ? npv : 65535, (npv + 65534) / 65535);
-  ts_flux_kernel<R, SPLIT><<<fg, TSF_WARPS * 32, 0, s>>>(A, npv, (int)chunk);
+  if constexpr (SPLIT)
+    ts_flux_kernel<R, SPLIT><<<fg, TSF_WARPS * 32, 0, s>>>(A, npv, (int)chunk);
+  else
+    ts_flux_f64_kernel<<<fg, TSF_WARPS * 32, 0, s>>>(A, npv, (int)chunk);
   return check_launch("rr_ts_flux");
 }
 

@@ -434,13 +434,15 @@ __device__ __forceinline__ void ts_fill_rows(const TsArgs<R>& A, int pv, int ta,
 // summaries), the runs of tiles that reach none are filled row by row, and
 // the others go through ts_tile.  The plain path has no tile summaries:
 // every tile of a valid pv goes through ts_tile.
+// ts_reach does all but the tiles that reach a box and returns those as bits.
 template <typename R, bool SPLIT>
-__device__ __forceinline__ void ts_range(const TsArgs<R>& A, int pv, int tb0, int tb1, const R* o, TsSmem<R>& S) {
+__device__ __forceinline__ unsigned ts_reach(const TsArgs<R>& A, int pv, int tb0, int tb1, const R* o,
+                                             unsigned& s_reach) {
   const int n = tb1 - tb0;
   const bool valid = o[15] != R(0);
   if (!valid) {
     ts_fill_rows<R>(A, pv, tb0, tb1, R(CUDART_NAN));
-    return;
+    return 0u;
   }
   unsigned reach = n >= 32 ? 0xffffffffu : (1u << n) - 1u;
   if constexpr (!SPLIT) {
@@ -450,7 +452,7 @@ __device__ __forceinline__ void ts_range(const TsArgs<R>& A, int pv, int tb0, in
     // ends' tc miss the box, holds 1.0 at every point (the same bits as the
     // per-point path).
     if (A.tiles64) {
-      __syncthreads();                 // S.reach of a previous range is consumed
+      __syncthreads();                 // s_reach of a previous range is consumed
       if ((threadIdx.x >> 5) == 0) {
         const int lane = threadIdx.x & 31;
         bool hit = false;
@@ -466,25 +468,25 @@ __device__ __forceinline__ void ts_range(const TsArgs<R>& A, int pv, int tb0, in
           }
         }
         const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0) S.reach = m;
+        if (lane == 0) s_reach = m;
       }
       __syncthreads();
-      reach = S.reach;
+      reach = s_reach;
     }
   }
   if constexpr (SPLIT) {
     if (!(o[22] != R(0))) {
-      __syncthreads();                 // S.reach of a previous range is consumed
+      __syncthreads();                 // s_reach of a previous range is consumed
       if ((threadIdx.x >> 5) == 0) {
         const int lane = threadIdx.x & 31;
         const float4* meta = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(A.times_ff) +
                                                              time_meta_offset(A.npt));
         const bool hit = lane < n && ts_tile_reaches_box(__ldg(meta + tb0 + lane), reinterpret_cast<const float*>(o));
         const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0) S.reach = m;
+        if (lane == 0) s_reach = m;
       }
       __syncthreads();
-      reach = S.reach;
+      reach = s_reach;
     }
   }
   // runs of tiles that reach no box copy, row by row
@@ -498,7 +500,13 @@ __device__ __forceinline__ void ts_range(const TsArgs<R>& A, int pv, int tb0, in
     ts_fill_rows<R>(A, pv, tb0 + a, tb0 + b, R(1));
     rest &= b >= 32 ? 0u : ~((1u << b) - 1u);
   }
-  for (unsigned m = reach; m; m &= m - 1u) ts_tile<R, SPLIT>(A, pv, tb0 + __ffs(m) - 1, o, S, true);
+  return reach;
+}
+
+template <typename R, bool SPLIT>
+__device__ __forceinline__ void ts_range(const TsArgs<R>& A, int pv, int tb0, int tb1, const R* o, TsSmem<R>& S) {
+  for (unsigned m = ts_reach<R, SPLIT>(A, pv, tb0, tb1, o, S.reach); m; m &= m - 1u)
+    ts_tile<R, SPLIT>(A, pv, tb0 + __ffs(m) - 1, o, S, true);
 }
 
 }  // namespace rr
