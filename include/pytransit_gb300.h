@@ -249,6 +249,17 @@ int rr_flux_split_transits(const float *times_ff, int npt, const int32_t *lcids,
 int rr_host_fill_f32(float *dst, size_t n, float value, int nthreads);
 int rr_host_fill_f64(double *dst, size_t n, double value, int nthreads);
 
+/* A call's small host arrays to the device (no counterpart in the reference,
+ * whose arrays stay on the host): bytes from a page-locked staging buffer src
+ * to dst on stream, and event recorded behind the copy; rr_event_wait returns
+ * when src may be written again.  An event belongs to the device that was
+ * current at rr_event_create. */
+int rr_event_create(void **event);
+int rr_event_destroy(void *event);
+int rr_event_wait(void *event);
+int rr_upload(void *dst, const void *src, size_t bytes, void *event, void *stream);
+
+
 /* rr_flux_split_range and rr_flux_split_transits with FP64 output rows (the
  * reference's output type, model_full.py:75): each FP32 result widened
  * exactly, the same values as the FP32 rows. */

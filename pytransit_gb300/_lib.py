@@ -62,6 +62,10 @@ def _sig(L):
     L.rr_flux_split_transits.argtypes = [_vp, _i, _vp, _i, _i, _i, _i, _d, _vp, _i, _i, _vp, _i, _vp]
     L.rr_host_fill_f32.argtypes = [_vp, _sz, C.c_float, _i]
     L.rr_host_fill_f64.argtypes = [_vp, _sz, _d, _i]
+    L.rr_event_create.argtypes = [C.POINTER(_vp)]
+    L.rr_event_destroy.argtypes = [_vp]
+    L.rr_event_wait.argtypes = [_vp]
+    L.rr_upload.argtypes = [_vp, _vp, _sz, _vp, _vp]
     L.rr_flux_split_range_f64.argtypes = [_vp, _i, _vp, _i, _i, _i, _i, _d, _vp, _i, _i, _vp, _i, _vp]
     L.rr_flux_split_transits_f64.argtypes = [_vp, _i, _vp, _i, _i, _i, _i, _d, _vp, _i, _i, _vp, _i, _vp]
     L.rr_time_tiles_f64_doubles.argtypes = [_i]
@@ -98,6 +102,15 @@ def _sig(L):
 
 # Signatures of entry points added in other translation units (name -> (argtypes, restype)).
 _EXTRA_SIGNATURES = {}
+
+
+def register(signatures):
+    """Declare a module's entry points, now if the library is loaded already."""
+    _EXTRA_SIGNATURES.update(signatures)
+    if _LIB is not None:
+        for name, (args, res) in signatures.items():
+            f = getattr(_LIB, name)
+            f.argtypes, f.restype = args, res
 
 
 def lib():
@@ -142,9 +155,11 @@ def to_host_f64(t, min_points: int = 1 << 17):
 
 
 def require_cuda(device=None) -> torch.device:
-    if not torch.cuda.is_available():
+    if not (torch.cuda.is_initialized() or torch.cuda.is_available()):
         raise RuntimeError("pytransit_gb300 needs a CUDA device (GB300, sm_103a); no CPU fallback exists")
-    dev = torch.device(device if device is not None else "cuda")
+    if device is None:
+        return torch.device("cuda", torch.cuda.current_device())
+    dev = torch.device(device)
     if dev.type != "cuda":
         raise RuntimeError(f"pytransit_gb300 runs on CUDA devices only, not {dev}")
     if dev.index is None:
@@ -157,5 +172,80 @@ def ptr(t):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
+def addr(t):
+    """ptr() as a plain int, for entry points whose argument types are
+    declared: ctypes converts it without an object per argument."""
+    return None if t is None else t.data_ptr()
+
+
 def stream_ptr(device=None):
     return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+
+
+def stream_addr(device):
+    """The current stream of a device (with an index) as a plain int."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+class Uploaded:
+    """A float64 array of the last Staging.put(): device address and shape; the
+    tensor itself only when asked for."""
+    __slots__ = ('base', 'off', 'shape', '_addr')
+
+    def __init__(self, base, base_addr, off, shape):
+        self.base, self.off, self.shape = base, off, shape
+        self._addr = base_addr + 8 * off
+
+    def data_ptr(self):
+        return self._addr
+
+    def numel(self):
+        n = 1
+        for s in self.shape:
+            n *= s
+        return n
+
+    def tensor(self):
+        return self.base[self.off:self.off + self.numel()].view(self.shape)
+
+
+class Staging:
+    """A page-locked buffer and its device twin for the float64 arrays of a
+    call, with the event that tells when the copy has left the buffer."""
+
+    def __init__(self, n, device):
+        import weakref
+        self.pin = torch.empty(n, dtype=torch.float64, pin_memory=True)
+        self.dev = torch.empty(n, dtype=torch.float64, device=device)
+        self.device, self.size = device, n
+        self._np, self._src, self._dst = self.pin.numpy(), self.pin.data_ptr(), self.dev.data_ptr()
+        self._event = C.c_void_p()
+        L = lib()
+        with torch.cuda.device(device):
+            check(L.rr_event_create(C.byref(self._event)), "rr_event_create")
+        self._busy = False
+        weakref.finalize(self, _release_staging, L, C.c_void_p(self._event.value), self.pin).atexit = False
+
+    def put(self, arrays):
+        """Copy a dict of float64 arrays (None values skipped) to the device on
+        its current stream, in one transfer; returns their Uploaded records."""
+        L = lib()
+        if self._busy:
+            check(L.rr_event_wait(self._event), "rr_event_wait")   # the previous copy has left the buffer
+            self._busy = False
+        hp, off, out = self._np, 0, {}
+        for n, v in arrays.items():
+            if v is not None:
+                sz = v.size
+                hp[off:off + sz] = v.reshape(-1)
+                out[n] = Uploaded(self.dev, self._dst, off, v.shape)
+                off += sz
+        self._busy = True
+        check(L.rr_upload(self._dst, self._src, 8 * off, self._event, stream_addr(self.device)), "rr_upload")
+        return out
+
+
+def _release_staging(L, event, pin):
+    """The last copy has left the buffer before its memory goes back."""
+    L.rr_event_wait(event)
+    L.rr_event_destroy(event)

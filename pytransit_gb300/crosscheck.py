@@ -25,15 +25,10 @@ _SIG = {
     'rr_ma_quad_flux_f64': ([_vp, _i, _vp, _i, _vp, _i, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                              _i, _vp], _i),
 }
-_lib._EXTRA_SIGNATURES.update(_SIG)
+_lib.register(_SIG)
 
 
-def _L():
-    L = _lib.lib()
-    for name, (args, res) in _SIG.items():
-        f = getattr(L, name)
-        f.argtypes, f.restype = args, res
-    return L
+_L = _lib.lib
 
 
 def ma_quadratic_z(z, k: float, u1: float, u2: float, device=None) -> np.ndarray:

@@ -44,15 +44,10 @@ _SIG = {
     'rr_es_split': ([_vp, _d, _d, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _d, _vp, _sz, _vp, _i,
                      _vp], _i),
 }
-_lib._EXTRA_SIGNATURES.update(_SIG)
+_lib.register(_SIG)
 
 
-def _L():
-    L = _lib.lib()
-    for name, (args, res) in _SIG.items():
-        f = getattr(L, name)
-        f.argtypes, f.restype = args, res
-    return L
+_L = _lib.lib
 
 
 def _vec(x, npv, name):
@@ -99,7 +94,7 @@ class EclipseModel(_GpuEclipseBase):
         dd = self._device_data(dev)
         g = self._upload(dict(k=k, t0=t0, **vecs), dev)   # one pinned host-to-device copy
         L = _L()
-        P = _lib.ptr
+        P = _lib.addr
         if self.precision == 'split':
             wsb = L.rr_eclipse_split_workspace_bytes(npv, self.nlc, 1)
             ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
@@ -108,14 +103,14 @@ class EclipseModel(_GpuEclipseBase):
                                           P(g['t0']), t0.shape[1], P(g['p']), P(g['a']), P(g['i']), P(g['e']),
                                           P(g['w']), P(g['rstar']), npv, self.nlc, P(dd['lcids']), P(dd['epids']),
                                           P(dd['nsamples']), P(dd['exptimes']), P(ws), wsb, P(out), self.npt,
-                                          _lib.stream_ptr(dev)), "rr_eclipse_split")
+                                          _lib.stream_addr(dev)), "rr_eclipse_split")
         else:
             wsb = L.rr_eclipse_workspace_bytes(npv)
             ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
             out = torch.empty((npv, self.npt), dtype=torch.float64, device=dev)
             rest = (self.npt, P(g['k']), P(g['t0']), t0.shape[1], P(g['p']), P(g['a']), P(g['i']), P(g['e']),
                     P(g['w']), P(g['rstar']), npv, self.nlc, P(dd['lcids']), P(dd['epids']), P(dd['nsamples']),
-                    P(dd['exptimes']), P(ws), wsb, P(out), self.npt, _lib.stream_ptr(dev))
+                    P(dd['exptimes']), P(ws), wsb, P(out), self.npt, _lib.stream_addr(dev))
             if self.fp64_cull:      # the same bits with the fold once per tile that reaches no box
                 _lib.check(L.rr_eclipse_f64_culled(P(dd['time']), P(dd['tiles64']), *rest), "rr_eclipse_f64")
             else:
@@ -153,7 +148,7 @@ class EclipseSpectroscopyModel(_GpuEclipseBase):
         dd = self._device_data(dev)
         g = self._upload(dict(k=k, f=f, **vecs), dev)
         L = _L()
-        P = _lib.ptr
+        P = _lib.addr
         ns0 = int(np.atleast_1d(self.nsamples)[0])
         ex0 = float(np.atleast_1d(self.exptimes)[0])
         if self.precision == 'split':
@@ -162,7 +157,7 @@ class EclipseSpectroscopyModel(_GpuEclipseBase):
             out = torch.empty((npv, npb, self.npt), dtype=torch.float32, device=dev)
             _lib.check(L.rr_es_split(P(dd['times_ff']), dd['t_ref'], dd['t_absmax'], self.npt, P(g['k']), P(g['t0']),
                                      P(g['p']), P(g['a']), P(g['i']), P(g['e']), P(g['w']), P(g['rstar']), P(g['f']),
-                                     npv, npb, ns0, ex0, P(ws), wsb, P(out), self.npt, _lib.stream_ptr(dev)),
+                                     npv, npb, ns0, ex0, P(ws), wsb, P(out), self.npt, _lib.stream_addr(dev)),
                        "rr_es_split")
         else:
             wsb = L.rr_eclipse_workspace_bytes(npv)
@@ -170,7 +165,7 @@ class EclipseSpectroscopyModel(_GpuEclipseBase):
             out = torch.empty((npv, npb, self.npt), dtype=torch.float64, device=dev)
             _lib.check(L.rr_es_f64(P(dd['time']), self.npt, P(g['k']), P(g['t0']), P(g['p']), P(g['a']), P(g['i']),
                                    P(g['e']), P(g['w']), P(g['rstar']), P(g['f']), npv, npb, ns0, ex0, P(ws), wsb,
-                                   P(out), self.npt, _lib.stream_ptr(dev)), "rr_es_f64")
+                                   P(out), self.npt, _lib.stream_addr(dev)), "rr_es_f64")
         return _lib.to_host_f64(out) if copy else out
 
     def __call__(self, *args, **kwargs):

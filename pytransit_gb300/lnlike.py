@@ -30,15 +30,10 @@ _SIG = {
                          _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _d, _d, _d, _d, _vp, _vp,
                          _vp, _vp, _sz, _vp, _vp, _vp], _i),
 }
-_lib._EXTRA_SIGNATURES.update(_SIG)
+_lib.register(_SIG)
 
 
-def _L():
-    L = _lib.lib()
-    for name, (args, res) in _SIG.items():
-        f = getattr(L, name)
-        f.argtypes, f.restype = args, res
-    return L
+_L = _lib.lib
 
 
 def grad_columns(nkc, nep, npb, npar):
@@ -65,16 +60,20 @@ def _run(model, obs, sigma, k, t0, p, a, i, e, w, ldc, want_grad):
     dd = model._device_data(device)
     nz = model.ze.size
     dt = torch.float32 if split else torch.float64
-    ldp = torch.empty((npv, npb, nz), dtype=dt, device=device)
-    istar = torch.empty((npv, npb), dtype=dt, device=device)
+    ld = torch.empty(npv * npb * (nz + 1), dtype=dt, device=device)   # ldp[npv, npb, nz], then istar[npv, npb]
+    ldp = ld.data_ptr()
+    istar = ldp + npv * npb * nz * ld.element_size()
     fn = L.rr_ld_tables_f32 if split else L.rr_ld_tables_f64
-    P = _lib.ptr
-    sp = _lib.stream_ptr(device)
-    _lib.check(fn(model.ld_law, P(ldc), npv, npb, npar, P(tb['mu']), nz, P(ldp), P(istar), sp), "rr_ld_tables")
+    P = _lib.addr
+    sp = _lib.stream_addr(device)
+    _lib.check(fn(model.ld_law, P(ldc), npv, npb, npar, P(tb['mu']), nz, ldp, istar, sp), "rr_ld_tables")
     obs = torch.as_tensor(obs, dtype=torch.float64).to(device).contiguous()
     if obs.numel() != npt:
         raise ValueError(f"obs should have {npt} values")
-    if torch.is_tensor(sigma):
+    if isinstance(sigma, (int, float)):
+        # filled on the device: no copy from pageable host memory to wait for
+        sig = torch.full((nlc,), float(sigma), dtype=torch.float64, device=device)
+    elif torch.is_tensor(sigma):
         sig = sigma.to(device=device, dtype=torch.float64).reshape(-1).expand(nlc).contiguous()
     else:
         sig = torch.as_tensor(np.broadcast_to(np.asarray(sigma, dtype=np.float64), (nlc,)).copy()).to(device)
@@ -84,7 +83,7 @@ def _run(model, obs, sigma, k, t0, p, a, i, e, w, ldc, want_grad):
     lnl = torch.empty(npv, dtype=torch.float64, device=device)
     g = torch.empty((npv, ngrad), dtype=torch.float64, device=device) if want_grad else None
     common_tail = (P(k), nkc, P(t0), nep, nep, P(p), P(a), P(i), P(e), P(w), npv, nlc, npb, P(dd['lcids']),
-                   P(dd['pbids']), P(dd['epids']), P(dd['nsamples']), P(dd['exptimes']), P(ldp), P(istar),
+                   P(dd['pbids']), P(dd['epids']), P(dd['nsamples']), P(dd['exptimes']), ldp, istar,
                    P(tb['W32'] if split else tb['W64']), model.nk, model.ng, nz, model.dk, float(model.klims[0]),
                    float(model.klims[1]), model.dg, P(tb['ze']), P(obs), P(sig), P(ws), ws.numel(), P(lnl), P(g))
     if split:
@@ -96,7 +95,7 @@ def _run(model, obs, sigma, k, t0, p, a, i, e, w, ldc, want_grad):
     return lnl, g
 
 
-def _as_params(model, k, t0, p, a, i, e, w, ldc, extra=None):
+def _upload_params(model, k, t0, p, a, i, e, w, ldc, extra):
     """Shape the parameters as evaluate() does and move them to the device, in
     one host-to-device copy through the model's pinned staging buffer (with
     the arrays of `extra`, a dict of float64 arrays, in the same copy)."""
@@ -105,11 +104,16 @@ def _as_params(model, k, t0, p, a, i, e, w, ldc, extra=None):
     k_, t0_, p_, a_, i_, e_, w_ = model._shape_params(*vals)
     ldc_ = ldc.detach().cpu().numpy() if torch.is_tensor(ldc) else ldc
     ldc3 = model._shape_ldc(ldc_, p_.size, model.npb)
-    arrays = dict(k=k_, t0=t0_, p=p_, a=a_, i=i_, e=e_, w=w_, ldc=ldc3)
-    arrays.update(extra or {})
-    dev = model._upload({n: np.ascontiguousarray(v, dtype=np.float64) for n, v in arrays.items()}, device)
-    out = [dev[n] for n in ('k', 't0', 'p', 'a', 'i', 'e', 'w', 'ldc')]
-    return (out, {n: dev[n] for n in (extra or {})}) if extra is not None else out
+    return model._upload(dict(k=k_, t0=t0_, p=p_, a=a_, i=i_, e=e_, w=w_, ldc=ldc3, **extra), device)
+
+
+_PARAMS = ('k', 't0', 'p', 'a', 'i', 'e', 'w', 'ldc')
+
+
+def _as_params(model, k, t0, p, a, i, e, w, ldc):
+    """_upload_params as a list of tensors."""
+    dev = _upload_params(model, k, t0, p, a, i, e, w, ldc, {})
+    return [dev[n].tensor() for n in _PARAMS]
 
 
 def lnlikelihood(model, obs, sigma, k, ldc, t0, p, a, i, e=0.0, w=0.0, grad=False, copy=True):
@@ -123,8 +127,9 @@ def lnlikelihood(model, obs, sigma, k, ldc, t0, p, a, i, e=0.0, w=0.0, grad=Fals
         extra['obs'] = np.asarray(obs, dtype=np.float64).reshape(-1)
     if not torch.is_tensor(sigma):
         extra['sigma'] = np.broadcast_to(np.asarray(sigma, dtype=np.float64), (model.nlc,)).copy()
-    (k_, t0_, p_, a_, i_, e_, w_, ldc3), dev = _as_params(model, k, t0, p, a, i, e, w, ldc, extra)
-    lnl, g = _run(model, dev.get('obs', obs), dev.get('sigma', sigma), k_, t0_, p_, a_, i_, e_, w_, ldc3, grad)
+    dev = _upload_params(model, k, t0, p, a, i, e, w, ldc, extra)
+    obs, sigma = (dev[n].tensor() if n in dev else v for n, v in (('obs', obs), ('sigma', sigma)))
+    lnl, g = _run(model, obs, sigma, *(dev[n] for n in _PARAMS), grad)
     if copy:
         lnl = lnl.cpu().numpy()
         g = g.cpu().numpy() if g is not None else None

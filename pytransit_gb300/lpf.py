@@ -17,15 +17,10 @@ __all__ = ['map_pv', 'transit_model', 'lnlikelihood']
 
 _vp, _i, _d = C.c_void_p, C.c_int, C.c_double
 _SIG = {'rr_lpf_map': ([_vp, _i, _i, _i, _i, _d, _vp, _vp, _vp, _vp, _vp, _vp, _vp], _i)}
-_lib._EXTRA_SIGNATURES.update(_SIG)
+_lib.register(_SIG)
 
 
-def _L():
-    L = _lib.lib()
-    for name, (args, res) in _SIG.items():
-        f = getattr(L, name)
-        f.argtypes, f.restype = args, res
-    return L
+_L = _lib.lib
 
 
 def map_pv(pv: torch.Tensor, tref: float, npb: int, ld_start: int = 5):

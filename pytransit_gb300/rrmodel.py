@@ -424,7 +424,7 @@ class RoadRunnerModel(TransitModel):
         (rr_flux_f64_range)."""
         k, t0 = args['k'], args['t0']
         common = (npt, P(k), k.shape[1], P(t0), t0.shape[1], P(args['p']), npv, nlc, npb, P(dd['lcids']),
-                  P(dd['pbids']), P(dd['epids']), P(dd['nsamples']), P(dd['exptimes']), P(istar), self.ng, self.dg,
+                  P(dd['pbids']), P(dd['epids']), P(dd['nsamples']), P(dd['exptimes']), istar, self.ng, self.dg,
                   P(ws), pv0, pv1, P(out), npt, stream)
         if self.fp64_cull:
             return L.rr_flux_f64_culled_range(P(dd['time']), P(dd['tiles64']), *common)
@@ -498,7 +498,7 @@ class RoadRunnerModel(TransitModel):
         k, t0, p, a, i, e, w = self._shape_params(k, t0, p, a, i, e, w)
         ldc3 = self._shape_ldc(ldc, p.size, self.npb) if self.ld_law is not None else None
         args = self._upload(dict(k=k, t0=t0, p=p, a=a, i=i, e=e, w=w, ldc=ldc3), device)
-        res = self._evaluate_device(args, ldc, out, copy)
+        res = self._evaluate_device(args, ldc, out, copy, device)
         return (res, self.last_error_bound) if return_error else res
 
     # ------------------------------------------------------------------
@@ -546,34 +546,43 @@ class RoadRunnerModel(TransitModel):
         b = self.error_bounds()
         return float(np.nanmax(b)) if b.size else 0.0
 
-    def _evaluate_device(self, args, ldc=None, out=None, copy=False):
-        """The device half of evaluate: args holds float64 device tensors k[npv,
+    def _evaluate_device(self, args, ldc=None, out=None, copy=False, device=None):
+        """The device half of evaluate: args holds float64 device tensors (or _lib.Uploaded) k[npv,
         nkc], t0[npv, nep], p, a, i, e, w[npv] and, for a named law, ldc[npv, npb,
         ncoef] (ldc: the host coefficients, used only by host LD models)."""
         import torch
         from . import _lib
         user_out = out
-        device = self._cuda_device()
+        if device is None:
+            device = self._cuda_device()
         k, t0 = args['k'], args['t0']
         npv, npt, npb, nlc = args['p'].numel(), self.npt, self.npb, self.nlc
         split = self.precision == 'split'
         tb = self._device_tables(device)
         dd = self._device_data(device)
         L = _lib.lib()
-        stream = _lib.stream_ptr(device)
+        stream = _lib.stream_addr(device)
         nz = self.ze.size
-        P = _lib.ptr
+        P = _lib.addr
         ldc_d = args.get('ldc')
         npar = int(ldc_d.shape[2]) if ldc_d is not None else 0
         basis, nb = self._basis(device, npar, split) if ldc_d is not None else (None, 0)
-        # a named law: the LD tables are made by the prologue call itself
+        nep = t0.shape[1]
+        wsb = (L.rr_full_split_workspace_bytes(npv, npb, nlc, nep, self.ng) if split
+               else L.rr_full_f64_workspace_bytes(npv, npb, self.ng))
+        # a named law: the LD tables are made by the prologue call itself, into
+        # the end of the workspace
         fused = self.ld_law is not None and ldc_d is not None
         if fused:
-            dt = torch.float32 if split else torch.float64
-            ldp = torch.empty((npv, npb, nz), dtype=dt, device=device)
-            istar = torch.empty((npv, npb), dtype=dt, device=device)
+            esize = 4 if split else 8
+            ws = self._workspace(wsb + 256 + esize * npv * npb * (nz + 1), device)
+            istar = ws.data_ptr() + (wsb + 255) // 256 * 256
+            ldp = istar + esize * npv * npb
         else:
             ldp, istar = self._ld_tables(ldc, npv, npb, device, split, ldc_d)
+            ws = self._workspace(wsb, device)
+            ldp_t, istar_t = ldp, istar          # kept until the launches below
+            ldp, istar = ldp.data_ptr(), istar.data_ptr()
         kmin, kmax = float(self.klims[0]), float(self.klims[1])
         # Host rows the flux goes to directly: a caller's contiguous pinned
         # buffer (float32 or float64 in the split path, float64 in the plain
@@ -594,24 +603,19 @@ class RoadRunnerModel(TransitModel):
         if split:
             ldf = (npt + 3) // 4 * 4
             res = None if pipe else torch.empty((npv, ldf), dtype=torch.float32, device=device)
-            nep = t0.shape[1]
-            wsb = L.rr_full_split_workspace_bytes(npv, npb, nlc, nep, self.ng)
-            ws = self._workspace(wsb, device)
             if fused:
                 st = L.rr_prepare_split_ld(dd['t_ref'], dd['t_absmax'], P(args['k']), k.shape[1], P(args['t0']),
                                            t0.shape[1], nep, P(args['p']), P(args['a']), P(args['i']),
                                            P(args['e']), P(args['w']), npv, nlc, npb, P(dd['pbids']),
                                            P(dd['epids']), P(dd['nsamples']), P(dd['exptimes']), self.ld_law,
                                            P(ldc_d), npar, P(tb['mu']), nz, P(basis), nb, P(tb['W32']), self.nk,
-                                           self.ng, self.dk, kmin, kmax, P(tb['ze']), P(ldp), P(istar), P(ws),
-                                           ws.numel(), stream)
+                                           self.ng, self.dk, kmin, kmax, P(tb['ze']), ldp, istar, P(ws), wsb, stream)
             else:
                 st = L.rr_prepare_split(dd['t_ref'], dd['t_absmax'], P(args['k']), k.shape[1], P(args['t0']),
                                         t0.shape[1], nep, P(args['p']), P(args['a']), P(args['i']), P(args['e']),
                                         P(args['w']), npv, nlc, npb, P(dd['pbids']), P(dd['epids']),
-                                        P(dd['nsamples']), P(dd['exptimes']), P(ldp), P(istar), P(tb['W32']),
-                                        self.nk, self.ng, nz, self.dk, kmin, kmax, P(tb['ze']), P(ws), ws.numel(),
-                                        stream, self.ld_law or 0, P(ldc_d), npar, P(basis), nb)
+                                        P(dd['nsamples']), P(dd['exptimes']), ldp, istar, P(tb['W32']),
+                                        self.nk, self.ng, nz, self.dk, kmin, kmax, P(tb['ze']), P(ws), wsb, stream, self.ld_law or 0, P(ldc_d), npar, P(basis), nb)
             if st == 0 and pipe:
                 if self.host_fill:
                     st = self._flux_to_pinned(dd, npt, npv, nlc, npb, ws, host_rows, device)
@@ -625,17 +629,15 @@ class RoadRunnerModel(TransitModel):
             res = None if pipe else res[:, :npt]
         else:
             res = None if pipe else torch.empty((npv, npt), dtype=torch.float64, device=device)
-            wsb = L.rr_full_f64_workspace_bytes(npv, npb, self.ng)
-            ws = self._workspace(wsb, device)
             orbit = (P(args['k']), k.shape[1], P(args['p']), P(args['a']), P(args['i']), P(args['e']), P(args['w']),
                      npv, npb)
             if fused:
                 st = L.rr_prepare_f64_ld(*orbit, self.ld_law, P(ldc_d), npar, P(tb['mu']), nz, P(basis), nb,
-                                         P(tb['W64']), self.nk, self.ng, self.dk, kmin, kmax, P(tb['ze']), P(ldp),
-                                         P(istar), P(ws), ws.numel(), stream)
+                                         P(tb['W64']), self.nk, self.ng, self.dk, kmin, kmax, P(tb['ze']), ldp,
+                                         istar, P(ws), wsb, stream)
             else:
-                st = L.rr_prepare_f64(*orbit, P(ldp), P(tb['W64']), self.nk, self.ng, nz, self.dk, kmin, kmax,
-                                      P(tb['ze']), P(ws), ws.numel(), stream, self.ld_law or 0, P(ldc_d), npar,
+                st = L.rr_prepare_f64(*orbit, ldp, P(tb['W64']), self.nk, self.ng, nz, self.dk, kmin, kmax,
+                                      P(tb['ze']), P(ws), wsb, stream, self.ld_law or 0, P(ldc_d), npar,
                                       P(basis), nb)
             if st == 0 and pipe:
                 st = self._flux64_to_host(args, dd, istar, npt, npv, nlc, npb, ws, host_rows, device)

@@ -143,31 +143,15 @@ class TransitModel:
 
     def _upload(self, arrays, device):
         """Send the small per-call arrays in one host-to-device copy through a
-        reused pinned staging buffer; returns device views of the same shapes."""
-        import torch
-        names = [n for n, v in arrays.items() if v is not None]
-        sizes = [int(arrays[n].size) for n in names]
-        total = sum(sizes)
-        if getattr(self, '_pin', None) is None or self._pin.numel() < total or self._pin_dev.device != device:
-            n = max(total, 1024)
-            self._pin = torch.empty(n, dtype=torch.float64, pin_memory=True)
-            self._pin_dev = torch.empty(n, dtype=torch.float64, device=device)
-            self._pin_evt = None
-        if self._pin_evt is not None:
-            self._pin_evt.synchronize()      # the previous copy has left the staging buffer
-        hp = self._pin.numpy()
-        off = 0
-        for n, sz in zip(names, sizes):
-            hp[off:off + sz] = np.asarray(arrays[n], dtype=np.float64).reshape(-1)
-            off += sz
-        self._pin_dev[:total].copy_(self._pin[:total], non_blocking=True)
-        self._pin_evt = torch.cuda.Event()
-        self._pin_evt.record()
-        out, off = {}, 0
-        for n, sz in zip(names, sizes):
-            out[n] = self._pin_dev[off:off + sz].view(arrays[n].shape)
-            off += sz
-        return out
+        reused pinned staging buffer; returns their device addresses and
+        shapes (_lib.Uploaded)."""
+        from . import _lib
+        arrays = {n: np.asarray(v, dtype=np.float64) for n, v in arrays.items() if v is not None}
+        total = sum(v.size for v in arrays.values())
+        st = self.__dict__.get('_staging')
+        if st is None or st.size < total or st.device != device:
+            st = self._staging = _lib.Staging(max(total, 1024), device)
+        return st.put(arrays)
 
     def __call__(self, *nargs, **kwargs):
         raise NotImplementedError

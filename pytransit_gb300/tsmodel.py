@@ -54,8 +54,8 @@ class TransmissionSpectroscopyModel(RoadRunnerModel):
         nz = self.ze.size
         dt = torch.float32 if split else torch.float64
         L = _lib.lib()
-        P = _lib.ptr
-        sp = _lib.stream_ptr(device)
+        P = _lib.addr
+        sp = _lib.stream_addr(device)
         ldc3 = np.ascontiguousarray(np.broadcast_to(ldc, (npv, npb, ldc.shape[2])))
         args = self._upload(dict(k=np.ascontiguousarray(k), t0=vecs[0], p=vecs[1], a=vecs[2], i=vecs[3],
                                  e=vecs[4], w=vecs[5], ldc=ldc3 if self.ld_law is not None else None), device)
