@@ -397,6 +397,7 @@ __device__ __forceinline__ void orbit_pv_split(const OrbitArgs& A, int pv) {
       if (hi + 2 * err >= 0.5 * p || lo - 2 * err <= -0.5 * p) flags |= FLAG_WIDE;
       const float d0h = __double2float_rn(d0[j]);
       const float kf = (float)kk[j];
+      if (ns[j] > 1) flags |= FLAG_MULTI;
       float4* q = q4 + (size_t)lc * (LC32 / 4);
       // LC_FLO, LC_FHI, LC_D0H, LC_D0L | LC_LO, LC_HI, LC_K, LC_INV1PK | LC_INVIS, LC_EXPT, LC_INVNS, LC_NS | LC_PB
       q[0] = make_float4((float)(lo - err), (float)(hi + err), d0h, __double2float_rn(d0[j] - (double)d0h));
@@ -742,9 +743,8 @@ flux_f64_culled_kernel(const __grid_constant__ FluxF64Args A, const double* tile
 // FP32-pair times (slot q of lane l holds point q * 32 + l) and take the
 // per-point path: the phase-folded time exact in FP32 pairs (error-free
 // transformations) and the box test; then, in FP32, z, the LD-table lerp and
-// the kite area on the limb, or, with several samples per point, a per-warp
-// list of (point, sample) pairs spread over the lanes and summed with a
-// segmented shuffle reduction.  Output F = 1 - deficit.
+// the kite area on the limb; points with several samples go through the warp's
+// queue (split_flush).  Output F = 1 - deficit.
 // ---------------------------------------------------------------------------
 constexpr int SPLIT_WARPS = 8;                // warps per block of the serving kernel
 constexpr int SPLIT_PTS = 4;                 // points per lane
@@ -789,20 +789,318 @@ constexpr int LC_SMEM = 64;                  // light-curve records staged in sh
 struct WarpList {
   float tc[WARP_TILE];
   int lc[WARP_TILE];
-  int off[WARP_TILE + 1];
   float acc[WARP_TILE];
 };
+
+// Points of supersampled light curves that the fast fold puts in the box, kept
+// by a warp over its tiles until they fill whole warps: at a 30-min cadence a
+// tile that reaches a transit holds ~10 of them.
+constexpr int SPLIT_Q = 256;       // points
+constexpr int SPLIT_ROWS = 10;     // rows of 32 samples evaluated at once
+struct SplitQueue {
+  int pt[SPLIT_Q];
+  float term[SPLIT_ROWS * 32], z[SPLIT_ROWS * 32];
+  unsigned short list[SPLIT_ROWS * 32];
+};
+
+// An output row of either type: one copy of the evaluating code serves both,
+// so their values are the same bits.
+struct SplitRow {
+  char* p;
+  bool f64;
+  __device__ __forceinline__ void put(int pt, float v) const {
+    if (f64) __stcs(reinterpret_cast<double*>(p) + pt, (double)v);
+    else __stcs(reinterpret_cast<float*>(p) + pt, v);
+  }
+  __device__ __forceinline__ void fill(int tile, int lane, float v) const {
+    if (f64) TileOut<double>::fill(reinterpret_cast<double*>(p), tile, lane, v);
+    else TileOut<float>::fill(reinterpret_cast<float*>(p), tile, lane, v);
+  }
+};
+
+// 1 / sqrt(x) of a normal x, without the scaling around it for denormals.
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Evaluates and stores queued points, all of the light curve record R: whole
+// warps of them, or, with all set, every one.  Returns the points left, moved
+// to the front.
+//
+// The kernel is bound by instruction issue.  A lane takes a point, folds its
+// time exactly and walks its samples, so that no index arithmetic is needed
+// per sample; the samples of up to SPLIT_ROWS rows (32 points x 1 sample) get
+// their separation and LD mean first, which finishes those inside the star,
+// and the overlap area of the samples on the limb (about a third) follows in
+// full warps from a list.  A point's terms are added in sample order.  4096 pv
+// x 118,526 times x 10 samples: 2682 us with each tile's (point, sample) pairs
+// by themselves (a binary search for a pair's point, the full area for every
+// pair, a segmented shuffle sum), 1706 us.  Ranges of 64, 128 and 256 tiles per
+// block instead of 32: 5, 8 and 14 % slower.
+__device__ __forceinline__ int split_flush(const float2* __restrict__ times, const float* orb, const float* R,
+                                           const float* ldm_pv, int ng, float inv_dg, SplitQueue& Q, int n, bool all,
+                                           const SplitRow& row) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  __syncwarp();
+  const float k = R[LC_K], ex = R[LC_EXPT], inv_ns = R[LC_INVNS], gsc = R[LC_INV1PK] * inv_dg, step = ex * inv_ns;
+  const int ns_all = __float_as_int(R[LC_NS]);
+  const float invis = R[LC_INVIS];
+  const float* lda = ldm_pv + __float_as_int(R[LC_PB]) * ng;
+  const float lim_out = 1.0f + k, lim_in = (k < 1.0f) ? 1.0f - k : -1.0f, area_in = float(PI) * k * k;
+  const float4 ca = *reinterpret_cast<const float4*>(orb);
+  const float4 cb = *reinterpret_cast<const float4*>(orb + 4);
+  const float2 cc = *reinterpret_cast<const float2*>(orb + 8);
+  const float4 fold = *reinterpret_cast<const float4*>(R), box = *reinterpret_cast<const float4*>(R + 4);
+  const int take = all ? n : n & ~31;
+  const int sc = min(max(ns_all, 1), SPLIT_ROWS), nb = SPLIT_ROWS / sc;   // samples, batches of 32 points at once
+  for (int i0 = 0; i0 < take; i0 += 32 * nb) {
+    float D = 0.0f;   // with more samples than rows (nb = 1): the point's sum so far
+    for (int s0 = 0; s0 < max(ns_all, 1); s0 += sc) {
+      const int ns = min(sc, ns_all - s0);
+      int nlimb = 0, r = 0;
+      for (int b = i0; b < min(take, i0 + 32 * nb); b += 32) {
+        // time_offset = exptime ((isample - 0.5)/ns - 0.5), isample = s0 + s + 1
+        float tb = 1e30f;   // no overlap past the last point and out of the box
+        if (b + lane < take) {
+          const float2 tt = __ldg(times + Q.pt[b + lane]);
+          const float ne = floorf(fmaf(tt.x - fold.z, orb[12], 0.5f));
+          const float tc = exact_tc(tt.x, tt.y, fold.z, fold.w, ne, orb[10], orb[11]);
+          if (box.x <= tc && tc <= box.y) tb = fmaf(-0.5f, ex, tc);
+        }
+        float sf = (float)s0 + 0.5f;
+#pragma unroll 2
+        for (int s = 0; s < ns; ++s, r += 32, sf += 1.0f) {
+          const float t = fmaf(sf, step, tb);
+          const float x = fmaf(t, fmaf(t, fmaf(t, fmaf(t, cb.x, ca.w), ca.z), ca.y), ca.x);
+          const float y = fmaf(t, fmaf(t, fmaf(t, fmaf(t, cc.y, cc.x), cb.w), cb.z), cb.y);
+          const float r2 = fmaf(x, x, y * y);
+          const float z = r2 * rsqrt_ftz(fmaxf(r2, 1e-30f));
+          const bool ovl = z < lim_out, limb = ovl && !(z <= lim_in);
+          const float gg = fminf(z, lim_out) * gsc;
+          const int i = min(max((int)gg, 0), ng - 2);
+          const float l0 = __ldg(lda + i), l1 = __ldg(lda + i + 1);
+          const float mean = fmaf(gg - (float)i, l1 - l0, l0);
+          Q.term[r + lane] = ovl ? (limb ? mean : mean * area_in) : 0.0f;
+          const unsigned m = __ballot_sync(FULL, limb);
+          if (limb) {
+            const int at = nlimb + __popc(m & below);
+            Q.z[at] = z;
+            Q.list[at] = (unsigned short)(r + lane);
+          }
+          nlimb += __popc(m);
+        }
+      }
+      __syncwarp();
+      for (int j = lane; j < nlimb; j += 32) {
+        const int f = Q.list[j];
+        const float z = Q.z[j];
+        float a;
+        if (k <= 0.25f) {          // uniform over the warp
+          a = kite_star_f32_smallk(k, z);
+        } else if (k < 1.0f) {
+          a = kite_star_f32(k, z);
+        } else {
+          float kap;
+          a = ccia_star<float>(k, z, kap);
+        }
+        Q.term[f] *= a;
+      }
+      __syncwarp();
+      const bool last = s0 + ns >= ns_all;
+      r = 0;
+      for (int b = i0; b < min(take, i0 + 32 * nb); b += 32) {
+        if (s0 == 0) D = 0.0f;
+        for (int s = 0; s < ns; ++s, r += 32) D += Q.term[r + lane];
+        // in the box without overlap: 1, or NaN with a NaN disk integral
+        const float f = 1.0f - D * invis * inv_ns;
+        if (last && b + lane < take) {
+          if (D != 0.0f) {
+            row.put(Q.pt[b + lane], f);
+          } else {
+            const float2 tt = __ldg(times + Q.pt[b + lane]);
+            const float ne = floorf(fmaf(tt.x - fold.z, orb[12], 0.5f));
+            const float tc = exact_tc(tt.x, tt.y, fold.z, fold.w, ne, orb[10], orb[11]);
+            row.put(Q.pt[b + lane], box.x <= tc && tc <= box.y ? f : 1.0f);
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+  const int left = n - take;
+  if (take > 0 && lane < left) Q.pt[lane] = Q.pt[take + lane];
+  __syncwarp();
+  return left;
+}
+
+union SplitSmem {   // a warp's lists: one of the two per pv
+  WarpList l;
+  SplitQueue q;
+};
+
+// The cull test of one tile: its time range (from its summary) misses every
+// box copy, the rounding of t - d0 and of j p covered by the error bound in
+// the box (flo, fhi).  Tiles of several light curves never miss.
+__device__ __forceinline__ bool split_tile_misses(const float4 tm, const float* LCR, float p_hi, float inv_p) {
+  const int tlc = __float_as_int(tm.z);
+  if (tlc < 0) return false;
+  const float4 f = *reinterpret_cast<const float4*>(LCR + tlc * LC32);  // flo, fhi, d0h, d0l
+  const float smin = tm.x - f.z, smax = tm.y - f.z;
+  const float j0f = ceilf((smin - f.y) * inv_p);
+  bool hit = false;
+#pragma unroll
+  for (int dj = -1; dj <= 1; ++dj) {
+    const float jj = j0f + (float)dj;
+    hit = hit || (fmaf(jj, p_hi, f.x) <= smax && fmaf(jj, p_hi, f.y) >= smin);
+  }
+  return !hit;
+}
+
+// The points of a tile of several light curves, a lane per point.
+__device__ __noinline__ void split_mixed_tile(const float2* __restrict__ times, const int32_t* __restrict__ lcids,
+                                              int npt, const float* orb, const float* LCR, const float* ldm_pv,
+                                              int ng, float inv_dg, int pt0, const SplitRow& row) {
+  const bool wide = __float_as_int(orb[14]) & FLAG_WIDE;
+  for (int q = 0; q < SPLIT_PTS; ++q) {
+    const int pt = pt0 + 32 * q;
+    if (pt >= npt) continue;
+    const float2 tt = __ldg(times + pt);
+    const float* R = LCR + __ldg(lcids + pt) * LC32;
+    const float sv = tt.x - R[LC_D0H], ne = floorf(fmaf(sv, orb[12], 0.5f)), r = fmaf(-ne, orb[10], sv);
+    float f = 1.0f;
+    if (wide || (r >= R[LC_FLO] && r <= R[LC_FHI])) {
+      const float tc = exact_tc(tt.x, tt.y, R[LC_D0H], R[LC_D0L], ne, orb[10], orb[11]);
+      if (R[LC_LO] <= tc && tc <= R[LC_HI]) {
+        const float* lda = ldm_pv + __float_as_int(R[LC_PB]) * ng;
+        const float k = R[LC_K];
+        const int ns = __float_as_int(R[LC_NS]);
+        float D = 0.0f;
+        for (int s = 0; s < ns; ++s) {
+          const float z = sep_c_f32(tc + R[LC_EXPT] * fmaf((float)s + 0.5f, R[LC_INVNS], -0.5f), orb);
+          if (!(z < 1.0f + k)) continue;
+          const float gg = z * R[LC_INV1PK] * inv_dg;
+          const int i = min(max((int)gg, 0), ng - 2);
+          const float l0 = __ldg(lda + i), l1 = __ldg(lda + i + 1);
+          float kap;
+          D += fmaf(gg - (float)i, l1 - l0, l0) * ccia_star<float>(k, z, kap);
+        }
+        f = 1.0f - D * R[LC_INVIS] * R[LC_INVNS];
+      }
+    }
+    row.put(pt, f);
+  }
+}
+
+// A warp's tiles of a valid pv with supersampled light curves: the same cull
+// test, every tile filled with 1, and of the tiles that reach a box the points
+// that the fast FP32 fold (its error allowed for in flo, fhi) puts in it to the
+// queue; their values overwrite the 1.  The queue is emptied at one place,
+// before a tile, so that no values of a tile live across it.
+__device__ __noinline__ void split_pv_multi(const FluxSplitArgs& A, int pv, int t_first, int t_step, int t_end,
+                                            const float* orb, const float* LCR, SplitQueue& Q, bool out_f64) {
+  const unsigned FULL = 0xffffffffu;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __builtin_assume(__isShared(&Q));
+  __builtin_assume(__isShared(orb));
+  // locals: a field of A would be read again after every store to the row
+  const int npt = A.npt, ng = A.ng;
+  const float inv_dg = A.inv_dg;
+  const float2* __restrict__ times = A.times_ff;
+  const bool wide = __float_as_int(orb[14]) & FLAG_WIDE;
+  const float p_hi = orb[10], inv_p = orb[12];
+  const float* __restrict__ ldm_pv = A.ldm + (size_t)pv * A.npb * ng;
+  const SplitRow row{static_cast<char*>(A.flux) + (size_t)pv * A.ldflux * (out_f64 ? 8 : 4), out_f64};
+  const bool row_vec = ((A.ldflux & 3) == 0) && ((reinterpret_cast<uintptr_t>(A.flux) & 15) == 0);
+  const bool fill = !A.transits_only;
+  const float4* meta = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(times) + time_meta_offset(npt));
+  const int tw0 = t_first + warp;
+  const int ntl = tw0 < t_end ? (t_end - tw0 + t_step - 1) / t_step : 0;
+  int n = 0, qlc = -1;   // queued points and their light curve
+  int j0 = -32, mylc = 0;
+  unsigned m = 0;        // tiles of the current group of 32 still to do
+  for (;;) {
+    while (m == 0 && j0 + 32 < ntl) {
+      j0 += 32;
+      const int jn = min(32, ntl - j0);
+      bool cull = false;
+      if (lane < jn) {
+        const float4 tm = __ldg(meta + tw0 + (j0 + lane) * t_step);
+        mylc = __float_as_int(tm.z);
+        cull = !wide && split_tile_misses(tm, LCR, p_hi, inv_p);
+      }
+      const unsigned jmask = jn == 32 ? FULL : (1u << jn) - 1u;
+      const unsigned cmask = __ballot_sync(FULL, cull) & jmask;
+      m = ~cmask & jmask;
+      for (unsigned c = fill ? jmask : m; c; c &= c - 1u) {
+        const int tile = tw0 + (j0 + __ffs(c) - 1) * t_step;
+        if (row_vec && (tile + 1) * WARP_TILE <= npt) {
+          row.fill(tile, lane, 1.0f);
+        } else {
+          for (int q = 0; q < SPLIT_PTS; ++q)
+            if (tile * WARP_TILE + 32 * q + lane < npt) row.put(tile * WARP_TILE + 32 * q + lane, 1.0f);
+        }
+      }
+    }
+    const bool done = m == 0;
+    const int j = done ? 0 : __ffs(m) - 1;
+    const int tlc = __shfl_sync(FULL, mylc, j);
+    const bool all = done || tlc != qlc;
+    if (n > 0 && (all || n > SPLIT_Q - WARP_TILE))
+      n = split_flush(times, orb, LCR + qlc * LC32, ldm_pv, ng, inv_dg, Q, n, all, row);
+    if (done) return;
+    m &= m - 1u;
+    const int p0 = (tw0 + (j0 + j) * t_step) * WARP_TILE;
+    if (tlc < 0) {
+      __syncwarp();   // after the fill
+      split_mixed_tile(times, A.lcids, npt, orb, LCR, ldm_pv, ng, inv_dg, p0 + lane, row);
+      continue;
+    }
+    qlc = tlc;
+    // points p0 + 4 lane + q
+    const float* R = LCR + tlc * LC32;
+    const float4 f = *reinterpret_cast<const float4*>(R);       // flo, fhi, d0h, d0l
+    const float lo = wide ? -INFINITY : f.x, hi = wide ? INFINITY : f.y;
+    const int pt = p0 + SPLIT_PTS * lane;
+    float t[SPLIT_PTS];
+    if (p0 + WARP_TILE <= npt) {
+      const float4 u = __ldg(reinterpret_cast<const float4*>(times + pt));
+      const float4 v = __ldg(reinterpret_cast<const float4*>(times + pt) + 1);
+      t[0] = u.x; t[1] = u.z; t[2] = v.x; t[3] = v.z;
+    } else {
+#pragma unroll
+      for (int q = 0; q < SPLIT_PTS; ++q)
+        t[q] = pt + q < npt ? __ldg(times + pt + q).x : __int_as_float(0x7fc00000);   // NaN: in no box
+    }
+    unsigned mask[SPLIT_PTS];
+    unsigned in = 0;
+#pragma unroll
+    for (int q = 0; q < SPLIT_PTS; ++q) {
+      const float sv = t[q] - f.z;
+      const float r = fmaf(-floorf(fmaf(sv, inv_p, 0.5f)), p_hi, sv);
+      const bool b = r >= lo && r <= hi;
+      in |= b ? 1u << q : 0u;
+      mask[q] = __ballot_sync(FULL, b);
+    }
+#pragma unroll
+    for (int q = 0; q < SPLIT_PTS; ++q) {
+      if (in >> q & 1u) Q.pt[n + __popc(mask[q] & ((1u << lane) - 1u))] = pt + q;
+      n += __popc(mask[q]);
+    }
+  }
+}
 
 // Per-point path for one warp tile of one pv (slot q of lane l = the tile's
 // point q * 32 + l).  Phase-folded times: for a tile of one light curve whose
 // span plus box half-width is below p/2, the exact time of the tile's first
 // point plus each point's (exact, small) offset from it; otherwise a fast
 // FP32 test per point and the exact reduction for candidates.  Then the
-// samples of the in-box points: with one sample per point, per point in
-// place, skipping slots without an in-box point as a whole warp; else a
-// per-warp list whose (point, sample) pairs are spread over the lanes and
-// summed with a segmented shuffle reduction.  res[] holds 1.0 on entry and
-// the flux of in-box points on exit.
+// flux of the in-box points in place, skipping slots without an in-box point as a whole warp.  res[] holds
+// 1.0 on entry and the flux of in-box points on exit.  For a pv whose light
+// curves take one sample per point; split_pv_multi does the others.
 __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb, const float* __restrict__ LCR,
                                                   const float* __restrict__ ldm_pv, int ng, float inv_dg,
                                                   bool wide, float4 tm, const float* hi, const float* lo,
@@ -853,17 +1151,7 @@ __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb,
   unsigned act = 0;
 #pragma unroll
   for (int q = 0; q < SPLIT_PTS; ++q) act |= (__ballot_sync(FULL, inb >> q & 1u) ? 1u : 0u) << q;
-  bool single;
-  if (tlc >= 0) {
-    single = __float_as_int(RT[LC_NS]) == 1;   // one light curve: warp-uniform
-  } else {
-    single = true;
-#pragma unroll
-    for (int q = 0; q < SPLIT_PTS; ++q)
-      if (inb >> q & 1u) single = single && (__float_as_int(LCR[lcv[q] * LC32 + LC_NS]) == 1);
-    single = __all_sync(FULL, single);
-  }
-  if (single) {
+  {
     // One sample per point.  A point whose planet disk is fully inside the
     // star (area pi k^2) is finished in place; points on the limb (kite area,
     // two atan2) are gathered into the warp's list and evaluated 32 at a time,
@@ -1003,90 +1291,7 @@ __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb,
     for (int q = 0; q < SPLIT_PTS; ++q)
       if (posq[q] >= 0) res[q] = 1.0f - L.acc[posq[q]] * LCR[lcv[q] * LC32 + LC_INVIS];
     __syncwarp();
-    return;
   }
-  int nitems = 0;
-  int posq[SPLIT_PTS];
-#pragma unroll
-  for (int q = 0; q < SPLIT_PTS; ++q) {
-    const bool in = inb >> q & 1u;
-    const unsigned m = __ballot_sync(FULL, in);
-    posq[q] = -1;
-    if (in) {
-      const int pos = nitems + __popc(m & ((1u << lane) - 1u));
-      L.tc[pos] = tcq[q];
-      L.lc[pos] = lcv[q];
-      posq[q] = pos;
-    }
-    nitems += __popc(m);
-  }
-  __syncwarp();
-  // exclusive prefix sum of the sample counts -> L.off
-  int carry = 0;
-  for (int c0 = 0; c0 < nitems; c0 += 32) {
-    const int it = c0 + lane;
-    const int v = (it < nitems) ? __float_as_int(LCR[L.lc[it] * LC32 + LC_NS]) : 0;
-    int incl = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int u = __shfl_up_sync(FULL, incl, d);
-      if (lane >= d) incl += u;
-    }
-    if (it < nitems) {
-      L.off[it] = carry + incl - v;
-      L.acc[it] = 0.0f;
-    }
-    carry += __shfl_sync(FULL, incl, 31);
-  }
-  __syncwarp();
-  const int total = carry;
-  for (int f0 = 0; f0 < total; f0 += 32) {
-    const int f = f0 + lane;
-    float d = 0.0f;
-    int item = -1;
-    if (f < total) {
-      int lo_i = 0, hi_i = nitems - 1;   // largest item with off[item] <= f
-      while (lo_i < hi_i) {
-        const int mid = (lo_i + hi_i + 1) >> 1;
-        if (L.off[mid] <= f) lo_i = mid; else hi_i = mid - 1;
-      }
-      item = lo_i;
-      const int smp = f - L.off[item];
-      const float* R = LCR + L.lc[item] * LC32;
-      const float k = R[LC_K];
-      // time_offset = exptime ((isample - 0.5)/ns - 0.5), isample = smp + 1
-      const float t = L.tc[item] + R[LC_EXPT] * fmaf(float(smp) + 0.5f, R[LC_INVNS], -0.5f);
-      const float z = sep_c_f32(t, orb);
-      if (z < 1.0f + k) {
-        const float gg = z * R[LC_INV1PK] * inv_dg;
-        int i = (int)gg;
-        i = min(max(i, 0), ng - 2);
-        const float fr = gg - (float)i;
-        const float* lda = ldm_pv + __float_as_int(R[LC_PB]) * ng;
-        const float l0 = __ldg(lda + i), l1 = __ldg(lda + i + 1);
-        float kap;
-        d = fmaf(fr, l1 - l0, l0) * ccia_star<float>(k, z, kap);
-      }
-    }
-    // segmented sum over lanes holding the same item
-#pragma unroll
-    for (int dd = 1; dd < 32; dd <<= 1) {
-      const float dv = __shfl_down_sync(FULL, d, dd);
-      const int iv = __shfl_down_sync(FULL, item, dd);
-      if (lane + dd < 32 && iv == item) d += dv;
-    }
-    const int iprev = __shfl_up_sync(FULL, item, 1);
-    if (item >= 0 && (lane == 0 || iprev != item)) L.acc[item] += d;
-    __syncwarp();
-  }
-#pragma unroll
-  for (int q = 0; q < SPLIT_PTS; ++q) {
-    if (posq[q] >= 0) {
-      const float* R = LCR + lcv[q] * LC32;
-      res[q] = 1.0f - L.acc[posq[q]] * R[LC_INVIS] * R[LC_INVNS];
-    }
-  }
-  __syncwarp();
 }
 
 // One block's share of one parameter vector: stage the pv's orbit and
@@ -1097,7 +1302,7 @@ __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb,
 // synchronises before staging another pv.
 template <typename OutT>
 __device__ __forceinline__ void split_pv_tiles(const FluxSplitArgs& A, int pv, int t_first, int t_step, int t_end,
-                                               float* recs, bool lc_in_smem, WarpList* lists) {
+                                               float* recs, bool lc_in_smem, SplitSmem* lists) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* lcg = A.lc32 + (size_t)pv * A.nlc * LC32;
   if (threadIdx.x < ORB32) recs[threadIdx.x] = __ldg(A.orb32 + (size_t)pv * ORB32 + threadIdx.x);
@@ -1109,13 +1314,17 @@ __device__ __forceinline__ void split_pv_tiles(const FluxSplitArgs& A, int pv, i
   const int flags = __float_as_int(orb[14]);
   const bool valid = flags & FLAG_VALID;
   const bool wide = flags & FLAG_WIDE;
+  if (valid && (flags & FLAG_MULTI)) {   // block-uniform
+    split_pv_multi(A, pv, t_first, t_step, t_end, orb, LCR, lists[warp].q, sizeof(OutT) == 8);
+    return;
+  }
   const float p_hi = orb[10], inv_p = orb[12];
   const float* ldm_pv = A.ldm + (size_t)pv * A.npb * A.ng;
   OutT* row = static_cast<OutT*>(A.flux) + (size_t)pv * A.ldflux;
   const bool row_vec = ((A.ldflux & 3) == 0) && ((reinterpret_cast<uintptr_t>(A.flux) & 15) == 0);
   const float4* meta = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(A.times_ff) +
                                                        time_meta_offset(A.npt));
-  WarpList& L = lists[warp];
+  WarpList& L = lists[warp].l;
   const unsigned FULL = 0xffffffffu;
   // The warp's tiles are t_first + warp + j t_step, j < ntl.  A culled tile is
   // one 16-byte store of the fill value per lane (ones; NaN for an invalid
@@ -1126,28 +1335,8 @@ __device__ __forceinline__ void split_pv_tiles(const FluxSplitArgs& A, int pv, i
   const int tile_part = (A.npt % WARP_TILE) ? A.npt / WARP_TILE : -1;
   const float fill = valid ? 1.0f : __int_as_float(0x7fc00000);
   for (int j0 = 0; j0 < ntl; j0 += 32) {
-    // The cull test of the warp's next 32 tiles, one tile per lane: the
-    // tile's time range (from its summary) against the box copies around it,
-    // the rounding of t - d0 and of j p covered by the error bound in the box
-    // (flo, fhi).
     const int tl = tw0 + (j0 + lane) * t_step;
-    bool cull = !valid;
-    if (valid && !wide && j0 + lane < ntl) {
-      const float4 tm = __ldg(meta + tl);
-      const int tlc = __float_as_int(tm.z);
-      if (tlc >= 0) {
-        const float4 f = *reinterpret_cast<const float4*>(LCR + tlc * LC32);  // flo, fhi, d0h, d0l
-        const float smin = tm.x - f.z, smax = tm.y - f.z;
-        const float j0f = ceilf((smin - f.y) * inv_p);
-        bool hit = false;
-#pragma unroll
-        for (int dj = -1; dj <= 1; ++dj) {
-          const float jj = j0f + (float)dj;
-          hit = hit || (fmaf(jj, p_hi, f.x) <= smax && fmaf(jj, p_hi, f.y) >= smin);
-        }
-        cull = !hit;
-      }
-    }
+    const bool cull = !valid || (!wide && j0 + lane < ntl && split_tile_misses(__ldg(meta + tl), LCR, p_hi, inv_p));
     const int jn = min(32, ntl - j0);
     const unsigned jmask = jn == 32 ? 0xffffffffu : (1u << jn) - 1u;
     const unsigned cmask = __ballot_sync(FULL, cull) & jmask;
@@ -1203,8 +1392,9 @@ constexpr int FLUX_NW = 2;
 constexpr int FLUX_CHUNK = 32;
 
 template <bool LC_IN_SMEM, typename OutT>
-__global__ void __launch_bounds__(FLUX_NW * 32) flux_split_kernel(FluxSplitArgs A, int chunk) {
-  __shared__ WarpList lists[FLUX_NW];
+__global__ void __launch_bounds__(FLUX_NW * 32, 16)
+flux_split_kernel(const __grid_constant__ FluxSplitArgs A, int chunk) {
+  __shared__ SplitSmem lists[FLUX_NW];
   extern __shared__ __align__(16) float flux_recs[];
   const int pv = block_pv();
   if (pv >= A.npv) return;  // block-uniform
@@ -1226,7 +1416,7 @@ serve_split_kernel(const rr_serve_request* __restrict__ reqs, const rr_serve_ite
   // the per-warp lists of the RoadRunner tiles and the tile state of the
   // transmission-spectroscopy tiles share the block's shared memory
   __shared__ union ServeSmem {
-    WarpList lists[SPLIT_WARPS];
+    SplitSmem lists[SPLIT_WARPS];
     TsSmem<float> ts;
   } U;
   __shared__ __align__(16) float recs[ORB32 + LC_SMEM * LC32];
@@ -1256,7 +1446,6 @@ serve_split_kernel(const rr_serve_request* __restrict__ reqs, const rr_serve_ite
       __syncthreads();
       continue;
     }
-    WarpList* lists = U.lists;
     FluxSplitArgs A{};
     A.times_ff = reinterpret_cast<const float2*>(r.times_ff);
     A.lcids = r.lcids;
@@ -1265,7 +1454,7 @@ serve_split_kernel(const rr_serve_request* __restrict__ reqs, const rr_serve_ite
     A.inv_dg = r.inv_dg; A.flux = r.flux;
     const bool lc_smem = r.nlc <= LC_SMEM;
     for (int pv = w.pv0; pv < w.pv1; ++pv) {
-      split_pv_tiles<float>(A, pv, w.tile0, SPLIT_WARPS, w.tile1, recs, lc_smem, lists);
+      split_pv_tiles<float>(A, pv, w.tile0, SPLIT_WARPS, w.tile1, recs, lc_smem, U.lists);
       __syncthreads();
     }
   }
