@@ -240,16 +240,14 @@ __global__ void __launch_bounds__(OBS_THREADS) obs_kernel(const double* __restri
 // r = do + D.  Block sums go to partials[pv][block][1 + ngrad] (FP64), summed
 // per pv in block order by lnlike_reduce_kernel: no step depends on timing.
 // ---------------------------------------------------------------------------
-template <typename R>
 struct GradArgs {
   // data
   const float2* times_ff;
   const int32_t *lcids, *pbids, *epids;
-  const R *dobs, *isig2;
+  const float *dobs, *isig2;
   int nkc, nep;
   // prologue tables
-  const float *orb32, *lc32;
-  const R *ldm, *dc, *tab, *dis;
+  const float *orb32, *lc32, *ldm, *dc, *tab, *dis;
   int npt, npv, npb, nlc, ng, npar, ngrad;
   double dg;
   double* partials;
@@ -271,19 +269,34 @@ constexpr int LNL_THREADS = 128;
 constexpr int LNL_PPT = 8;
 constexpr int LNL_CHUNK = LNL_THREADS * LNL_PPT;
 constexpr int LNL_NW = LNL_THREADS / 32;
+constexpr int DC_ROW = 12;   // a row of dc in shared memory: ten coefficients, 16-byte aligned
+
+// a b + c d with one rounding fewer, in FP32: the first product is exact.
+// The likelihood's arithmetic is written out in fused operations, so that its
+// bits do not depend on how the compiler contracts and schedules it.
+__device__ __forceinline__ float fma2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
+
+// The kite of ccia_star (|1 - k| < z < 1 + k): its area and the half-angles
+// of planet and star.
+__device__ __forceinline__ float kite_area(float k, float z) {
+  const float a = fmaxf(1.0f, k), b = fminf(1.0f, k);
+  const float x = fmaxf(a, z), t = fminf(a, z);
+  const float y = fmaxf(b, t), w = fminf(b, t);
+  return 0.5f * sqrtf((x + (y + w)) * (w - (x - y)) * (w + (x - y)) * (x + (y - w)));
+}
+constexpr int LNL_STASH = 8;   // samples per point kept in shared memory for the second pass
 
 // Adds one point's terms to the slot accumulators acc (the lnL term and, with
-// GRAD, the gradient terms of GS_KK ... GS_C0 + npar - 1); nothing for a point
-// out of the box.  Two passes over the samples: the first gives the point's
-// deficit D and with it the residual weight -(r / sigma^2) / (ns istar); the
-// second recomputes each sample and adds its derivative terms, already
-// scaled by that weight, straight into acc (no per-point sums are kept).
-template <typename R, bool GRAD>
-__device__ __forceinline__ void lnlike_point(const GradArgs<R>& A, int pv, int pt, int lc, const float* lcs,
-                                             bool lc_smem, const R* orbc, const R* dcs, R* acc) {
-  const int pb = A.pbids[lc], ep = A.epids[lc];
-  bool inbox;
-  R tc, nep_count;
+// GRAD, the gradient terms of GS_KK ... GS_C0 + npar - 1); false for a point
+// out of the box, which adds nothing.  Two passes over the samples: the first
+// gives the point's deficit D and with it the residual weight
+// -(r / sigma^2) / (ns istar); the second adds each sample's derivative terms,
+// already scaled by that weight, straight into acc (no per-point sums are
+// kept).  The first LNL_STASH samples' separations and areas are kept in
+// shared memory between the passes.
+template <bool GRAD>
+__device__ __forceinline__ bool lnlike_point(const GradArgs& A, int pv, int pt, int lc, const float* lcs, bool lc_smem,
+                                             const float* orbc, const float* dcs, float4* stash, float* acc) {
   const float* LCR = lc_smem ? lcs + lc * LC32 : A.lc32 + ((size_t)pv * A.nlc + lc) * LC32;
   const float* o = A.orb32 + (size_t)pv * ORB32;
   const float p_hi = o[10], p_lo = o[11], inv_p = o[12];
@@ -294,152 +307,201 @@ __device__ __forceinline__ void lnlike_point(const GradArgs<R>& A, int pv, int p
   two_sum(tt.x, -d0h, s1, e1);
   two_prod(n, p_hi, q1, e2);
   two_sum(s1, -q1, s2, e3);
-  float t = s2 + (((e1 + e3) - e2) + (tt.y - d0l) - n * p_lo);
-  if (t >= 0.5f * p_hi || t < -0.5f * p_hi) {
-    n += (t >= 0.5f * p_hi) ? 1.0f : -1.0f;
+  float tc = s2 + (((e1 + e3) - e2) + (tt.y - d0l) - n * p_lo);
+  if (tc >= 0.5f * p_hi || tc < -0.5f * p_hi) {
+    n += (tc >= 0.5f * p_hi) ? 1.0f : -1.0f;
     two_prod(n, p_hi, q1, e2);
     two_sum(s1, -q1, s2, e3);
-    t = s2 + (((e1 + e3) - e2) + (tt.y - d0l) - n * p_lo);
+    tc = s2 + (((e1 + e3) - e2) + (tt.y - d0l) - n * p_lo);
   }
-  inbox = (LCR[LC_LO] <= t && t <= LCR[LC_HI]);
-  tc = (R)t;
-  nep_count = (R)n;
-  if (!inbox) return;
-  const R kk = (R)LCR[LC_K], inv_is = (R)LCR[LC_INVIS], ex = (R)LCR[LC_EXPT], inv_ns = (R)LCR[LC_INVNS];
+  if (!(LCR[LC_LO] <= tc && tc <= LCR[LC_HI])) return false;
+  const float kk = LCR[LC_K], inv_is = LCR[LC_INVIS], ex = LCR[LC_EXPT], inv_ns = LCR[LC_INVNS];
   const int ns = __float_as_int(LCR[LC_NS]);
-  const R inv1pk = R(1) / (R(1) + kk);
-  const R inv_dg = R(1) / (R)A.dg;
-  const size_t ppb = (size_t)pv * A.npb + pb;
-  const R* L = A.ldm + ppb * A.ng;
+  const float inv1pk = 1.0f / (1.0f + kk);
+  const float inv_dg = 1.0f / (float)A.dg;
+  const size_t ppb = (size_t)pv * A.npb + A.pbids[lc];
+  const float* L = A.ldm + ppb * A.ng;
+  const float lim = 1.0f + kk, lim_in = fabsf(1.0f - kk), area_in = kk < 1.0f ? float(PI) * kk * kk : float(PI);
   // pass 1: the deficit D = sum_s I A / (ns istar)
-  R SQ = R(0);
+  float SQ = 0.0f;
   for (int s = 0; s < ns; ++s) {
-    const R t = tc + ex * ((R(s) + R(0.5)) * inv_ns - R(0.5));
-    R x = orbc[4], y = orbc[9];
+    const float t = fmaf(ex, fmaf((float)s + 0.5f, inv_ns, -0.5f), tc);
+    float x = orbc[4], y = orbc[9];
+#pragma unroll
     for (int m = 3; m >= 0; --m) {
-      x = x * t + orbc[m];
-      y = y * t + orbc[5 + m];
+      x = fmaf(x, t, orbc[m]);
+      y = fmaf(y, t, orbc[5 + m]);
     }
-    const R z = sqrt(x * x + y * y);
-    if (!(z < R(1) + kk)) continue;  // A = 0 and I A = 0 beyond first contact
-    const R gg = z * inv1pk * inv_dg;
-    const int i = min(max((int)gg, 0), A.ng - 2);
-    const R fr = gg - (R)i;
-    const R l0 = L[i], l1 = L[i + 1];
-    R kap;
-    SQ += (l0 + fr * (l1 - l0)) * ccia_star<R>(kk, z, kap);
+    const float z = sqrtf(fma2(x, x, y, y));
+    float a_kite = 0.0f;
+    if (z < lim) {   // A = 0 and I A = 0 beyond first contact
+      const float gg = z * inv1pk * inv_dg;
+      const int i = min(max((int)gg, 0), A.ng - 2);
+      const float fr = __fsub_rn(gg, (float)i);
+      const float l0 = L[i], l1 = L[i + 1];
+      float area = area_in;
+      if (lim_in < z) {
+        a_kite = kite_area(kk, z);
+        const float k0 = atan2f(2.0f * a_kite, fma2(z, z, kk - 1.0f, kk + 1.0f));
+        const float k1 = atan2f(2.0f * a_kite, fma2(z, z, 1.0f - kk, 1.0f + kk));
+        area = __fsub_rn(fmaf(kk * kk, k0, k1), a_kite);
+      }
+      SQ = fmaf(fmaf(fr, l1 - l0, l0), area, SQ);
+    }
+    if (GRAD && s < LNL_STASH) stash[s * LNL_THREADS] = make_float4(x, y, z, a_kite);
   }
-  const R sc = inv_is * inv_ns;
-  const R D = SQ * sc;
-  const R do_ = A.dobs[pt], w = A.isig2[pt];
-  acc[GS_LNL] += -(do_ + R(0.5) * D) * D * w;
+  const float sc = inv_is * inv_ns;
+  const float D = __fmul_rn(SQ, sc);
+  const float do_ = A.dobs[pt], w = A.isig2[pt];
+  acc[GS_LNL] = fmaf(__fmul_rn(-fmaf(0.5f, D, do_), D), w, acc[GS_LNL]);
   if constexpr (GRAD) {
-    const R gsc = -(do_ + D) * w * sc;    // -(r / sigma^2) / (ns istar)
-    const R* T = A.tab + ppb * (size_t)(1 + A.npar) * A.ng;
+    const float r = __fadd_rn(do_, D);
+    const float gsc = -r * w * sc;    // -(r / sigma^2) / (ns istar)
+    const float* T = A.tab + ppb * (size_t)(1 + A.npar) * A.ng;
     // pass 2: the derivative terms of every sample, times gsc
     for (int s = 0; s < ns; ++s) {
-      const R t = tc + ex * ((R(s) + R(0.5)) * inv_ns - R(0.5));
-      R x = orbc[4], y = orbc[9], xd = R(4) * orbc[4], yd = R(4) * orbc[9];
-      for (int m = 3; m >= 0; --m) {
-        x = x * t + orbc[m];
-        y = y * t + orbc[5 + m];
-        if (m >= 1) {
-          xd = xd * t + R(m) * orbc[m];
-          yd = yd * t + R(m) * orbc[5 + m];
+      asm volatile("" ::: "memory");   // keeps the 50 derivative coefficients out of registers: see below
+      const float t = fmaf(ex, fmaf((float)s + 0.5f, inv_ns, -0.5f), tc);
+      float x, y, z, a_kite = 0.0f;
+      if (s < LNL_STASH) {
+        const float4 st = stash[s * LNL_THREADS];
+        x = st.x; y = st.y; z = st.z; a_kite = st.w;
+        if (!(z < lim)) continue;
+      } else {
+        x = orbc[4]; y = orbc[9];
+#pragma unroll
+        for (int m = 3; m >= 0; --m) {
+          x = fmaf(x, t, orbc[m]);
+          y = fmaf(y, t, orbc[5 + m]);
         }
+        z = sqrtf(fma2(x, x, y, y));
+        if (!(z < lim)) continue;
+        if (lim_in < z) a_kite = kite_area(kk, z);
       }
-      const R z = sqrt(x * x + y * y);
-      if (!(z < R(1) + kk)) continue;
-      const R g = z * inv1pk;
-      const R gg = g * inv_dg;
+      // d(x, y)/dt from m c_m
+      float xd = orbc[10 + 3], yd = orbc[14 + 3];
+#pragma unroll
+      for (int m = 2; m >= 0; --m) {
+        xd = fmaf(xd, t, orbc[10 + m]);
+        yd = fmaf(yd, t, orbc[14 + m]);
+      }
+      // the area with its partial derivatives dA/dk = 2 k kappa0 and
+      // dA/dz = -2 A_kite / z (ccia_star_grad)
+      float ar = area_in, dadk = kk < 1.0f ? 2.0f * float(PI) * kk : 0.0f, dadz = 0.0f;
+      if (lim_in < z) {
+        const float k0 = atan2f(2.0f * a_kite, fma2(kk - 1.0f, kk + 1.0f, z, z));
+        const float k1 = atan2f(2.0f * a_kite, fma2(1.0f - kk, 1.0f + kk, z, z));
+        dadk = 2.0f * kk * k0;
+        dadz = -2.0f * a_kite / z;
+        ar = __fsub_rn(fmaf(kk * kk, k0, k1), a_kite);
+      }
+      const float g = z * inv1pk;
+      const float gg = g * inv_dg;
       const int i = min(max((int)gg, 0), A.ng - 2);
-      const R fr = gg - (R)i;
-      const R l0 = L[i], l1 = L[i + 1];
-      const R ip = l0 + fr * (l1 - l0);
-      R dadk, dadz;
-      const R ar = ccia_star_grad<R>(kk, z, dadk, dadz);
-      const R gar = gsc * ar;
-      const R iz = R(1) / z;
-      const R dzdt = (x * xd + y * yd) * iz;
-      const R dIdg = (l1 - l0) * inv_dg;
-      const R gdz = gsc * (dIdg * inv1pk * ar + ip * dadz);   // gsc dQ/dz
-      acc[GS_KK] += gsc * (-dIdg * g * inv1pk * ar + ip * dadk);
-      acc[GS_KW] += (T[i] + fr * (T[i + 1] - T[i])) * gar;
+      const float fr = __fsub_rn(gg, (float)i);
+      const float l0 = L[i], l1 = L[i + 1];
+      const float ip = fmaf(fr, l1 - l0, l0);
+      const float gar = gsc * ar;
+      const float iz = 1.0f / z;
+      const float dzdt = fma2(x, xd, y, yd) * iz;
+      const float dIdg = (l1 - l0) * inv_dg;
+      const float gdz = gsc * fma2(ip, dadz, dIdg * inv1pk, ar);   // gsc dQ/dz
+      acc[GS_KK] = fmaf(gsc, fma2(ip, dadk, -dIdg * g * inv1pk, ar), acc[GS_KK]);
+      acc[GS_KW] = fmaf(fmaf(fr, T[i + 1] - T[i], T[i]), gar, acc[GS_KW]);
 #pragma unroll
       for (int j = 0; j < MAX_GRAD_PAR; ++j) {
         if (j < A.npar) {
-          const R* Tj = T + (size_t)(1 + j) * A.ng;
-          acc[GS_C0 + j] += (Tj[i] + fr * (Tj[i + 1] - Tj[i])) * gar;
+          const float* Tj = T + (size_t)(1 + j) * A.ng;
+          acc[GS_C0 + j] = fmaf(fmaf(fr, Tj[i + 1] - Tj[i], Tj[i]), gar, acc[GS_C0 + j]);
         }
       }
       // dz/dtheta: orbit coefficients (p, a, i, e, w) and the time shift of t0, p
-      acc[GS_T0] += gdz * (-dzdt);
+      acc[GS_T0] = fmaf(gdz, -dzdt, acc[GS_T0]);
 #pragma unroll
       for (int jj = 0; jj < 5; ++jj) {
-        const R* d = dcs + jj * 10;
-        R dx = d[4], dy = d[9];
+        const float4 da = *reinterpret_cast<const float4*>(dcs + jj * DC_ROW);
+        const float4 db = *reinterpret_cast<const float4*>(dcs + jj * DC_ROW + 4);
+        const float2 de = *reinterpret_cast<const float2*>(dcs + jj * DC_ROW + 8);
+        const float d[10] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w, de.x, de.y};
+        float dx = d[4], dy = d[9];
+#pragma unroll
         for (int m = 3; m >= 0; --m) {
-          dx = dx * t + d[m];
-          dy = dy * t + d[5 + m];
+          dx = fmaf(dx, t, d[m]);
+          dy = fmaf(dy, t, d[5 + m]);
         }
-        R dz = (x * dx + y * dy) * iz;
-        if (jj == 0) dz += dzdt * (-nep_count);
-        acc[GS_P + jj] += gdz * dz;
+        const float q = fma2(x, dx, y, dy);
+        const float dz = jj == 0 ? fma2(q, iz, dzdt, -n) : __fmul_rn(q, iz);
+        acc[GS_P + jj] = fmaf(gdz, dz, acc[GS_P + jj]);
       }
     }
     // the disk integral's dependence on the LD coefficients
-    const R* dI = A.dis + ppb * A.npar;
+    const float* dI = A.dis + ppb * A.npar;
 #pragma unroll
     for (int j = 0; j < MAX_GRAD_PAR; ++j)
-      if (j < A.npar) acc[GS_C0 + j] += (do_ + D) * w * D * inv_is * dI[j];
+      if (j < A.npar) acc[GS_C0 + j] = fmaf(r * w * D * inv_is, dI[j], acc[GS_C0 + j]);
   }
+  return true;
 }
 
 // Adds the accumulators of the lanes in `pending` to the warp's row of
 // shared FP64 sums, one group of lanes sharing a light curve at a time
 // (lowest lane first), each slot by the same shuffle tree; then clears them.
-// Every step is in a fixed order, so the sums are reproducible bit for bit.
-template <typename R, int NS>
-__device__ __forceinline__ void lnlike_flush(const GradArgs<R>& A, R* acc, int key, bool pending, double* row) {
+// Groups without a point in the box add nothing.  The tree sums FP32 (hi, lo)
+// pairs with error-free two-sums, as accurate as an FP64 tree; lane s keeps
+// slot s's pair, so that one FP64 addition serves all slots (one per slot, on
+// the pipe of 1/64 rate, held that pipe for a quarter of the adjoint's time).  Every step is
+// in a fixed order, so the sums are reproducible bit for bit.
+template <int NS>
+__device__ __forceinline__ void lnlike_flush(const GradArgs& A, float* acc, int key, bool pending, bool& dirty,
+                                             double* row) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int nsl = NS > 1 ? GS_C0 + A.npar : 1;
   unsigned pend = __ballot_sync(FULL, pending);
+  const unsigned live = __ballot_sync(FULL, dirty);
   while (pend) {
     const int leader = __ffs(pend) - 1;
     const int kl = __shfl_sync(FULL, key, leader);
     const unsigned mem = __ballot_sync(FULL, pending && key == kl) & pend;
+    pend &= ~mem;
+    if (!(mem & live)) continue;
     const bool in = (mem >> lane) & 1u;
-    const int pb = A.pbids[kl], ep = A.epids[kl];
+    float my_hi = 0.0f, my_lo = 0.0f;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       if (s >= nsl) break;
-      const int col = (s == GS_LNL) ? -1 : grad_col(s, A.nkc, A.nep, A.npar, pb, ep, s - GS_C0);
-      double tot;
-      if constexpr (sizeof(R) == 4) {
-        // FP32 (hi, lo) pairs summed with error-free two-sums: as accurate as
-        // an FP64 tree without the FP64 pipe (1/64 rate)
-        float hi = in ? acc[s] : 0.0f, lo = 0.0f;
-        for (int o = 16; o > 0; o >>= 1) {
-          const float h2 = __shfl_down_sync(FULL, hi, o), l2 = __shfl_down_sync(FULL, lo, o);
-          float sh, se;
-          two_sum(hi, h2, sh, se);
-          lo = lo + l2 + se;
-          hi = sh;
-        }
-        tot = (double)hi + (double)lo;
-      } else {
-        double vv = in ? (double)acc[s] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) vv += __shfl_down_sync(FULL, vv, o);
-        tot = vv;
+      float hi = in ? acc[s] : 0.0f, lo = 0.0f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float h2 = __shfl_down_sync(FULL, hi, o), l2 = __shfl_down_sync(FULL, lo, o);
+        float sh, se;
+        two_sum(hi, h2, sh, se);
+        lo = lo + l2 + se;
+        hi = sh;
       }
-      if (lane == 0) row[col + 1] += tot;
+      if (NS > 1) {
+        hi = __shfl_sync(FULL, hi, 0);
+        lo = __shfl_sync(FULL, lo, 0);
+      }
+      if (lane == s) { my_hi = hi; my_lo = lo; }
     }
+    if (lane < nsl) {
+      const int pb = A.pbids[kl], ep = A.epids[kl];
+      const int col = lane == GS_LNL ? -1 : grad_col(lane, A.nkc, A.nep, A.npar, pb, ep, lane - GS_C0);
+      const double tot = (double)my_hi + (double)my_lo;
+      if (lane != GS_KK && lane != GS_KW) row[col + 1] += tot;
+      // both slots of the radius ratio can share a column
+      __syncwarp((1u << nsl) - 1u);
+      if (lane == GS_KK) row[col + 1] += tot;
+      __syncwarp((1u << nsl) - 1u);
+      if (lane == GS_KW) row[col + 1] += tot;
+    }
+    __syncwarp();
     if (in) {
 #pragma unroll
-      for (int s = 0; s < NS; ++s) acc[s] = R(0);
+      for (int s = 0; s < NS; ++s) acc[s] = 0.0f;
+      dirty = false;
     }
-    pend &= ~mem;
   }
 }
 
@@ -448,40 +510,55 @@ __device__ __forceinline__ void lnlike_flush(const GradArgs<R>& A, R* acc, int k
 // depend on its passband and epoch), flushing to its warp's row of shared
 // sums when the light curve changes and at the end; the block writes the sum
 // of the warps' rows, in warp order, to its slot of partials.
-template <typename R, bool GRAD>
-__global__ void __launch_bounds__(LNL_THREADS, 4) lnlike_kernel(GradArgs<R> A) {
+//
+// Bound by instruction issue and, at few warps, by its latency.  With the orbit
+// coefficients' derivatives read from shared memory as 16-byte words for each
+// sample instead of held in 50 registers, 20 warps fit on an SM instead of 16.
+// Adjoint of 4096 pv x 5000 times x 5 samples: 887 us before, 890 with the FP64
+// additions and the second pass's separations alone taken out (registers
+// spilled), 819 with the coefficients out of the registers, 743 at 20 warps
+// (739 at 24, which spills and costs the likelihood alone 2 %: 242 us, not 238).
+template <bool GRAD>
+__global__ void __launch_bounds__(LNL_THREADS, 5) lnlike_kernel(const __grid_constant__ GradArgs A) {
   constexpr int NS = GRAD ? GS_NSLOT : 1;
   __shared__ double wred[LNL_NW][1 + MAX_NGRAD];
   __shared__ __align__(16) float lcs[GLC_SMEM * LC32];
-  __shared__ R orbc[10];
-  __shared__ R dcs[50];
+  __shared__ __align__(16) float orbc[18];   // c_m of x and y; m c_m (m = 1..4) of x and y
+  __shared__ __align__(16) float dcs[5 * DC_ROW];
+  __shared__ float4 stash[GRAD ? LNL_STASH * LNL_THREADS : 1];
   const int pv = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5;
   for (int i = tid; i < LNL_NW * (1 + MAX_NGRAD); i += blockDim.x) (&wred[0][0])[i] = 0.0;
-  if (tid < 10) orbc[tid] = (R)A.orb32[(size_t)pv * ORB32 + tid];
-  if (GRAD && tid < 50) dcs[tid] = A.dc[(size_t)pv * 50 + tid];
+  if (tid < 10) {
+    const float c = A.orb32[(size_t)pv * ORB32 + tid];
+    const int m = tid % 5;
+    orbc[tid] = c;
+    if (m > 0) orbc[10 + tid / 5 * 4 + m - 1] = __fmul_rn((float)m, c);
+  }
+  if (GRAD && tid < 50) dcs[tid / 10 * DC_ROW + tid % 10] = A.dc[(size_t)pv * 50 + tid];
   const bool lc_smem = A.nlc <= GLC_SMEM;
   if (lc_smem)
     for (int i = tid; i < A.nlc * LC32; i += blockDim.x) lcs[i] = A.lc32[(size_t)pv * A.nlc * LC32 + i];
   __syncthreads();
   const bool valid = __float_as_int(A.orb32[(size_t)pv * ORB32 + 14]) & FLAG_VALID;
-  R acc[NS];
+  float acc[NS];
 #pragma unroll
-  for (int s = 0; s < NS; ++s) acc[s] = R(0);
+  for (int s = 0; s < NS; ++s) acc[s] = 0.0f;
   int key = -1;
+  bool dirty = false;   // acc holds a point's terms
   for (int j = 0; j < LNL_PPT; ++j) {
     const int pt = blockIdx.x * LNL_CHUNK + j * LNL_THREADS + tid;
     const int lc = (valid && pt < A.npt) ? A.lcids[pt] : -1;
     const bool flush = key >= 0 && lc >= 0 && lc != key;
     if (__any_sync(0xffffffffu, flush)) {
-      lnlike_flush<R, NS>(A, acc, key, flush, wred[warp]);
+      lnlike_flush<NS>(A, acc, key, flush, dirty, wred[warp]);
       if (flush) key = -1;
     }
     if (lc < 0) continue;
-    lnlike_point<R, GRAD>(A, pv, pt, lc, lcs, lc_smem, orbc, dcs, acc);
+    dirty |= lnlike_point<GRAD>(A, pv, pt, lc, lcs, lc_smem, orbc, dcs, stash + (GRAD ? tid : 0), acc);
     key = lc;
   }
-  lnlike_flush<R, NS>(A, acc, key, key >= 0, wred[warp]);
+  lnlike_flush<NS>(A, acc, key, key >= 0, dirty, wred[warp]);
   __syncthreads();
   double* out = A.partials + ((size_t)pv * gridDim.x + blockIdx.x) * (1 + A.ngrad);
   for (int i = tid; i <= A.ngrad; i += blockDim.x) {
@@ -892,7 +969,7 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
   const int nobs = (npt + OBS_CHUNK - 1) / OBS_CHUNK;
   obs_kernel<R><<<nobs, OBS_THREADS, 0, s>>>(obs, sigma, lcids, npt, nlc, g.dobs, g.isig2, g.cconst, times, g.tiles64);
   if constexpr (sizeof(R) == 4) {
-    GradArgs<R> A{};
+    GradArgs A{};
     A.times_ff = reinterpret_cast<const float2*>(times_ff);
     A.lcids = lcids; A.pbids = pbids; A.epids = epids;
     A.dobs = g.dobs; A.isig2 = g.isig2; A.nkc = nkc; A.nep = nep;
@@ -901,8 +978,8 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
     A.npt = npt; A.npv = npv; A.npb = npb; A.nlc = nlc; A.ng = ng; A.npar = npar; A.ngrad = ngrad;
     A.dg = dg; A.partials = g.partials;
     const dim3 grid(nblk, npv);
-    if (grad) lnlike_kernel<R, true><<<grid, LNL_THREADS, 0, s>>>(A);
-    else lnlike_kernel<R, false><<<grid, LNL_THREADS, 0, s>>>(A);
+    if (grad) lnlike_kernel<true><<<grid, LNL_THREADS, 0, s>>>(A);
+    else lnlike_kernel<false><<<grid, LNL_THREADS, 0, s>>>(A);
   } else {
     LnlF64Args A{};
     A.times = times; A.k = k; A.t0 = t0; A.p = p; A.exptimes = exptimes; A.istar = (const double*)istar;
