@@ -56,6 +56,26 @@ __device__ inline float cci_kite_f32(float r1, float r2, float b) {
   return r1 * r1 * k1 + r2 * r2 * k0 - ak;
 }
 
+template <typename R> struct Word16;   // 16 bytes of R
+template <> struct Word16<float> {
+  using T = float4;
+  static __device__ __forceinline__ T lerp(float a0, const T& u, float a1, const T& v) {
+    return {fmaf(a0, u.x, a1 * v.x), fmaf(a0, u.y, a1 * v.y), fmaf(a0, u.z, a1 * v.z), fmaf(a0, u.w, a1 * v.w)};
+  }
+  static __device__ __forceinline__ void dot(float& d, const T& u, const T& v) {
+    d = fmaf(u.x, v.x, d); d = fmaf(u.y, v.y, d); d = fmaf(u.z, v.z, d); d = fmaf(u.w, v.w, d);
+  }
+};
+template <> struct Word16<double> {
+  using T = double2;
+  static __device__ __forceinline__ T lerp(double a0, const T& u, double a1, const T& v) {
+    return {fma(a0, u.x, a1 * v.x), fma(a0, u.y, a1 * v.y)};
+  }
+  static __device__ __forceinline__ void dot(double& d, const T& u, const T& v) {
+    d = fma(u.x, v.x, d); d = fma(u.y, v.y, d);
+  }
+};
+
 // Area of the overlap of the unit stellar disk and a planet of radius k at
 // separation z: circle_circle_intersection_area_kite(1, k, z), common.py:53-73
 // (Agol et al. 2020).  kappa0 receives the second return value.

@@ -14,7 +14,7 @@ namespace rr {
 
 constexpr int LDM_PBB = 4;      // passbands per block of the LD-means kernel
 constexpr int MAX_NZ = 64;      // radial grid points staged in shared memory
-constexpr int LDM_SCRATCH = 2048;   // FP64 areas of the 2D table per chunk of rows (FP32 tables)
+constexpr int LDM_SCRATCH = 512;   // FP64 areas of the 2D table per chunk of rows (FP32 tables)
 
 // ---------------------------------------------------------------------------
 // Limb-darkening means, model_full.py:43-55:
@@ -24,11 +24,20 @@ constexpr int LDM_SCRATCH = 2048;   // FP64 areas of the 2D table per chunk of r
 // would run past the table.  mode 1: the transmission-spectroscopy rule
 // kmin <= k <= kmax_pv[pv] (model_trspec.py:48); mode 2: always the 2D table.
 // One block per (pv, share of the passband groups): the k-interpolated weight
-// slab (or the 2D table, computed once per block) is staged in shared memory
-// with coalesced loads (rows padded to nz+1 words so the dot products are
-// free of bank conflicts), then the block walks its groups of LDM_PBB
-// passbands and every (pb, g) output is a dot product from shared memory:
-// ldm[pv][pb][g].
+// slab (or the 2D table, computed once per block) is staged in shared memory,
+// then the block walks its groups of LDM_PBB passbands and every (pb, g) output
+// is a dot product from shared memory: ldm[pv][pb][g].
+//
+// In FP32, with one passband, bound by the latency of the slab's loads, the issue
+// of their index arithmetic and the FP64 divisions that place k in the table.  So
+// where rows are whole 16-byte words (VEC: nz a multiple of 4 (FP32) or 2 (FP64),
+// W aligned) both go by words, four pairs of loads in flight and rows unpadded (at
+// nz = 40 a word-wise dot product meets two-way bank conflicts); else element by
+// element, rows padded to nz + 1.  The divisions are one warp's, and the scratch
+// of the 2D table is small, so that the shared memory leaves 9 blocks on an SM.
+// 4096 pv, ng = 100, nz = 40: 55.4 us by elements, 35.5 by words, 26.1 with
+// 4 KB of scratch instead of 16, 17.9 with one warp's divisions.  In FP64 the
+// pipe bounds it: 49 -> 39 us for 1500 pv.
 // ---------------------------------------------------------------------------
 // Byte offset of the FP64 scratch after the slab [ng][nz+1] and the LD
 // profiles [LDM_PBB][MAX_NZ] (8-byte aligned).
@@ -37,7 +46,7 @@ __host__ __device__ inline size_t ldm_scratch_offset(int ng, int nz) {
   return (sizeof(R) * ((size_t)ng * (nz + 1) + (size_t)LDM_PBB * MAX_NZ) + 7) & ~size_t(7);
 }
 
-template <typename R>
+template <typename R, bool VEC>
 __global__ void __launch_bounds__(128)
 ldm_kernel(const R* __restrict__ ldp, int npb, int nz, const double* __restrict__ kw, int kw_stride,
            const R* __restrict__ W, int nk, int ng, double dk, double kmin, double kmax,
@@ -45,36 +54,65 @@ ldm_kernel(const R* __restrict__ ldp, int npb, int nz, const double* __restrict_
            R* __restrict__ ldm) {
   extern __shared__ __align__(16) unsigned char ldm_smem[];
   R* Wk = reinterpret_cast<R*>(ldm_smem);                  // [ng][nz + 1]
-  R* l = Wk + (size_t)ng * (nz + 1);                       // [LDM_PBB][nz]
-  const int ldw = nz + 1;
+  using W16 = typename Word16<R>::T;
+  constexpr int PER = 16 / sizeof(R);
+  const int ldw = VEC ? nz : nz + 1;
+  R* l = Wk + (((size_t)ng * ldw + PER - 1) & ~size_t(PER - 1));   // [LDM_PBB][nz]
   const int pv = blockIdx.x;
 
+  // the block's place in the table, by one warp: FP64 divisions
+  __shared__ int s_ik;
+  __shared__ double s_ak;
   const double k = kw[(size_t)pv * kw_stride];
-  int ik = -1;
-  double ak = 0.0;
-  double kup = (mode == 1) ? kmax_pv[pv] : kmax;
-  if (mode != 2 && W != nullptr && kmin <= k && k <= kup) {
-    ik = (int)floor((k - kmin) / dk);
-    ak = (k - kmin - ik * dk) / dk;
-    if (ik + 1 >= nk || ik < 0) ik = -1;
+  if (threadIdx.x < 32) {
+    int ik = -1;
+    double ak = 0.0;
+    double kup = (mode == 1) ? kmax_pv[pv] : kmax;
+    if (mode != 2 && W != nullptr && kmin <= k && k <= kup) {
+      ik = (int)floor((k - kmin) / dk);
+      ak = (k - kmin - ik * dk) / dk;
+      if (ik + 1 >= nk || ik < 0) ik = -1;
+    }
+    if (threadIdx.x == 0) { s_ik = ik; s_ak = ak; }
   }
+  __syncthreads();
+  const int ik = s_ik;
   if (ik >= 0) {
+    const R ak = (R)s_ak;
     const R* W0 = W + (size_t)ik * ng * nz;
     const R* W1 = W0 + (size_t)ng * nz;
-    const R a1 = (R)ak, a0 = R(1) - (R)ak;
-    for (int i = threadIdx.x; i < ng * nz; i += blockDim.x)
-      Wk[(i / nz) * ldw + (i % nz)] = a0 * __ldg(W0 + i) + a1 * __ldg(W1 + i);
+    const R a1 = ak, a0 = R(1) - ak;
+    if constexpr (VEC) {
+      const W16 *V0 = reinterpret_cast<const W16*>(W0), *V1 = reinterpret_cast<const W16*>(W1);
+      W16* S = reinterpret_cast<W16*>(Wk);
+      const int n = ng * nz / PER;
+      for (int i0 = threadIdx.x; i0 < n; i0 += 4 * 128) {
+        W16 u[4], v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int i = min(i0 + q * 128, n - 1);
+          u[q] = __ldg(V0 + i);
+          v[q] = __ldg(V1 + i);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (i0 + q * 128 < n) S[i0 + q * 128] = Word16<R>::lerp(a0, u[q], a1, v[q]);
+      }
+    } else {
+      for (int i = threadIdx.x; i < ng * nz; i += blockDim.x)
+        Wk[(i / nz) * ldw + (i % nz)] = a0 * __ldg(W0 + i) + a1 * __ldg(W1 + i);
+    }
   } else {
     // 2D table at this k (calculate_weights_2d, common.py:153-185) in FP64:
     // the areas A(ze_z) at every (g, z) in parallel, then per row the
     // differences w_z = A(ze_z) - A(ze_{z-1}) and their sum, normalised.  The
     // areas go to the table itself (FP64) or, for an FP32 table, to an FP64
-    // scratch in chunks of rows.
+    // scratch in chunks of rows, each row's sum in the word after it.
     const double gstep = (1.0 - 1e-7) / (double)(ng - 1);
     double* A2 = (sizeof(R) == 8) ? reinterpret_cast<double*>(Wk)
                                   : reinterpret_cast<double*>(ldm_smem + ldm_scratch_offset<R>(ng, nz));
-    const int rows = (sizeof(R) == 8) ? ng : max(1, LDM_SCRATCH / nz);
-    const int lda = (sizeof(R) == 8) ? ldw : nz;
+    const int rows = (sizeof(R) == 8) ? ng : LDM_SCRATCH / (nz + 1);
+    const int lda = (sizeof(R) == 8) ? ldw : nz + 1;
     for (int g0 = 0; g0 < ng; g0 += rows) {
       const int nr = min(rows, ng - g0);
       for (int i = threadIdx.x; i < nr * nz; i += blockDim.x) {
@@ -84,15 +122,27 @@ ldm_kernel(const R* __restrict__ ldp, int npb, int nz, const double* __restrict_
       }
       __syncthreads();
       for (int rr = threadIdx.x; rr < nr; rr += blockDim.x) {
-        const double* a = A2 + (size_t)rr * lda;
-        R* row = Wk + (size_t)(g0 + rr) * ldw;
+        double* a = A2 + (size_t)rr * lda;
         double s = a[0];
         for (int z = 1; z < nz; ++z) s += a[z] - a[z - 1];
-        // in place for an FP64 table: walk down so a[z-1] is still the area
-        for (int z = nz - 1; z >= 1; --z) row[z] = (R)((a[z] - a[z - 1]) / s);
-        row[0] = (R)(a[0] / s);
+        if constexpr (sizeof(R) == 8) {
+          // in place: walk down so a[z-1] is still the area
+          R* row = Wk + (size_t)(g0 + rr) * ldw;
+          for (int z = nz - 1; z >= 1; --z) row[z] = (a[z] - a[z - 1]) / s;
+          row[0] = a[0] / s;
+        } else {
+          a[nz] = s;
+        }
       }
       __syncthreads();
+      if constexpr (sizeof(R) == 4) {
+        for (int i = threadIdx.x; i < nr * nz; i += blockDim.x) {
+          const int rr = i / nz, z = i % nz;
+          const double* a = A2 + (size_t)rr * lda;
+          Wk[(size_t)(g0 + rr) * ldw + z] = (R)((z ? a[z] - a[z - 1] : a[0]) / a[nz]);
+        }
+        __syncthreads();
+      }
     }
   }
   const int ngroups = (npb + LDM_PBB - 1) / LDM_PBB;
@@ -108,7 +158,13 @@ ldm_kernel(const R* __restrict__ ldp, int npb, int nz, const double* __restrict_
       const R* row = Wk + (size_t)g * ldw;
       const R* lb = l + b * nz;
       R d = R(0);
-      for (int z = 0; z < nz; ++z) d += row[z] * lb[z];
+      if constexpr (VEC) {
+        const W16 *rw = reinterpret_cast<const W16*>(row), *lw = reinterpret_cast<const W16*>(lb);
+#pragma unroll 5
+        for (int z = 0; z < nz / PER; ++z) Word16<R>::dot(d, rw[z], lw[z]);
+      } else {
+        for (int z = 0; z < nz; ++z) d += row[z] * lb[z];
+      }
       ldm[((size_t)pv * npb + pb0 + b) * ng + g] = d;
     }
   }
@@ -123,24 +179,19 @@ static dim3 ldm_grid(int npv, int npb, int mode) {
   return dim3(npv, (unsigned)std::max(1, std::min(ngroups, want)));
 }
 
-// Dynamic shared memory of ldm_kernel<R>; above the default 48 KB (large ng)
-// the kernel is opted in to the larger carve-out first.
-template <typename R>
-static size_t ldm_smem_bytes(int ng, int nz) {
-  const size_t scratch = (sizeof(R) == 8) ? 0 : sizeof(double) * LDM_SCRATCH;
-  const size_t bytes = ldm_scratch_offset<R>(ng, nz) + scratch;
-  if (bytes > 48 * 1024)
-    cudaFuncSetAttribute(ldm_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  return bytes;
-}
-
-// Host launchers of the LD-means kernel for the other translation units.
+// Host launcher of the LD-means kernel; dynamic shared memory above the default
+// 48 KB (large ng) opts in to the larger carve-out first.
 template <typename R>
 static void launch_ldm_impl(const R* ldp, int npv, int npb, int nz, const double* kw, int kw_stride, const R* W,
                             int nk, int ng, double dk, double kmin, double kmax, const double* ze, int mode,
                             const double* kmax_pv, R* ldm, cudaStream_t s) {
-  ldm_kernel<R><<<ldm_grid(npv, npb, mode), 128, ldm_smem_bytes<R>(ng, nz), s>>>(
-      ldp, npb, nz, kw, kw_stride, W, nk, ng, dk, kmin, kmax, ze, mode, kmax_pv, ldm);
+  const size_t scratch = (sizeof(R) == 8) ? 0 : sizeof(double) * LDM_SCRATCH;
+  const size_t bytes = ldm_scratch_offset<R>(ng, nz) + scratch;
+  const bool vec = W && nz % (16 / sizeof(R)) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
+  auto fn = vec ? ldm_kernel<R, true> : ldm_kernel<R, false>;
+  if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  fn<<<ldm_grid(npv, npb, mode), 128, bytes, s>>>(ldp, npb, nz, kw, kw_stride, W, nk, ng, dk, kmin, kmax, ze, mode,
+                                                  kmax_pv, ldm);
 }
 void launch_ldm_f32(const float* ldp, int npv, int npb, int nz, const double* kw, int kw_stride, const float* W,
                     int nk, int ng, double dk, double kmin, double kmax, const double* ze, int mode,
@@ -1520,8 +1571,7 @@ int rr_prepare_f64(const double* k, int nkc, const double* p, const double* a, c
     ldm_basis_kernel<double><<<npv, 128, sizeof(double) * npb * nb, s>>>(
         law, ldc, npar, npb, k, nkc, basis, nb, nk, ng, dk, kmin, kmax, ldp, nz, z_edges, ldm);
   } else {
-    ldm_kernel<double><<<ldm_grid(npv, npb, 0), 128, ldm_smem_bytes<double>(ng, nz), s>>>(
-        ldp, npb, nz, k, nkc, weights, nk, ng, dk, kmin, kmax, z_edges, 0, nullptr, ldm);
+    launch_ldm_impl<double>(ldp, npv, npb, nz, k, nkc, weights, nk, ng, dk, kmin, kmax, z_edges, 0, nullptr, ldm, s);
   }
   OrbitArgs oa{};
   oa.k = k; oa.p = p; oa.a = a; oa.inc = inc; oa.e = e; oa.w = w;
@@ -1632,8 +1682,7 @@ int rr_prepare_split(double t_ref, double t_absmax, const double* k, int nkc, co
     ldm_basis_kernel<float><<<npv, 128, sizeof(float) * npb * nb, s>>>(
         law, ldc, npar, npb, k, nkc, basis, nb, nk, ng, dk, kmin, kmax, ldp, nz, z_edges, t.ldm);
   } else {
-    ldm_kernel<float><<<ldm_grid(npv, npb, 0), 128, ldm_smem_bytes<float>(ng, nz), s>>>(
-        ldp, npb, nz, k, nkc, weights, nk, ng, dk, kmin, kmax, z_edges, 0, nullptr, t.ldm);
+    launch_ldm_impl<float>(ldp, npv, npb, nz, k, nkc, weights, nk, ng, dk, kmin, kmax, z_edges, 0, nullptr, t.ldm, s);
   }
   OrbitArgs oa{};
   oa.k = k; oa.t0 = t0; oa.p = p; oa.a = a; oa.inc = inc; oa.e = e; oa.w = w; oa.exptimes = exptimes;

@@ -24,6 +24,7 @@ namespace rr {
 
 constexpr int MAX_GRAD_PAR = 4;    // LD coefficients per passband in the adjoint
 constexpr int MAX_NGRAD = 64;      // nkc + nep + 5 + npb * npar
+constexpr size_t GLD_SMEM = 64 * 1024;   // weight slabs staged by the LD-table derivatives
 constexpr int GLC_SMEM = 64;       // light-curve records staged in shared memory (split)
 
 // Slots of one point's gradient contribution: destinations vary per point.
@@ -52,22 +53,63 @@ __global__ void grad_orbit_kernel(const double* __restrict__ p, const double* __
 //                central difference of the 2D table at k +- h;
 //   dL/dc_j[g] = Wk @ (d ldp / d c_j), Wk the table the forward pass uses;
 //   d istar / d c_j analytic, or the 200-point trapezoid of z dI/dc_j.
+// FP32 is bound by the reads of W: a thread's rows element by element from global
+// memory (95.5 us for 4096 pv, ng = 100, nz = 40), or, where rows are whole 16-byte
+// words and the two slabs fit (STAGE), staged by words in shared memory (65.3 us;
+// 51.2 with the FP64 divisions that place k in the table done by one warp).
 // tab layout per (pv, pb): [dL/dk (ng)][dL/dc_0 (ng)]...[dL/dc_{npar-1} (ng)],
 // dis layout: [d istar/dc_j] (npar).
 // ---------------------------------------------------------------------------
-template <typename R>
+template <typename R, bool STAGE>
 __global__ void __launch_bounds__(128)
 grad_ld_kernel(int law, const double* __restrict__ ldc, int npb, int npar, const double* __restrict__ mu,
                int nz, const R* __restrict__ ldp, const double* __restrict__ kw, int kw_stride,
                const R* __restrict__ W, int nk, int ng, double dk, double kmin, double kmax,
                const double* __restrict__ ze, R* __restrict__ tab, R* __restrict__ dis) {
-  __shared__ R l[64];
-  __shared__ R dl[MAX_GRAD_PAR][64];
+  extern __shared__ __align__(16) unsigned char gld_smem[];   // STAGE: the slabs of W at ik and ik + 1
+  __shared__ __align__(16) R l[64];
+  __shared__ __align__(16) R dl[MAX_GRAD_PAR][64];
   __shared__ R pvs[16];
   const int pv = blockIdx.x, pb = blockIdx.y;
   const size_t ppb = (size_t)pv * npb + pb;
+  // the block's place in the table, by one warp: FP64 divisions
+  __shared__ int s_ik;
+  __shared__ double s_ak;
+  const double k = kw[(size_t)pv * kw_stride];
+  if (threadIdx.x < 32) {
+    int ik = -1;
+    double ak = 0.0;
+    if (kmin <= k && k <= kmax) {
+      ik = (int)floor((k - kmin) / dk);
+      ak = (k - kmin - ik * dk) / dk;
+      if (ik + 1 >= nk || ik < 0) ik = -1;
+    }
+    if (threadIdx.x == 0) { s_ik = ik; s_ak = ak; }
+  }
   if (threadIdx.x < npar) pvs[threadIdx.x] = (R)ldc[ppb * npar + threadIdx.x];
   __syncthreads();
+  const int ik = s_ik;
+  const double ak = s_ak;
+  using W16 = typename Word16<R>::T;
+  constexpr int PER = 16 / sizeof(R);
+  const R* slab = nullptr;
+  if constexpr (STAGE) {
+    // the two slabs are consecutive: one stretch of 2 ng nz elements
+    W16* S = reinterpret_cast<W16*>(gld_smem);
+    slab = reinterpret_cast<const R*>(gld_smem);
+    if (ik >= 0) {
+      const W16* V = reinterpret_cast<const W16*>(W + (size_t)ik * ng * nz);
+      const int n = 2 * ng * nz / PER;
+      for (int i0 = threadIdx.x; i0 < n; i0 += 8 * 128) {
+        W16 v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = __ldg(V + min(i0 + q * 128, n - 1));
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (i0 + q * 128 < n) S[i0 + q * 128] = v[q];
+      }
+    }
+  }
   for (int z = threadIdx.x; z < nz; z += blockDim.x) {
     l[z] = ldp[ppb * nz + z];
     for (int j = 0; j < npar; ++j) dl[j][z] = ld_dvalue<R>(law, (R)mu[z], pvs, npar, j);
@@ -91,29 +133,39 @@ grad_ld_kernel(int law, const double* __restrict__ ldc, int npb, int npar, const
     dis[ppb * npar + j] = d;
   }
   __syncthreads();
-  const double k = kw[(size_t)pv * kw_stride];
-  int ik = -1;
-  double ak = 0.0;
-  if (kmin <= k && k <= kmax) {
-    ik = (int)floor((k - kmin) / dk);
-    ak = (k - kmin - ik * dk) / dk;
-    if (ik + 1 >= nk || ik < 0) ik = -1;
-  }
   R* out = tab + ppb * (size_t)(1 + npar) * ng;
   const double gstep = (1.0 - 1e-7) / (double)(ng - 1);
   for (int g = threadIdx.x; g < ng; g += blockDim.x) {
     if (ik >= 0) {
-      const R* w0 = W + ((size_t)ik * ng + g) * nz;
-      const R* w1 = w0 + (size_t)ng * nz;
       R d0 = R(0), d1 = R(0);
       R c0[MAX_GRAD_PAR] = {}, c1[MAX_GRAD_PAR] = {};
-      for (int z = 0; z < nz; ++z) {
-        const R a0 = __ldg(w0 + z), a1 = __ldg(w1 + z);
-        d0 += a0 * l[z];
-        d1 += a1 * l[z];
-        for (int j = 0; j < npar; ++j) {
-          c0[j] += a0 * dl[j][z];
-          c1[j] += a1 * dl[j][z];
+      if constexpr (STAGE) {
+        const W16 *w0 = reinterpret_cast<const W16*>(slab + (size_t)g * nz);
+        const W16 *w1 = reinterpret_cast<const W16*>(slab + (size_t)(ng + g) * nz);
+#pragma unroll 2
+        for (int z = 0; z < nz / PER; ++z) {
+          const W16 a0 = w0[z], a1 = w1[z], lz = reinterpret_cast<const W16*>(l)[z];
+          Word16<R>::dot(d0, a0, lz);
+          Word16<R>::dot(d1, a1, lz);
+#pragma unroll
+          for (int j = 0; j < MAX_GRAD_PAR; ++j)
+            if (j < npar) {
+              const W16 dz = reinterpret_cast<const W16*>(dl[j])[z];
+              Word16<R>::dot(c0[j], a0, dz);
+              Word16<R>::dot(c1[j], a1, dz);
+            }
+        }
+      } else {
+        const R* w0 = W + ((size_t)ik * ng + g) * nz;
+        const R* w1 = w0 + (size_t)ng * nz;
+        for (int z = 0; z < nz; ++z) {
+          const R a0 = __ldg(w0 + z), a1 = __ldg(w1 + z);
+          d0 += a0 * l[z];
+          d1 += a1 * l[z];
+          for (int j = 0; j < npar; ++j) {
+            c0[j] += a0 * dl[j][z];
+            c1[j] += a1 * dl[j][z];
+          }
         }
       }
       out[g] = (R)(((double)d1 - (double)d0) / dk);
@@ -963,8 +1015,13 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
   }
   if (grad) {   // the derivative tables, read by the adjoint alone
     grad_orbit_kernel<R><<<(npv + 63) / 64, 64, 0, s>>>(p, a, inc, e, w, npv, g.dc);
-    grad_ld_kernel<R><<<dim3(npv, npb), 128, 0, s>>>(law, ldc, npb, npar, mu, nz, ldp, k, nkc, weights, nk, ng, dk,
-                                                     kmin, kmax, z_edges, g.tab, g.dis);
+    // rows of whole 16-byte words, two slabs within what four blocks of an SM can have
+    const size_t slabs = 2 * sizeof(R) * (size_t)ng * nz;
+    const bool stage = nz % (16 / sizeof(R)) == 0 && (reinterpret_cast<uintptr_t>(weights) & 15) == 0 && slabs <= GLD_SMEM;
+    auto fn = stage ? grad_ld_kernel<R, true> : grad_ld_kernel<R, false>;
+    if (stage && slabs > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slabs);
+    fn<<<dim3(npv, npb), 128, stage ? slabs : 0, s>>>(law, ldc, npb, npar, mu, nz, ldp, k, nkc, weights, nk, ng, dk, kmin,
+                                                      kmax, z_edges, g.tab, g.dis);
   }
   const int nobs = (npt + OBS_CHUNK - 1) / OBS_CHUNK;
   obs_kernel<R><<<nobs, OBS_THREADS, 0, s>>>(obs, sigma, lcids, npt, nlc, g.dobs, g.isig2, g.cconst, times, g.tiles64);
