@@ -119,6 +119,15 @@ __device__ __forceinline__ bool f64_moderate(double d) {
   return (unsigned)__double2hiint(d) - ((1023u - 100u) << 20) < (200u << 20);
 }
 
+// FP32 of any double, rounded to nearest even as the conversion does.
+__device__ __forceinline__ float f32_near(double d) {
+  if (!f64_moderate(fabs(d))) return (float)d;
+  const unsigned long long u = __double_as_longlong(d);
+  const unsigned long long b = u + 0x0fffffffull + ((u >> 29) & 1u);   // a carry goes into the exponent
+  const unsigned hi = (unsigned)(b >> 32);
+  return __uint_as_float(__funnelshift_l((unsigned)b, (hi & 0x7fffffffu) - F64_BIAS, 3) | (hi & 0x80000000u));
+}
+
 // Square root of a moderate x and its reciprocal, from the FP32 reciprocal
 // root g: with e = 1 - x g^2 (|e| < 4e-7), 1/sqrt(x) = g (1 + e/2 + 3 e^2/8 +
 // O(e^3)), the quadratic term (below 1e-13) in FP32.

@@ -143,7 +143,8 @@ constexpr int TS_L2_ROWS = 16;   // g rows of the 2D table per LD block
 //   blocks [0, npv): per-pv blocks: mean and largest k, orbit, box, record;
 //   blocks [npv, ...): LD blocks (pv, chunk of TS_L2_ROWS rows, chunk of
 //     channels): the same k statistics (the same reduction, so the same
-//     bits), the channels' LD profiles (from the law's coefficients, or read
+//     bits; the split path's inner row chunks, which need the mean in FP32
+//     alone, sum it in FP32 pairs), the channels' LD profiles (from the law's coefficients, or read
 //     from ldp for a host-evaluated law) staged in shared memory, the 2D
 //     table rows at kmean, the LD means by 16-byte shared-memory loads; the
 //     blocks of the first row chunk also write the channel records (afac,
@@ -151,6 +152,9 @@ constexpr int TS_L2_ROWS = 16;   // g rows of the 2D table per LD block
 //     reference's 200-point trapezoid (rrmodel.py:222-227).
 // The orbit blocks come first in the grid, so their serial chains start at
 // once and the LD blocks fill the SMs around them.
+// The split path is bound by what is left in FP64: 64 pv x 200 channels 35.3 us
+// with the statistics, the step in g and every conversion of its inner row
+// chunks on that pipe, 27.1 us without.
 // ---------------------------------------------------------------------------
 constexpr int TSP_MAXPAR = 16;
 constexpr int MAX_BASIS_TS = 16;   // basis_coefs writes up to npar values
@@ -161,7 +165,7 @@ struct TsProArgs {
   const double *ldc, *mu, *ze;   // law >= 0: coefficients [npv, npb, npar] and the mu grid
   const R *ldp, *istar;          // law < 0: host-evaluated profiles and integrals
   int law, npar, npv, npb, nz, ng, nrc, ncc;
-  double exptime0, t_ref, t_absmax;
+  double exptime0, t_ref, t_absmax, gstep;   // gstep: the 2D table's step in g
   R *orb, *ch, *ldm;
 };
 
@@ -188,11 +192,29 @@ __device__ __forceinline__ void ts_kstats(const double* __restrict__ kp, int npb
   }
 }
 
+// Mean of pv's radius ratios in FP32: each warp's lanes sum their channels, and
+// the lanes' sums are added, as (sum, error) pairs.
+__device__ __forceinline__ float ts_kmean_f32(const double* __restrict__ kp, int npb) {
+  float sm = 0.0f, er = 0.0f, t, e;
+  for (int b = threadIdx.x & 31; b < npb; b += 32) {
+    two_sum(sm, f32_near(kp[b]), t, e);
+    sm = t;
+    er += e;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    two_sum(sm, __shfl_xor_sync(0xffffffffu, sm, o), t, e);
+    er += __shfl_xor_sync(0xffffffffu, er, o) + e;
+    sm = t;
+  }
+  return (sm + er) / (float)npb;
+}
+
 template <typename R, bool SPLIT>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 4) ts_prologue_kernel(TsProArgs<R> P) {
   __shared__ double s_sum[3], s_max[3];
   __shared__ __align__(16) R Wr[TS_L2_ROWS][64];
   __shared__ R s_mu[64];
+  __shared__ float s_ze[SPLIT ? 64 : 1];
   __shared__ R s_cf[128][TSP_MAXPAR + 1];   // each thread's channel coefficients (law >= 0)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int npb = P.npb, nz = P.nz, ng = P.ng;
@@ -277,14 +299,23 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 4) ts_prologue_kerne
   const double* kp = P.k + (size_t)pv * npb;
   if (P.law >= 0)   // a host-evaluated law (law < 0) passes no mu grid
     for (int i = tid; i < nz4; i += blockDim.x) s_mu[i] = i < nz ? (R)P.mu[i] : R(0);
-  ts_kstats(kp, npb, s_sum, s_max);
+  if (SPLIT && tid >= 64 && tid - 64 < nz) s_ze[tid - 64] = f32_near(P.ze[tid - 64]);
+  // FP64 mean: the channel records (first row chunk), the grazing last row
+  const bool exact = !SPLIT || rc == 0 || rc == P.nrc - 1;
+  double k = 0.0;
+  float kf = 0.0f;
+  if (exact) ts_kstats(kp, npb, s_sum, s_max);
+  else kf = ts_kmean_f32(kp, npb);
   __syncthreads();
-  const double k = ((s_sum[0] + s_sum[1]) + s_sum[2]) / npb;
+  if (exact) {
+    k = ((s_sum[0] + s_sum[1]) + s_sum[2]) / npb;
+    kf = (float)k;
+  }
   // the 2D table rows at kmean (calculate_weights_2d, common.py:153-185): a
   // warp per row, lanes over z (z and z + 32), the differences through
   // shuffles, the row sum by a shuffle tree
-  const double gstep = (1.0 - 1e-7) / (double)(ng - 1);
-  const float kf = (float)k, gstep_f = (float)gstep, opk_f = (float)(1.0 + k);
+  const double gstep = P.gstep;
+  const float gstep_f = (float)gstep, opk_f = 1.0f + kf;
   for (int r = warp; r < nr; r += blockDim.x >> 5) {
     const int g = g0 + r;
     const bool f64 = !SPLIT || g == ng - 1;   // the split path's grazing last row: FP64 areas
@@ -293,7 +324,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 4) ts_prologue_kerne
       float af[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h)
-        af[h] = cci_kite_f32((float)P.ze[min(lane + 32 * h, nz - 1)], kf, (float)g * gstep_f * opk_f);
+        af[h] = cci_kite_f32(s_ze[min(lane + 32 * h, nz - 1)], kf, (float)g * gstep_f * opk_f);
       const float q0 = __shfl_up_sync(0xffffffffu, af[0], 1), q1 = __shfl_up_sync(0xffffffffu, af[1], 1);
       const float l0 = __shfl_sync(0xffffffffu, af[0], 31);
       const float df0 = lane == 0 ? af[0] : af[0] - q0;
@@ -308,6 +339,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 4) ts_prologue_kerne
         continue;
       }
       // a row left without area in FP32: the FP64 path below
+      if (!exact) k = (double)kf;
     }
     const double gg = (g == ng - 1) ? 1.0 - 1e-7 : (double)g * gstep;
     double av[2];
@@ -400,7 +432,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 4) ts_prologue_kerne
     R* cf = s_cf[tid];
     if (P.law >= 0) {
       const double* src = P.ldc + ((size_t)pv * npb + b) * P.npar;
-      for (int q = 0; q < P.npar; ++q) cf[q] = (R)src[q];
+      for (int q = 0; q < P.npar; ++q) cf[q] = sizeof(R) == 4 ? (R)f32_near(src[q]) : (R)src[q];
     }
     if (rc == 0) {
       R is;
@@ -713,7 +745,7 @@ static int ts_prepare_impl(double t_ref, double t_absmax, const double* k, const
     // are cheap to repeat); the plain path computes its FP64 areas once per
     // row chunk and loops over all channels in the block
     P.ncc = SPLIT ? (npb + 127) / 128 : 1;
-    P.exptime0 = exptime0; P.t_ref = t_ref; P.t_absmax = t_absmax;
+    P.exptime0 = exptime0; P.t_ref = t_ref; P.t_absmax = t_absmax; P.gstep = (1.0 - 1e-7) / (double)(ng - 1);
     P.orb = orb; P.ch = ch; P.ldm = ldm;
     if constexpr (!SPLIT) {
       // an affine law with a few basis functions, and channels enough that the
