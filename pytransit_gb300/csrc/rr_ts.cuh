@@ -136,6 +136,15 @@ __device__ __forceinline__ void ts_store4(double* dst, double a, double b, doubl
   __stcs(reinterpret_cast<double2*>(dst) + 1, make_double2(c, d));
 }
 
+__device__ __forceinline__ void ts_load4(const float* src, float* v) {   // 16-byte aligned
+  const float4 x = *reinterpret_cast<const float4*>(src);
+  v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+}
+__device__ __forceinline__ void ts_load4(const double* src, double* v) {
+  const double2 x = *reinterpret_cast<const double2*>(src), y = *(reinterpret_cast<const double2*>(src) + 1);
+  v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+}
+
 // The tile `tile` of parameter vector pv (record o, in shared or global
 // memory), by every thread of the block (blockDim.x a multiple of 32, at
 // least TS_TILE); every branch around a barrier is block-uniform.  A tile that
@@ -173,9 +182,12 @@ __device__ __forceinline__ void ts_tile(const TsArgs<R>& A, int pv, int tile, co
       int nrow = 0, jlo = 0;
       const int pt = pt0 + tid;
       if (tid < TS_TILE) {
-        // rows 0 and 1 are read for every point by the two-row path of phase 2
+        // read for every point by phase 2: rows 0 and 1 by its two-row path, with
+        // several samples any up to the largest of the tile by the other
+        const int nz = A.nsamples0 > 1 ? TS_MW : 2;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) S.w[k][0][tid] = S.w[k][1][tid] = R(0);
+        for (int k = 0; k < 3; ++k)
+          for (int j = 0; j < nz; ++j) S.w[k][j][tid] = R(0);
       }
       if (tid < TS_TILE && pt < npt) {
         const double tz = SPLIT ? 0.0 : A.t0[pv], pp = SPLIT ? 0.0 : A.p[pv];
@@ -211,7 +223,6 @@ __device__ __forceinline__ void ts_tile(const TsArgs<R>& A, int pv, int tile, co
           // (a row outside the window of pass 1, possible only through a
           // different rounding of z, sends the point to the warp path)
           if (nwin > 0 && !wide) {
-            for (int j = 2; j < nwin; ++j) S.w[0][j][tid] = S.w[1][j][tid] = S.w[2][j][tid] = R(0);
             for (int s = 0; s < ns; ++s) {
               const R t = tc + ex * ((R(s) + R(0.5)) * inv_ns - R(0.5));
               R a, dadk, fr;
@@ -327,33 +338,60 @@ __device__ __forceinline__ void ts_tile(const TsArgs<R>& A, int pv, int tile, co
       }
     }
   } else {
-    const int mrow = max(max(nr[0], nr[1]), max(nr[2], nr[3]));
-    for (int b = warp; b < npb; b += nwarps) {
-      const R* cr = ch_pv + (size_t)b * TS_CH;
-      const R afac = __ldg(cr), dkb = __ldg(cr + 1), scale = __ldg(cr + 2) * inv_ns;
-      const R* Lb = ldm_pv + (size_t)b * ng;
-      R acc[4];
+    // A point's row count differs from its neighbours': rows past it have zero
+    // weights and are not read, without a branch, so that the loads of two rows
+    // and U channels are in flight together.  (With a branch per point and row,
+    // one load after the other: 107.5 us for 100 pv x 200 channels x 1203 times x 5
+    // samples; 46.4 us so.)
+    constexpr int U = sizeof(R) == 4 ? 2 : 1;
+    const int mrow = __reduce_max_sync(FULL, max(max(nr[0], nr[1]), max(nr[2], nr[3])));
+    for (int b = warp; b < npb; b += U * nwarps) {
+      R cf[U][3], acc[U][4];
+      const R* Lb[U];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] = R(0);
-      for (int j = 0; j < mrow; ++j) {
+      for (int u = 0; u < U; ++u) {
+        const int bc = min(b + u * nwarps, npb - 1);
+        const R* cr = ch_pv + (size_t)bc * TS_CH;
+        cf[u][0] = __ldg(cr);
+        cf[u][1] = __ldg(cr + 1);
+        cf[u][2] = __ldg(cr + 2) * inv_ns;
+        Lb[u] = ldm_pv + (size_t)bc * ng;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (j < nr[q]) {
-            const R l = __ldg(Lb + jl[q] + j);
-            acc[q] += l * (afac * S.w[0][j][4 * lane + q] + S.w[1][j][4 * lane + q] +
-                           dkb * S.w[2][j][4 * lane + q]);
-          }
+        for (int q = 0; q < 4; ++q) acc[u][q] = R(0);
+      }
+      for (int j = 0; j < mrow; j += 2) {
+        R l[U][2][4];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) l[u][h][q] = j + h < nr[q] ? __ldg(Lb[u] + (jl[q] + j + h)) : R(0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          R w[3][4];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) ts_load4(&S.w[k][j + h][4 * lane], w[k]);
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              acc[u][q] += l[u][h][q] * (cf[u][0] * w[0][q] + w[1][q] + cf[u][1] * w[2][q]);
         }
       }
-      R v[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = nr[q] > 0 ? R(1) - acc[q] * scale : R(1);   // out of box: exactly 1
-      R* dst = fpv + (size_t)b * A.ldflux + p0;
-      if (vec) {
-        ts_store4(dst, v[0], v[1], v[2], v[3]);
-      } else {
-        for (int q = 0; q < 4; ++q)
-          if (p0 + q < npt) dst[q] = v[q];
+      for (int u = 0; u < U; ++u) {
+        if (u > 0 && b + u * nwarps >= npb) break;
+        R v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = nr[q] > 0 ? R(1) - acc[u][q] * cf[u][2] : R(1);   // out of box: exactly 1
+        R* dst = fpv + (size_t)(b + u * nwarps) * A.ldflux + p0;
+        if (vec) {
+          ts_store4(dst, v[0], v[1], v[2], v[3]);
+        } else {
+          for (int q = 0; q < 4; ++q)
+            if (p0 + q < npt) dst[q] = v[q];
+        }
       }
     }
   }
