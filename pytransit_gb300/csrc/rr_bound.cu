@@ -41,6 +41,7 @@ struct BoundArgs {
   const double *p, *a, *inc, *e, *w;
   const float *orb, *lc, *ldm;   // split RR: orb32 [npv][ORB32], lc32 [npv][nlc][LC32]; TS: orb [npv][TS_ORB], ch [npv][npb][TS_CH]
   int npv, npb, nlc, ng, ts, nsamples0;
+  int share;                     // warps of a block that share a pv
   double dg, exptime0;
   double* bound;                 // [npv]
   unsigned long long* bound_max; // max over pv (bits of a non-negative double), zeroed by the caller
@@ -72,14 +73,19 @@ constexpr float BOUND_SAFETY = 1.0f + 1e-4f;
 // part of each z error, one lane of warp 0 per pv, so that every FP64
 // instruction serves up to 32 pvs (the FP64 pipe is the scarce one); then a
 // warp per pv over the LD-table rows.  RoadRunner populations take 32 pvs a
-// block; transmission-spectroscopy ones, with every channel on every row,
-// take 4, which spreads few pvs over more SMs.
+// block, of a warp each.  In transmission spectroscopy, with every channel on
+// every row, several warps share a pv's channels (a maximum: the same value in any
+// order): 8, at 4 pvs a block, or all 32 while 4 pvs a block leave SMs idle, when
+// the latency of the channel loop bounds the kernel (32 pv x 200 channels: 244 us
+// with a warp per pv, 41 with 8, 29 with 32).
 constexpr int BOUND_PV_MAX = 32;
 
 __global__ void __launch_bounds__(BOUND_PV_MAX * 32) error_bound_kernel(BoundArgs B) {
   __shared__ double s_dz[BOUND_PV_MAX];
+  __shared__ float s_worst[BOUND_PV_MAX];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int npb_blk = blockDim.x >> 5;   // pvs of this block
+  const int share = B.share;                            // warps of a pv
+  const int npb_blk = (int)(blockDim.x >> 5) / share;   // pvs of this block
   const int pv0 = blockIdx.x * npb_blk;
   const unsigned FULL = 0xffffffffu;
   if (warp == 0) {
@@ -112,9 +118,9 @@ __global__ void __launch_bounds__(BOUND_PV_MAX * 32) error_bound_kernel(BoundArg
   const int ng = B.ng;
   const float dg = (float)B.dg;
   {
-    const int i = warp;
+    const int i = warp / share, part = warp % share;
     const int pv = pv0 + i;
-    if (pv >= B.npv) return;   // warp-uniform
+    if (!B.ts && pv >= B.npv) return;   // warp-uniform
     float worst = 0.0f;
     if (!B.ts) {
       const float* o = B.orb + (size_t)pv * ORB32;
@@ -143,7 +149,7 @@ __global__ void __launch_bounds__(BOUND_PV_MAX * 32) error_bound_kernel(BoundArg
           }
         }
       }
-    } else {
+    } else if (pv < B.npv) {
       const float* o = B.orb + (size_t)pv * TS_ORB;
       const bool valid = o[15] != 0.0f;
       if (valid) {
@@ -167,8 +173,8 @@ __global__ void __launch_bounds__(BOUND_PV_MAX * 32) error_bound_kernel(BoundArg
           float kap;
           const float A0 = ccia_star<float>(km, (float)j * gz, kap);
           const float rj = 3.0f * u * (float)(j + 1);
-          const float* L = B.ldm + (size_t)pv * B.npb * ng + j;
-          for (int b = 0; b < B.npb; ++b, L += ng) {
+          const float* L = B.ldm + ((size_t)pv * B.npb + part) * ng + j;
+          for (int b = part; b < B.npb; b += share, L += (size_t)share * ng) {
             const float afac = ch[b * TS_CH], dk = fabsf(ch[b * TS_CH + 1]), inv_is = fabsf(ch[b * TS_CH + 2]);
             if (!isfinite(inv_is)) continue;
             const float kb = km * sqrtf(afac);
@@ -183,6 +189,12 @@ __global__ void __launch_bounds__(BOUND_PV_MAX * 32) error_bound_kernel(BoundArg
       }
     }
     for (int off = 16; off > 0; off >>= 1) worst = fmaxf(worst, __shfl_xor_sync(FULL, worst, off));
+    if (B.ts) {   // block-uniform
+      if (lane == 0) s_worst[warp] = worst;
+      __syncthreads();
+      if (part != 0 || pv >= B.npv) return;
+      for (int q = 1; q < share; ++q) worst = fmaxf(worst, s_worst[warp + q]);
+    }
     if (lane == 0) {
       const double bnd = worst > 0.0f ? (double)(worst * BOUND_SAFETY) + BOUND_U : 0.0;
       B.bound[pv] = bnd;
@@ -202,9 +214,10 @@ static int launch_bounds(BoundArgs& B, void* stream) {
     }
   }
   if (B.npv == 0) return RR_OK;
-  const int per = B.ts ? 4 : BOUND_PV_MAX;
+  const int per = !B.ts ? BOUND_PV_MAX : (B.npv >= 4 * sm_count() ? 4 : 1);
+  B.share = B.ts ? BOUND_PV_MAX / per : 1;
   const unsigned nblk = (unsigned)((B.npv + per - 1) / per);
-  error_bound_kernel<<<nblk, per * 32, 0, s>>>(B);
+  error_bound_kernel<<<nblk, BOUND_PV_MAX * 32, 0, s>>>(B);
   return check_launch("rr_error_bounds");
 }
 
