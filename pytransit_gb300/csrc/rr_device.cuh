@@ -56,6 +56,16 @@ __device__ inline float cci_kite_f32(float r1, float r2, float b) {
   return r1 * r1 * k1 + r2 * r2 * k0 - ak;
 }
 
+// Overlap of the small kernels that prepare a call (each bound by latency and
+// independent of the others): every one of them lets the next start as soon as
+// its own blocks have, and one thread of a kernel started that way (launch_overlap)
+// waits, when its own work is done, for the kernel before, so that the last one's
+// end is the end of all.  Neither does anything in an ordinary launch.
+__device__ __forceinline__ void overlap_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void overlap_end() {
+  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <typename R> struct Word16;   // 16 bytes of R
 template <> struct Word16<float> {
   using T = float4;

@@ -172,6 +172,45 @@ __device__ __forceinline__ double f64_floor_div(double a, double b, float inv_b)
   return floor(__ddiv_rn(a, b));
 }
 
+// FP64 of any FP32 value, on the integer pipe where it is a normal one.
+__device__ __forceinline__ double f64_of_f32(float f) {
+  const unsigned e = (__float_as_uint(f) >> 23) & 0xffu;
+  return e - 1u < 254u ? f64_of(f) : (double)f;
+}
+
+// FP32 of the FP64 quotient a / b (rounded to FP64, then to FP32), from the product
+// with inv_b = 1 / b, whose error is below two units in the last place: the
+// division itself only where the product comes within 8 of the middle of two FP32
+// values.
+__device__ __forceinline__ float f32_quotient(double a, double b, double inv_b) {
+  const double q = __dmul_rn(a, inv_b);
+  const unsigned tail = (unsigned)__double2loint(q) & 0x1fffffffu;
+  if (f64_moderate(fabs(q)) && tail - (0x10000000u - 8u) > 16u) return f32_near(q);
+  return (float)__ddiv_rn(a, b);
+}
+
+// A radius ratio's place in the weight table: rows ik and ik + 1, the second's
+// share ak (ik = -1: past the table's end).
+__device__ __forceinline__ void table_place(double k, double kmin, double dk, double, int nk, int& ik, double& ak) {
+  ik = (int)floor((k - kmin) / dk);
+  ak = (k - kmin - ik * dk) / dk;
+  if (ik + 1 >= nk || ik < 0) ik = -1;
+}
+__device__ __forceinline__ void table_place(double k, double kmin, double dk, double inv_dk, int nk, int& ik, float& ak) {
+  const double x = __dsub_rn(k, kmin);
+  float n;
+  double nd;
+  if (f64_floor_sure(f32_of(x) * f32_of(inv_dk), n)) {
+    nd = f64_int(n);
+  } else {
+    nd = floor(__ddiv_rn(x, dk));
+    n = (float)nd;
+  }
+  ik = (int)n;
+  ak = f32_quotient(__fma_rn(-nd, dk, x), dk, inv_dk);
+  if (ik + 1 >= nk || ik < 0) ik = -1;
+}
+
 // ---------------------------------------------------------------------------
 // Outer contact times for the bounding box, by the FP32 bisection
 // (contact_points14_f32) on the rounded coefficients.  The box decides only

@@ -36,8 +36,8 @@ constexpr int LDM_SCRATCH = 512;   // FP64 areas of the 2D table per chunk of ro
 // element, rows padded to nz + 1.  The divisions are one warp's, and the scratch
 // of the 2D table is small, so that the shared memory leaves 9 blocks on an SM.
 // 4096 pv, ng = 100, nz = 40: 55.4 us by elements, 35.5 by words, 26.1 with
-// 4 KB of scratch instead of 16, 17.9 with one warp's divisions.  In FP64 the
-// pipe bounds it: 49 -> 39 us for 1500 pv.
+// 4 KB of scratch instead of 16, 17.9 with one warp's divisions, 15.5 with products
+// in their place.  In FP64 the pipe bounds it: 49 -> 39 us for 1500 pv.
 // ---------------------------------------------------------------------------
 // Byte offset of the FP64 scratch after the slab [ng][nz+1] and the LD
 // profiles [LDM_PBB][MAX_NZ] (8-byte aligned).
@@ -49,7 +49,7 @@ __host__ __device__ inline size_t ldm_scratch_offset(int ng, int nz) {
 template <typename R, bool VEC>
 __global__ void __launch_bounds__(128)
 ldm_kernel(const R* __restrict__ ldp, int npb, int nz, const double* __restrict__ kw, int kw_stride,
-           const R* __restrict__ W, int nk, int ng, double dk, double kmin, double kmax,
+           const R* __restrict__ W, int nk, int ng, double dk, double inv_dk, double kmin, double kmax,
            const double* __restrict__ ze, int mode, const double* __restrict__ kmax_pv,
            R* __restrict__ ldm) {
   extern __shared__ __align__(16) unsigned char ldm_smem[];
@@ -60,25 +60,22 @@ ldm_kernel(const R* __restrict__ ldp, int npb, int nz, const double* __restrict_
   R* l = Wk + (((size_t)ng * ldw + PER - 1) & ~size_t(PER - 1));   // [LDM_PBB][nz]
   const int pv = blockIdx.x;
 
-  // the block's place in the table, by one warp: FP64 divisions
+  overlap_next();
+  // the block's place in the table, by one warp: FP64 work
   __shared__ int s_ik;
-  __shared__ double s_ak;
+  __shared__ R s_ak;
   const double k = kw[(size_t)pv * kw_stride];
   if (threadIdx.x < 32) {
     int ik = -1;
-    double ak = 0.0;
+    R ak = R(0);
     double kup = (mode == 1) ? kmax_pv[pv] : kmax;
-    if (mode != 2 && W != nullptr && kmin <= k && k <= kup) {
-      ik = (int)floor((k - kmin) / dk);
-      ak = (k - kmin - ik * dk) / dk;
-      if (ik + 1 >= nk || ik < 0) ik = -1;
-    }
+    if (mode != 2 && W != nullptr && kmin <= k && k <= kup) table_place(k, kmin, dk, inv_dk, nk, ik, ak);
     if (threadIdx.x == 0) { s_ik = ik; s_ak = ak; }
   }
   __syncthreads();
   const int ik = s_ik;
   if (ik >= 0) {
-    const R ak = (R)s_ak;
+    const R ak = s_ak;
     const R* W0 = W + (size_t)ik * ng * nz;
     const R* W1 = W0 + (size_t)ng * nz;
     const R a1 = ak, a0 = R(1) - ak;
@@ -168,6 +165,7 @@ ldm_kernel(const R* __restrict__ ldp, int npb, int nz, const double* __restrict_
       ldm[((size_t)pv * npb + pb0 + b) * ng + g] = d;
     }
   }
+  overlap_end();
 }
 
 // Blocks per pv of the LD-means kernel: the 2D table (mode 2) is costly FP64
@@ -184,14 +182,18 @@ static dim3 ldm_grid(int npv, int npb, int mode) {
 template <typename R>
 static void launch_ldm_impl(const R* ldp, int npv, int npb, int nz, const double* kw, int kw_stride, const R* W,
                             int nk, int ng, double dk, double kmin, double kmax, const double* ze, int mode,
-                            const double* kmax_pv, R* ldm, cudaStream_t s) {
+                            const double* kmax_pv, R* ldm, cudaStream_t s, bool overlap = false) {
   const size_t scratch = (sizeof(R) == 8) ? 0 : sizeof(double) * LDM_SCRATCH;
   const size_t bytes = ldm_scratch_offset<R>(ng, nz) + scratch;
   const bool vec = W && nz % (16 / sizeof(R)) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
   auto fn = vec ? ldm_kernel<R, true> : ldm_kernel<R, false>;
   if (bytes > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  fn<<<ldm_grid(npv, npb, mode), 128, bytes, s>>>(ldp, npb, nz, kw, kw_stride, W, nk, ng, dk, kmin, kmax, ze, mode,
-                                                  kmax_pv, ldm);
+  if (overlap)
+    launch_overlap(fn, ldm_grid(npv, npb, mode), 128, bytes, s, ldp, npb, nz, kw, kw_stride, W, nk, ng, dk, 1.0 / dk, kmin, kmax,
+                   ze, mode, kmax_pv, ldm);
+  else
+    fn<<<ldm_grid(npv, npb, mode), 128, bytes, s>>>(ldp, npb, nz, kw, kw_stride, W, nk, ng, dk, 1.0 / dk, kmin, kmax, ze, mode,
+                                                    kmax_pv, ldm);
 }
 void launch_ldm_f32(const float* ldp, int npv, int npb, int nz, const double* kw, int kw_stride, const float* W,
                     int nk, int ng, double dk, double kmin, double kmax, const double* ze, int mode,
@@ -270,6 +272,7 @@ ldm_basis_kernel(int law, const double* __restrict__ ldc, int npar, int npb, con
   __shared__ int s_ik;
   __shared__ double s_ak;
   const int pv = blockIdx.x;
+  overlap_next();
   if (threadIdx.x == 0) {
     const double k = kw[(size_t)pv * kw_stride];
     int ik = -1;
@@ -308,6 +311,7 @@ ldm_basis_kernel(int law, const double* __restrict__ ldc, int npar, int npb, con
     for (int g = threadIdx.x; g < ng; g += blockDim.x)
       ldm_direct_g(k, g, ng, nz, ze, ldp + (size_t)pv * npb * nz, npb, out);
   }
+  overlap_end();
 }
 
 // ---------------------------------------------------------------------------
@@ -474,6 +478,7 @@ __device__ __forceinline__ void orbit_pv(const OrbitArgs& A, int pv) {
 
 template <bool SPLIT>
 __global__ void orbit_kernel(OrbitArgs A) {
+  overlap_next();
   const int pv = blockIdx.x * blockDim.x + threadIdx.x;
   if (pv < A.npv) orbit_pv<SPLIT>(A, pv);
 }
@@ -1567,17 +1572,19 @@ int rr_prepare_f64(const double* k, int nkc, const double* p, const double* a, c
   Carve cv(workspace);
   double* orb = cv.take<double>((size_t)npv * ORB64);
   double* ldm = cv.take<double>((size_t)npv * npb * ng);
-  if (basis && nb > 0 && nb <= MAX_BASIS && ldc) {
-    ldm_basis_kernel<double><<<npv, 128, sizeof(double) * npb * nb, s>>>(
-        law, ldc, npar, npb, k, nkc, basis, nb, nk, ng, dk, kmin, kmax, ldp, nz, z_edges, ldm);
-  } else {
-    launch_ldm_impl<double>(ldp, npv, npb, nz, k, nkc, weights, nk, ng, dk, kmin, kmax, z_edges, 0, nullptr, ldm, s);
-  }
   OrbitArgs oa{};
   oa.k = k; oa.p = p; oa.a = a; oa.inc = inc; oa.e = e; oa.w = w;
   oa.nkc = nkc; oa.npv = npv; oa.npb = npb; oa.nz = nz;
   oa.ldp = ldp; oa.ldp_is_f32 = 0; oa.orb64 = orb;
   orbit_kernel<false><<<(npv + 31) / 32, 32, 0, s>>>(oa);
+  // beside the orbits' chains
+  if (basis && nb > 0 && nb <= MAX_BASIS && ldc) {
+    launch_overlap(ldm_basis_kernel<double>, npv, 128, sizeof(double) * npb * nb, s, law, ldc, npar, npb, k, nkc, basis, nb,
+                   nk, ng, dk, kmin, kmax, ldp, nz, z_edges, ldm);
+  } else {
+    launch_ldm_impl<double>(ldp, npv, npb, nz, k, nkc, weights, nk, ng, dk, kmin, kmax, z_edges, 0, nullptr, ldm, s,
+                            true);
+  }
   return check_launch("rr_prepare_f64");
 }
 
@@ -1678,12 +1685,6 @@ int rr_prepare_split(double t_ref, double t_absmax, const double* k, int nkc, co
   if (workspace_bytes < rr_full_split_workspace_bytes(npv, npb, nlc, nep, ng)) return RR_ERR_WORKSPACE;
   cudaStream_t s = as_stream(stream);
   SplitTables t = carve_split(workspace, npv, npb, nlc, ng);
-  if (basis && nb > 0 && nb <= MAX_BASIS && ldc) {
-    ldm_basis_kernel<float><<<npv, 128, sizeof(float) * npb * nb, s>>>(
-        law, ldc, npar, npb, k, nkc, basis, nb, nk, ng, dk, kmin, kmax, ldp, nz, z_edges, t.ldm);
-  } else {
-    launch_ldm_impl<float>(ldp, npv, npb, nz, k, nkc, weights, nk, ng, dk, kmin, kmax, z_edges, 0, nullptr, t.ldm, s);
-  }
   OrbitArgs oa{};
   oa.k = k; oa.t0 = t0; oa.p = p; oa.a = a; oa.inc = inc; oa.e = e; oa.w = w; oa.exptimes = exptimes;
   oa.pbids = pbids; oa.epids = epids; oa.nsamples = nsamples;
@@ -1691,6 +1692,14 @@ int rr_prepare_split(double t_ref, double t_absmax, const double* k, int nkc, co
   oa.ldp = ldp; oa.ldp_is_f32 = 1; oa.orb32 = t.orb; oa.lc32 = t.lc;
   oa.istar32 = istar; oa.t_ref = t_ref; oa.t_absmax = t_absmax;
   orbit_kernel<true><<<(npv + 31) / 32, 32, 0, s>>>(oa);
+  // beside the orbits' chains
+  if (basis && nb > 0 && nb <= MAX_BASIS && ldc) {
+    launch_overlap(ldm_basis_kernel<float>, npv, 128, sizeof(float) * npb * nb, s, law, ldc, npar, npb, k, nkc, basis, nb,
+                   nk, ng, dk, kmin, kmax, ldp, nz, z_edges, t.ldm);
+  } else {
+    launch_ldm_impl<float>(ldp, npv, npb, nz, k, nkc, weights, nk, ng, dk, kmin, kmax, z_edges, 0, nullptr, t.ldm, s,
+                            true);
+  }
   return check_launch("rr_prepare_split");
 }
 

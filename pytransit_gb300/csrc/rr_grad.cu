@@ -32,19 +32,51 @@ enum GSlot { GS_LNL = 0, GS_KK, GS_KW, GS_T0, GS_P, GS_A, GS_I, GS_E, GS_W, GS_C
 
 // ---------------------------------------------------------------------------
 // Prologue 1: derivatives of the orbit's Taylor coefficients, one thread per
-// pv: dc[pv][j][m] = d c_m / d theta_j, theta = (p, a, i, e, w).
+// (pv, j): dc[pv][j][m] = d c_m / d theta_j, theta = (p, a, i, e, w).  Bound by
+// the thread's chain of FP64 instructions: with the five directions in one
+// thread 37 us for 4096 pv, 24.8 us so.
 // ---------------------------------------------------------------------------
 template <typename R>
 __global__ void grad_orbit_kernel(const double* __restrict__ p, const double* __restrict__ a,
                                   const double* __restrict__ inc, const double* __restrict__ e,
                                   const double* __restrict__ w, int npv, R* __restrict__ dc) {
-  const int pv = blockIdx.x * blockDim.x + threadIdx.x;
+  overlap_next();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, pv = i / 5;
   if (pv >= npv) return;
-  D5 c[10];
-  solve2d_conj_dual(p[pv], a[pv], inc[pv], e[pv], w[pv], c);
-  R* o = dc + (size_t)pv * 50;
-  for (int j = 0; j < 5; ++j)
-    for (int m = 0; m < 10; ++m) o[j * 10 + m] = (R)c[m].d[j];
+  Dual c[10];
+  solve2d_conj_dual(p[pv], a[pv], inc[pv], e[pv], w[pv], i % 5, c);
+  R* o = dc + (size_t)i * 10;
+  for (int m = 0; m < 10; ++m) o[m] = (R)c[m].d;
+}
+
+// Row g of the derivatives from the 2D table at k (and at k +- h for the k
+// derivative), FP64 rows; dl: [npar][64].  Not inlined: the rows of the 3D table,
+// the common case, keep their registers.
+template <typename R>
+static __device__ __noinline__ void grad_ld_row_2d(double k, int g, int ng, int nz, int npar,
+                                                   const double* __restrict__ ze, const R* l, const R* dl, R* out) {
+  const double gstep = (1.0 - 1e-7) / (double)(ng - 1);
+  double gg = (g == ng - 1) ? (1.0 - 1e-7) : (double)g * gstep;
+  const double h = 1e-6 * fmax(k, 1e-3);
+  double res[3][1 + MAX_GRAD_PAR];
+  for (int v = 0; v < 3; ++v) {
+    const double kv = k + (v - 1) * h;
+    const double bb = gg * (1.0 + kv);
+    double a0 = cci_acos(ze[0], kv, bb), s = a0;
+    double acc[1 + MAX_GRAD_PAR];
+    acc[0] = a0 * (double)l[0];
+    for (int j = 0; j < npar; ++j) acc[1 + j] = a0 * (double)dl[j * 64];
+    for (int z = 1; z < nz; ++z) {
+      const double a1 = cci_acos(ze[z], kv, bb), wz = a1 - a0;
+      a0 = a1;
+      s += wz;
+      acc[0] += wz * (double)l[z];
+      for (int j = 0; j < npar; ++j) acc[1 + j] += wz * (double)dl[j * 64 + z];
+    }
+    for (int j = 0; j <= npar; ++j) res[v][j] = acc[j] / s;
+  }
+  out[g] = (R)((res[2][0] - res[0][0]) / (2.0 * h));
+  for (int j = 0; j < npar; ++j) out[(size_t)(1 + j) * ng + g] = (R)res[1][1 + j];
 }
 
 // ---------------------------------------------------------------------------
@@ -56,7 +88,9 @@ __global__ void grad_orbit_kernel(const double* __restrict__ p, const double* __
 // FP32 is bound by the reads of W: a thread's rows element by element from global
 // memory (95.5 us for 4096 pv, ng = 100, nz = 40), or, where rows are whole 16-byte
 // words and the two slabs fit (STAGE), staged by words in shared memory (65.3 us;
-// 51.2 with the FP64 divisions that place k in the table done by one warp).
+// 51.2 with the FP64 divisions that place k in the table done by one warp; 41.2
+// without divisions and with the 2D table's rows, which took registers and local
+// memory, in a function of their own).
 // tab layout per (pv, pb): [dL/dk (ng)][dL/dc_0 (ng)]...[dL/dc_{npar-1} (ng)],
 // dis layout: [d istar/dc_j] (npar).
 // ---------------------------------------------------------------------------
@@ -64,7 +98,7 @@ template <typename R, bool STAGE>
 __global__ void __launch_bounds__(128)
 grad_ld_kernel(int law, const double* __restrict__ ldc, int npb, int npar, const double* __restrict__ mu,
                int nz, const R* __restrict__ ldp, const double* __restrict__ kw, int kw_stride,
-               const R* __restrict__ W, int nk, int ng, double dk, double kmin, double kmax,
+               const R* __restrict__ W, int nk, int ng, double dk, double inv_dk, double kmin, double kmax,
                const double* __restrict__ ze, R* __restrict__ tab, R* __restrict__ dis) {
   extern __shared__ __align__(16) unsigned char gld_smem[];   // STAGE: the slabs of W at ik and ik + 1
   __shared__ __align__(16) R l[64];
@@ -72,24 +106,24 @@ grad_ld_kernel(int law, const double* __restrict__ ldc, int npb, int npar, const
   __shared__ R pvs[16];
   const int pv = blockIdx.x, pb = blockIdx.y;
   const size_t ppb = (size_t)pv * npb + pb;
-  // the block's place in the table, by one warp: FP64 divisions
+  overlap_next();
+  // the block's place in the table, by one warp: FP64 work
   __shared__ int s_ik;
-  __shared__ double s_ak;
+  __shared__ R s_ak;
   const double k = kw[(size_t)pv * kw_stride];
+  const bool has_z = threadIdx.x < nz;
+  const R lz0 = has_z ? ldp[ppb * nz + threadIdx.x] : R(0);   // nz <= 64 threads: loads with k's
+  const double mu0 = has_z ? mu[threadIdx.x] : 0.0;
   if (threadIdx.x < 32) {
     int ik = -1;
-    double ak = 0.0;
-    if (kmin <= k && k <= kmax) {
-      ik = (int)floor((k - kmin) / dk);
-      ak = (k - kmin - ik * dk) / dk;
-      if (ik + 1 >= nk || ik < 0) ik = -1;
-    }
+    R ak = R(0);
+    if (kmin <= k && k <= kmax) table_place(k, kmin, dk, inv_dk, nk, ik, ak);
     if (threadIdx.x == 0) { s_ik = ik; s_ak = ak; }
   }
   if (threadIdx.x < npar) pvs[threadIdx.x] = (R)ldc[ppb * npar + threadIdx.x];
   __syncthreads();
   const int ik = s_ik;
-  const double ak = s_ak;
+  const R ak = s_ak;
   using W16 = typename Word16<R>::T;
   constexpr int PER = 16 / sizeof(R);
   const R* slab = nullptr;
@@ -110,9 +144,9 @@ grad_ld_kernel(int law, const double* __restrict__ ldc, int npb, int npar, const
       }
     }
   }
-  for (int z = threadIdx.x; z < nz; z += blockDim.x) {
-    l[z] = ldp[ppb * nz + z];
-    for (int j = 0; j < npar; ++j) dl[j][z] = ld_dvalue<R>(law, (R)mu[z], pvs, npar, j);
+  if (has_z) {
+    l[threadIdx.x] = lz0;
+    for (int j = 0; j < npar; ++j) dl[j][threadIdx.x] = ld_dvalue<R>(law, (R)mu0, pvs, npar, j);
   }
   if (threadIdx.x < npar) {
     const int j = threadIdx.x;
@@ -134,7 +168,6 @@ grad_ld_kernel(int law, const double* __restrict__ ldc, int npb, int npar, const
   }
   __syncthreads();
   R* out = tab + ppb * (size_t)(1 + npar) * ng;
-  const double gstep = (1.0 - 1e-7) / (double)(ng - 1);
   for (int g = threadIdx.x; g < ng; g += blockDim.x) {
     if (ik >= 0) {
       R d0 = R(0), d1 = R(0);
@@ -162,39 +195,26 @@ grad_ld_kernel(int law, const double* __restrict__ ldc, int npb, int npar, const
           const R a0 = __ldg(w0 + z), a1 = __ldg(w1 + z);
           d0 += a0 * l[z];
           d1 += a1 * l[z];
-          for (int j = 0; j < npar; ++j) {
-            c0[j] += a0 * dl[j][z];
-            c1[j] += a1 * dl[j][z];
-          }
+#pragma unroll
+          for (int j = 0; j < MAX_GRAD_PAR; ++j)
+            if (j < npar) {
+              c0[j] += a0 * dl[j][z];
+              c1[j] += a1 * dl[j][z];
+            }
         }
       }
-      out[g] = (R)(((double)d1 - (double)d0) / dk);
-      for (int j = 0; j < npar; ++j) out[(size_t)(1 + j) * ng + g] = (R(1) - (R)ak) * c0[j] + (R)ak * c1[j];
+      if constexpr (sizeof(R) == 4)
+        out[g] = f32_quotient(f64_of_f32(d1) - f64_of_f32(d0), dk, inv_dk);
+      else
+        out[g] = (d1 - d0) / dk;
+#pragma unroll
+      for (int j = 0; j < MAX_GRAD_PAR; ++j)
+        if (j < npar) out[(size_t)(1 + j) * ng + g] = (R(1) - ak) * c0[j] + ak * c1[j];
     } else {
-      // 2D table at k (and at k +- h for the k derivative), FP64 rows
-      double gg = (g == ng - 1) ? (1.0 - 1e-7) : (double)g * gstep;
-      const double h = 1e-6 * fmax(k, 1e-3);
-      double res[3][1 + MAX_GRAD_PAR];
-      for (int v = 0; v < 3; ++v) {
-        const double kv = k + (v - 1) * h;
-        const double bb = gg * (1.0 + kv);
-        double a0 = cci_acos(ze[0], kv, bb), s = a0;
-        double acc[1 + MAX_GRAD_PAR];
-        acc[0] = a0 * (double)l[0];
-        for (int j = 0; j < npar; ++j) acc[1 + j] = a0 * (double)dl[j][0];
-        for (int z = 1; z < nz; ++z) {
-          const double a1 = cci_acos(ze[z], kv, bb), wz = a1 - a0;
-          a0 = a1;
-          s += wz;
-          acc[0] += wz * (double)l[z];
-          for (int j = 0; j < npar; ++j) acc[1 + j] += wz * (double)dl[j][z];
-        }
-        for (int j = 0; j <= npar; ++j) res[v][j] = acc[j] / s;
-      }
-      out[g] = (R)((res[2][0] - res[0][0]) / (2.0 * h));
-      for (int j = 0; j < npar; ++j) out[(size_t)(1 + j) * ng + g] = (R)res[1][1 + j];
+      grad_ld_row_2d<R>(k, g, ng, nz, npar, ze, l, &dl[0][0], out);
     }
   }
+  overlap_end();
 }
 
 // ---------------------------------------------------------------------------
@@ -281,6 +301,7 @@ __global__ void __launch_bounds__(OBS_THREADS) obs_kernel(const double* __restri
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) sm += red[i];
     cpart[blockIdx.x] = sm;
   }
+  overlap_end();
 }
 
 // ---------------------------------------------------------------------------
@@ -1014,17 +1035,20 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
     ldm = (const R*)pcv.take<double>((size_t)npv * npb * ng);
   }
   if (grad) {   // the derivative tables, read by the adjoint alone
-    grad_orbit_kernel<R><<<(npv + 63) / 64, 64, 0, s>>>(p, a, inc, e, w, npv, g.dc);
+    // an ordinary launch: beside the end of the LD means its blocks crowd the first
+    // SMs with room, where they share a few FP64 pipes (77 us, against 25)
+    grad_orbit_kernel<R><<<(5 * npv + 63) / 64, 64, 0, s>>>(p, a, inc, e, w, npv, g.dc);
     // rows of whole 16-byte words, two slabs within what four blocks of an SM can have
     const size_t slabs = 2 * sizeof(R) * (size_t)ng * nz;
     const bool stage = nz % (16 / sizeof(R)) == 0 && (reinterpret_cast<uintptr_t>(weights) & 15) == 0 && slabs <= GLD_SMEM;
     auto fn = stage ? grad_ld_kernel<R, true> : grad_ld_kernel<R, false>;
     if (stage && slabs > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slabs);
-    fn<<<dim3(npv, npb), 128, stage ? slabs : 0, s>>>(law, ldc, npb, npar, mu, nz, ldp, k, nkc, weights, nk, ng, dk, kmin,
-                                                      kmax, z_edges, g.tab, g.dis);
+    launch_overlap(fn, dim3(npv, npb), 128, stage ? slabs : 0, s, law, ldc, npb, npar, mu, nz, ldp, k, nkc, weights, nk,
+                   ng, dk, 1.0 / dk, kmin, kmax, z_edges, g.tab, g.dis);
   }
   const int nobs = (npt + OBS_CHUNK - 1) / OBS_CHUNK;
-  obs_kernel<R><<<nobs, OBS_THREADS, 0, s>>>(obs, sigma, lcids, npt, nlc, g.dobs, g.isig2, g.cconst, times, g.tiles64);
+  launch_overlap(obs_kernel<R>, nobs, OBS_THREADS, 0, s, obs, sigma, lcids, npt, nlc, g.dobs, g.isig2, g.cconst, times,
+                 g.tiles64);
   if constexpr (sizeof(R) == 4) {
     GradArgs A{};
     A.times_ff = reinterpret_cast<const float2*>(times_ff);

@@ -25,6 +25,20 @@ void launch_ldm_f64(const double* ldp, int npv, int npb, int nz, const double* k
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// Launches f so that it may start before the kernel before it on the stream has
+// ended: that kernel calls overlap_next, f reads nothing it writes, writes nothing
+// it reads, and ends with overlap_end.
+template <typename... P, typename... A>
+inline void launch_overlap(void (*f)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+  cfg.attrs = &at; cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, f, static_cast<P>(args)...);
+}
+
 // Multiprocessor count of the current device (queried once per device), for
 // launch shapes.
 int sm_count();
