@@ -182,6 +182,91 @@ __global__ void __launch_bounds__(128) ld_tables_kernel(int law, const double* _
   if (lane == 0) istar[j] = is;
 }
 
+// The same in FP64 for the affine laws whose disk integral has no closed form and
+// whose basis functions are finite on [0, 1]: the trapezoid is a sum over fixed
+// nodes, so it is taken once per block for each basis function, and a (pv, pb)
+// needs nb multiply-adds for its integral and for each point of its profile.
+// Bound by the FP64 pipe: nonlinear law, 2000 pv, 285 us with a trapezoid per
+// (pv, pb) (square roots and powers at 200 nodes), 10.3 us so.
+constexpr int AFF_NB = 5, AFF_NZ = 64, AFF_PAIRS = 16, AFF_THREADS = 256;
+
+__device__ __forceinline__ void affine_basis(int law, int nb, double mu, double* phi) {
+  if (law == LD_GENERAL) {
+    double m = 1.0;
+    for (int b = 0; b < AFF_NB; ++b) {
+      m *= mu;
+      phi[b] = 1.0 - m;
+    }
+    return;
+  }
+  const double s = sqrt(mu);
+  phi[0] = 1.0;
+  if (law == LD_SQUARE_ROOT) {
+    phi[1] = -(1.0 - mu);
+    phi[2] = -(1.0 - s);
+    phi[3] = phi[4] = 0.0;
+  } else {   // LD_NONLINEAR
+    phi[1] = -(1.0 - s);
+    phi[2] = -(1.0 - mu);
+    phi[3] = -(1.0 - mu * s);
+    phi[4] = -(1.0 - mu * mu);
+  }
+}
+
+__global__ void __launch_bounds__(AFF_THREADS) ld_tables_affine_kernel(int law, int nb, const double* __restrict__ ldc,
+                                                                      int npvpb, int npar,
+                                                                      const double* __restrict__ mu, int nz,
+                                                                      double* __restrict__ ldp,
+                                                                      double* __restrict__ istar) {
+  __shared__ double s_z[NTRAP], s_y[AFF_NB][NTRAP], s_phi[AFF_NB][AFF_NZ], s_J[AFF_NB];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  double phi[AFF_NB];
+  if (tid < NTRAP) {
+    const double m = (double)(NTRAP - 1 - tid) / (double)(NTRAP - 1), z = sqrt(1.0 - m * m);   // as ld_tables_kernel
+    affine_basis(law, nb, m, phi);
+    s_z[tid] = z;
+#pragma unroll
+    for (int b = 0; b < AFF_NB; ++b) s_y[b][tid] = z * phi[b];
+  }
+  if (tid >= AFF_THREADS - AFF_NZ && tid - (AFF_THREADS - AFF_NZ) < nz) {
+    const int i = tid - (AFF_THREADS - AFF_NZ);
+    affine_basis(law, nb, mu[i], phi);
+#pragma unroll
+    for (int b = 0; b < AFF_NB; ++b) s_phi[b][i] = phi[b];
+  }
+  __syncthreads();
+  if (warp < nb) {
+    double s = 0.0;
+    for (int i = lane + 1; i < NTRAP; i += 32) s += 0.5 * ((s_z[i] - s_z[i - 1]) * (s_y[warp][i] + s_y[warp][i - 1]));
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) s_J[warp] = 2.0 * PI * s;
+  }
+  __syncthreads();
+  for (int q = warp; q < AFF_PAIRS; q += AFF_THREADS / 32) {
+    const long long j = (long long)blockIdx.x * AFF_PAIRS + q;
+    if (j >= npvpb) return;   // warp-uniform
+    double c[AFF_NB];
+    const double* src = ldc + (size_t)j * npar;
+    const int shift = law == LD_GENERAL ? 0 : 1;
+#pragma unroll
+    for (int b = 0; b < AFF_NB; ++b) c[b] = b < nb ? (b < shift ? 1.0 : src[b - shift]) : 0.0;
+    if (lane == 0) {
+      double is = c[0] * s_J[0];
+#pragma unroll
+      for (int b = 1; b < AFF_NB; ++b)
+        if (b < nb) is = fma(c[b], s_J[b], is);
+      istar[j] = is;
+    }
+    for (int i = lane; i < nz; i += 32) {
+      double v = c[0] * s_phi[0][i];
+#pragma unroll
+      for (int b = 1; b < AFF_NB; ++b)
+        if (b < nb) v = fma(c[b], s_phi[b][i], v);
+      ldp[(size_t)j * nz + i] = v;
+    }
+  }
+}
+
 template <typename R>
 static int ld_tables(int law, const double* ldc, int npv, int npb, int npar, const double* mu, int nz,
                      R* ldp, R* istar, void* stream) {
@@ -189,6 +274,16 @@ static int ld_tables(int law, const double* ldc, int npv, int npb, int npar, con
   if (npv < 0 || npb < 1 || npar < 0 || npar > MAX_LDPAR || nz < 1) return RR_ERR_ARG;
   const long long n = (long long)npv * npb;
   if (n == 0) return RR_OK;
+  if constexpr (sizeof(R) == 8) {
+    const int nb = basis_count(law, npar);
+    // all of the law's coefficients given (their count is the caller's) and few
+    const bool affine = (law == LD_NONLINEAR && npar >= 4) || (law == LD_SQUARE_ROOT && npar >= 2) || law == LD_GENERAL;
+    if (affine && nb > 0 && nb <= AFF_NB && nz <= AFF_NZ) {
+      ld_tables_affine_kernel<<<(unsigned)((n + AFF_PAIRS - 1) / AFF_PAIRS), AFF_THREADS, 0, as_stream(stream)>>>(
+          law, nb, ldc, (int)n, npar, mu, nz, ldp, istar);
+      return check_launch("rr_ld_tables");
+    }
+  }
   ld_tables_kernel<R><<<(unsigned)((n + 3) / 4), 128, 0, as_stream(stream)>>>(law, ldc, (int)n, npar, mu, nz, ldp,
                                                                               istar);
   return check_launch("rr_ld_tables");
