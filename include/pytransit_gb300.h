@@ -361,6 +361,17 @@ int rr_lnlike_f64(int law, const double *ldc, int npar, const double *mu, const 
                   const double *weights, int nk, int ng, int nz, double dk, double kmin, double kmax,
                   double dg, const double *z_edges, const double *obs, const double *sigma, void *workspace,
                   size_t workspace_bytes, double *lnl, double *grad, void *stream);
+/* rr_lnlike_f64 with the LD tables made inside, as rr_prepare_f64_ld makes them
+ * (basis, nb: rr_basis_tables of the law, or NULL, 0); ldp[npv, npb, nz] and
+ * istar[npv, npb] are written where they are read. */
+int rr_lnlike_f64_ld(int law, const double *ldc, int npar, const double *mu, const double *basis, int nb,
+                     const double *times, int npt, const double *k, int nkc, const double *t0, int ldt0, int nep,
+                     const double *p, const double *a, const double *inc, const double *e, const double *w,
+                     int npv, int nlc, int npb, const int32_t *lcids, const int32_t *pbids, const int32_t *epids,
+                     const int32_t *nsamples, const double *exptimes, double *ldp, double *istar,
+                     const double *weights, int nk, int ng, int nz, double dk, double kmin, double kmax,
+                     double dg, const double *z_edges, const double *obs, const double *sigma, void *workspace,
+                     size_t workspace_bytes, double *lnl, double *grad, void *stream);
 /* Same, split precision (FP32 per-sample arithmetic and residuals formed from
  * the deficit, FP64 block sums). */
 int rr_lnlike_split(int law, const double *ldc, int npar, const double *mu, const float *times_ff,

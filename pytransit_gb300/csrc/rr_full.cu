@@ -618,6 +618,7 @@ template <int LAW>
 __global__ void __launch_bounds__(PRO_THREADS) prologue_f64_kernel(Pro64Args P, int norb) {
   constexpr int NB = LAW == LD_UNIFORM ? 1 : (LAW == LD_LINEAR ? 2 : 3);   // basis_count of the law
   __shared__ double s_coef[PRO_WARPS][PRO_MAX_COEF];
+  overlap_next();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if ((int)blockIdx.x < norb) {
     if (warp != 0) return;
@@ -1516,6 +1517,12 @@ serve_split_kernel(const rr_serve_request* __restrict__ reqs, const rr_serve_ite
   }
 }
 
+bool prepare_f64_fused(int law, int npar, int npb, const double* ldc, const double* mu, const double* basis, int nb) {
+  const bool analytic = law == LD_UNIFORM || law == LD_LINEAR || law == LD_QUADRATIC || law == LD_QUADRATIC_TRI;
+  return analytic && basis && ldc && mu && nb > 0 && nb <= MAX_BASIS && nb == basis_count(law, npar) && npar >= 0 &&
+         npar <= ORB_MAX_LDPAR && npb * nb <= PRO_MAX_COEF;
+}
+
 }  // namespace rr
 
 using namespace rr;
@@ -1757,10 +1764,7 @@ int rr_prepare_f64_ld(const double* k, int nkc, const double* p, const double* a
                       int nz, const double* basis, int nb, const double* weights, int nk, int ng, double dk,
                       double kmin, double kmax, const double* z_edges, double* ldp, double* istar, void* workspace,
                       size_t workspace_bytes, void* stream) {
-  const bool analytic = law == LD_UNIFORM || law == LD_LINEAR || law == LD_QUADRATIC || law == LD_QUADRATIC_TRI;
-  const bool fused = analytic && basis && ldc && mu && nb > 0 && nb <= MAX_BASIS && nb == basis_count(law, npar) &&
-                     npar >= 0 && npar <= ORB_MAX_LDPAR && npb * nb <= PRO_MAX_COEF;
-  if (!fused) {
+  if (!prepare_f64_fused(law, npar, npb, ldc, mu, basis, nb)) {
     const int st = rr_ld_tables_f64(law, ldc, npv, npb, npar, mu, nz, ldp, istar, stream);
     if (st) return st;
     return rr_prepare_f64(k, nkc, p, a, inc, e, w, npv, npb, ldp, weights, nk, ng, nz, dk, kmin, kmax, z_edges,

@@ -995,7 +995,8 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
                        const double* exptimes, const R* ldp, const R* istar, const R* weights, int nk, int ng,
                        int nz, double dk, double kmin, double kmax, double dg, const double* z_edges,
                        const double* obs, const double* sigma, void* workspace, size_t workspace_bytes,
-                       double* lnl, double* grad, void* stream) {
+                       double* lnl, double* grad, void* stream, const double* basis = nullptr, int nb = 0,
+                       bool make_ld = false) {
   if (nkc > 1 && nkc != npb) return RR_ERR_SHAPE;
   if (law < 0 || law >= LD_NLAWS) return RR_ERR_LAW;
   if (npt < 1 || npv < 0 || nlc < 1 || npb < 1 || nk < 2 || ng < 2 || nz < 1 || nz > 64 || nkc < 1 || nep < 1 ||
@@ -1014,7 +1015,17 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
     st = rr_prepare_split(t_ref, t_absmax, k, nkc, t0, ldt0, nep, p, a, inc, e, w, npv, nlc, npb, pbids, epids,
                           nsamples, exptimes, (const float*)ldp, (const float*)istar, (const float*)weights, nk, ng,
                           nz, dk, kmin, kmax, z_edges, workspace, base, stream, 0, nullptr, 0, nullptr, 0);
-  else
+  else if (make_ld) {
+    // the adjoint reads the whole profile, which the fused prologue leaves out
+    double *ldp64 = (double*)const_cast<R*>(ldp), *istar64 = (double*)const_cast<R*>(istar);
+    st = grad && prepare_f64_fused(law, npar, npb, ldc, mu, basis, nb)
+             ? rr_ld_tables_f64(law, ldc, npv, npb, npar, mu, nz, ldp64, istar64, stream)
+             : RR_OK;
+    if (st == RR_OK)
+      st = rr_prepare_f64_ld(k, nkc, p, a, inc, e, w, npv, npb, law, ldc, npar, mu, nz, basis, nb,
+                             (const double*)weights, nk, ng, dk, kmin, kmax, z_edges, ldp64, istar64, workspace, base,
+                             stream);
+  } else
     st = rr_prepare_f64(k, nkc, p, a, inc, e, w, npv, npb, (const double*)ldp, (const double*)weights, nk, ng, nz,
                         dk, kmin, kmax, z_edges, workspace, base, stream, 0, nullptr, 0, nullptr, 0);
   if (st) return st;
@@ -1094,6 +1105,21 @@ int rr_lnlike_f64(int law, const double* ldc, int npar, const double* mu, const 
                              e, w, npv, nlc, npb, lcids, pbids, epids, nsamples, exptimes, ldp, istar, weights, nk,
                              ng, nz, dk, kmin, kmax, dg, z_edges, obs, sigma, workspace, workspace_bytes, lnl, grad,
                              stream);
+}
+
+int rr_lnlike_f64_ld(int law, const double* ldc, int npar, const double* mu, const double* basis, int nb,
+                     const double* times, int npt, const double* k, int nkc, const double* t0, int ldt0, int nep,
+                     const double* p, const double* a, const double* inc, const double* e, const double* w, int npv,
+                     int nlc, int npb, const int32_t* lcids, const int32_t* pbids, const int32_t* epids,
+                     const int32_t* nsamples, const double* exptimes, double* ldp, double* istar,
+                     const double* weights, int nk, int ng, int nz, double dk, double kmin, double kmax, double dg,
+                     const double* z_edges, const double* obs, const double* sigma, void* workspace,
+                     size_t workspace_bytes, double* lnl, double* grad, void* stream) {
+  if (!mu || !ldp || !istar) return RR_ERR_ARG;
+  return lnlike_impl<double>(0, law, ldc, npar, mu, times, nullptr, 0.0, 0.0, npt, k, nkc, t0, ldt0, nep, p, a, inc,
+                             e, w, npv, nlc, npb, lcids, pbids, epids, nsamples, exptimes, ldp, istar, weights, nk,
+                             ng, nz, dk, kmin, kmax, dg, z_edges, obs, sigma, workspace, workspace_bytes, lnl, grad,
+                             stream, basis, nb, true);
 }
 
 int rr_lnlike_split(int law, const double* ldc, int npar, const double* mu, const float* times_ff, double t_ref,

@@ -23,6 +23,10 @@ void launch_ldm_f64(const double* ldp, int npv, int npb, int nz, const double* k
                     int nk, int ng, double dk, double kmin, double kmax, const double* ze, int mode,
                     const double* kmax_pv, double* ldm, cudaStream_t s);
 
+// rr_prepare_f64_ld takes its fused kernel (which writes the profile only for a k
+// outside the tables).
+bool prepare_f64_fused(int law, int npar, int npb, const double* ldc, const double* mu, const double* basis, int nb);
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // Launches f so that it may start before the kernel before it on the stream has

@@ -5,7 +5,7 @@ The reference evaluates the model (rr_full) and then the log-likelihood
 parameter vector.  Here both run in one CUDA kernel (the flux is never
 stored), and ``d lnL / d theta`` for theta = (k, t0, p, a, i, e, w, ldc) comes
 from a hand-written adjoint kernel that recomputes z per sample
-(rr_lnlike_f64 / rr_lnlike_split in the C ABI).
+(rr_lnlike_f64_ld / rr_lnlike_split in the C ABI).
 
 ``LogLikelihood`` is a torch.autograd.Function: its forward runs the
 likelihood kernel without derivatives, its backward re-runs it with them.
@@ -26,6 +26,9 @@ _SIG = {
     'rr_lnlike_f64': ([_i, _vp, _i, _vp, _vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i,
                        _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _d, _d, _d, _d, _vp, _vp, _vp, _vp,
                        _sz, _vp, _vp, _vp], _i),
+    'rr_lnlike_f64_ld': ([_i, _vp, _i, _vp, _vp, _i, _vp, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i,
+                          _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _d, _d, _d, _d, _vp, _vp, _vp, _vp,
+                          _sz, _vp, _vp, _vp], _i),
     'rr_lnlike_split': ([_i, _vp, _i, _vp, _vp, _d, _d, _i, _vp, _i, _vp, _i, _i, _vp, _vp, _vp, _vp, _vp, _i,
                          _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _d, _d, _d, _d, _vp, _vp,
                          _vp, _vp, _sz, _vp, _vp, _vp], _i),
@@ -63,10 +66,13 @@ def _run(model, obs, sigma, k, t0, p, a, i, e, w, ldc, want_grad):
     ld = torch.empty(npv * npb * (nz + 1), dtype=dt, device=device)   # ldp[npv, npb, nz], then istar[npv, npb]
     ldp = ld.data_ptr()
     istar = ldp + npv * npb * nz * ld.element_size()
-    fn = L.rr_ld_tables_f32 if split else L.rr_ld_tables_f64
     P = _lib.addr
     sp = _lib.stream_addr(device)
-    _lib.check(fn(model.ld_law, P(ldc), npv, npb, npar, P(tb['mu']), nz, ldp, istar, sp), "rr_ld_tables")
+    if split:
+        _lib.check(L.rr_ld_tables_f32(model.ld_law, P(ldc), npv, npb, npar, P(tb['mu']), nz, ldp, istar, sp),
+                   "rr_ld_tables")
+    else:
+        basis, nb = model._basis(device, npar, False)
     obs = torch.as_tensor(obs, dtype=torch.float64).to(device).contiguous()
     if obs.numel() != npt:
         raise ValueError(f"obs should have {npt} values")
@@ -90,7 +96,8 @@ def _run(model, obs, sigma, k, t0, p, a, i, e, w, ldc, want_grad):
         st = L.rr_lnlike_split(model.ld_law, P(ldc), npar, P(tb['mu']), P(dd['times_ff']), dd['t_ref'],
                                dd['t_absmax'], npt, *common_tail, sp)
     else:
-        st = L.rr_lnlike_f64(model.ld_law, P(ldc), npar, P(tb['mu']), P(dd['time']), npt, *common_tail, sp)
+        st = L.rr_lnlike_f64_ld(model.ld_law, P(ldc), npar, P(tb['mu']), P(basis), nb, P(dd['time']), npt,
+                                *common_tail, sp)
     _lib.check(st, "rr_lnlike")
     return lnl, g
 
