@@ -852,7 +852,7 @@ struct WarpList {
 // Points of supersampled light curves that the fast fold puts in the box, kept
 // by a warp over its tiles until they fill whole warps: at a 30-min cadence a
 // tile that reaches a transit holds ~10 of them.
-constexpr int SPLIT_Q = 256;       // points
+constexpr int SPLIT_Q = 160;       // points: what a tile adds to a queue of whole warps' remainder, and a warp
 constexpr int SPLIT_ROWS = 10;     // rows of 32 samples evaluated at once
 struct SplitQueue {
   int pt[SPLIT_Q];
@@ -894,7 +894,7 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
 // full warps from a list.  A point's terms are added in sample order.  4096 pv
 // x 118,526 times x 10 samples: 2682 us with each tile's (point, sample) pairs
 // by themselves (a binary search for a pair's point, the full area for every
-// pair, a segmented shuffle sum), 1706 us.  Ranges of 64, 128 and 256 tiles per
+// pair, a segmented shuffle sum), 1691 us.  Ranges of 64, 128 and 256 tiles per
 // block instead of 32: 5, 8 and 14 % slower.
 __device__ __forceinline__ int split_flush(const float2* __restrict__ times, const float* orb, const float* R,
                                            const float* ldm_pv, int ng, float inv_dg, SplitQueue& Q, int n, bool all,
