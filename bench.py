@@ -28,6 +28,7 @@ Reported (one JSON line from rank 0):
 path restated in C; the reference itself is Python + numba, absent here).
 """
 import argparse
+import gc
 import json
 import os
 import statistics
@@ -902,6 +903,7 @@ def main():
                                  P(dd["exptimes"]), P(ist64), ng, model.dg, P(ws64), P(flux64), npt, sp))
 
     def timed(fn, steps, warmup, per_step_events=False):
+        gc.collect()   # a collection of the imported modules' objects takes about eight steps
         for _ in range(warmup):
             fn()
         barrier()
