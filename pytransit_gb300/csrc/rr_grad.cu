@@ -781,8 +781,10 @@ template <bool GRAD>
 __device__ __noinline__ void lnl_f64_flush(const LnlF64Args& A, const F64Orbit& P, F64Lc* recs, F64Queue& Q,
                                            const double* o, LnlF64Smem<GRAD>& S, int pv, int lc, int n) {
   const int lane = threadIdx.x & 31, nrec = min(A.nlc, F64_LC_SMEM);
-  if (lc != S.lc) {
-    if (S.lc >= 0) lnl_f64_reduce<GRAD>(A, S, pv);
+  const int before = S.lc;
+  __syncwarp();   // every lane has read it
+  if (lc != before) {
+    if (before >= 0) lnl_f64_reduce<GRAD>(A, S, pv);
     if (lane == 0) S.lc = lc;
     __syncwarp();
   }
