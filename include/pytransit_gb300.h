@@ -349,7 +349,8 @@ int rr_ts_split(const float *times_ff, double t_ref, double t_absmax, int npt, c
  * interpolations, kite area, orbit Taylor coefficients), recomputing z per
  * sample.  The reference has no adjoint (its dfdk/dfdb, common.py:105-128, are
  * unused partials).  Named LD laws only (law, ldc[npv, npb, npar], npar <= 4);
- * ldp/istar as from rr_ld_tables_*. */
+ * ldp/istar as from rr_ld_tables_*.  FP64: a vector whose flux is NaN at a
+ * point (a NaN radius ratio, say) has a NaN lnl and gradient. */
 int rr_lnlike_ngrad(int nkc, int nep, int npb, int npar);
 size_t rr_lnlike_workspace_bytes(int split, int npv, int npb, int nlc, int nep, int ng, int npar, int npt,
                                  int nkc);

@@ -163,10 +163,12 @@ void rro_weights_3d(int nk, double k0, double k1, const double *ze, int nz, int 
 
 /* interpolate_mean_limb_darkening_s, common.py:225-233.  The reference reads
  * lda[ng] for g in [1-1e-7, 1]; here the index is clamped to ng-2 (linear
- * extrapolation from the last cell), which is what the GPU path does too. */
+ * extrapolation from the last cell), which is what the GPU path does too.  NaN
+ * passes neither of the reference's two tests: it is taken with g < 0, for its
+ * index would be any number. */
 double rro_interp_ldm(double g, double dg, const double *lda, int ng)
 {
-    if (g < 0.0) return NAN;
+    if (!(g >= 0.0)) return NAN;
     if (g > 1.0) return 0.0;
     int i = (int)floor(g / dg);
     if (i > ng - 2) i = ng - 2;

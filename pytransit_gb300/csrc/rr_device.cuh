@@ -165,9 +165,11 @@ __device__ inline R ccia_star_grad(R k, R z, R& dadk, R& dadz) {
 }
 
 // interpolate_mean_limb_darkening_s, common.py:225-233.  The reference reads
-// lda[ng] for g in [1-1e-7, 1]; the index is clamped to ng-2 here.
+// lda[ng] for g in [1-1e-7, 1]; the index is clamped to ng-2 here.  NaN (a NaN
+// radius ratio or separation) passes neither of the reference's two tests and
+// has no index: it is taken with g < 0.
 __device__ inline double interp_ldm_f64(double g, double dg, const double* lda, int ng) {
-  if (g < 0.0) return CUDART_NAN;
+  if (!(g >= 0.0)) return CUDART_NAN;
   if (g > 1.0) return 0.0;
   int i = (int)floor(g / dg);
   if (i > ng - 2) i = ng - 2;

@@ -688,7 +688,7 @@ struct F64Partials {
 static __device__ __noinline__ void f64_partials_general(const F64Disk& K, const F64Transit& T, double r2, F64Partials& S) {
   const double z = sqrt(r2);
   S.z = z;
-  S.none = !(z < 1.0 + K.k);
+  S.none = z >= 1.0 + K.k;   // NaN has partial derivatives: NaN
   S.iz = 1.0 / z;
   const double gg = z / (1.0 + K.k) / T.dg;
   S.i = min(max((int)gg, 0), T.ng - 2);
