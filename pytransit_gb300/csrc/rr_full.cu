@@ -39,11 +39,15 @@ constexpr int LDM_SCRATCH = 512;   // FP64 areas of the 2D table per chunk of ro
 // 4 KB of scratch instead of 16, 17.9 with one warp's divisions, 15.5 with products
 // in their place.  In FP64 the pipe bounds it: 49 -> 39 us for 1500 pv.
 // ---------------------------------------------------------------------------
-// Byte offset of the FP64 scratch after the slab [ng][nz+1] and the LD
-// profiles [LDM_PBB][MAX_NZ] (8-byte aligned).
+// Shared memory: the slab [ng][nz + 1 at most], the LD profiles [LDM_PBB][MAX_NZ at
+// most] at the next 16-byte boundary, and the FP64 scratch.  Byte offsets:
+template <typename R>
+__host__ __device__ inline size_t ldm_profile_offset(int ng, int ldw) {
+  return (sizeof(R) * (size_t)ng * ldw + 15) & ~size_t(15);
+}
 template <typename R>
 __host__ __device__ inline size_t ldm_scratch_offset(int ng, int nz) {
-  return (sizeof(R) * ((size_t)ng * (nz + 1) + (size_t)LDM_PBB * MAX_NZ) + 7) & ~size_t(7);
+  return ldm_profile_offset<R>(ng, nz + 1) + sizeof(R) * (size_t)LDM_PBB * MAX_NZ;
 }
 
 template <typename R, bool VEC>
@@ -57,7 +61,7 @@ ldm_kernel(const R* __restrict__ ldp, int npb, int nz, const double* __restrict_
   using W16 = typename Word16<R>::T;
   constexpr int PER = 16 / sizeof(R);
   const int ldw = VEC ? nz : nz + 1;
-  R* l = Wk + (((size_t)ng * ldw + PER - 1) & ~size_t(PER - 1));   // [LDM_PBB][nz]
+  R* l = reinterpret_cast<R*>(ldm_smem + ldm_profile_offset<R>(ng, ldw));   // [LDM_PBB][nz]
   const int pv = blockIdx.x;
 
   overlap_next();
