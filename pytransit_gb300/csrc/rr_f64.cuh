@@ -114,6 +114,8 @@ __device__ __forceinline__ double f64_of(float f) {
   const unsigned b = __float_as_uint(f);
   return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + F64_BIAS)), (int)(b << 29));
 }
+// Neither infinite nor NaN.
+__device__ __forceinline__ bool f64_finite(double d) { return (__double2hiint(d) & 0x7ff00000) != 0x7ff00000; }
 // Magnitude between 2^-100 and 2^100 and a positive sign (excludes NaN).
 __device__ __forceinline__ bool f64_moderate(double d) {
   return (unsigned)__double2hiint(d) - ((1023u - 100u) << 20) < (200u << 20);

@@ -44,14 +44,18 @@ struct F64Orbit {
   float df[R2_N];
   float t1, t4;        // contacts
   int even;
+  int finite;          // every coefficient is
 };
 
 __device__ __forceinline__ void f64_orbit(const double* o, F64Orbit& P) {
+  bool fin = true;
 #pragma unroll
   for (int m = 0; m < R2_N; ++m) {
     P.d[m] = o[ORB64_R2 + m];
     P.df[m] = f32_of(P.d[m]);
+    fin = fin && f64_finite(P.d[m]);
   }
+  P.finite = fin;
   P.t1 = (float)o[10];
   P.t4 = (float)o[11];
   P.even = r2_is_even(P.d);
@@ -84,6 +88,12 @@ __device__ __forceinline__ void f64_lc(const F64Args& A, int pv, int lc, const F
 #pragma unroll
   for (int m = R2_N - 2; m >= 0; --m) sum = fmaf(sum, tb, fabsf(P.df[m]));
   f64_disk<IK>(A.k[(size_t)pv * A.nkc + (A.nkc == A.npb ? R.pb : 0)], A.dg, fmaf(4e-6f, sum, 2e-6f), R.disk);
+  // f32_of knows no NaN: with a coefficient that is not finite (a NaN inclination,
+  // say) no sample is sure, and general() gives the reference's NaN
+  if (!P.finite) {
+    R.disk.r2out = INFINITY;
+    R.disk.r2in = -INFINITY;
+  }
   const double is = A.istar ? A.istar[(size_t)pv * A.npb + R.pb] : 1.0;
   R.w = isfinite(is) || !A.nan_istar ? f64_recip(R.ns == 1 ? is : __dmul_rn(is, (double)R.ns)) : CUDART_NAN;
 }

@@ -37,7 +37,8 @@ def args(prm):
     return tuple(prm[n] for n in ('k', 'ldc', 't0', 'p', 'a', 'i', 'e', 'w'))
 
 
-NAN = ['k']
+# NaN k, i: NaN in the box; the others move the box away, and every point is 1
+NAN = ['k', 'i', 'p', 't0', 'e', 'w']
 
 
 @pytest.mark.gpu
@@ -53,7 +54,7 @@ def test_flux(name, npt, ns, npb):
     ref = oracle.OracleRoadRunner(LAW)
     ref.set_data(**data)
     want = ref.evaluate(*args(prm))
-    assert np.isnan(want[2]).any()
+    assert np.isnan(want[2]).any() == (name in 'ki')
     m = RoadRunnerModel(LAW)
     m.set_data(**data)
     for cull in (False, True):
@@ -79,7 +80,9 @@ def test_lnlikelihood(name, npt, ns, npb):
     m.set_data(**data)
     lnl0, g0 = lnlikelihood(m, obs, 1e-3, *args(good), grad=True)
     lnl, g = lnlikelihood(m, obs, 1e-3, *args(prm), grad=True)
-    assert np.isnan(lnl[2]) and np.isnan(g[2]).all()
+    flux = m.evaluate(*args(prm))
+    assert np.isnan(lnl[2]) == np.isnan(flux[2]).any() == (name in 'ki')
+    assert np.isnan(g[2]).all() == (name in 'ki')
     rest = [0, 1, 3, 4]
     np.testing.assert_array_equal(lnl[rest], lnl0[rest])
     np.testing.assert_array_equal(g[rest], g0[rest])
@@ -102,3 +105,31 @@ def test_walker_with_negative_area_ratio():
     got = lpf.lnlikelihood(m, obs, 1e-3, torch.as_tensor(pv).cuda(), 0.0).cpu().numpy()
     assert np.isnan(got[1])
     np.testing.assert_array_equal(got[[0, 2, 3]], good[[0, 2, 3]])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ['k', 'i', 'w', 'p'])
+@pytest.mark.parametrize("ns", [1, 3])
+def test_eclipses(name, ns):
+    from pytransit_gb300 import EclipseModel, EclipseSpectroscopyModel
+    npv, time = 3, np.concatenate([np.linspace(-0.2, 0.2, 200), 1.5 + np.linspace(-0.4, 0.4, 400)])
+    a = np.array([8.0, 5.0, 11.0])
+    prm = dict(k=np.full(npv, 0.1), t0=np.zeros(npv), p=np.full(npv, 3.0), a=a, i=np.arccos(0.3 / a),
+               e=np.full(npv, 0.1), w=np.array([0.3, 2.0, 5.0]))
+    prm[name][1] = np.nan
+    order = tuple(prm[n] for n in ('k', 't0', 'p', 'a', 'i', 'e', 'w'))
+    ex = 0.02 if ns > 1 else 0.0
+    want = oracle.eclipse_full(time, order[0], prm['t0'].reshape(npv, 1), *order[2:], 1.0, np.zeros(time.size, int), [0],
+                               [ns], [ex])
+    m = EclipseModel()
+    m.set_data(time, nsamples=[ns], exptimes=[ex])
+    for cull in (False, True):
+        m.fp64_cull = cull
+        np.testing.assert_allclose(m.evaluate(order[0], prm['t0'].reshape(npv, 1), *order[2:], copy=False).cpu().numpy(),
+                                   want, rtol=0, atol=2e-13)
+    f = np.full((npv, 2), 1e-3)
+    want = oracle.es_full(time, *order, np.ones(npv), f, ns, ex)
+    m = EclipseSpectroscopyModel()
+    m.set_data(time, nsamples=[ns], exptimes=[ex])
+    got = m.evaluate(f, *order, copy=False).cpu().numpy()
+    np.testing.assert_allclose(got, want.reshape(got.shape), rtol=0, atol=2e-13)
