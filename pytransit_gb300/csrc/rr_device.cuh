@@ -384,11 +384,19 @@ __device__ inline void basis_coefs(int law, const double* pv, int npar, double* 
 // One thread's FP64 instructions are issued ~75 cycles apart, so their number
 // is the kernel's time: 4 divisions and a root here, against 12 and 2 for the
 // general recurrence, and no sine of w for a circular orbit.
-// (sf, cf): sine and cosine of the true anomaly there, read for e != 0.
+// (sf, cf): sine and cosine of the true anomaly there, from apsis_sincos.
+// sin f = cos w and cos f = sin w at f = pi/2 - w, where they matter: for a
+// circular orbit (1, 0), or NaN with a w that has neither (as e sin w is NaN).
+__device__ inline void apsis_sincos(double e, double w, double& sf, double& cf) {
+  sf = 1.0;
+  cf = 0.0;
+  if (e != 0.0) sincos(w, &cf, &sf);
+  else if (!isfinite(w)) sf = cf = CUDART_NAN;
+}
 __device__ inline void solve2d_apsis(double p, double a, double inc, double e, double sf, double cf, double* c) {
   const double n = 2.0 * PI / p;
   double r = a, vr = 0.0, vt = n * a;
-  if (e != 0.0) {
+  if (e != 0.0 || isnan(cf)) {
     const double se2 = 1.0 - e * e, q = 1.0 + e * cf;
     const double v = n * a / sqrt(se2);
     r = a * se2 / q;
@@ -413,8 +421,8 @@ __device__ inline void solve2d_apsis(double p, double a, double inc, double e, d
 }
 
 __device__ inline void solve2d_conj(double p, double a, double inc, double e, double w, double* c) {
-  double sf = 1.0, cf = 0.0;
-  if (e != 0.0) sincos(w, &cf, &sf);   // f = pi/2 - w: sin f = cos w, cos f = sin w
+  double sf, cf;
+  apsis_sincos(e, w, sf, cf);
   solve2d_apsis(p, a, inc, e, sf, cf, c);
 }
 
@@ -423,8 +431,8 @@ __device__ inline void solve2d_conj(double p, double a, double inc, double e, do
 // propagated there from the transit by Newton's method on Kepler's equation,
 // as the reference's solve2d(eclipse offset, ...) takes it, agrees to 2e-15.)
 __device__ inline void solve2d_ecl(double p, double a, double inc, double e, double w, double* c) {
-  double sf = 1.0, cf = 0.0;
-  if (e != 0.0) sincos(w, &cf, &sf);
+  double sf, cf;
+  apsis_sincos(e, w, sf, cf);
   solve2d_apsis(p, a, inc, e, -sf, -cf, c);
 #pragma unroll
   for (int i = 0; i < 10; ++i) c[i] = -c[i];

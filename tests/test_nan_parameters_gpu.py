@@ -133,3 +133,36 @@ def test_eclipses(name, ns):
     m.set_data(time, nsamples=[ns], exptimes=[ex])
     got = m.evaluate(f, *order, copy=False).cpu().numpy()
     np.testing.assert_allclose(got, want.reshape(got.shape), rtol=0, atol=2e-13)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w", [np.nan, np.inf])
+def test_argument_of_periastron_of_a_circular_orbit(w):
+    """e = 0 does not hide a w that is no angle: e sin w is NaN."""
+    from pytransit_gb300 import EclipseModel, RoadRunnerModel, TSModel
+    from pytransit_gb300.lnlike import lnlikelihood
+    data, prm = problem(300, 1, 1)
+    prm['e'][:] = 0.0
+    prm['w'][2] = w
+    ref = oracle.OracleRoadRunner(LAW)
+    ref.set_data(**data)
+    want = ref.evaluate(*args(prm))
+    assert (want[2] == 1.0).all() and (want[1] < 1.0).any()
+    m = RoadRunnerModel(LAW)
+    m.set_data(**data)
+    np.testing.assert_allclose(m.evaluate(*args(prm)), want, rtol=0, atol=TOL)
+    obs = np.ones(300)
+    np.testing.assert_allclose(lnlikelihood(m, obs, 1e-3, *args(prm)), oracle.lnlike_normal(obs, want, 1e-3), rtol=1e-9)
+    ref = oracle.OracleRoadRunner(LAW, ts=True)
+    ref.set_data(data['time'])
+    m = TSModel(LAW)
+    m.set_data(data['time'])
+    prm['t0'] = prm['t0'][:, 0]
+    got = m.evaluate(*args(prm))
+    np.testing.assert_allclose(got, ref.evaluate(*args(prm)).reshape(got.shape), rtol=0, atol=TOL)
+    order = (prm['k'][:, 0], prm['t0'].reshape(-1, 1), *(prm[n] for n in ('p', 'a', 'i', 'e', 'w')))
+    time = np.linspace(1.2, 1.8, 200)
+    m = EclipseModel()
+    m.set_data(time)
+    np.testing.assert_allclose(m.evaluate(*order), oracle.eclipse_full(time, *order, 1.0, np.zeros(200, int), [0], [1], [0.0]),
+                               rtol=0, atol=2e-13)
