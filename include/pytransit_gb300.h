@@ -350,7 +350,11 @@ int rr_ts_split(const float *times_ff, double t_ref, double t_absmax, int npt, c
  * sample.  The reference has no adjoint (its dfdk/dfdb, common.py:105-128, are
  * unused partials).  Named LD laws only (law, ldc[npv, npb, npar], npar <= 4);
  * ldp/istar as from rr_ld_tables_*.  FP64: a vector whose flux is NaN at a
- * point (a NaN radius ratio, say) has a NaN lnl and gradient. */
+ * point (a NaN radius ratio, say) has a NaN lnl and gradient.
+ * The workspace size never falls as npv or npt grows and is the same for every
+ * device: one for the largest population serves every smaller call.  The sums'
+ * order is fixed for given npt and npv (the same bits in every run); in FP64 it
+ * depends on npv, so that a vector's last bits can differ between batches. */
 int rr_lnlike_ngrad(int nkc, int nep, int npb, int npar);
 size_t rr_lnlike_workspace_bytes(int split, int npv, int npb, int nlc, int nep, int ng, int npar, int npt,
                                  int nkc);

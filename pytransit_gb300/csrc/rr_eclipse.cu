@@ -637,7 +637,7 @@ static int eclipse_f64_launch(const double* times, const double* tiles64, int np
   A.nsamples = nsamples; A.exptimes = exptimes; A.orb64 = rec; A.shift = rec + ECL_SHIFT; A.npv = npv; A.nlc = nlc;
   A.nkc = A.npb = 1; A.dg = 1.0; A.flux = flux; A.ldflux = ldflux;
   if (tiles64) {
-    const int slots = f64_slots(npt, npv);
+    const int slots = f64_slots(npt, npv, sm_count());
     dim3 fg(f64_warps(npt, slots), npv < 65535 ? npv : 65535, (npv + 65534) / 65535);
     const size_t smem = sizeof(F64Lc) * (std::min(nlc, F64_LC_SMEM) + 1);
     eclipse_flux_culled_kernel<<<fg, 32, smem, s>>>(A, tiles64, slots);

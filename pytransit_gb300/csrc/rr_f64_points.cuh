@@ -407,9 +407,9 @@ __device__ __forceinline__ void f64_fill_tile(double* row, int npt, int p0, int 
 // warp, 491 with 64, 493 with 96), and down to 8 while that leaves one, since a
 // warp's own cost (constants, cull test, partly filled last lists) is that of
 // about two tiles (log-likelihood of 1500 x 2999: 156 us with 3, 142 with 8).
-inline int f64_slots(int npt, int npv) {
+inline int f64_slots(int npt, int npv, int sms) {
   const int ntiles = (npt + TIME_TILE - 1) / TIME_TILE;
-  const long long tiles = (long long)ntiles * npv, round = 16LL * sm_count();
+  const long long tiles = (long long)ntiles * npv, round = 16LL * sms;
   if (tiles < round) return 4 * tiles <= round ? 1 : (4 * tiles <= 2 * round ? 2 : 4);
   long long want = tiles / (4 * round);
   const long long least = tiles / round < 8 ? tiles / round : 8;

@@ -1647,7 +1647,7 @@ int rr_flux_f64_culled_range(const double* times, const double* tiles64, int npt
   fa.nsamples = nsamples; fa.npt = npt; fa.npv = pv1 - pv0; fa.nkc = nkc; fa.ldt0 = ldt0; fa.npb = npb;
   fa.nlc = nlc; fa.ng = ng; fa.ldflux = ldflux; fa.dg = dg; fa.nan_istar = true; fa.flux = flux;
   const int n = pv1 - pv0;
-  const int slots = f64_slots(npt, n);
+  const int slots = f64_slots(npt, n, sm_count());
   dim3 fg(f64_warps(npt, slots), n < 65535 ? n : 65535, (n + 65534) / 65535);
   const size_t smem = sizeof(F64Lc) * (std::min(nlc, F64_LC_SMEM) + 1);
   flux_f64_culled_kernel<<<fg, 32, smem, as_stream(stream)>>>(fa, tiles64, slots);

@@ -949,22 +949,40 @@ struct GradWs {
 };
 
 template <typename R>
-static GradWs<R> carve_grad(Carve& cv, int npv, int npb, int npar, int ng, int npt, int nblk, int ngrad) {
+static GradWs<R> carve_grad(Carve& cv, int npv, int npb, int npar, int ng, int npt, size_t npart, int ngrad) {
   GradWs<R> g;
   g.dc = cv.take<R>((size_t)npv * 50);
   g.tab = cv.take<R>((size_t)npv * npb * (1 + npar) * ng);
   g.dis = cv.take<R>((size_t)npv * npb * (npar > 0 ? npar : 1));
   g.dobs = cv.take<R>((size_t)npt);
   g.isig2 = cv.take<R>((size_t)npt);
-  g.partials = cv.take<double>((size_t)npv * nblk * (1 + ngrad));
+  g.partials = cv.take<double>(npart * (1 + ngrad));
   g.cconst = cv.take<double>((size_t)(npt + OBS_CHUNK - 1) / OBS_CHUNK);
   g.tiles64 = sizeof(R) == 8 ? cv.take<double>(4 * (((size_t)npt + TIME_TILE - 1) / TIME_TILE)) : nullptr;
   return g;
 }
 
-// Shares of a pv's row: the partial sums' count.
+// Shares of a pv's row.  In FP64 they follow the launch's size, counted for the
+// GB300's 152 SMs whatever device is current, so that a workspace holds for every
+// device.  (A partial sum per 2, 4 or 8 tiles in every launch would make the last
+// bits independent of the vectors beside one, and one vector's adjoint over 3000 x 5
+// samples 311, 411 or 712 us instead of 116.)
+constexpr int LNL64_SMS = 152;
+static int lnlike_f64_slots(int npt, int npv) { return f64_slots(npt, npv, LNL64_SMS); }
 static int lnlike_blocks(int split, int npt, int npv) {
-  return split ? (npt + LNL_CHUNK - 1) / LNL_CHUNK : f64_warps(npt, f64_slots(npt, npv));
+  return split ? (npt + LNL_CHUNK - 1) / LNL_CHUNK : f64_warps(npt, lnlike_f64_slots(npt, npv));
+}
+
+// Partial sums that a workspace has room for: at least npv lnlike_blocks(...) of
+// this and of every smaller call, so that one workspace for the largest population
+// serves all.  In FP64, with R = 16 x 152 warps a round and T = npv ntiles, f64_slots
+// gives a row at most four shares a tile, at most R shares in all below R tiles,
+// less than 2 R below 9 R tiles, and above T / w rounded up per row with w = 8, or
+// T / 4 R from 36 R on, or 64.
+static size_t lnlike_partials(int split, int npt, int npv) {
+  if (split) return (size_t)npv * lnlike_blocks(split, npt, npv);
+  const size_t ntiles = ((size_t)npt + TIME_TILE - 1) / TIME_TILE, n = (size_t)npv;
+  return std::min(4 * ntiles * n, 5 * 16 * (size_t)LNL64_SMS + n * (1 + ntiles / 64 + 1));
 }
 
 }  // namespace rr
@@ -977,12 +995,12 @@ int rr_lnlike_ngrad(int nkc, int nep, int npb, int npar) { return nkc + nep + 5 
 
 size_t rr_lnlike_workspace_bytes(int split, int npv, int npb, int nlc, int nep, int ng, int npar, int npt,
                                  int nkc) {
-  const int nblk = lnlike_blocks(split, npt, npv);
+  const size_t npart = lnlike_partials(split, npt, npv);
   const int ngrad = rr_lnlike_ngrad(nkc, nep, npb, npar);
   size_t base = split ? rr_full_split_workspace_bytes(npv, npb, nlc, nep, ng) : rr_full_f64_workspace_bytes(npv, npb, ng);
   Carve c(nullptr);
-  if (split) carve_grad<float>(c, npv, npb, npar, ng, npt, nblk, ngrad);
-  else carve_grad<double>(c, npv, npb, npar, ng, npt, nblk, ngrad);
+  if (split) carve_grad<float>(c, npv, npb, npar, ng, npt, npart, ngrad);
+  else carve_grad<double>(c, npv, npb, npar, ng, npt, npart, ngrad);
   return base + c.used + 512;
 }
 
@@ -1010,6 +1028,9 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
   if (npv > 65535) return RR_ERR_ARG;
   if (workspace_bytes < rr_lnlike_workspace_bytes(split, npv, npb, nlc, nep, ng, npar, npt, nkc))
     return RR_ERR_WORKSPACE;
+  const int nblk = lnlike_blocks(split, npt, npv);
+  const size_t npart = lnlike_partials(split, npt, npv);
+  if ((size_t)npv * nblk > npart) return RR_ERR_WORKSPACE;   // never: see lnlike_partials
   cudaStream_t s = as_stream(stream);
   size_t base = split ? rr_full_split_workspace_bytes(npv, npb, nlc, nep, ng) : rr_full_f64_workspace_bytes(npv, npb, ng);
   int st;
@@ -1031,9 +1052,8 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
     st = rr_prepare_f64(k, nkc, p, a, inc, e, w, npv, npb, (const double*)ldp, (const double*)weights, nk, ng, nz,
                         dk, kmin, kmax, z_edges, workspace, base, stream, 0, nullptr, 0, nullptr, 0);
   if (st) return st;
-  const int nblk = lnlike_blocks(split, npt, npv);
   Carve cv(static_cast<char*>(workspace) + base);
-  GradWs<R> g = carve_grad<R>(cv, npv, npb, npar, ng, npt, nblk, ngrad);
+  GradWs<R> g = carve_grad<R>(cv, npv, npb, npar, ng, npt, npart, ngrad);
   // prologue tables of the forward pass (inside the base workspace)
   Carve pcv(workspace);
   const double* orb64 = nullptr;
@@ -1083,7 +1103,7 @@ static int lnlike_impl(int split, int law, const double* ldc, int npar, const do
     A.dobs = g.dobs; A.isig2 = g.isig2; A.dc = g.dc; A.tab = g.tab; A.dis = g.dis;
     A.npar = npar; A.nep = nep; A.ngrad = ngrad; A.partials = g.partials;
     const dim3 grid(nblk, npv);
-    const int slots = f64_slots(npt, npv);
+    const int slots = lnlike_f64_slots(npt, npv);
     const size_t smem = sizeof(F64Lc) * (std::min(nlc, F64_LC_SMEM) + 1);
     if (grad) lnlike_f64_kernel<true><<<grid, 32, smem, s>>>(A, g.tiles64, slots);
     else lnlike_f64_kernel<false><<<grid, 32, smem, s>>>(A, g.tiles64, slots);
