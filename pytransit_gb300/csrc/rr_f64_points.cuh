@@ -33,9 +33,11 @@ __device__ __forceinline__ double f64_t0(const F64Args& A, int pv, int lc) {
 
 // Phase fold of the reference (model_full.py:84-86) with its rounding: the
 // epoch's conjunction t0 + epoch p, epoch = floor(((t - t0) + p/2) / p).
+__device__ __forceinline__ double f64_epoch(double t, double t0, double p, float inv_p) {
+  return f64_floor_div(__dadd_rn(__dsub_rn(t, t0), __dmul_rn(0.5, p)), p, inv_p);
+}
 __device__ __forceinline__ double f64_conjunction(double t, double t0, double p, float inv_p) {
-  const double epoch = f64_floor_div(__dadd_rn(__dsub_rn(t, t0), __dmul_rn(0.5, p)), p, inv_p);
-  return __dadd_rn(t0, __dmul_rn(epoch, p));
+  return __dadd_rn(t0, __dmul_rn(f64_epoch(t, t0, p, inv_p), p));
 }
 
 // Constants of one parameter vector: r^2(t) in FP64 and FP32.

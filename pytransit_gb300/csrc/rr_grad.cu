@@ -674,7 +674,7 @@ struct LnlF64Smem {
   double tot[NS];
   double row[GRAD ? 1 + MAX_NGRAD : 1];    // the share's columns
   double g[GRAD ? F64_Q : 1];              // per point of a chunk: -(r / sigma^2) w
-  float ep[GRAD ? F64_Q : 1];              // per point of a chunk: epoch
+  double ep[GRAD ? F64_Q : 1];             // per point of a chunk: epoch
   int lc;                                  // light curve of acc, or -1
 };
 
@@ -796,8 +796,8 @@ __device__ __noinline__ void lnl_f64_flush(const LnlF64Args& A, const F64Orbit& 
   const size_t ppb = (size_t)pv * A.npb + R.pb;
   const F64Transit T{o, A.ldm + ppb * A.ng, A.ng, A.dg};
   double lnl = S.acc[FS_LNL][lane], is = GRAD ? S.acc[GRAD ? FS_IS : 0][lane] : 0.0;
-  const double t0 = GRAD ? A.t0[(size_t)pv * A.ldt0 + A.epids[lc]] : 0.0;
-  const float inv_p = 1.0f / f32_of(A.p[pv]);
+  const double t0 = GRAD ? A.t0[(size_t)pv * A.ldt0 + A.epids[lc]] : 0.0, p = A.p[pv];
+  const float inv_p = 1.0f / f32_of(p);
   f64_sums(
       R, P, T, Q, n,
       [&](int i, double SQ) {
@@ -809,7 +809,7 @@ __device__ __noinline__ void lnl_f64_flush(const LnlF64Args& A, const F64Orbit& 
           const double rw = __dmul_rn(__dadd_rn(d, D), w);
           S.g[j] = __dmul_rn(-rw, R.w);
           is = __fma_rn(rw, D, is);
-          S.ep[j] = rintf(f32_of(__dsub_rn(__dsub_rn(A.times[pt], t0), Q.tc[i])) * inv_p);
+          S.ep[j] = f64_epoch(A.times[pt], t0, p, inv_p);   // the fold's
         }
       },
       [&](int i0, int ni) {
@@ -850,7 +850,7 @@ __device__ __noinline__ void lnl_f64_flush(const LnlF64Args& A, const F64Orbit& 
             }
             const double gt = __fma_rn(u, xd, __dmul_rn(v, yd));   // dL/dz dz/dt
             a[FS_T] = __dadd_rn(a[FS_T], gt);
-            if (S.ep[it] != 0.0f) a[FS_P] = __fma_rn(gt, f64_of(S.ep[it]), a[FS_P]);
+            a[FS_P] = __fma_rn(gt, S.ep[it], a[FS_P]);
 #pragma unroll
             for (int m = 0; m < 5; ++m) {
               a[FS_M0 + m] = __dadd_rn(a[FS_M0 + m], u);
