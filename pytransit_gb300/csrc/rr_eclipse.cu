@@ -48,7 +48,7 @@ __device__ inline double eclipse_ltt(double a, double inc, double e, double w, d
 // thread's FP64 instructions are issued ~75 cycles apart, so the four parts
 // run on four warps, lane = pv: the mean anomalies at the two conjunctions, the
 // orbit, and the light travel time (1000 pv: 76 us on one thread per pv, with
-// the FP64 bisections and Kepler's equation; 12 us).
+// the FP64 bisections and Kepler's equation; 14 us).
 constexpr int ECL_PREP_THREADS = 128;
 
 __global__ void __launch_bounds__(ECL_PREP_THREADS)
@@ -64,13 +64,14 @@ eclipse_prepare_kernel(const double* __restrict__ k, const double* __restrict__ 
     if (warp < 2) {
       s_m[warp][lane] = conjunction_anomaly(e[pv], w[pv], warp == 0 ? 0.0 : PI);
     } else if (warp == 2) {
-      double c[10], t1, t4;
+      double c[10], d[R2_N], t1, t4;
       solve2d_ecl(p[pv], a[pv], inc[pv], e[pv], w[pv], c);
-      contact_box(k[pv], c, t1, t4);
+      r2_poly(c, d);
+      contact_times(k[pv], c, d, t1, t4);
       for (int i = 0; i < 10; ++i) o[i] = c[i];
       o[10] = t1;
       o[11] = t4;
-      r2_poly(c, o + ORB64_R2);
+      for (int i = 0; i < R2_N; ++i) o[ORB64_R2 + i] = d[i];
     } else {
       s_ltt[lane] = eclipse_ltt(a[pv], inc[pv], e[pv], w[pv], rstar[pv]);
     }
@@ -103,7 +104,7 @@ __device__ __noinline__ double ecl_point_f64(const EclF64Args& A, int pv, int lc
   F64Lc R;
   f64_lc(A, pv, lc, P, R);
   const float tf = f32_of(tc);
-  if (!(R.lo <= tf && tf <= R.hi)) return R.disk.area_in;
+  if (!(R.lo <= tf && tf <= R.hi && f64_in_box(A, P, R, tc))) return R.disk.area_in;
   return f64_point_value(R, P, F64Eclipse{o}, tc);
 }
 
@@ -132,7 +133,11 @@ static __device__ __noinline__ void ecl_flush(const EclF64Args& A, const F64Orbi
   const F64Lc& R = recs[min(lc, nrec)];
   const F64Eclipse T{o};
   double* row = A.flux + (size_t)pv * A.ldflux;
-  f64_sums(R, P, T, Q, n, [&](int i, double D) { __stcs(row + Q.pt[i], T.value(R, D)); }, [](int, int) {});
+  f64_sums(R, P, T, Q, n,
+           [&](int i, double D) {
+             __stcs(row + Q.pt[i], f64_in_box(A, P, R, Q.tc[i]) ? T.value(R, D) : R.disk.area_in);
+           },
+           [](int, int) {});
 }
 
 struct EclSink {
@@ -265,7 +270,7 @@ __global__ void __launch_bounds__(32, 20) es_flux_kernel(const __grid_constant__
       if (!(r < R.lo - err || r > R.hi + err) || fabsf(r) > 0.5f * fabsf(pf) - err || !(fabsf(sf * inv_p) < 1e5f)) {
         tc = __dsub_rn(t, f64_conjunction(t, te, p, inv_p));
         const float tf = f32_of(tc);
-        in = R.lo <= tf && tf <= R.hi;
+        in = R.lo <= tf && tf <= R.hi && f64_in_box(A, P, R, tc);
       }
     }
     const unsigned bm = __ballot_sync(FULL, in);
@@ -680,7 +685,7 @@ int rr_es_f64(const double* times, int npt, const double* k, const double* t0, c
   EsF64Args A{};
   A.times = times; A.npt = npt; A.k = k; A.t0 = t0; A.ldt0 = 1; A.p = p;
   A.orb64 = rec; A.shift = rec + ECL_SHIFT; A.npv = npv; A.nlc = 1; A.nkc = A.npb = 1; A.dg = 1.0;
-  A.pad0 = 0.0015f; A.ns0 = nsamples0; A.ex0 = exptime0;
+  A.pad0 = 0.0015; A.pad0f = 0.001500005f; A.ns0 = nsamples0; A.ex0 = exptime0;
   A.fratio = fratio; A.nch = npb; A.flux = flux; A.ldflux = ldflux;
   // 32-point slots per warp: four rounds of 16 warps per SM, at most 32 slots
   const long long total = (long long)((npt + 31) / 32) * npv, want = total / (64LL * sm_count());

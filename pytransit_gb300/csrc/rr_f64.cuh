@@ -104,6 +104,12 @@ __device__ __forceinline__ float f32_of(double d) {
   const unsigned m = min(max((int)(hi & 0x7fffffffu), F64_BIAS), F64_BIAS + (254 << 20)) - F64_BIAS;
   return __uint_as_float(__funnelshift_l(__double2loint(d), m, 3) | (hi & 0x80000000u));
 }
+// Neither infinite nor NaN.
+__device__ __forceinline__ bool f64_finite(double d) { return (__double2hiint(d) & 0x7ff00000) != 0x7ff00000; }
+// FP32 of a double, its magnitude rounded up by an ulp; NaN and infinity stay.
+__device__ __forceinline__ float f32_up(double d) {
+  return f64_finite(d) ? __uint_as_float(__float_as_uint(f32_of(d)) + 1u) : (float)d;
+}
 // FP64 of a non-negative FP32 value (0 becomes 2^-127).
 __device__ __forceinline__ double f64_of_pos(float f) {
   const unsigned b = __float_as_uint(f);
@@ -114,8 +120,6 @@ __device__ __forceinline__ double f64_of(float f) {
   const unsigned b = __float_as_uint(f);
   return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + F64_BIAS)), (int)(b << 29));
 }
-// Neither infinite nor NaN.
-__device__ __forceinline__ bool f64_finite(double d) { return (__double2hiint(d) & 0x7ff00000) != 0x7ff00000; }
 // Magnitude between 2^-100 and 2^100 and a positive sign (excludes NaN).
 __device__ __forceinline__ bool f64_moderate(double d) {
   return (unsigned)__double2hiint(d) - ((1023u - 100u) << 20) < (200u << 20);
@@ -214,25 +218,6 @@ __device__ __forceinline__ void table_place(double k, double kmin, double dk, do
 }
 
 // ---------------------------------------------------------------------------
-// Outer contact times for the bounding box, by the FP32 bisection
-// (contact_points14_f32) on the rounded coefficients.  The box decides only
-// which points are evaluated: F = 1 from the contacts outwards, in or out of
-// it.  So the FP32 times are moved outwards by their own error, the shift dt
-// with |d(z^2)| = 2 z v dt below 4e-6 or, for a grazing orbit, the whole time
-// in which z^2 moves by that much.
-// ---------------------------------------------------------------------------
-__device__ inline void contact_box(double k, const double* c, double& t1, double& t4) {
-  float cf[10];
-#pragma unroll
-  for (int i = 0; i < 10; ++i) cf[i] = (float)c[i];
-  float a, b;
-  contact_points14_f32((float)k, cf, a, b);
-  const float iv = 1.0f / fabsf(cf[1]), most = 2e-3f * iv;
-  t1 = (double)(a - fmaf(fabsf(a), 1e-6f, fminf(most, 2e-6f * iv * iv / fabsf(a))));
-  t4 = (double)(b + fmaf(fabsf(b), 1e-6f, fminf(most, 2e-6f * iv * iv / fabsf(b))));
-}
-
-// ---------------------------------------------------------------------------
 // r^2(t) = x(t)^2 + y(t)^2 of a Taylor orbit c[0..9], degree 8.
 // ---------------------------------------------------------------------------
 constexpr int R2_N = 9;
@@ -273,6 +258,129 @@ __device__ __forceinline__ bool r2_is_even(const double* d) {
 #pragma unroll
   for (int m = 1; m < R2_N; m += 2) any |= (__double2hiint(d[m]) << 1) | __double2loint(d[m]);
   return any == 0;
+}
+
+// ---------------------------------------------------------------------------
+// Outer contact times for the bounding box: contact_point's bisection (bracket [0,
+// +-2/vx], 1e-6 d), whose end is a fixed fraction of the bracket that the signs of z -
+// (1 + k) at the midpoints choose.  The box belongs to the vector's first radius
+// ratio (and a grazing or close orbit may have no contact in the bracket), so its edge
+// can cut through a transit and has to be that fraction exactly.  But a sign does not
+// need FP64: most are sure in FP32 within its error bound, and the others, next to
+// the contact, from r^2's value in FP64 at one point and its derivatives in FP32.
+// (FP64 throughout: ~1350 dependent FP64 instructions, 40 us; a sign in FP64 or in
+// FP32 pairs wherever FP32 leaves a doubt: 7 or 5 us more than FP32 alone.)
+// ---------------------------------------------------------------------------
+static __device__ __noinline__ void contact_times_general(double k, const double* c, double& t1, double& t4) {
+  t1 = contact_point(k, 1, c);
+  t4 = contact_point(k, 4, c);
+}
+
+// Sign of r^2 - zt2 at t; 0 for neither, as NaN.
+static __device__ __noinline__ int r2_sign(const double* d, double zt2, double t) {
+  const double D = __dadd_rn(r2_at(d, false, t), -zt2);
+  return D < 0.0 ? -1 : (D > 0.0 ? 1 : 0);
+}
+
+// One contact (dir -1 or 1): FP32 bisection of [0, dir T].
+struct ContactBisection {
+  int a, sign0;        // bracket [a, a + 1] / 2^n of T; sign at its lower end
+  int n_u, a_u, s_u;   // level and state at the first sign in doubt, n_u < 0: none
+};
+
+__device__ __forceinline__ void contact_step(const float* cf, float zt2, float T, float dir, int n, ContactBisection& B) {
+  const float t = dir * T * ((float)(2 * B.a + 1) * __int_as_float((126 - n) << 23)), ta = fabsf(t);
+  float x = cf[4], y = cf[9], xa = fabsf(cf[4]), ya = fabsf(cf[9]);
+#pragma unroll
+  for (int j = 3; j >= 0; --j) {
+    x = fmaf(x, t, cf[j]);
+    y = fmaf(y, t, cf[5 + j]);
+    xa = fmaf(xa, ta, fabsf(cf[j]));
+    ya = fmaf(ya, ta, fabsf(cf[5 + j]));
+  }
+  // 56 roundings of the partial sums' magnitudes: coefficients (1), time (4 in t, up to
+  // the fourth power), Horner (9), each twice in the squares
+  const float diff = fmaf(x, x, fmaf(y, y, -zt2)), tol = 3.5e-6f * fmaf(xa, xa, fmaf(ya, ya, zt2));
+  const int s = diff < 0.0f ? -1 : 1;
+  if (!(fabsf(diff) > tol) && B.n_u < 0) {
+    B.n_u = n;
+    B.a_u = B.a;
+    B.s_u = B.sign0;
+  }
+  const bool lower = B.sign0 * s < 0;
+  B.a = 2 * B.a + (lower ? 0 : 1);
+  if (!lower) B.sign0 = s;
+}
+
+// The bisection again from its first sign in doubt, with r^2 - zt2 about its end tc:
+// f0 in FP64, and in x = t / tc - 1 its first two derivatives g1, g2 in FP32 and a bound of
+// the rest.
+__device__ __forceinline__ int contact_refine(const double* d, const float* df, double zt2, double T, float dir,
+                                              int halvings, const ContactBisection& B) {
+  const int mc = 2 * B.a + 1;   // tc in units of T / 2^(halvings + 1)
+  const double unit = __dmul_rn(dir < 0.0f ? -T : T, __hiloint2double((1022 - halvings) << 20, 0));
+  const double tc = __dmul_rn(unit, (double)mc);
+  const float f0 = (float)__dadd_rn(r2_at(d, false, tc), -zt2), t = f32_of(tc), ta = fabsf(t);
+  float g1 = 8.0f * df[8], g2 = 28.0f * df[8], mag = fabsf(df[8]);
+#pragma unroll
+  for (int m = 7; m >= 0; --m) {
+    g1 = fmaf(g1, t, (float)m * df[m]);
+    g2 = fmaf(g2, t, (float)(m * (m - 1) / 2) * df[m]);
+    mag = fmaf(mag, ta, fabsf(df[m]));
+  }
+  int a = B.a_u, s0 = B.s_u;
+  const float ic = 1.0f / (float)mc;
+  for (int n = B.n_u; n < halvings; ++n) {
+    const int g = (2 * a + 1) << (halvings - n);
+    const float x = (float)(g - mc) * ic, xa = fabsf(x);
+    const float L = fmaf(x, fmaf(x, g2, g1), f0);
+    // g1 and g2 within 2e-5 and 6e-5, the third derivative's share within 60 of the magnitude
+    const float tol = fmaf(2e-7f, fabsf(f0) + fabsf(x * g1), mag * fmaf(xa, fmaf(xa, fmaf(xa, 60.0f, 6e-5f), 2e-5f), 1e-13f));
+    int s = L < 0.0f ? -1 : 1;
+    if (!(fabsf(L) > tol && xa < 0.01f)) s = r2_sign(d, zt2, __dmul_rn(unit, (double)g));
+    const bool lower = s0 * s < 0;
+    a = 2 * a + (lower ? 0 : 1);
+    if (!lower) s0 = s;
+  }
+  return a;
+}
+
+// c: the orbit, d: its r^2.
+__device__ __forceinline__ void contact_times(double k, const double* c, const double* d, double& t1, double& t4) {
+  const double zt = __dadd_rn(1.0, k), vx = fabs(c[1]);
+  // brackets of at most 512 d, so that a midpoint's number is an int; k > -1
+  if (!f64_moderate(vx) || vx < 1.0 / 256 || __double2hiint(zt) <= 0) {
+    contact_times_general(k, c, t1, t4);
+    return;
+  }
+  double T = f64_recip(vx);
+  T = __dadd_rn(T, T);
+  const double zt2 = __dmul_rn(zt, zt);
+  float cf[10];
+#pragma unroll
+  for (int i = 0; i < 10; ++i) cf[i] = f32_near(c[i]);
+  const float Tf = f32_of(T), zt2f = f32_near(zt2);
+  // halvings until the bracket is no longer than 1e-6 d: at most 29
+  const long long bt = __double_as_longlong(T), b6 = __double_as_longlong(1e-6), frac = (1ll << 52) - 1;
+  const int halvings = max((int)((bt >> 52) - (b6 >> 52)) + ((bt & frac) > (b6 & frac) ? 1 : 0), 0);
+  const double D0 = __dadd_rn(d[0], -zt2);
+  const int s0 = D0 < 0.0 ? -1 : (D0 > 0.0 ? 1 : 0);
+  ContactBisection A{0, s0, -1, 0, 0}, B = A;
+#pragma unroll 1
+  for (int n = 0; n < halvings; ++n) {
+    contact_step(cf, zt2f, Tf, -1.0f, n, A);
+    contact_step(cf, zt2f, Tf, 1.0f, n, B);
+  }
+  if (A.n_u >= 0 || B.n_u >= 0) {
+    float df[R2_N];
+#pragma unroll
+    for (int m = 0; m < R2_N; ++m) df[m] = f32_near(d[m]);
+    if (A.n_u >= 0) A.a = contact_refine(d, df, zt2, T, -1.0f, halvings, A);
+    if (B.n_u >= 0) B.a = contact_refine(d, df, zt2, T, 1.0f, halvings, B);
+  }
+  const double unit = __dmul_rn(T, __hiloint2double((1022 - halvings) << 20, 0));
+  t1 = -__dmul_rn(unit, (double)(2 * A.a + 1));
+  t4 = __dmul_rn(unit, (double)(2 * B.a + 1));
 }
 
 // ---------------------------------------------------------------------------

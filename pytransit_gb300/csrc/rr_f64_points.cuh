@@ -18,7 +18,8 @@ struct F64Args {
   // the eclipse models: no LD tables (istar, pbids null, npb = nkc = 1); the
   // eclipse's shift and light travel time at shift[pv * ORB64]
   const double* shift;
-  float pad0 = 0.003f; // box padding beyond the contacts and the exposure
+  double pad0 = 0.003; // box padding beyond the contacts and the exposure
+  float pad0f = 0.00300001f;
   int ns0;             // for null nsamples / exptimes
   double ex0;
 };
@@ -44,7 +45,8 @@ __device__ __forceinline__ double f64_conjunction(double t, double t0, double p,
 struct F64Orbit {
   double d[R2_N];
   float df[R2_N];
-  float t1, t4;        // contacts
+  double t1, t4;       // contacts
+  float t1f, t4f;      // rounded outwards
   int even;
   int finite;          // every coefficient is
 };
@@ -58,8 +60,10 @@ __device__ __forceinline__ void f64_orbit(const double* o, F64Orbit& P) {
     fin = fin && f64_finite(P.d[m]);
   }
   P.finite = fin;
-  P.t1 = (float)o[10];
-  P.t4 = (float)o[11];
+  P.t1 = o[10];
+  P.t4 = o[11];
+  P.t1f = f32_up(P.t1);
+  P.t4f = f32_up(P.t4);
   P.even = r2_is_even(P.d);
 }
 
@@ -68,9 +72,31 @@ struct F64Lc {
   F64Disk disk;
   double w;            // 1 / (istar nsamples); NaN for a non-finite istar (A.nan_istar)
   double ex, step;     // exposure time and its share of one sample
-  float lo, hi;        // box
+  float lo, hi;        // box, its edges rounded outwards
+  int hlo, hhi;        // upper words of FP64 magnitudes surely inside them
   int ns, pb;
 };
+
+// Box: the contact times padded by 0.003 d + exposure (model_full.py:87-89), the
+// edges rounded outwards to FP32 (by less than 5e-7 of its width).
+__device__ __forceinline__ void f64_box_edges(const F64Args& A, const F64Orbit& P, double ex, float& lo, float& hi) {
+  const float pad = __fadd_ru(A.pad0f, f32_up(ex));
+  lo = __fsub_rd(P.t1f, pad);
+  hi = __fadd_ru(P.t4f, pad);
+}
+
+// Is a point that the FP32 edges put in the box there by the FP64 ones?  They decide
+// close to an edge: the flux need not be 1 on its inside (several radius ratios with
+// the first one's box, contacts that are not in the bisection's bracket).  A walk
+// queues points by the FP32 edges and its flush asks this of each.
+static __device__ __noinline__ bool f64_in_box_exact(const F64Args& A, const F64Orbit& P, double ex, double tc) {
+  const double pad = __dadd_rn(A.pad0, ex);
+  return __dsub_rn(P.t1, pad) <= tc && tc <= __dadd_rn(P.t4, pad);
+}
+__device__ __forceinline__ bool f64_in_box(const F64Args& A, const F64Orbit& P, const F64Lc& R, double tc) {
+  const int h = __double2hiint(tc);
+  return (h & 0x7fffffff) < (h < 0 ? R.hlo : R.hhi) || f64_in_box_exact(A, P, R.ex, tc);
+}
 
 template <bool IK = false>
 __device__ __forceinline__ void f64_lc(const F64Args& A, int pv, int lc, const F64Orbit& P, F64Lc& R) {
@@ -78,12 +104,11 @@ __device__ __forceinline__ void f64_lc(const F64Args& A, int pv, int lc, const F
   R.ns = max(A.nsamples ? A.nsamples[lc] : A.ns0, 0);
   R.ex = A.exptimes ? A.exptimes[lc] : A.ex0;
   R.step = R.ns > 1 ? __ddiv_rn(R.ex, (double)R.ns) : R.ex;
-  // Box: the contact times padded by 0.003 d + exposure (model_full.py:87-89).
-  // It only separates points that may overlap the star from points that
-  // cannot (F = 1 on both sides of its edges), so it is FP32.
-  const float ex = f32_of(R.ex), pad = A.pad0 + ex;
-  R.lo = P.t1 - pad;
-  R.hi = P.t4 + pad;
+  const float ex = f32_up(R.ex);
+  f64_box_edges(A, P, R.ex, R.lo, R.hi);
+  // an upper word's last place is 5e-7 to 1e-6 of the value, the edges' rounding 5e-7
+  R.hlo = (int)((__float_as_uint(R.lo) & 0x7fffffffu) >> 3) + F64_BIAS - 2;
+  R.hhi = (int)((__float_as_uint(R.hi) & 0x7fffffffu) >> 3) + F64_BIAS - 2;
   // bound of the FP32 r^2's error at any sample: 16 roundings of the largest partial sums
   const float tb = fmaxf(fabsf(R.lo), fabsf(R.hi)) + ex;
   float sum = fabsf(P.df[R2_N - 1]);
@@ -199,9 +224,7 @@ __device__ __forceinline__ void f64_box(const F64Args& A, const F64Orbit& P, int
     lo = recs[lc].lo;
     hi = recs[lc].hi;
   } else {
-    const float pad = A.pad0 + f32_of(A.exptimes[lc]);
-    lo = P.t1 - pad;
-    hi = P.t4 + pad;
+    f64_box_edges(A, P, A.exptimes[lc], lo, hi);
   }
 }
 

@@ -365,21 +365,20 @@ __device__ __forceinline__ void orbit_pv_f64(const OrbitArgs& A, int pv) {
                          : isnan(((const double*)A.ldp)[(size_t)pv * A.npb * A.nz]);
   }
   const bool valid = !(isnan(a) || a <= 1.0 || e < 0.0 || ldbad);
-  double c[10];
+  double c[10] = {}, d[R2_N] = {};
   double t1 = 0.0, t4 = 0.0;
   const double k0 = A.k[(size_t)pv * A.nkc];
   if (valid) {
     solve2d_conj(p, a, A.inc[pv], e, A.w[pv], c);
-    contact_box(k0, c, t1, t4);
-  } else {
-    for (int i = 0; i < 10; ++i) c[i] = 0.0;
+    r2_poly(c, d);
+    contact_times(k0, c, d, t1, t4);
   }
   double* o = A.orb64 + (size_t)pv * ORB64;
   for (int i = 0; i < 10; ++i) o[i] = c[i];
   o[10] = t1;
   o[11] = t4;
   o[12] = valid ? 1.0 : 0.0;
-  r2_poly(c, o + ORB64_R2);
+  for (int i = 0; i < R2_N; ++i) o[ORB64_R2 + i] = d[i];
 }
 
 // Split path: the FP32 orbit record [ORB32] and the per-light-curve records
@@ -602,8 +601,8 @@ __global__ void __launch_bounds__(PRO_THREADS, 8) prologue_split_kernel(ProArgs 
 // The same for the plain FP64 path: ld_tables_kernel<double>,
 // ldm_basis_kernel<double> and orbit_kernel<false> in one launch.  The three
 // took 74 + 63 + 53 us for 8192 pv x 4 passbands, each bound by the FP64 pipe
-// or by one thread's chain of FP64 instructions; this one takes 52 us (77 pv
-// x 1: 9 us, against 4 + 4 + 51).  Here the chains run beside
+// or by one thread's chain of FP64 instructions; this one takes 54 us (77 pv
+// x 1: 12 us, against 4 + 4 + 51).  Here the chains run beside
 // the LD blocks; the two k rows of a basis column are blended once for all
 // passbands (2 NB + NB npb FP64 instructions per column instead of
 // 2 (NB + 1) npb); and the profile on the mu grid is evaluated only for a k
@@ -691,7 +690,7 @@ __device__ __noinline__ double f64_point(const F64Args& A, int pv, int lc, doubl
   F64Lc R;
   f64_lc(A, pv, lc, P, R);
   const float tf = f32_of(tc);
-  if (!(R.lo <= tf && tf <= R.hi)) return 1.0;
+  if (!(R.lo <= tf && tf <= R.hi && f64_in_box(A, P, R, tc))) return 1.0;
   return f64_point_value(R, P, F64Transit{o, A.ldm + ((size_t)pv * A.npb + R.pb) * A.ng, A.ng, A.dg}, tc);
 }
 
@@ -748,7 +747,10 @@ static __device__ __noinline__ void f64_flux_flush(const FluxF64Args& A, const F
   const F64Lc& R = recs[min(lc, nrec)];
   const F64Transit T{o, A.ldm + ((size_t)pv * A.npb + R.pb) * A.ng, A.ng, A.dg};
   double* row = A.flux + (size_t)pv * A.ldflux;
-  f64_sums(R, P, T, Q, n, [&](int i, double D) { __stcs(row + Q.pt[i], T.value(R, D)); },
+  f64_sums(R, P, T, Q, n,
+           [&](int i, double D) {
+             __stcs(row + Q.pt[i], f64_in_box(A, P, R, Q.tc[i]) ? T.value(R, D) : 1.0);
+           },
            [](int, int) {});
 }
 

@@ -802,12 +802,13 @@ __device__ __noinline__ void lnl_f64_flush(const LnlF64Args& A, const F64Orbit& 
       R, P, T, Q, n,
       [&](int i, double SQ) {
         const int pt = Q.pt[i];
-        const double D = __dmul_rn(SQ, R.w), d = A.dobs[pt], w = A.isig2[pt];
+        const bool in = f64_in_box(A, P, R, Q.tc[i]);
+        const double D = in ? __dmul_rn(SQ, R.w) : 0.0, d = A.dobs[pt], w = A.isig2[pt];
         lnl = __fma_rn(-__dmul_rn(__fma_rn(0.5, D, d), D), w, lnl);
         if constexpr (GRAD) {
           const int j = i % (F64_Q / min(max(R.ns, 1), F64_Q));   // the point's place in its chunk
           const double rw = __dmul_rn(__dadd_rn(d, D), w);
-          S.g[j] = __dmul_rn(-rw, R.w);
+          S.g[j] = in ? __dmul_rn(-rw, R.w) : 0.0;
           is = __fma_rn(rw, D, is);
           S.ep[j] = f64_epoch(A.times[pt], t0, p, inv_p);   // the fold's
         }

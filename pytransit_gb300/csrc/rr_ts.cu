@@ -529,13 +529,14 @@ __global__ void __launch_bounds__(128) ts64_prologue_kernel(TsProArgs<double> P,
     const double km = ((s_sum[0] + s_sum[1]) + s_sum[2]) / npb;
     const double kx = fmax(fmax(s_max[0], s_max[1]), s_max[2]);
     if (valid && tid == 0) {
-      double t1, t4;
-      contact_box(km, s_c, t1, t4);
+      double d[R2_N], t1, t4;
+      r2_poly(s_c, d);
+      for (int i = 0; i < R2_N; ++i) s_d[i] = d[i];
+      contact_times(km, s_c, d, t1, t4);
       const double pad = 0.0015 + P.exptime0;
       s_t[0] = t1 - pad;
       s_t[1] = t4 + pad;
     }
-    if (valid && tid == 32) r2_poly(s_c, s_d);
     double* u = P.ldm + (size_t)pv * npb * ng + (size_t)nb * ng;
     const double ikm2 = 1.0 / (km * km);
     for (int b = tid; b < npb; b += blockDim.x) {
