@@ -134,6 +134,15 @@ __device__ __forceinline__ float f32_near(double d) {
   return __uint_as_float(__funnelshift_l((unsigned)b, (hi & 0x7fffffffu) - F64_BIAS, 3) | (hi & 0x80000000u));
 }
 
+// FP32 pair (48 bits) of a double: its upper 24 bits and the rest.  Below 2^-70, where
+// FP32 does not hold the rest, the rounded value alone; so too above 2^100 and for NaN.
+__device__ __forceinline__ float2 f32_pair(double d) {
+  const int e = (__double2hiint(d) >> 20) & 0x7ff;
+  if (e < 1023 - 70 || e > 1023 + 100) return make_float2((float)d, 0.0f);
+  const float h = f32_of(d), rest = (float)(__double2loint(d) & 0x1fffffff) * __int_as_float((e - 1023 - 52 + 127) << 23);
+  return make_float2(h, copysignf(rest, h));
+}
+
 // Square root of a moderate x and its reciprocal, from the FP32 reciprocal
 // root g: with e = 1 - x g^2 (|e| < 4e-7), 1/sqrt(x) = g (1 + e/2 + 3 e^2/8 +
 // O(e^3)), the quadratic term (below 1e-13) in FP32.

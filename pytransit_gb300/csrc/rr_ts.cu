@@ -143,8 +143,8 @@ constexpr int TS_L2_ROWS = 16;   // g rows of the 2D table per LD block
 //   blocks [0, npv): per-pv blocks: mean and largest k, orbit, box, record;
 //   blocks [npv, ...): LD blocks (pv, chunk of TS_L2_ROWS rows, chunk of
 //     channels): the same k statistics (the same reduction, so the same
-//     bits; the split path's inner row chunks, which need the mean in FP32
-//     alone, sum it in FP32 pairs), the channels' LD profiles (from the law's coefficients, or read
+//     bits; the split path's inner row chunks, which need the mean rounded to
+//     FP32 alone, sum it in FP32 pairs), the channels' LD profiles (from the law's coefficients, or read
 //     from ldp for a host-evaluated law) staged in shared memory, the 2D
 //     table rows at kmean, the LD means by 16-byte shared-memory loads; the
 //     blocks of the first row chunk also write the channel records (afac,
@@ -192,21 +192,35 @@ __device__ __forceinline__ void ts_kstats(const double* __restrict__ kp, int npb
   }
 }
 
-// Mean of pv's radius ratios in FP32: each warp's lanes sum their channels, and
-// the lanes' sums are added, as (sum, error) pairs.
-__device__ __forceinline__ float ts_kmean_f32(const double* __restrict__ kp, int npb) {
+// Mean of pv's radius ratios as an FP32 pair (hi the mean's FP32 value, 2^-44 in all)
+// without the FP64 pipe: the ratios as pairs, summed with their errors by each warp.
+__device__ __forceinline__ float2 ts_kmean_pair(const double* __restrict__ kp, int npb) {
   float sm = 0.0f, er = 0.0f, t, e;
   for (int b = threadIdx.x & 31; b < npb; b += 32) {
-    two_sum(sm, f32_near(kp[b]), t, e);
+    const float2 k = f32_pair(kp[b]);
+    two_sum(sm, k.x, t, e);
     sm = t;
-    er += e;
+    er += e + k.y;
   }
   for (int o = 16; o > 0; o >>= 1) {
     two_sum(sm, __shfl_xor_sync(0xffffffffu, sm, o), t, e);
     er += __shfl_xor_sync(0xffffffffu, er, o) + e;
     sm = t;
   }
-  return (sm + er) / (float)npb;
+  const float n = (float)npb, q = (sm + er) / n, rest = (fmaf(-q, n, sm) + er) / n;
+  return make_float2(q + rest, rest - ((q + rest) - q));
+}
+
+// The mean of ts_kstats, the same bits, by one warp.
+static __device__ __noinline__ double ts_kmean_f64(const double* __restrict__ kp, int npb) {
+  double total = 0.0;
+  for (int w = 0; w < 3; ++w) {
+    double sm = 0.0;
+    for (int b = 32 * w + (threadIdx.x & 31); b < npb; b += 96) sm += kp[b];
+    for (int o = 16; o > 0; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
+    total = w == 0 ? sm : total + sm;
+  }
+  return total / npb;
 }
 
 template <typename R, bool SPLIT>
@@ -303,19 +317,27 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 4) ts_prologue_kerne
   // FP64 mean: the channel records (first row chunk), the grazing last row
   const bool exact = !SPLIT || rc == 0 || rc == P.nrc - 1;
   double k = 0.0;
-  float kf = 0.0f;
-  if (exact) ts_kstats(kp, npb, s_sum, s_max);
-  else kf = ts_kmean_f32(kp, npb);
+  float kf = 0.0f, opk_f = 1.0f;   // k and 1 + k rounded to FP32
+  if (exact) {
+    ts_kstats(kp, npb, s_sum, s_max);
+  } else {
+    const float2 m = ts_kmean_pair(kp, npb);
+    float e;
+    kf = m.x;
+    two_sum(1.0f, m.x, opk_f, e);
+    opk_f += e + m.y;
+  }
   __syncthreads();
   if (exact) {
     k = ((s_sum[0] + s_sum[1]) + s_sum[2]) / npb;
     kf = (float)k;
+    opk_f = (float)(1.0 + k);
   }
   // the 2D table rows at kmean (calculate_weights_2d, common.py:153-185): a
   // warp per row, lanes over z (z and z + 32), the differences through
   // shuffles, the row sum by a shuffle tree
   const double gstep = P.gstep;
-  const float gstep_f = (float)gstep, opk_f = 1.0f + kf;
+  const float gstep_f = (float)gstep;
   for (int r = warp; r < nr; r += blockDim.x >> 5) {
     const int g = g0 + r;
     const bool f64 = !SPLIT || g == ng - 1;   // the split path's grazing last row: FP64 areas
@@ -339,7 +361,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 8 : 4) ts_prologue_kerne
         continue;
       }
       // a row left without area in FP32: the FP64 path below
-      if (!exact) k = (double)kf;
+      if (!exact) k = ts_kmean_f64(kp, npb);   // warp-uniform
     }
     const double gg = (g == ng - 1) ? 1.0 - 1e-7 : (double)g * gstep;
     double av[2];
