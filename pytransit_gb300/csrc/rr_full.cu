@@ -897,11 +897,16 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
 // per sample; the samples of up to SPLIT_ROWS rows (32 points x 1 sample) get
 // their separation and LD mean first, which finishes those inside the star,
 // and the overlap area of the samples on the limb (about a third) follows in
-// full warps from a list.  A point's terms are added in sample order.  4096 pv
+// full warps from a list.  A point's terms are added as a tree within SPLIT_ROWS
+// samples, and the sums of more rounds (each folds its points again) with their
+// rounding errors.  4096 pv
 // x 118,526 times x 10 samples: 2682 us with each tile's (point, sample) pairs
 // by themselves (a binary search for a pair's point, the full area for every
-// pair, a segmented shuffle sum), 1691 us.  Ranges of 64, 128 and 256 tiles per
+// pair, a segmented shuffle sum), 1672 us.  Ranges of 64, 128 and 256 tiles per
 // block instead of 32: 5, 8 and 14 % slower.
+// MANY: more samples than SPLIT_ROWS, so that a point's sum so far and its error live across
+// rounds (two registers that the common case does without).
+template <bool MANY>
 __device__ __forceinline__ int split_flush(const float2* __restrict__ times, const float* orb, const float* R,
                                            const float* ldm_pv, int ng, float inv_dg, SplitQueue& Q, int n, bool all,
                                            const SplitRow& row) {
@@ -919,11 +924,11 @@ __device__ __forceinline__ int split_flush(const float2* __restrict__ times, con
   const float2 cc = *reinterpret_cast<const float2*>(orb + 8);
   const float4 fold = *reinterpret_cast<const float4*>(R), box = *reinterpret_cast<const float4*>(R + 4);
   const int take = all ? n : n & ~31;
-  const int sc = min(max(ns_all, 1), SPLIT_ROWS), nb = SPLIT_ROWS / sc;   // samples, batches of 32 points at once
+  const int sc = MANY ? SPLIT_ROWS : max(ns_all, 1), nb = MANY ? 1 : SPLIT_ROWS / sc;   // samples, batches of 32 points at once
   for (int i0 = 0; i0 < take; i0 += 32 * nb) {
-    float D = 0.0f;   // with more samples than rows (nb = 1): the point's sum so far
-    for (int s0 = 0; s0 < max(ns_all, 1); s0 += sc) {
-      const int ns = min(sc, ns_all - s0);
+    float Dh = 0.0f, Dl = 0.0f;
+    for (int s0 = 0; s0 < (MANY ? ns_all : 1); s0 += sc) {
+      const int ns = MANY ? min(sc, ns_all - s0) : ns_all;
       int nlimb = 0, r = 0;
       for (int b = i0; b < min(take, i0 + 32 * nb); b += 32) {
         // time_offset = exptime ((isample - 0.5)/ns - 0.5), isample = s0 + s + 1
@@ -973,11 +978,27 @@ __device__ __forceinline__ int split_flush(const float2* __restrict__ times, con
         Q.term[f] *= a;
       }
       __syncwarp();
-      const bool last = s0 + ns >= ns_all;
+      const bool last = !MANY || s0 + ns >= ns_all;
       r = 0;
       for (int b = i0; b < min(take, i0 + 32 * nb); b += 32) {
-        if (s0 == 0) D = 0.0f;
-        for (int s = 0; s < ns; ++s, r += 32) D += Q.term[r + lane];
+        float D = 0.0f;
+        const float* q = Q.term + r + lane;
+        int s = 0;
+        for (; s + 4 <= ns; s += 4) D += (q[32 * s] + q[32 * (s + 1)]) + (q[32 * (s + 2)] + q[32 * (s + 3)]);
+        if (s < ns) {
+          float rest = q[32 * s];
+          if (s + 1 < ns) rest += q[32 * (s + 1)];
+          if (s + 2 < ns) rest += q[32 * (s + 2)];
+          D += rest;
+        }
+        r += 32 * max(ns, 0);
+        if constexpr (MANY) {
+          float sum, err;
+          two_sum(Dh, D, sum, err);
+          Dh = sum;
+          Dl += err;
+          D = Dh + Dl;
+        }
         // in the box without overlap: 1, or NaN with a NaN disk integral
         const float f = 1.0f - D * invis * inv_ns;
         if (last && b + lane < take) {
@@ -998,6 +1019,14 @@ __device__ __forceinline__ int split_flush(const float2* __restrict__ times, con
   if (take > 0 && lane < left) Q.pt[lane] = Q.pt[take + lane];
   __syncwarp();
   return left;
+}
+
+static __device__ __noinline__ int split_flush_many(const float2* __restrict__ times, const float* orb, const float* R,
+                                                    const float* ldm_pv, int ng, float inv_dg, SplitQueue& Q, int n,
+                                                    bool all, const SplitRow& row) {
+  __builtin_assume(__isShared(&Q));
+  __builtin_assume(__isShared(orb));
+  return split_flush<true>(times, orb, R, ldm_pv, ng, inv_dg, Q, n, all, row);
 }
 
 union SplitSmem {   // a warp's lists: one of the two per pv
@@ -1041,7 +1070,7 @@ __device__ __noinline__ void split_mixed_tile(const float2* __restrict__ times, 
         const float* lda = ldm_pv + __float_as_int(R[LC_PB]) * ng;
         const float k = R[LC_K];
         const int ns = __float_as_int(R[LC_NS]);
-        float D = 0.0f;
+        float D = 0.0f, low = 0.0f;   // the sum and its error
         for (int s = 0; s < ns; ++s) {
           const float z = sep_c_f32(tc + R[LC_EXPT] * fmaf((float)s + 0.5f, R[LC_INVNS], -0.5f), orb);
           if (!(z < 1.0f + k)) continue;
@@ -1049,8 +1078,13 @@ __device__ __noinline__ void split_mixed_tile(const float2* __restrict__ times, 
           const int i = min(max((int)gg, 0), ng - 2);
           const float l0 = __ldg(lda + i), l1 = __ldg(lda + i + 1);
           float kap;
-          D += fmaf(gg - (float)i, l1 - l0, l0) * ccia_star<float>(k, z, kap);
+          const float term = fmaf(gg - (float)i, l1 - l0, l0) * ccia_star<float>(k, z, kap);
+          float sum, err;
+          two_sum(D, term, sum, err);
+          D = sum;
+          low += err;
         }
+        D += low;
         f = 1.0f - D * R[LC_INVIS] * R[LC_INVNS];
       }
     }
@@ -1112,8 +1146,11 @@ __device__ __noinline__ void split_pv_multi(const FluxSplitArgs& A, int pv, int 
     const int j = done ? 0 : __ffs(m) - 1;
     const int tlc = __shfl_sync(FULL, mylc, j);
     const bool all = done || tlc != qlc;
-    if (n > 0 && (all || n > SPLIT_Q - WARP_TILE))
-      n = split_flush(times, orb, LCR + qlc * LC32, ldm_pv, ng, inv_dg, Q, n, all, row);
+    if (n > 0 && (all || n > SPLIT_Q - WARP_TILE)) {
+      const float* R = LCR + qlc * LC32;
+      n = __float_as_int(R[LC_NS]) <= SPLIT_ROWS ? split_flush<false>(times, orb, R, ldm_pv, ng, inv_dg, Q, n, all, row)
+                                                 : split_flush_many(times, orb, R, ldm_pv, ng, inv_dg, Q, n, all, row);
+    }
     if (done) return;
     m &= m - 1u;
     const int p0 = (tw0 + (j0 + j) * t_step) * WARP_TILE;
