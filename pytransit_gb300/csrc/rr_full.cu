@@ -424,7 +424,7 @@ __device__ __forceinline__ void orbit_pv_split(const OrbitArgs& A, int pv) {
   const float p_lo = __double2float_rn(p - (double)p_hi);
   // Bound of |fast-test tc - true tc|: 2^-24 (4 (T + |d0|) + 2 p), doubled.
   const double err = ldexp(1.0, -21) * (A.t_absmax + d0max + p) + 1e-9;
-  int flags = valid ? FLAG_VALID : 0;
+  int flags = (valid ? FLAG_VALID : 0) | FLAG_MULTI;
   for (int lc0 = 0; lc0 < A.nlc; lc0 += ORB_LCG) {
     double d0[ORB_LCG], kk[ORB_LCG], ex[ORB_LCG];
     int pb[ORB_LCG], ns[ORB_LCG];
@@ -455,7 +455,7 @@ __device__ __forceinline__ void orbit_pv_split(const OrbitArgs& A, int pv) {
       if (hi + 2 * err >= 0.5 * p || lo - 2 * err <= -0.5 * p) flags |= FLAG_WIDE;
       const float d0h = __double2float_rn(d0[j]);
       const float kf = (float)kk[j];
-      if (ns[j] > 1) flags |= FLAG_MULTI;
+      if (ns[j] == 1) flags &= ~FLAG_MULTI;
       float4* q = q4 + (size_t)lc * (LC32 / 4);
       // LC_FLO, LC_FHI, LC_D0H, LC_D0L | LC_LO, LC_HI, LC_K, LC_INV1PK | LC_INVIS, LC_EXPT, LC_INVNS, LC_NS | LC_PB
       q[0] = make_float4((float)(lo - err), (float)(hi + err), d0h, __double2float_rn(d0[j] - (double)d0h));
@@ -852,7 +852,8 @@ constexpr int LC_SMEM = 64;                  // light-curve records staged in sh
 struct WarpList {
   float tc[WARP_TILE];
   int lc[WARP_TILE];
-  float acc[WARP_TILE];
+  int off[WARP_TILE + 1];
+  float acc[WARP_TILE], err[WARP_TILE];
 };
 
 // Points of supersampled light curves that the fast fold puts in the box, kept
@@ -1199,8 +1200,10 @@ __device__ __noinline__ void split_pv_multi(const FluxSplitArgs& A, int pv, int 
 // point plus each point's (exact, small) offset from it; otherwise a fast
 // FP32 test per point and the exact reduction for candidates.  Then the
 // flux of the in-box points in place, skipping slots without an in-box point as a whole warp.  res[] holds
-// 1.0 on entry and the flux of in-box points on exit.  For a pv whose light
-// curves take one sample per point; split_pv_multi does the others.
+// 1.0 on entry and the flux of in-box points on exit.  With several samples per point
+// the in-box points' (point, sample) pairs are spread over the lanes, whatever each light
+// curve's count, and summed by a segmented shuffle reduction and, over groups of 32 pairs,
+// with their rounding errors.
 __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb, const float* __restrict__ LCR,
                                                   const float* __restrict__ ldm_pv, int ng, float inv_dg,
                                                   bool wide, float4 tm, const float* hi, const float* lo,
@@ -1251,7 +1254,17 @@ __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb,
   unsigned act = 0;
 #pragma unroll
   for (int q = 0; q < SPLIT_PTS; ++q) act |= (__ballot_sync(FULL, inb >> q & 1u) ? 1u : 0u) << q;
-  {
+  bool single;
+  if (tlc >= 0) {
+    single = __float_as_int(RT[LC_NS]) == 1;   // one light curve: warp-uniform
+  } else {
+    single = true;
+#pragma unroll
+    for (int q = 0; q < SPLIT_PTS; ++q)
+      if (inb >> q & 1u) single = single && (__float_as_int(LCR[lcv[q] * LC32 + LC_NS]) == 1);
+    single = __all_sync(FULL, single);
+  }
+  if (single) {
     // One sample per point.  A point whose planet disk is fully inside the
     // star (area pi k^2) is finished in place; points on the limb (kite area,
     // two atan2) are gathered into the warp's list and evaluated 32 at a time,
@@ -1391,7 +1404,89 @@ __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb,
     for (int q = 0; q < SPLIT_PTS; ++q)
       if (posq[q] >= 0) res[q] = 1.0f - L.acc[posq[q]] * LCR[lcv[q] * LC32 + LC_INVIS];
     __syncwarp();
+    return;
   }
+  int nitems = 0;
+  int posq[SPLIT_PTS];
+#pragma unroll
+  for (int q = 0; q < SPLIT_PTS; ++q) {
+    const bool in = inb >> q & 1u;
+    const unsigned m = __ballot_sync(FULL, in);
+    posq[q] = -1;
+    if (in) {
+      const int pos = nitems + __popc(m & ((1u << lane) - 1u));
+      L.tc[pos] = tcq[q];
+      L.lc[pos] = lcv[q];
+      L.acc[pos] = L.err[pos] = 0.0f;
+      posq[q] = pos;
+    }
+    nitems += __popc(m);
+  }
+  __syncwarp();
+  // exclusive prefix sum of the sample counts -> L.off
+  int total = 0;
+  for (int c0 = 0; c0 < nitems; c0 += 32) {
+    const int it = c0 + lane;
+    const int v = (it < nitems) ? max(__float_as_int(LCR[L.lc[it] * LC32 + LC_NS]), 0) : 0;
+    int incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(FULL, incl, d);
+      if (lane >= d) incl += u;
+    }
+    if (it < nitems) L.off[it] = total + incl - v;
+    total += __shfl_sync(FULL, incl, 31);
+  }
+  __syncwarp();
+  for (int f0 = 0; f0 < total; f0 += 32) {
+    const int f = f0 + lane;
+    float d = 0.0f;
+    int item = -1;
+    if (f < total) {
+      int lo_i = 0, hi_i = nitems - 1;   // largest item with off[item] <= f
+      while (lo_i < hi_i) {
+        const int mid = (lo_i + hi_i + 1) >> 1;
+        if (L.off[mid] <= f) lo_i = mid; else hi_i = mid - 1;
+      }
+      item = lo_i;
+      const int smp = f - L.off[item];
+      const float* R = LCR + L.lc[item] * LC32;
+      const float k = R[LC_K];
+      // time_offset = exptime ((isample - 0.5)/ns - 0.5), isample = smp + 1
+      const float t = L.tc[item] + R[LC_EXPT] * fmaf((float)smp + 0.5f, R[LC_INVNS], -0.5f);
+      const float z = sep_c_f32(t, orb);
+      if (z < 1.0f + k) {
+        const float gg = z * R[LC_INV1PK] * inv_dg;
+        const int i = min(max((int)gg, 0), ng - 2);
+        const float* lda = ldm_pv + __float_as_int(R[LC_PB]) * ng;
+        const float l0 = __ldg(lda + i), l1 = __ldg(lda + i + 1);
+        float kap;
+        d = fmaf(gg - (float)i, l1 - l0, l0) * ccia_star<float>(k, z, kap);
+      }
+    }
+    // segmented sum over lanes holding the same item
+#pragma unroll
+    for (int dd = 1; dd < 32; dd <<= 1) {
+      const float dv = __shfl_down_sync(FULL, d, dd);
+      const int iv = __shfl_down_sync(FULL, item, dd);
+      if (lane + dd < 32 && iv == item) d += dv;
+    }
+    const int before = __shfl_up_sync(FULL, item, 1);
+    if (item >= 0 && (lane == 0 || before != item)) {
+      float sum, err;
+      two_sum(L.acc[item], d, sum, err);
+      L.acc[item] = sum;
+      L.err[item] += err;
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int q = 0; q < SPLIT_PTS; ++q)
+    if (posq[q] >= 0) {
+      const float* R = LCR + lcv[q] * LC32;
+      res[q] = 1.0f - (L.acc[posq[q]] + L.err[posq[q]]) * R[LC_INVIS] * R[LC_INVNS];
+    }
+  __syncwarp();
 }
 
 // One block's share of one parameter vector: stage the pv's orbit and
@@ -1414,7 +1509,15 @@ __device__ __forceinline__ void split_pv_tiles(const FluxSplitArgs& A, int pv, i
   const int flags = __float_as_int(orb[14]);
   const bool valid = flags & FLAG_VALID;
   const bool wide = flags & FLAG_WIDE;
-  if (valid && (flags & FLAG_MULTI)) {   // block-uniform
+  // Which way a pv's tiles go (block-uniform): through the queue over tiles where every
+  // light curve is supersampled and most tiles are of one (light curves of two tiles
+  // on average), else each tile by itself, which keeps tiles of single samples, or of
+  // several light curves with counts of any kind, at their own cost.  Flux kernel, us,
+  // queue / by itself: 4096 pv x 118,526 30-min times x 10 samples 1672 / 2682; a 30-min
+  // light curve x 10 beside three 2-min ones (4096 x 21,015) 136 / 115; 60 light
+  // curves of 73 points x 5 (1024 pv) 140 / 110; points of four interleaved, x 10,
+  // (1024 x 19,700) 164 / 181.
+  if (valid && (flags & FLAG_MULTI) && A.npt >= 2 * WARP_TILE * A.nlc) {
     split_pv_multi(A, pv, t_first, t_step, t_end, orb, LCR, lists[warp].q, sizeof(OutT) == 8);
     return;
   }

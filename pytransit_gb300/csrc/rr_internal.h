@@ -87,7 +87,7 @@ enum LcField {
 constexpr int TIME_TILE = 128;
 __host__ __device__ inline size_t time_meta_offset(int npt) { return 2 * (((size_t)npt + 1) / 2 * 2); }
 constexpr int FLAG_VALID = 1;
-constexpr int FLAG_MULTI = 4; // a light curve with several samples per point
+constexpr int FLAG_MULTI = 4; // no light curve takes one sample per point
 constexpr int FLAG_WIDE = 2;  // box too close to +-p/2: take the exact path for every point
 
 }  // namespace rr
