@@ -888,8 +888,8 @@ def main():
                                          P(ist32), P(ws32), ws32.numel(), sp))
         if ev is not None:
             ev[0].record(stream)
-        _lib.check(L.rr_flux_split(P(dd["times_ff"]), npt, P(dd["lcids"]), npv, nlc, npb, ng, model.dg,
-                                   P(ws32), P(flux32), ldf, sp))
+        _lib.check(L.rr_flux_split_rows(P(dd["times_ff"]), npt, P(dd["lcids"]), npv, nlc, npb, ng, model.dg,
+                                        P(ws32), 0, npv, P(flux32), ldf, dd["rows"], sp))
         if ev is not None:
             ev[1].record(stream)
 

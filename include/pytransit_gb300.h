@@ -241,6 +241,16 @@ int rr_flux_split_transits(const float *times_ff, int npt, const int32_t *lcids,
                            int ng, double dg, const void *workspace, int pv0, int pv1, float *flux, int ldflux,
                            void *stream);
 
+/* Either of the two with FP32 or FP64 rows, as kind says (a sum of RR_ROWS_*).
+ * RR_ROWS_TILES: not every light curve takes several samples per point (nsamples),
+ * or they are shorter than 256 points on average.  Without it the launch also holds
+ * the code that data sets of long supersampled light curves need, which costs the
+ * others about 2 %; the values are right either way. */
+enum { RR_ROWS_F64 = 1, RR_ROWS_TRANSITS = 2, RR_ROWS_TILES = 4 };
+int rr_flux_split_rows(const float *times_ff, int npt, const int32_t *lcids, int npv, int nlc, int npb, int ng,
+                       double dg, const void *workspace, int pv0, int pv1, void *flux, int ldflux, int kind,
+                       void *stream);
+
 /* Host memory fill on the library's own threads: dst[0..n) = value, split
  * over nthreads threads (the calling thread included; nthreads <= 0 or 1:
  * the calling thread alone).  The threads are started on first use and kept;

@@ -60,6 +60,7 @@ def _sig(L):
     L.rr_flux_split.argtypes = [_vp, _i, _vp, _i, _i, _i, _i, _d, _vp, _vp, _i, _vp]
     L.rr_flux_split_range.argtypes = [_vp, _i, _vp, _i, _i, _i, _i, _d, _vp, _i, _i, _vp, _i, _vp]
     L.rr_flux_split_transits.argtypes = [_vp, _i, _vp, _i, _i, _i, _i, _d, _vp, _i, _i, _vp, _i, _vp]
+    L.rr_flux_split_rows.argtypes = [_vp, _i, _vp, _i, _i, _i, _i, _d, _vp, _i, _i, _vp, _i, _i, _vp]
     L.rr_host_fill_f32.argtypes = [_vp, _sz, C.c_float, _i]
     L.rr_host_fill_f64.argtypes = [_vp, _sz, _d, _i]
     L.rr_event_create.argtypes = [C.POINTER(_vp)]
@@ -102,6 +103,8 @@ def _sig(L):
 
 # Signatures of entry points added in other translation units (name -> (argtypes, restype)).
 _EXTRA_SIGNATURES = {}
+
+ROWS_F64, ROWS_TRANSITS, ROWS_TILES = 1, 2, 4    # rr_flux_split_rows
 
 
 def register(signatures):

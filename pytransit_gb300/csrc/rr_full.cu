@@ -4,6 +4,7 @@
 // precision.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "rr_device.cuh"
 #include "rr_f64_points.cuh"
@@ -853,7 +854,7 @@ struct WarpList {
   float tc[WARP_TILE];
   int lc[WARP_TILE];
   int off[WARP_TILE + 1];
-  float acc[WARP_TILE], err[WARP_TILE];
+  float acc[WARP_TILE], sum[WARP_TILE];
 };
 
 // Points of supersampled light curves that the fast fold puts in the box, kept
@@ -1034,6 +1035,9 @@ union SplitSmem {   // a warp's lists: one of the two per pv
   WarpList l;
   SplitQueue q;
 };
+struct ListSmem {   // without the queue
+  WarpList l;
+};
 
 // The cull test of one tile: its time range (from its summary) misses every
 // box copy, the rounding of t - d0 and of j p covered by the error bound in
@@ -1202,8 +1206,8 @@ __device__ __noinline__ void split_pv_multi(const FluxSplitArgs& A, int pv, int 
 // flux of the in-box points in place, skipping slots without an in-box point as a whole warp.  res[] holds
 // 1.0 on entry and the flux of in-box points on exit.  With several samples per point
 // the in-box points' (point, sample) pairs are spread over the lanes, whatever each light
-// curve's count, and summed by a segmented shuffle reduction and, over groups of 32 pairs,
-// with their rounding errors.
+// curve's count, and summed by a segmented shuffle reduction, over groups of 32 pairs and
+// over 16 of those at a time, so that the error grows little with the samples.
 __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb, const float* __restrict__ LCR,
                                                   const float* __restrict__ ldm_pv, int ng, float inv_dg,
                                                   bool wide, float4 tm, const float* hi, const float* lo,
@@ -1417,7 +1421,7 @@ __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb,
       const int pos = nitems + __popc(m & ((1u << lane) - 1u));
       L.tc[pos] = tcq[q];
       L.lc[pos] = lcv[q];
-      L.acc[pos] = L.err[pos] = 0.0f;
+      L.acc[pos] = L.sum[pos] = 0.0f;
       posq[q] = pos;
     }
     nitems += __popc(m);
@@ -1472,19 +1476,21 @@ __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb,
       if (lane + dd < 32 && iv == item) d += dv;
     }
     const int before = __shfl_up_sync(FULL, item, 1);
-    if (item >= 0 && (lane == 0 || before != item)) {
-      float sum, err;
-      two_sum(L.acc[item], d, sum, err);
-      L.acc[item] = sum;
-      L.err[item] += err;
-    }
+    if (item >= 0 && (lane == 0 || before != item)) L.acc[item] += d;
     __syncwarp();
+    if ((f0 & 511) == 480) {   // after 16 groups of pairs
+      for (int it = lane; it < nitems; it += 32) {
+        L.sum[it] += L.acc[it];
+        L.acc[it] = 0.0f;
+      }
+      __syncwarp();
+    }
   }
 #pragma unroll
   for (int q = 0; q < SPLIT_PTS; ++q)
     if (posq[q] >= 0) {
       const float* R = LCR + lcv[q] * LC32;
-      res[q] = 1.0f - (L.acc[posq[q]] + L.err[posq[q]]) * R[LC_INVIS] * R[LC_INVNS];
+      res[q] = 1.0f - (L.sum[posq[q]] + L.acc[posq[q]]) * R[LC_INVIS] * R[LC_INVNS];
     }
   __syncwarp();
 }
@@ -1495,9 +1501,9 @@ __device__ __forceinline__ void split_tile_points(const float* __restrict__ orb,
 // the stores of the culled tiles (walking the set bits of the cull mask),
 // then the per-point path of the others.  Ends without a barrier: the caller
 // synchronises before staging another pv.
-template <typename OutT>
+template <typename OutT, bool QUEUE, typename Smem>
 __device__ __forceinline__ void split_pv_tiles(const FluxSplitArgs& A, int pv, int t_first, int t_step, int t_end,
-                                               float* recs, bool lc_in_smem, SplitSmem* lists) {
+                                               float* recs, bool lc_in_smem, Smem* lists) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* lcg = A.lc32 + (size_t)pv * A.nlc * LC32;
   if (threadIdx.x < ORB32) recs[threadIdx.x] = __ldg(A.orb32 + (size_t)pv * ORB32 + threadIdx.x);
@@ -1514,12 +1520,14 @@ __device__ __forceinline__ void split_pv_tiles(const FluxSplitArgs& A, int pv, i
   // on average), else each tile by itself, which keeps tiles of single samples, or of
   // several light curves with counts of any kind, at their own cost.  Flux kernel, us,
   // queue / by itself: 4096 pv x 118,526 30-min times x 10 samples 1672 / 2682; a 30-min
-  // light curve x 10 beside three 2-min ones (4096 x 21,015) 136 / 115; 60 light
-  // curves of 73 points x 5 (1024 pv) 140 / 110; points of four interleaved, x 10,
+  // light curve x 10 beside three 2-min ones (4096 x 21,015) 136 / 118; 60 light
+  // curves of 73 points x 5 (1024 pv) 140 / 111; points of four interleaved, x 10,
   // (1024 x 19,700) 164 / 181.
-  if (valid && (flags & FLAG_MULTI) && A.npt >= 2 * WARP_TILE * A.nlc) {
-    split_pv_multi(A, pv, t_first, t_step, t_end, orb, LCR, lists[warp].q, sizeof(OutT) == 8);
-    return;
+  if constexpr (QUEUE) {
+    if (valid && (flags & FLAG_MULTI) && A.npt >= 2LL * WARP_TILE * A.nlc) {
+      split_pv_multi(A, pv, t_first, t_step, t_end, orb, LCR, lists[warp].q, sizeof(OutT) == 8);
+      return;
+    }
   }
   const float p_hi = orb[10], inv_p = orb[12];
   const float* ldm_pv = A.ldm + (size_t)pv * A.npb * A.ng;
@@ -1594,17 +1602,19 @@ __device__ __forceinline__ void split_pv_tiles(const FluxSplitArgs& A, int pv, i
 constexpr int FLUX_NW = 2;
 constexpr int FLUX_CHUNK = 32;
 
-template <bool LC_IN_SMEM, typename OutT>
+// QUEUE: with the queue over tiles, whose call and shared memory cost the tiles by
+// themselves 2 %: 117.4 us for 8192 x 19,700 points of single samples, 115.3 without.
+template <bool LC_IN_SMEM, typename OutT, bool QUEUE>
 __global__ void __launch_bounds__(FLUX_NW * 32, 16)
 flux_split_kernel(const __grid_constant__ FluxSplitArgs A, int chunk) {
-  __shared__ SplitSmem lists[FLUX_NW];
+  __shared__ typename std::conditional<QUEUE, SplitSmem, ListSmem>::type lists[FLUX_NW];
   extern __shared__ __align__(16) float flux_recs[];
   const int pv = block_pv();
   if (pv >= A.npv) return;  // block-uniform
   const int ntiles = (A.npt + WARP_TILE - 1) / WARP_TILE;
   const int t0 = blockIdx.x * chunk;
   const int t1 = t0 + chunk < ntiles ? t0 + chunk : ntiles;
-  split_pv_tiles<OutT>(A, pv, t0, FLUX_NW, t1, flux_recs, LC_IN_SMEM, lists);
+  split_pv_tiles<OutT, QUEUE>(A, pv, t0, FLUX_NW, t1, flux_recs, LC_IN_SMEM, lists);
 }
 
 // ---------------------------------------------------------------------------
@@ -1657,7 +1667,7 @@ serve_split_kernel(const rr_serve_request* __restrict__ reqs, const rr_serve_ite
     A.inv_dg = r.inv_dg; A.flux = r.flux;
     const bool lc_smem = r.nlc <= LC_SMEM;
     for (int pv = w.pv0; pv < w.pv1; ++pv) {
-      split_pv_tiles<float>(A, pv, w.tile0, SPLIT_WARPS, w.tile1, recs, lc_smem, U.lists);
+      split_pv_tiles<float, true>(A, pv, w.tile0, SPLIT_WARPS, w.tile1, recs, lc_smem, U.lists);
       __syncthreads();
     }
   }
@@ -1955,7 +1965,8 @@ static int flux_split_args(int npt, int npv, int nlc, int npb, int ng, int pv0, 
 
 static int flux_split_launch(const float* times_ff, int npt, const int32_t* lcids, int npv, int nlc, int npb,
                              int ng, double dg, const void* workspace, int pv0, int pv1, void* flux, int ldflux,
-                             void* stream, int transits_only, bool out_f64) {
+                             void* stream, int kind) {
+  const bool transits_only = kind & RR_ROWS_TRANSITS, out_f64 = kind & RR_ROWS_F64;
   const int st = flux_split_args(npt, npv, nlc, npb, ng, pv0, pv1, ldflux);
   if (st != RR_OK) return st;
   if (pv1 == pv0 || npt == 0) return RR_OK;
@@ -1980,17 +1991,15 @@ static int flux_split_launch(const float* times_ff, int npt, const int32_t* lcid
   const bool lc_smem = nlc <= LC_SMEM;
   const size_t smem = sizeof(float) * (ORB32 + (lc_smem ? (size_t)nlc * LC32 : 0));
   cudaStream_t s = as_stream(stream);
-  if (out_f64) {
-    if (lc_smem)
-      flux_split_kernel<true, double><<<fg, FLUX_NW * 32, smem, s>>>(fa, (int)chunk);
-    else
-      flux_split_kernel<false, double><<<fg, FLUX_NW * 32, smem, s>>>(fa, (int)chunk);
-  } else {
-    if (lc_smem)
-      flux_split_kernel<true, float><<<fg, FLUX_NW * 32, smem, s>>>(fa, (int)chunk);
-    else
-      flux_split_kernel<false, float><<<fg, FLUX_NW * 32, smem, s>>>(fa, (int)chunk);
-  }
+  const bool queue = !(kind & RR_ROWS_TILES) && npt >= 2LL * WARP_TILE * nlc;
+  auto fn = flux_split_kernel<false, float, false>;
+  if (queue)
+    fn = out_f64 ? (lc_smem ? flux_split_kernel<true, double, true> : flux_split_kernel<false, double, true>)
+                 : (lc_smem ? flux_split_kernel<true, float, true> : flux_split_kernel<false, float, true>);
+  else
+    fn = out_f64 ? (lc_smem ? flux_split_kernel<true, double, false> : flux_split_kernel<false, double, false>)
+                 : (lc_smem ? flux_split_kernel<true, float, false> : flux_split_kernel<false, float, false>);
+  fn<<<fg, FLUX_NW * 32, smem, s>>>(fa, (int)chunk);
   return check_launch("rr_flux_split");
 }
 
@@ -2018,40 +2027,44 @@ static void* device_rows(void* flux, int* status) {
   return dst;
 }
 
+int rr_flux_split_rows(const float* times_ff, int npt, const int32_t* lcids, int npv, int nlc, int npb, int ng,
+                       double dg, const void* workspace, int pv0, int pv1, void* flux, int ldflux, int kind,
+                       void* stream) {
+  if (kind & ~(RR_ROWS_F64 | RR_ROWS_TRANSITS | RR_ROWS_TILES)) return RR_ERR_ARG;
+  int st = flux_split_args(npt, npv, nlc, npb, ng, pv0, pv1, ldflux);
+  if (st != RR_OK || pv1 == pv0 || npt == 0) return st;
+  if (kind & RR_ROWS_TRANSITS) {
+    flux = device_rows(flux, &st);
+    if (!flux) return st;
+  }
+  return flux_split_launch(times_ff, npt, lcids, npv, nlc, npb, ng, dg, workspace, pv0, pv1, flux, ldflux, stream, kind);
+}
+
 int rr_flux_split_range(const float* times_ff, int npt, const int32_t* lcids, int npv, int nlc, int npb, int ng,
                         double dg, const void* workspace, int pv0, int pv1, float* flux, int ldflux,
                         void* stream) {
-  return flux_split_launch(times_ff, npt, lcids, npv, nlc, npb, ng, dg, workspace, pv0, pv1, flux, ldflux, stream,
-                           0, false);
+  return rr_flux_split_rows(times_ff, npt, lcids, npv, nlc, npb, ng, dg, workspace, pv0, pv1, flux, ldflux, 0, stream);
 }
 
 int rr_flux_split_range_f64(const float* times_ff, int npt, const int32_t* lcids, int npv, int nlc, int npb,
                             int ng, double dg, const void* workspace, int pv0, int pv1, double* flux, int ldflux,
                             void* stream) {
-  return flux_split_launch(times_ff, npt, lcids, npv, nlc, npb, ng, dg, workspace, pv0, pv1, flux, ldflux, stream,
-                           0, true);
+  return rr_flux_split_rows(times_ff, npt, lcids, npv, nlc, npb, ng, dg, workspace, pv0, pv1, flux, ldflux,
+                            RR_ROWS_F64, stream);
 }
 
 int rr_flux_split_transits(const float* times_ff, int npt, const int32_t* lcids, int npv, int nlc, int npb, int ng,
                            double dg, const void* workspace, int pv0, int pv1, float* flux, int ldflux,
                            void* stream) {
-  int st = flux_split_args(npt, npv, nlc, npb, ng, pv0, pv1, ldflux);
-  if (st != RR_OK || pv1 == pv0 || npt == 0) return st;
-  void* dst = device_rows(flux, &st);
-  if (!dst) return st;
-  return flux_split_launch(times_ff, npt, lcids, npv, nlc, npb, ng, dg, workspace, pv0, pv1, dst, ldflux, stream,
-                           1, false);
+  return rr_flux_split_rows(times_ff, npt, lcids, npv, nlc, npb, ng, dg, workspace, pv0, pv1, flux, ldflux,
+                            RR_ROWS_TRANSITS, stream);
 }
 
 int rr_flux_split_transits_f64(const float* times_ff, int npt, const int32_t* lcids, int npv, int nlc, int npb,
                                int ng, double dg, const void* workspace, int pv0, int pv1, double* flux,
                                int ldflux, void* stream) {
-  int st = flux_split_args(npt, npv, nlc, npb, ng, pv0, pv1, ldflux);
-  if (st != RR_OK || pv1 == pv0 || npt == 0) return st;
-  void* dst = device_rows(flux, &st);
-  if (!dst) return st;
-  return flux_split_launch(times_ff, npt, lcids, npv, nlc, npb, ng, dg, workspace, pv0, pv1, dst, ldflux, stream,
-                           1, true);
+  return rr_flux_split_rows(times_ff, npt, lcids, npv, nlc, npb, ng, dg, workspace, pv0, pv1, flux, ldflux,
+                            RR_ROWS_TRANSITS | RR_ROWS_F64, stream);
 }
 
 int rr_full_split(const float* times_ff, double t_ref, double t_absmax, int npt, const double* k, int nkc,

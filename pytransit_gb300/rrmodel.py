@@ -344,8 +344,8 @@ class RoadRunnerModel(TransitModel):
             b = bufs[c % 2]
             if copied[c % 2] is not None:
                 comp.wait_event(copied[c % 2])
-            st = L.rr_flux_split_range(P(dd['times_ff']), npt, P(dd['lcids']), npv, nlc, npb, self.ng, self.dg,
-                                       P(ws), pv0, pv1, P(b), npt, sp)
+            st = L.rr_flux_split_rows(P(dd['times_ff']), npt, P(dd['lcids']), npv, nlc, npb, self.ng, self.dg,
+                                      P(ws), pv0, pv1, P(b), npt, dd['rows'], sp)
             if st != 0:
                 return st
             done = torch.cuda.Event()
@@ -372,7 +372,7 @@ class RoadRunnerModel(TransitModel):
         rows to 1, a pv chunk at a time, on the library's threads
         (rr_host_fill_f32/_f64), and after each chunk the GPU writes that
         chunk's transit tiles and invalid rows straight into it
-        (rr_flux_split_transits[_f64]): tiles that reach no transit window
+        (rr_flux_split_rows, RR_ROWS_TRANSITS): tiles that reach no transit window
         never cross the link.  The current stream waits for the copy; the
         caller synchronises it.  Returns the first non-zero status."""
         import torch
@@ -380,8 +380,7 @@ class RoadRunnerModel(TransitModel):
         L, P = _lib.lib(), _lib.ptr
         f64 = out2d.dtype == torch.float64
         esize = 8 if f64 else 4
-        dense = L.rr_flux_split_range_f64 if f64 else L.rr_flux_split_range
-        transits = L.rr_flux_split_transits_f64 if f64 else L.rr_flux_split_transits
+        kind = dd['rows'] | (_lib.ROWS_F64 if f64 else 0)
         fill = L.rr_host_fill_f64 if f64 else L.rr_host_fill_f32
         comp = torch.cuda.current_stream(device)
         sp = C.c_void_p(comp.cuda_stream)
@@ -394,8 +393,8 @@ class RoadRunnerModel(TransitModel):
                 self._stage = (key, torch.empty((ncopy, npt), dtype=out2d.dtype, device=device),
                                torch.cuda.Stream(device))
             _, buf, cs = self._stage
-            st = dense(P(dd['times_ff']), npt, P(dd['lcids']), npv, nlc, npb, self.ng, self.dg, P(ws), 0, ncopy,
-                       P(buf), npt, sp)
+            st = L.rr_flux_split_rows(P(dd['times_ff']), npt, P(dd['lcids']), npv, nlc, npb, self.ng, self.dg, P(ws),
+                                      0, ncopy, P(buf), npt, kind, sp)
             if st != 0:
                 return st
             cs.wait_stream(comp)
@@ -409,8 +408,8 @@ class RoadRunnerModel(TransitModel):
             rows = C.c_void_p(base + pv0 * npt * esize)
             st = fill(rows, (pv1 - pv0) * npt, 1.0, int(self.host_threads))
             if st == 0:
-                st = transits(P(dd['times_ff']), npt, P(dd['lcids']), npv, nlc, npb, self.ng, self.dg, P(ws),
-                              pv0, pv1, rows, npt, sp)
+                st = L.rr_flux_split_rows(P(dd['times_ff']), npt, P(dd['lcids']), npv, nlc, npb, self.ng, self.dg,
+                                          P(ws), pv0, pv1, rows, npt, kind | _lib.ROWS_TRANSITS, sp)
             if st != 0:
                 return st
         if cs is not None:
@@ -624,8 +623,8 @@ class RoadRunnerModel(TransitModel):
                 else:
                     st = self._flux_to_pinned(dd, npt, npv, nlc, npb, ws, host_rows, device, fill_fraction=0.0)
             elif st == 0:
-                st = L.rr_flux_split(P(dd['times_ff']), npt, P(dd['lcids']), npv, nlc, npb, self.ng, self.dg,
-                                     P(ws), P(res), ldf, stream)
+                st = L.rr_flux_split_rows(P(dd['times_ff']), npt, P(dd['lcids']), npv, nlc, npb, self.ng, self.dg,
+                                          P(ws), 0, npv, P(res), ldf, dd['rows'], stream)
             res = None if pipe else res[:, :npt]
         else:
             res = None if pipe else torch.empty((npv, npt), dtype=torch.float64, device=device)

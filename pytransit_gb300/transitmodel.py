@@ -123,6 +123,8 @@ class TransitModel:
         d['epids'] = torch.as_tensor(ep).to(device)
         d['nsamples'] = torch.as_tensor(ns).to(device)
         d['exptimes'] = torch.as_tensor(ex).to(device)
+        # rr_flux_split_rows: each tile by itself, unless every light curve is supersampled and long
+        d['rows'] = 0 if (ns > 1).all() and self.npt >= 256 * self.nlc else _lib.ROWS_TILES
         if self.npt > 0:
             tmin, tmax = float(self.time.min()), float(self.time.max())
         else:
