@@ -9,10 +9,16 @@
 //   * the z error: the FP32 Taylor coefficients against the FP64 jet
 //     recomputed here (the difference itself, not an estimate of it) summed
 //     over the bounding box, |t|^j sum_j |dc_j|, plus the FP32 Horner, the
-//     FP32 sample time and the square root: dz <= sum_j |dc_j| tb^j
-//     + 4u M + u tb V + 4u (1 + k) + 1e-11 V, with u = 2^-24,
+//     FP32 sample time and the root: dz <= sum_j |dc_j| tb^j
+//     + 4u M + dt V + 6u (1 + k) + 1e-11 V, with u = 2^-24,
 //     M = sum_j |c_j| tb^j and V = sum_j j |c_j| tb^(j-1) (the largest sky
-//     speed), tb the largest |t| a sample of the box reaches;
+//     speed), tb the largest |t| a sample of the box reaches.  The sample
+//     time's dt is the point's rounding, u tb; with several samples per point of
+//     exposure ex also those of tc - ex / 2 and of the sum (u tb each), of the
+//     exposure (ex / 2 u at the ends) and of the step ex (1 / ns) (2u of at most
+//     ex): u (3 tb + 2.5 ex).  The other form, tc + ex ((s + 1/2) (1 / ns) - 1/2), has
+//     u (2 tb + 2 ex).  The root, r^2 times the FP32 reciprocal root (2^-22.9),
+//     has 2.2u + u, and r^2's two roundings u;
 //   * the flux's sensitivity to z on every LD-table row j (a sample in row j
 //     has z in [z_j, z_j+1]): |dF/dz| <= (2 min(k, 1) I + A |dI/dz|) / istar
 //     with I <= max(L_j, L_j+1), A <= A(z_j) (the area falls with z) and
@@ -47,10 +53,10 @@ struct BoundArgs {
   unsigned long long* bound_max; // max over pv (bits of a non-negative double), zeroed by the caller
 };
 
-// The z error of pv on |t| <= tb, without the square root's term
-// 4u (1 + kmax), which the per-pv pass adds: the FP32 coefficients of the
+// The z error of pv on |t| <= tb with a sample time's error of u tu, without the root's
+// term 6u (1 + kmax), which the per-pv pass adds: the FP32 coefficients of the
 // record against the FP64 jet.
-__device__ inline double z_error_part(const BoundArgs& B, int pv, const float* c32, double tb) {
+__device__ inline double z_error_part(const BoundArgs& B, int pv, const float* c32, double tb, double tu) {
   double c[10];
   solve2d_conj(B.p[pv], B.a[pv], B.inc[pv], B.e[pv], B.w[pv], c);
   double dcz = 0.0, M = 0.0, V = 0.0, tp = 1.0;
@@ -60,7 +66,7 @@ __device__ inline double z_error_part(const BoundArgs& B, int pv, const float* c
     if (j < 4) V += (j + 1) * (fabs(c[j + 1]) + fabs(c[6 + j])) * tp;
     tp *= tb;
   }
-  return dcz + 4 * BOUND_U * M + BOUND_U * tb * V + 1e-11 * V;
+  return dcz + 4 * BOUND_U * M + BOUND_U * tu * V + 1e-11 * V;
 }
 
 // Per-row terms in FP32 (the FP64 rate of this GPU is 1/64 of its FP32
@@ -96,18 +102,20 @@ __global__ void __launch_bounds__(BOUND_PV_MAX * 32) error_bound_kernel(BoundArg
         const float* o = B.orb + (size_t)pv * ORB32;
         if (__float_as_int(o[14]) & FLAG_VALID) {
           const float* L0 = B.lc + (size_t)pv * B.nlc * LC32;
-          double tb = 0.0;
+          double tb = 0.0, tu = 0.0;
           for (int lc = 0; lc < B.nlc; ++lc) {
             const float* r = L0 + (size_t)lc * LC32;
-            tb = fmax(tb, fmax(fabs((double)r[LC_LO]), fabs((double)r[LC_HI])) + 0.5 * r[LC_EXPT]);
+            const double t = fmax(fabs((double)r[LC_LO]), fabs((double)r[LC_HI])) + 0.5 * r[LC_EXPT];
+            tb = fmax(tb, t);
+            tu = fmax(tu, __float_as_int(r[LC_NS]) > 1 ? 3.0 * t + 2.5 * r[LC_EXPT] : t);
           }
-          part = z_error_part(B, pv, o, tb);
+          part = z_error_part(B, pv, o, tb, tu);
         }
       } else {
         const float* o = B.orb + (size_t)pv * TS_ORB;
         if (o[15] != 0.0f) {
           const double tb = fmax(fabs((double)o[10]), fabs((double)o[11])) + 0.5 * B.exptime0;
-          part = z_error_part(B, pv, o, tb);
+          part = z_error_part(B, pv, o, tb, B.nsamples0 > 1 ? 3.0 * tb + 2.5 * B.exptime0 : tb);
         }
       }
     }
@@ -129,7 +137,7 @@ __global__ void __launch_bounds__(BOUND_PV_MAX * 32) error_bound_kernel(BoundArg
         const float* L0 = B.lc + (size_t)pv * B.nlc * LC32;
         double kmax = 0.0;
         for (int lc = 0; lc < B.nlc; ++lc) kmax = fmax(kmax, (double)L0[(size_t)lc * LC32 + LC_K]);
-        const float dz = __double2float_ru(s_dz[i] + 4 * BOUND_U * (1.0 + kmax));
+        const float dz = __double2float_ru(s_dz[i] + 6 * BOUND_U * (1.0 + kmax));
         for (int lc = 0; lc < B.nlc; ++lc) {
           const float* r = L0 + (size_t)lc * LC32;
           const float k = r[LC_K], inv_is = fabsf(r[LC_INVIS]);
@@ -159,7 +167,7 @@ __global__ void __launch_bounds__(BOUND_PV_MAX * 32) error_bound_kernel(BoundArg
         for (int b = lane; b < B.npb; b += 32) afmax = fmaxf(afmax, ch[b * TS_CH]);
         for (int off = 16; off > 0; off >>= 1) afmax = fmaxf(afmax, __shfl_xor_sync(FULL, afmax, off));
         const double kmax = (double)km * sqrt((double)afmax);
-        const double dz64 = s_dz[i] + 4 * BOUND_U * (1.0 + kmax);
+        const double dz64 = s_dz[i] + 6 * BOUND_U * (1.0 + kmax);
         const float dz = __double2float_ru(dz64);
         // kappa_0 near the outer (inner) contact goes as sqrt(2 eps / (k (1 +- k))):
         // a z error dz moves it by at most sqrt(2 dz / (k (1 - k)))
