@@ -168,9 +168,17 @@ extern "C" int rr_event_destroy(void* event) {
   return RR_OK;
 }
 
+// The event belongs to no capture, so the wait is safe beside one; but unless the
+// thread says so it invalidates a capture that this or another thread has under way.
 extern "C" int rr_event_wait(void* event) {
   if (!event) return RR_ERR_ARG;
-  const cudaError_t st = cudaEventSynchronize(static_cast<cudaEvent_t>(event));
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaError_t st = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (st == cudaSuccess) {
+    st = cudaEventSynchronize(static_cast<cudaEvent_t>(event));
+    const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (st == cudaSuccess) st = back;
+  }
   if (st != cudaSuccess) {
     rr::set_cuda_error(st, "rr_event_wait");
     return RR_ERR_CUDA;
