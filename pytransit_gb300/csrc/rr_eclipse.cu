@@ -141,6 +141,7 @@ static __device__ __noinline__ void ecl_flush(const EclF64Args& A, const F64Orbi
 }
 
 struct EclSink {
+  static constexpr bool BY_LIGHT_CURVE = false;
   const EclF64Args& A;
   const F64Orbit& P;
   F64Lc* recs;

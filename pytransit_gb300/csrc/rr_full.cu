@@ -756,6 +756,7 @@ static __device__ __noinline__ void f64_flux_flush(const FluxF64Args& A, const F
 }
 
 struct F64FluxSink {
+  static constexpr bool BY_LIGHT_CURVE = false;
   const FluxF64Args& A;
   const F64Orbit& P;
   F64Lc* recs;

@@ -675,7 +675,7 @@ struct LnlF64Smem {
   double row[GRAD ? 1 + MAX_NGRAD : 1];    // the share's columns
   double g[GRAD ? F64_Q : 1];              // per point of a chunk: -(r / sigma^2) w
   double ep[GRAD ? F64_Q : 1];             // per point of a chunk: epoch
-  int lc;                                  // light curve of acc, or -1
+  int lc;                                  // a light curve of acc's passband and epoch, or -1
 };
 
 // I(z) A(z)'s value and partial derivatives at one sample.
@@ -735,7 +735,7 @@ __device__ __forceinline__ void f64_partials(const F64Lc& R, const F64Transit& T
   }
 }
 
-// The lanes' sums of light curve S.lc into the share's columns.
+// The lanes' sums into the share's columns of the passband and epoch of light curve S.lc.
 template <bool GRAD>
 __device__ __noinline__ void lnl_f64_reduce(const LnlF64Args& A, LnlF64Smem<GRAD>& S, int pv) {
   const int lane = threadIdx.x & 31;
@@ -784,7 +784,9 @@ __device__ __noinline__ void lnl_f64_flush(const LnlF64Args& A, const F64Orbit& 
   const int before = S.lc;
   __syncwarp();   // every lane has read it
   if (lc != before) {
-    if (before >= 0) lnl_f64_reduce<GRAD>(A, S, pv);
+    // the sums' columns are those of the passband and the epoch
+    if (before >= 0 && (A.pbids[lc] != A.pbids[before] || A.epids[lc] != A.epids[before]))
+      lnl_f64_reduce<GRAD>(A, S, pv);
     if (lane == 0) S.lc = lc;
     __syncwarp();
   }
@@ -879,6 +881,7 @@ __device__ __noinline__ void lnl_f64_flush(const LnlF64Args& A, const F64Orbit& 
 
 template <bool GRAD>
 struct LnlF64Sink {
+  static constexpr bool BY_LIGHT_CURVE = true;   // with and without the gradient: the same sums
   const LnlF64Args& A;
   const F64Orbit& P;
   F64Lc* recs;
