@@ -506,11 +506,6 @@ __device__ inline double contact_point(double k, int point, const double* c) {
   return t1;
 }
 
-// The same bisection on the FP32 coefficients, for the split path: the contact
-// times only place the bounding box, which is padded by 0.003 d beyond
-// contact, so a ~1e-7 d error in them changes no flux value.
-__device__ inline float contact_point_f32(float k, int point, const float* c);
-
 // ---------------------------------------------------------------------------
 // Float-float helpers (error-free transformations, Knuth / Dekker)
 // ---------------------------------------------------------------------------
@@ -561,32 +556,10 @@ __device__ __forceinline__ float sep_c_f32(float t, const float* c) {
   return sqrtf(fmaf(x, x, y * y));
 }
 
-__device__ inline float contact_point_f32(float k, int point, const float* c) {
-  const float s = (point == 1 || point == 2) ? -1.0f : 1.0f;
-  const float zt = (point == 1 || point == 4) ? 1.0f + k : 1.0f - k;
-  float t0 = 0.0f;
-  float t2 = s * 2.0f / fabsf(c[1]);
-  float t1 = 0.5f * t2;
-  float z0 = sep_c_f32(t0, c) - zt;
-  float z1 = sep_c_f32(t1, c) - zt;
-  for (int i = 0; fabsf(t2 - t0) > 1e-6f && i < 100; ++i) {
-    if (z0 * z1 < 0.0f) {
-      t2 = t1;
-      t1 = 0.5f * (t0 + t1);
-      z1 = sep_c_f32(t1, c) - zt;
-    } else {
-      t0 = t1;
-      t1 = 0.5f * (t1 + t2);
-      z0 = z1;
-      z1 = sep_c_f32(t1, c) - zt;
-    }
-  }
-  return t1;
-}
-
-// Points 1 and 4 of contact_point_f32 (the outer contacts) bisected in one
-// loop: each keeps its own bracket and stops on its own test, so the results
-// are those of the two separate calls, while the two dependent chains overlap.
+// contact_point for points 1 and 4 (the outer contacts) on the FP32 coefficients, for
+// the split path: the contact times only place the bounding box, which is padded by
+// 0.003 d beyond contact.  Bisected in one loop: each keeps its own bracket and stops on
+// its own test, as in two calls, while the two dependent chains overlap.
 __device__ inline void contact_points14_f32(float k, const float* c, float& t1, float& t4) {
   const float zt = 1.0f + k;
   float a0 = 0.0f, a2 = -2.0f / fabsf(c[1]);

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(128) ld_tables_kernel(int law, const double* _
 // (pv, pb) (square roots and powers at 200 nodes), 10.3 us so.
 constexpr int AFF_NB = 5, AFF_NZ = 64, AFF_PAIRS = 16, AFF_THREADS = 256;
 
-__device__ __forceinline__ void affine_basis(int law, int nb, double mu, double* phi) {
+__device__ __forceinline__ void affine_basis(int law, double mu, double* phi) {
   if (law == LD_GENERAL) {
     double m = 1.0;
     for (int b = 0; b < AFF_NB; ++b) {
@@ -223,14 +223,14 @@ __global__ void __launch_bounds__(AFF_THREADS) ld_tables_affine_kernel(int law, 
   double phi[AFF_NB];
   if (tid < NTRAP) {
     const double m = (double)(NTRAP - 1 - tid) / (double)(NTRAP - 1), z = sqrt(1.0 - m * m);   // as ld_tables_kernel
-    affine_basis(law, nb, m, phi);
+    affine_basis(law, m, phi);
     s_z[tid] = z;
 #pragma unroll
     for (int b = 0; b < AFF_NB; ++b) s_y[b][tid] = z * phi[b];
   }
   if (tid >= AFF_THREADS - AFF_NZ && tid - (AFF_THREADS - AFF_NZ) < nz) {
     const int i = tid - (AFF_THREADS - AFF_NZ);
-    affine_basis(law, nb, mu[i], phi);
+    affine_basis(law, mu[i], phi);
 #pragma unroll
     for (int b = 0; b < AFF_NB; ++b) s_phi[b][i] = phi[b];
   }

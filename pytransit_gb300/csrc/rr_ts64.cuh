@@ -36,7 +36,6 @@ struct Ts64Smem {
   double cin[TS64_CH][TS64_MAXNB], cout[TS64_CH][TS64_MAXNB], dk[TS64_CH];
   int act[TS_TILE];                    // points with an overlapped sample
   int flags[TS_TILE / 32];             // per 32-point slot: 1 inside sums, 2 limb sums
-  unsigned reach;
   F64Disk disk;                        // at kmean
   float df[R2_N];
   int even;
