@@ -375,10 +375,16 @@ __device__ __forceinline__ void contact_times(double k, const double* c, const d
   const double D0 = __dadd_rn(d[0], -zt2);
   const int s0 = D0 < 0.0 ? -1 : (D0 > 0.0 ? 1 : 0);
   ContactBisection A{0, s0, -1, 0, 0}, B = A;
+  const bool even = r2_is_even(d);   // a circular orbit: the two are mirror images, in every rounding
+  if (even) {
 #pragma unroll 1
-  for (int n = 0; n < halvings; ++n) {
-    contact_step(cf, zt2f, Tf, -1.0f, n, A);
-    contact_step(cf, zt2f, Tf, 1.0f, n, B);
+    for (int n = 0; n < halvings; ++n) contact_step(cf, zt2f, Tf, -1.0f, n, A);
+  } else {
+#pragma unroll 1
+    for (int n = 0; n < halvings; ++n) {
+      contact_step(cf, zt2f, Tf, -1.0f, n, A);
+      contact_step(cf, zt2f, Tf, 1.0f, n, B);
+    }
   }
   if (A.n_u >= 0 || B.n_u >= 0) {
     float df[R2_N];
@@ -387,6 +393,7 @@ __device__ __forceinline__ void contact_times(double k, const double* c, const d
     if (A.n_u >= 0) A.a = contact_refine(d, df, zt2, T, -1.0f, halvings, A);
     if (B.n_u >= 0) B.a = contact_refine(d, df, zt2, T, 1.0f, halvings, B);
   }
+  if (even) B.a = A.a;
   const double unit = __dmul_rn(T, __hiloint2double((1022 - halvings) << 20, 0));
   t1 = -__dmul_rn(unit, (double)(2 * A.a + 1));
   t4 = __dmul_rn(unit, (double)(2 * B.a + 1));
