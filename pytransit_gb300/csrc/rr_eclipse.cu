@@ -99,12 +99,12 @@ struct EclF64Args : F64Args {
 
 // One point of a valid pv by one thread.
 __device__ __noinline__ double ecl_point_f64(const EclF64Args& A, int pv, int lc, double tc, const double* o) {
+  const double pad = __dadd_rn(A.pad0, A.exptimes[lc]), k = A.k[pv];
+  if (!(__dsub_rn(o[10], pad) <= tc && tc <= __dadd_rn(o[11], pad))) return __dmul_rn(PI, __dmul_rn(k, k));
   F64Orbit P;
   f64_orbit(o, P);
   F64Lc R;
   f64_lc(A, pv, lc, P, R);
-  const float tf = f32_of(tc);
-  if (!(R.lo <= tf && tf <= R.hi && f64_in_box(A, P, R, tc))) return R.disk.area_in;
   return f64_point_value(R, P, F64Eclipse{o}, tc);
 }
 

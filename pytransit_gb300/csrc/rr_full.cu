@@ -686,12 +686,12 @@ struct FluxF64Args : F64Args {
 // The flux of one point at tc from conjunction, in or out of the box, by one
 // thread.
 __device__ __noinline__ double f64_point(const F64Args& A, int pv, int lc, double tc, const double* o) {
+  const double pad = __dadd_rn(A.pad0, A.exptimes[lc]);
+  if (!(__dsub_rn(o[10], pad) <= tc && tc <= __dadd_rn(o[11], pad))) return 1.0;
   F64Orbit P;
   f64_orbit(o, P);
   F64Lc R;
   f64_lc(A, pv, lc, P, R);
-  const float tf = f32_of(tc);
-  if (!(R.lo <= tf && tf <= R.hi && f64_in_box(A, P, R, tc))) return 1.0;
   return f64_point_value(R, P, F64Transit{o, A.ldm + ((size_t)pv * A.npb + R.pb) * A.ng, A.ng, A.dg}, tc);
 }
 
